@@ -305,31 +305,42 @@ __global__ void k_get_receivers(long long n, int m, int nrec, const int *__restr
     out[q] = acc;
 }
 
-// Xs = S R (new ordering, engine precision); S the Jacobi scaling of the factor.
+// Xs = S R (new ordering, engine precision, rows of nc >= m columns); S the
+// Jacobi scaling of the factor.  Columns m .. nc - 1 and the pass's other two
+// blocks are zeroed.
 template <class T>
-__global__ void k_gather_new(long long n, int m, const int *__restrict__ perm, const double *__restrict__ s,
-                             const double2 *__restrict__ R, cx<T> *__restrict__ Xs)
+__global__ void k_gather_new(long long n, int m, int nc, const int *__restrict__ perm, const double *__restrict__ s,
+                             const double2 *__restrict__ R, cx<T> *__restrict__ Xs, cx<T> *__restrict__ Zs,
+                             cx<T> *__restrict__ Ys)
 {
     long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n * m) return;
-    long long i = q / m;
-    int j = (int)(q % m);
-    const long long o = perm[i];
-    double2 v = R[o * MAXRHS + j];
-    const double w = s[o];
-    Xs[i * MAXRHS + j] = cx<T>((T)(v.x * w), (T)(v.y * w));
+    if (q >= n * nc) return;
+    long long i = q / nc;
+    int j = (int)(q % nc);
+    cx<T> x(0);
+    if (j < m) {
+        const long long o = perm[i];
+        const double2 v = R[o * MAXRHS + j];
+        const double w = s[o];
+        x = cx<T>((T)(v.x * w), (T)(v.y * w));
+    }
+    Xs[q] = x;
+    Zs[q] = cx<T>(0);
+    Ys[q] = cx<T>(0);
 }
 
-// Xn += S Xs (natural ordering, FP64 accumulate).
+// Xn += S Ys (natural ordering, FP64 accumulate).
 template <class T>
-__global__ void k_scatter_add_nat(long long n, int m, const int *__restrict__ perm, const double *__restrict__ s,
-                                  const cx<T> *__restrict__ Xs, double2 *__restrict__ Xn)
+__global__ void k_scatter_add_nat(long long n, int m, int nc, const int *__restrict__ perm,
+                                  const double *__restrict__ s, const cx<T> *__restrict__ Ys,
+                                  double2 *__restrict__ Xn)
 {
     long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n * m) return;
-    long long i = q / m;
-    int j = (int)(q % m);
-    cx<T> v = Xs[i * MAXRHS + j];
+    if (q >= n * nc) return;
+    long long i = q / nc;
+    int j = (int)(q % nc);
+    if (j >= m) return;
+    const cx<T> v = Ys[q];
     const long long o = perm[i];
     const double w = s[o];
     double2 *d = Xn + o * MAXRHS + j;
@@ -529,7 +540,8 @@ int fgmres(wt3d_solver *h, Engine<T> &E, Schedule<T> *sc, int m, bool adjoint, d
     } release{h};
     double2 *V = h->gmV.p, *Z = h->gmZ.p;
     const int th = 256;
-    const unsigned nbm = (unsigned)ceil_div(n * m, th), nbb = (unsigned)ceil_div(blk, th);
+    const int nc = sk_columns(m);
+    const unsigned nbm = (unsigned)ceil_div(n * nc, th), nbb = (unsigned)ceil_div(blk, th);
     typedef std::complex<double> C;
     std::vector<double> sc_h(MAXRHS);
     std::vector<double2> hb((kr + 1) * MAXRHS), hb2((kr + 1) * MAXRHS), coef((kr + 1) * MAXRHS);
@@ -570,10 +582,10 @@ int fgmres(wt3d_solver *h, Engine<T> &E, Schedule<T> *sc, int m, bool adjoint, d
             if (all || it >= maxit) break;
             // z_j = M^-1 v_j
             double2 *Vj = V + (long long)j * blk, *Zj = Z + (long long)j * blk, *W = V + (long long)(j + 1) * blk;
-            k_gather_new<T><<<nbm, th, 0, st>>>(n, m, h->perm.p, E.scale.p, Vj, E.X.p);
+            k_gather_new<T><<<nbm, th, 0, st>>>(n, m, nc, h->perm.p, E.scale.p, Vj, E.X.p, E.Z.p, E.Y.p);
             if ((rc = E.run(*sc, st))) return rc;
             WT_CUDA(cudaMemsetAsync(Zj, 0, sizeof(double2) * blk, st));
-            k_scatter_add_nat<T><<<nbm, th, 0, st>>>(n, m, h->perm.p, E.scale.p, E.X.p, Zj);
+            k_scatter_add_nat<T><<<nbm, th, 0, st>>>(n, m, nc, h->perm.p, E.scale.p, E.Y.p, Zj);
             // w = op(A) z_j
             WT_CUDA(cudaMemsetAsync(h->norms.p, 0, sizeof(double) * 2 * MAXRHS, st));
             residual(h, st, m, Zj, nullptr, W, adjoint);
@@ -684,13 +696,14 @@ int refine(wt3d_solver *h, Engine<T> &E, int m, bool adjoint, double tol, int ma
     // the first pass is a refinement step from x = 0, whose relative residual is 1
     double prev_worst = 1.0;
     const int th = 256;
-    const unsigned nb = (unsigned)ceil_div(n * m, th);
+    const int nc = sk_columns(m);
+    const unsigned nb = (unsigned)ceil_div(n * nc, th);
     for (;;) {
-        k_gather_new<T><<<nb, th, 0, st>>>(n, m, h->perm.p, E.scale.p, h->Rn.p, E.X.p);
+        k_gather_new<T><<<nb, th, 0, st>>>(n, m, nc, h->perm.p, E.scale.p, h->Rn.p, E.X.p, E.Z.p, E.Y.p);
         rc = E.run(*sc, st);
         if (rc) return rc;
         h->kernels_solve += sc->kernels() + 3;   // + gather, scatter-add, residual
-        k_scatter_add_nat<T><<<nb, th, 0, st>>>(n, m, h->perm.p, E.scale.p, E.X.p, h->Xn.p);
+        k_scatter_add_nat<T><<<nb, th, 0, st>>>(n, m, nc, h->perm.p, E.scale.p, E.Y.p, h->Xn.p);
         WT_CUDA(cudaMemsetAsync(h->norms.p, 0, sizeof(double) * 2 * MAXRHS, st));
         residual(h, st, m, h->Xn.p, h->Bn.p, h->Rn.p, adjoint);
         WT_CUDA(cudaGetLastError());
@@ -812,9 +825,9 @@ std::shared_ptr<FactorWorkspace<T>> pick_workspace(std::vector<std::weak_ptr<Fac
 void handle_bytes(const Symbolic &S, long long nnz, int prec, double *out)
 {
     const double n = (double)S.n, nn = n / 3, sz = prec == WT3D_PREC_MIXED ? 8.0 : 16.0;
-    long long npan = 0;
-    for (const Front &F : S.fronts) npan += (F.p + KB - 1) / KB;
-    const double engine = (double)S.fac_total * sz + n * MAXRHS * sz + (double)npan * 2 * KB * KB * sz + n * 4 +
+    long long ninv = 0;
+    for (const Front &F : S.fronts) ninv += inv_entries(F.p);
+    const double engine = (double)S.fac_total * sz + 3 * n * MAXRHS * sz + (double)ninv * sz + 2 * n * 4 +
                           (double)(S.border.size() + S.rel.size()) * 4 + (double)S.fronts.size() * sizeof(FrontDev) +
                           (double)nnz * 8 + n * 8;
     const double api = (n + 1) * 4 + (double)nnz * (4 + 16 + 4) + n * 4 + 3 * n * MAXRHS * 16 + nn * (12 + 32 + 8);

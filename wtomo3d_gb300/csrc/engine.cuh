@@ -2,7 +2,7 @@
 // schedule of the factorisation and of the solves, and their execution.
 #pragma once
 #include "internal.h"
-#include "mf_kernels.cuh"
+#include "sub_kernels.cuh"
 #include "devvec.cuh"
 #include "tc_gemm.h"
 #include <type_traits>
@@ -25,6 +25,7 @@ struct LaunchRec {
     int kind;
     double flops;        // real-flop count of a GEMM launch (sum of 8 M N K)
     double bytes = 0;    // operand bytes of a GEMM launch (A, B read; C read and written)
+    bool side = false;   // off the factorisation's chain: nothing of the factorisation reads its results
 };
 
 // A list of launches plus the task arrays they read.
@@ -42,8 +43,8 @@ struct Schedule {
     DevVec<ColTask> col;
     DevVec<GemmTask<T>> gemm;
     DevVec<EATask> ea;
-    DevVec<StepTask> step;                                    // fused substitution steps
-    DevVec<cx<T>> zs;                                         // their per-front scratch slots
+    DevVec<InvTask> inv;                                      // block-inverse columns
+    DevVec<SkUnit> sk;                                        // units of the substitution products
     std::vector<std::vector<GemmTask<float>>> tc_pending;   // tensor-core task lists, built after allocation
     std::vector<std::unique_ptr<TcLaunch>> tc;
     std::vector<std::vector<GemmTask<float>>> ts_pending;   // tall-skinny tensor-core task lists (solves)
@@ -72,24 +73,36 @@ template <class T>
 class Engine {
 public:
     const Symbolic *S = nullptr;
-    DevVec<cx<T>> fac, X, dinv;   // dinv: per KB panel L_D^{-1}, U_D^{-1} (KB x KB each)
+    DevVec<cx<T>> fac, binv;      // factors; inverses of the diagonal blocks (see k_tile_inverse)
+    // right-hand sides of a pass, [row][sk_columns(m)] in the new ordering: X the
+    // sources (then the forward sweep's partial sums), Z the forward sweep's
+    // solution (then the backward sweep's partial sums), Y the solution.  Z and
+    // Y are zero when a pass starts (k_gather_new).
+    DevVec<cx<T>> X, Z, Y;
     std::shared_ptr<FactorWorkspace<T>> ws;
     DevVec<int> ipiv, border;
-    DevVec<int> pord;   // per KB panel: the stored row at each position after its interchanges
+    DevVec<int> gord;   // per pivot position (new ordering): the row that the interchanges leave there
     DevVec<int> rel;
     DevVec<FrontDev> fr;
+    std::vector<FrontDev> hfr;
     DevVec<long long> map;
     DevVec<int> npert;
     DevVec<unsigned long long> maxabs;
     std::unique_ptr<Schedule<T>> fsched;
     std::map<int, std::unique_ptr<Schedule<T>>> ssched[2];   // [adjoint][m]
+    // products of at least this many factor entries go to the tall-skinny
+    // tensor-core kernel
+    static constexpr double TS_MIN_ENTRIES = 4e6;
+    // units a launch of k_skinny is cut into, and the shortest K of a unit
+    static constexpr int SK_SLOTS = 152 * 4, SK_KMIN = 64;
     // outer block width of the two-level LU (WT3D_WB: a multiple of KB, 512 by default)
     const int WB = [] {
         const char *e = getenv("WT3D_WB");
         const int v = e ? atoi(e) : 512;
         return (v >= KB && v % KB == 0) ? v : 512;
     }();
-    static constexpr int WS = 512;   // outer block width of the blocked substitutions
+    cudaStream_t side = nullptr;     // branch of the factorisation's graph for the launches off its chain
+    cudaEvent_t side_ev = nullptr;
     // pivots below pivot_rel times the largest entry are perturbed: only
     // (near-)zero ones, since Dirichlet rows carry unit pivots next to O(1e8)
     // stiffness entries
@@ -98,7 +111,6 @@ public:
     bool use_tc = std::is_same<T, float>::value && !(getenv("WT3D_TC") && getenv("WT3D_TC")[0] == '0');
     // tcgen05 path for the large blocks of complex64 substitution passes (WT3D_TS=0: SIMT)
     bool use_ts = std::is_same<T, float>::value && !(getenv("WT3D_TS") && getenv("WT3D_TS")[0] == '0');
-    bool building_solve = false;   // set while a solve schedule is built: only those route to the TS kernel
     DevVec<float> own_tcws;   // private split workspace, only if the shared one is too small
     DevVec<int> tc_err;                                 // barrier-timeout flag of the tensor-core kernel
     std::vector<Schedule<T> *> built_tc;   // schedules whose tensor maps point into the split workspace
@@ -111,7 +123,8 @@ public:
         size_t sw = 0;   // the solve schedules' tall-skinny workspaces
         for (const auto &m : ssched)
             for (const auto &kv : m) sw += kv.second->tsws.n * sizeof(float);
-        return (fac.n + X.n + dinv.n) * sizeof(cx<T>) + (ipiv.n + border.n + rel.n + pord.n) * 4 + fr.n * sizeof(FrontDev) +
+        return (fac.n + X.n + Z.n + Y.n + binv.n) * sizeof(cx<T>) + (ipiv.n + border.n + rel.n + gord.n) * 4 +
+               fr.n * sizeof(FrontDev) +
                map.n * 8 + scale.n * 8 + own_tcws.n * sizeof(float) + sw;
     }
 
@@ -149,7 +162,8 @@ public:
             if (ws->upd0.n < n0 && (rc = ws->upd0.alloc(n0))) return rc;
             if (ws->upd1.n < n1 && (rc = ws->upd1.alloc(n1))) return rc;
         }
-        if ((rc = X.alloc((size_t)sym.n * MAXRHS))) return rc;
+        const size_t nx = (size_t)sym.n * MAXRHS;
+        if ((rc = X.alloc(nx)) || (rc = Z.alloc(nx)) || (rc = Y.alloc(nx))) return rc;
         if ((rc = ipiv.alloc(sym.n))) return rc;
         if ((rc = border.upload(sym.border))) return rc;
         if ((rc = rel.upload(sym.rel))) return rc;
@@ -162,11 +176,11 @@ public:
         if (use_tc && (rc = tc_init())) return rc;
         if (use_ts && (rc = ts_init())) return rc;
         std::vector<FrontDev> h(sym.fronts.size());
-        long long npan = 0;
+        long long ninv = 0;
         for (size_t f = 0; f < h.size(); f++) {
-            h[f].pan = (int)npan;
-            npan += (sym.fronts[f].p + KB - 1) / KB;
             const Front &F = sym.fronts[f];
+            h[f].inv = ninv;
+            ninv += inv_entries(F.p);
             h[f].fac = F.fac_off;
             h[f].upd = F.upd_off;
             h[f].border = F.border_off;
@@ -176,8 +190,11 @@ public:
             h[f].parity = F.level & 1;
         }
         if ((rc = fr.upload(h))) return rc;
-        if ((rc = dinv.alloc((size_t)npan * 2 * KB * KB))) return rc;
-        if ((rc = pord.alloc((size_t)npan * KB))) return rc;
+        hfr = h;
+        if ((rc = binv.alloc((size_t)ninv))) return rc;
+        if ((rc = gord.alloc((size_t)sym.n))) return rc;
+        WT_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+        WT_CUDA(cudaEventCreateWithFlags(&side_ev, cudaEventDisableTiming));
         // kernel attributes are per device: once for each device this process uses
         static std::once_flag attr_once[64];
         int dev = 0;
@@ -196,10 +213,60 @@ public:
                 cudaFuncSetAttribute(k_trsm_col_h<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)band_col_smem());
             }
-            cudaFuncSetAttribute(k_sub_step<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(cx<T>) * sub_step_smem_elems()));
+            sk_attr<1>();
+            sk_attr<4>();
+            sk_attr<8>();
+            sk_attr<16>();
+            sk_attr<32>();
         });
         return build_factor_schedule();
+    }
+    Engine() = default;
+    Engine(const Engine &) = delete;
+    Engine &operator=(const Engine &) = delete;
+    ~Engine()
+    {
+        if (side_ev) cudaEventDestroy(side_ev);
+        if (side) cudaStreamDestroy(side);
+    }
+
+    template <int NC>
+    static void sk_attr()
+    {
+        cudaFuncSetAttribute(k_skinny<T, NC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)SkCfg<T, NC>::smem(false));
+        cudaFuncSetAttribute(k_skinny<T, NC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)SkCfg<T, NC>::smem(true));
+    }
+
+    template <int NC, bool H>
+    static void sk_launch_t(const SkUnit *u, int n, const cx<T> *in, cx<T> *out, cudaStream_t st)
+    {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)n);
+        cfg.blockDim = dim3(SK_TH);
+        cfg.dynamicSmemBytes = SkCfg<T, NC>::smem(H);
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see k_skinny
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        cudaLaunchKernelEx(&cfg, k_skinny<T, NC, H>, u, in, out);
+    }
+    template <int NC>
+    static void sk_launch_n(bool herm, const SkUnit *u, int n, const cx<T> *in, cx<T> *out, cudaStream_t st)
+    {
+        if (herm) sk_launch_t<NC, true>(u, n, in, out, st);
+        else sk_launch_t<NC, false>(u, n, in, out, st);
+    }
+    static void sk_launch(int nc, bool herm, const SkUnit *u, int n, const cx<T> *in, cx<T> *out, cudaStream_t st)
+    {
+        if (nc == 1) sk_launch_n<1>(herm, u, n, in, out, st);
+        else if (nc == 4) sk_launch_n<4>(herm, u, n, in, out, st);
+        else if (nc == 8) sk_launch_n<8>(herm, u, n, in, out, st);
+        else if (nc == 16) sk_launch_n<16>(herm, u, n, in, out, st);
+        else sk_launch_n<32>(herm, u, n, in, out, st);
     }
 
     // ---------------------------------------------------------------------
@@ -245,28 +312,6 @@ public:
                 sc.launches.push_back({[psc, idx](cudaStream_t st) { tc_split(*psc->tc[idx], st); }, LK_SPLIT, 0});
                 sc.launches.push_back({[psc, idx, this](cudaStream_t st) { tc_mma(*psc->tc[idx], tc_err.p, st); },
                                        LK_TCGEMM, fl, by});
-            }
-            if (use_ts && building_solve) {
-                // blocks TMA can address (16-byte aligned, even stride) and the rest:
-                // one tall-skinny launch each
-                std::vector<GemmTask<float>> tsv[2], rest;
-                for (auto &g : simt) {
-                    if (!ts_eligible(g)) rest.push_back(g);
-                    else tsv[ts_tma_ok(g) ? 1 : 0].push_back(g);
-                }
-                for (int tma = 0; tma < 2; tma++) {
-                    if (tsv[tma].empty()) continue;
-                    double fl = 0, by = 0;
-                    for (auto &g : tsv[tma]) { fl += 8.0 * g.M * (double)g.N * g.K; by += gemm_bytes(g); }
-                    const int idx = (int)sc.ts_pending.size();
-                    sc.ts_pending.push_back(std::move(tsv[tma]));
-                    sc.ts_tma.push_back((char)tma);
-                    Schedule<T> *psc = &sc;
-                    sc.launches.push_back({[psc, idx](cudaStream_t st) { ts_expand(*psc->ts[idx], st); }, LK_SPLIT, 0});
-                    sc.launches.push_back({[psc, idx, this](cudaStream_t st) { ts_mma(*psc->ts[idx], tc_err.p, st); },
-                                           LK_TCGEMM, fl, by});
-                }
-                simt.swap(rest);
             }
         } else {
             simt.assign(all.begin() + b, all.end());
@@ -393,6 +438,51 @@ public:
         return WT3D_OK;
     }
 
+    // The inverses of the diagonal blocks that end in [k0, k1) of the fronts fl,
+    // once the panels [p0, end) of hp are factored.  Off the factorisation's
+    // chain (only the substitutions read them): a branch of its graph.
+    void push_inverses(Schedule<T> &sc, const std::vector<int> &fl, const std::vector<PanelTask> &hp, size_t p0,
+                       std::vector<InvTask> &hi, int k0, int k1)
+    {
+        Schedule<T> *psc = &sc;
+        const int np = (int)(hp.size() - p0);
+        const size_t smi = sizeof(cx<T>) * (KB * (KB + 1) + 2 * KB * (KB + 1));
+        if (np) {
+            sc.launches.push_back({[psc, this, p0, np, smi](cudaStream_t st) {
+                k_tile_inverse<T><<<np, 2 * KB, smi, st>>>(psc->panel.p + p0, fr.p, fac.p, binv.p);
+            }, LK_PANEL, 0});
+            sc.launches.back().side = true;
+        }
+        const size_t i0 = hi.size();
+        for (int f : fl) {
+            const int p = S->fronts[f].p;
+            for (int c0 = 0; c0 < p; c0 += SB) {
+                const int end = std::min(c0 + SB, p), w = end - c0, nt = (w + KB - 1) / KB;
+                if (end - 1 < k0 || end - 1 >= k1) continue;
+                for (int up = 0; up < 2; up++)
+                    for (int t = 0; t < nt; t++) {
+                        if (up ? t == 0 : t == nt - 1) continue;
+                        for (int h = 0; h < 2; h++)
+                            if (KB * t + IV_N * h < w) hi.push_back(InvTask{f, c0, t, h, up});
+                    }
+            }
+        }
+        // longest chains first
+        std::stable_sort(hi.begin() + i0, hi.end(), [this](const InvTask &a, const InvTask &b) {
+            auto len = [this](const InvTask &x) {
+                return x.upper ? x.t : (std::min(SB, S->fronts[x.f].p - x.c0) + KB - 1) / KB - 1 - x.t;
+            };
+            return len(a) > len(b);
+        });
+        const int ni = (int)(hi.size() - i0);
+        if (ni) {
+            sc.launches.push_back({[psc, this, i0, ni](cudaStream_t st) {
+                k_block_inverse<T><<<ni, IV_TH, 0, st>>>(psc->inv.p + i0, fr.p, fac.p, gord.p, binv.p);
+            }, LK_PANEL, 0});
+            sc.launches.back().side = true;
+        }
+    }
+
     int build_factor_schedule()
     {
         auto sc = std::make_unique<Schedule<T>>();
@@ -401,6 +491,7 @@ public:
         std::vector<ColTask> hc;
         std::vector<GemmTask<T>> hg;
         std::vector<EATask> he;
+        std::vector<InvTask> hi;
         Schedule<T> *psc = sc.get();
         const Symbolic &sym = *S;
         cx<T> *F = fac.p;
@@ -462,6 +553,7 @@ public:
             int maxp = 0;
             for (int f : fl) maxp = std::max(maxp, sym.fronts[f].p);
             for (int c0 = 0; c0 < maxp; c0 += WB) {
+                const size_t pblk = hp.size();   // first panel of this outer block
                 for (int k = c0; k < std::min(c0 + WB, maxp); k += KB) {
                     size_t p0 = hp.size(), r0 = hr.size(), cc0 = hc.size(), g0 = hg.size();
                     long long tiles = 0;
@@ -491,14 +583,14 @@ public:
                     size_t smc = sizeof(cx<T>) * (KB * (KB + 1) + TCR * (KB + 1));
                     sc->launches.push_back({[psc, this, p0, np, smp](cudaStream_t st) {
                         k_panel<T><<<np, 256, smp, st>>>(psc->panel.p + p0, fr.p, fac.p, ipiv.p, maxabs.p, pivot_rel,
-                                                         npert.p, pord.p);
+                                                         npert.p, gord.p);
                     }, LK_PANEL, 0});
                     if (nr)
                         sc->launches.push_back({[psc, this, r0, nr, smr](cudaStream_t st) {
                             if constexpr (std::is_same<T, float>::value)
-                                k_trsm_row_h<0><<<nr, TRW, band_row_smem(), st>>>(psc->row.p + r0, fr.p, fac.p, pord.p);
+                                k_trsm_row_h<0><<<nr, TRW, band_row_smem(), st>>>(psc->row.p + r0, fr.p, fac.p, gord.p);
                             else
-                                k_trsm_row<T><<<nr, TRW, smr, st>>>(psc->row.p + r0, fr.p, fac.p, pord.p);
+                                k_trsm_row<T><<<nr, TRW, smr, st>>>(psc->row.p + r0, fr.p, fac.p, gord.p);
                         }, LK_TRSM, 0});
                     if (ncl)
                         sc->launches.push_back({[psc, this, cc0, ncl, smc](cudaStream_t st) {
@@ -509,6 +601,7 @@ public:
                         }, LK_TRSM, 0});
                     push_gemm_launch(*sc, hg, g0, tiles);
                 }
+                push_inverses(*sc, fl, hp, pblk, hi, c0, std::min(c0 + WB, maxp));
                 // rank-WB update of everything below and right of the outer block
                 size_t g0 = hg.size();
                 long long tiles = 0;
@@ -540,190 +633,199 @@ public:
                 push_gemm_launch(*sc, hg, g0, tiles);
             }
         }
-        // the tile inverses the solves use, for every panel at once
-        {
-            const int npall = (int)hp.size();
-            const size_t smi = sizeof(cx<T>) * (KB * (KB + 1) + 2 * KB * (KB + 1));
-            if (npall)
-                sc->launches.push_back({[psc, this, npall, smi](cudaStream_t st) {
-                    k_tile_inverse<T><<<npall, 2 * KB, smi, st>>>(psc->panel.p, fr.p, fac.p, dinv.p);
-                }, LK_PANEL, 0});
-        }
         int rc;
         if ((rc = sc->panel.upload(hp))) return rc;
         if ((rc = sc->row.upload(hr))) return rc;
         if ((rc = sc->col.upload(hc))) return rc;
         if ((rc = sc->gemm.upload(hg))) return rc;
         if ((rc = sc->ea.upload(he))) return rc;
+        if ((rc = sc->inv.upload(hi))) return rc;
         if ((rc = finish_tc(*sc))) return rc;
         fsched = std::move(sc);
         return WT3D_OK;
     }
 
-    // Solve schedule for m right-hand sides in X (new ordering, row-major n x MAXRHS).
+    // One product of a substitution pass: out (=, -=) op(A) in, A a factor block
+    // or (flags SK_LOWER / SK_UPPER) a packed block inverse.
+    struct Product {
+        const cx<T> *A;
+        int lda, M, K;
+        const int *bmap;   // input rows bmap[k], or b0 + k
+        int b0;
+        const int *cmap;   // output rows cmap[i], or c0 + i
+        int c0;
+        int flags;
+    };
+
+    // Appends the launches of the products of one step.
+    void push_products(Schedule<T> &sc, std::vector<SkUnit> &hu, std::vector<Product> v, bool herm, const cx<T> *in,
+                       cx<T> *out, int m)
+    {
+        const int nc = sk_columns(m);
+        Schedule<T> *psc = &sc;
+        if constexpr (std::is_same<T, float>::value) {
+            // large blocks go to the tall-skinny tensor-core kernel: those that TMA
+            // can address (16-byte aligned, even stride) and the rest, one launch each
+            std::vector<GemmTask<float>> tsv[2];
+            std::vector<Product> rest;
+            for (const Product &q : v) {
+                GemmTask<float> g{};
+                g.A = q.A; g.lda = q.lda; g.M = q.M; g.K = q.K; g.N = m; g.conjA = herm;
+                g.B = in + (q.bmap ? 0 : (long long)q.b0 * nc); g.brow = q.bmap; g.ldb = nc;
+                g.C = out + (q.cmap ? 0 : (long long)q.c0 * nc); g.crow = q.cmap; g.ldc = nc;
+                const bool tri = (q.flags & (SK_LOWER | SK_UPPER)) != 0;
+                if (use_ts && !tri && nc >= 8 && (double)q.M * q.K >= TS_MIN_ENTRIES && ts_eligible(g))
+                    tsv[ts_tma_ok(g) ? 1 : 0].push_back(g);
+                else rest.push_back(q);
+            }
+            v.swap(rest);
+            for (int tma = 0; tma < 2; tma++) {
+                if (tsv[tma].empty()) continue;
+                double fl = 0, by = 0;
+                for (auto &g : tsv[tma]) { fl += 8.0 * g.M * (double)g.N * g.K; by += gemm_bytes(g); }
+                const int idx = (int)sc.ts_pending.size();
+                sc.ts_pending.push_back(std::move(tsv[tma]));
+                sc.ts_tma.push_back((char)tma);
+                sc.launches.push_back({[psc, idx](cudaStream_t st) { ts_expand(*psc->ts[idx], st); }, LK_SPLIT, 0});
+                sc.launches.push_back({[psc, idx, this](cudaStream_t st) { ts_mma(*psc->ts[idx], tc_err.p, st); },
+                                       LK_TCGEMM, fl, by});
+            }
+        }
+        if (v.empty()) return;
+        // K range of the 64 rows from r0: all of it, or the triangle's part
+        auto range = [&](const Product &q, int r0, int &k0, int &k1) {
+            k0 = 0;
+            k1 = q.K;
+            if (!(q.flags & (SK_LOWER | SK_UPPER))) return;
+            if (((q.flags & SK_LOWER) != 0) != herm) k1 = std::min(q.K, r0 + SK_M);
+            else k0 = r0;
+        };
+        double work = 0, fl = 0;
+        for (const Product &q : v)
+            for (int r0 = 0; r0 < q.M; r0 += SK_M) {
+                int k0, k1;
+                range(q, r0, k0, k1);
+                work += k1 - k0;
+                fl += 8.0 * std::min(SK_M, q.M - r0) * (double)(k1 - k0) * m;
+            }
+        // K chunk for about SK_SLOTS units
+        const int chunk = std::min<long long>(SK_KMAX, std::max<long long>(SK_KMIN, (long long)(work / SK_SLOTS / 64 + 1) * 64));
+        const size_t u0 = hu.size();
+        for (const Product &q : v)
+            for (int r0 = 0; r0 < q.M; r0 += SK_M) {
+                int k0, k1;
+                range(q, r0, k0, k1);
+                const int n = std::max(1, (k1 - k0 + chunk / 2) / chunk);   // chunks of about the same length
+                const int len = std::min<int>(SK_KMAX, ((k1 - k0 + n - 1) / n + 31) / 32 * 32);
+                for (int k = k0; k < k1; k += len) {
+                    SkUnit u{};
+                    u.A = herm ? q.A + (long long)k * q.lda + r0 : q.A + (long long)r0 * q.lda + k;
+                    u.bmap = q.bmap ? q.bmap + k : nullptr;
+                    u.b0 = q.b0 + k;
+                    u.cmap = q.cmap ? q.cmap + r0 : nullptr;
+                    u.c0 = q.c0 + r0;
+                    u.lda = q.lda;
+                    u.M = std::min(SK_M, q.M - r0);
+                    u.K = std::min(len, k1 - k);
+                    u.flags = q.flags | (k1 - k0 > len ? SK_ATOM : 0);
+                    u.d = k - r0;
+                    hu.push_back(u);
+                }
+            }
+        const int nu = (int)(hu.size() - u0);
+        const bool tri = (v[0].flags & (SK_LOWER | SK_UPPER)) != 0;
+        sc.launches.push_back({[psc, u0, nu, nc, herm, in, out](cudaStream_t st) {
+            sk_launch(nc, herm, psc->sk.p + u0, nu, in, out, st);
+        }, tri ? LK_SUBSTEP : LK_GEMM, fl, fl / m * sizeof(cx<T>) / 8});
+    }
+
+    // Solve schedule for m right-hand sides: X (sources, new ordering) to Y.
+    // Every level of a sweep walks the SB-wide diagonal blocks of its fronts: the
+    // block inverse gives the block's unknowns, then the rows outside the block
+    // are updated with them.
     Schedule<T> *solve_schedule(int m, bool adjoint)
     {
         auto it = ssched[adjoint].find(m);
         if (it != ssched[adjoint].end()) return it->second.get();
         auto sc = std::make_unique<Schedule<T>>();
-        Schedule<T> *psc = sc.get();
-        std::vector<PanelTask> hp;
-        std::vector<GemmTask<T>> hg;
+        std::vector<SkUnit> hu;
         const Symbolic &sym = *S;
-        cx<T> *F = fac.p;
-        cx<T> *Xp = X.p;
-        struct Flag {
-            bool &f;
-            Flag(bool &x) : f(x) { f = true; }
-            ~Flag() { f = false; }
-        } building(building_solve);
-        const int ldx = MAXRHS;
         const int nlev = (int)sym.levels.size();
-        // Two-level blocking of the in-front substitutions, like the
-        // factorisation's: inside each WS-wide outer block the KB panels are
-        // solved one by one, each step one fused launch (k_sub_step: the
-        // diagonal-tile product and the update of the block's other rows);
-        // the rows outside the block then receive one K = WS update, which
-        // the tall-skinny tensor-core kernel takes.
-        std::vector<StepTask> hs;
-        size_t smd_step = sizeof(cx<T>) * sub_step_smem_elems();
-        int maxslots = 0;
-        // one fused launch over the step tasks [s0, end)
-        auto step_launch = [&](size_t s0, int mode) {
-            const int ns = (int)(hs.size() - s0);
-            if (!ns) return;
-            sc->launches.push_back({[psc, this, s0, ns, smd_step, m, mode, Xp, ldx](cudaStream_t st) {
-                // programmatic dependent launch: see k_sub_step
-                cudaLaunchConfig_t cfg = {};
-                cfg.gridDim = dim3((unsigned)ns);
-                cfg.blockDim = dim3(SUB_THREADS);
-                cfg.dynamicSmemBytes = smd_step;
-                cfg.stream = st;
-                cudaLaunchAttribute at[1];
-                at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-                at[0].val.programmaticStreamSerializationAllowed = 1;
-                cfg.attrs = at;
-                cfg.numAttrs = 1;
-                cudaLaunchKernelEx(&cfg, k_sub_step<T>, (const StepTask *)(psc->step.p + s0), (const FrontDev *)fr.p,
-                                   (const cx<T> *)fac.p, (const cx<T> *)dinv.p, (const int *)pord.p, Xp, ldx, m, mode,
-                                   psc->zs.p);
-            }, LK_SUBSTEP, 0, (double)ns * (KB * KB + 2.0 * KB * m) * sizeof(cx<T>)});
-        };
-        // the tasks of one panel step of front f (slot = its position in the level)
-        auto add_step = [&](int f, int slot, int k, int kprev, int u0, int u1) {
-            const int nup = u1 > u0 ? (u1 - u0 + SUB_RB - 1) / SUB_RB : 0;
-            hs.push_back(StepTask{f, k, 0, 0, nup ? 0 : 3, kprev, slot});
-            for (int r = u0; r < u1; r += SUB_RB) hs.push_back(StepTask{f, k, r, std::min(r + SUB_RB, u1), 1, -1, slot});
+        auto block = [&](int f, int c0) {   // the packed inverse of block c0
+            return binv.p + hfr[f].inv + (long long)(c0 / SB) * SB * SB;
         };
         // ---- forward sweep: leaves to root ----
         for (int L = nlev - 1; L >= 0; L--) {
             const std::vector<int> &fl = sym.levels[L];
-            maxslots = std::max(maxslots, (int)fl.size());
             int maxp = 0;
             for (int f : fl) maxp = std::max(maxp, sym.fronts[f].p);
-            for (int c0 = 0; c0 < maxp; c0 += WS) {
-                for (int k = c0; k < std::min(c0 + WS, maxp); k += KB) {
-                    const size_t s0 = hs.size();
-                    for (int si = 0; si < (int)fl.size(); si++) {
-                        const Front &Fr = sym.fronts[fl[si]];
-                        if (Fr.p <= k) continue;
-                        const int k2 = k + std::min(KB, Fr.p - k), cend = std::min(c0 + WS, Fr.p);
-                        add_step(fl[si], si, k, k > c0 ? k - KB : -1, k2, cend);
-                    }
-                    step_launch(s0, adjoint ? 2 : 0);
-                }
-                // rows below the outer block
-                size_t g0 = hg.size();
-                long long tiles = 0;
+            for (int c0 = 0; c0 < maxp; c0 += SB) {
+                std::vector<Product> ap, up;
                 for (int f : fl) {
                     const Front &Fr = sym.fronts[f];
                     if (Fr.p <= c0) continue;
-                    const int nf = Fr.nf(), cend = std::min(c0 + WS, Fr.p);
-                    cx<T> *Pb = F + Fr.fac_off;
-                    cx<T> *Y = Xp + (long long)Fr.first * ldx;
-                    if (!adjoint)   // Y[cend:p] -= L[cend:p, c0:cend] Y[c0:cend]
-                        add_gemm(hg, tiles, Pb + (long long)cend * nf + c0, nf, Y + (long long)c0 * ldx, ldx,
-                                 Y + (long long)cend * ldx, ldx, Fr.p - cend, m, cend - c0);
-                    else            // Y[cend:p] -= U[c0:cend, cend:p]^H Y[c0:cend]
-                        add_gemm(hg, tiles, Pb + (long long)c0 * nf + cend, nf, Y + (long long)c0 * ldx, ldx,
-                                 Y + (long long)cend * ldx, ldx, Fr.p - cend, m, cend - c0, nullptr, nullptr, 1);
+                    const int nf = Fr.nf(), cend = std::min(c0 + SB, Fr.p), w = cend - c0, r = Fr.first + c0;
+                    const cx<T> *Pb = fac.p + Fr.fac_off;
+                    const cx<T> *W = block(f, c0);
+                    if (!adjoint) ap.push_back({W, inv_ld(w), w, w, gord.p + r, 0, nullptr, r, SK_LOWER});
+                    else ap.push_back({W, inv_ld(w), w, w, nullptr, r, nullptr, r, SK_UPPER});
+                    if (cend == Fr.p) continue;
+                    if (!adjoint)   // x[cend:p] -= L[cend:p, c0:cend] z[c0:cend]
+                        up.push_back({Pb + (long long)cend * nf + c0, nf, Fr.p - cend, w, nullptr, r, nullptr,
+                                      Fr.first + cend, SK_SUB});
+                    else            // x[cend:p] -= U[c0:cend, cend:p]^H z[c0:cend]
+                        up.push_back({Pb + (long long)c0 * nf + cend, nf, Fr.p - cend, w, nullptr, r, nullptr,
+                                      Fr.first + cend, SK_SUB});
                 }
-                push_gemm_launch(*sc, hg, g0, tiles);
+                push_products(*sc, hu, std::move(ap), adjoint, X.p, Z.p, m);
+                push_products(*sc, hu, std::move(up), adjoint, Z.p, X.p, m);
             }
-            // border update  X[border] -= L21 Y   (adjoint: U12^H Y)
-            size_t g0 = hg.size();
-            long long tiles = 0;
+            // x[border] -= L21 z   (adjoint: U12^H z); siblings share border rows
+            std::vector<Product> bo;
             for (int f : fl) {
                 const Front &Fr = sym.fronts[f];
                 if (Fr.b == 0) continue;
-                const int nf = Fr.nf();
-                cx<T> *Pb = F + Fr.fac_off;
-                cx<T> *Lo = Pb + (long long)Fr.p * nf;
-                cx<T> *Y = Xp + (long long)Fr.first * ldx;
-                const int *crow = border.p + Fr.border_off;
-                if (!adjoint) add_gemm(hg, tiles, Lo, Fr.p, Y, ldx, Xp, ldx, Fr.b, m, Fr.p, nullptr, crow, 0);
-                else add_gemm(hg, tiles, Pb + Fr.p, nf, Y, ldx, Xp, ldx, Fr.b, m, Fr.p, nullptr, crow, 1);
+                const cx<T> *Pb = fac.p + Fr.fac_off, *Lo = Pb + (long long)Fr.p * Fr.nf();
+                bo.push_back({adjoint ? Pb + Fr.p : Lo, adjoint ? Fr.nf() : Fr.p, Fr.b, Fr.p, nullptr, Fr.first,
+                              border.p + Fr.border_off, 0, SK_SUB | SK_ATOM});
             }
-            push_gemm_launch(*sc, hg, g0, tiles);
+            push_products(*sc, hu, std::move(bo), adjoint, Z.p, X.p, m);
         }
         // ---- backward sweep: root to leaves ----
         for (int L = 0; L < nlev; L++) {
             const std::vector<int> &fl = sym.levels[L];
-            size_t g0 = hg.size();
-            long long tiles = 0;
             int maxp = 0;
+            std::vector<Product> bo;
             for (int f : fl) {
                 const Front &Fr = sym.fronts[f];
                 maxp = std::max(maxp, Fr.p);
                 if (Fr.b == 0) continue;
-                const int nf = Fr.nf();
-                cx<T> *Pb = F + Fr.fac_off;
-                cx<T> *Lo = Pb + (long long)Fr.p * nf;
-                cx<T> *Y = Xp + (long long)Fr.first * ldx;
-                const int *brow = border.p + Fr.border_off;
-                if (!adjoint)   // Y -= U12 X[border]
-                    add_gemm(hg, tiles, Pb + Fr.p, nf, Xp, ldx, Y, ldx, Fr.p, m, Fr.b, brow, nullptr, 0);
-                else            // Y -= L21^H X[border]
-                    add_gemm(hg, tiles, Lo, Fr.p, Xp, ldx, Y, ldx, Fr.p, m, Fr.b, brow, nullptr, 1);
+                const cx<T> *Pb = fac.p + Fr.fac_off, *Lo = Pb + (long long)Fr.p * Fr.nf();
+                // z -= U12 y[border]   (adjoint: L21^H y[border])
+                bo.push_back({adjoint ? Lo : Pb + Fr.p, adjoint ? Fr.p : Fr.nf(), Fr.p, Fr.b,
+                              border.p + Fr.border_off, 0, nullptr, Fr.first, SK_SUB});
             }
-            push_gemm_launch(*sc, hg, g0, tiles);
-            for (int c0 = (maxp - 1) / WS * WS; c0 >= 0; c0 -= WS) {
-                const int nsteps = (std::min(c0 + WS, maxp) - c0 + KB - 1) / KB;
-                for (int s = nsteps - 1; s >= 0; s--) {
-                    const int k = c0 + s * KB;
-                    const size_t s0 = hs.size();
-                    for (int si = 0; si < (int)fl.size(); si++) {
-                        const Front &Fr = sym.fronts[fl[si]];
-                        if (Fr.p <= k) continue;
-                        const int cend = std::min(c0 + WS, Fr.p);
-                        // the rows above the panel inside the block (right-looking for both modes)
-                        add_step(fl[si], si, k, k + KB < cend ? k + KB : -1, c0, k);
-                    }
-                    step_launch(s0, adjoint ? 3 : 1);
+            push_products(*sc, hu, std::move(bo), adjoint, Y.p, Z.p, m);
+            for (int c0 = (maxp - 1) / SB * SB; c0 >= 0; c0 -= SB) {
+                std::vector<Product> ap, up;
+                for (int f : fl) {
+                    const Front &Fr = sym.fronts[f];
+                    if (Fr.p <= c0) continue;
+                    const int nf = Fr.nf(), w = std::min(c0 + SB, Fr.p) - c0, r = Fr.first + c0;
+                    const cx<T> *Pb = fac.p + Fr.fac_off;
+                    const cx<T> *W = block(f, c0);
+                    if (!adjoint) ap.push_back({W, inv_ld(w), w, w, nullptr, r, nullptr, r, SK_UPPER});
+                    else ap.push_back({W, inv_ld(w), w, w, nullptr, r, gord.p + r, 0, SK_LOWER});
+                    if (c0 == 0) continue;
+                    // z[0:c0] -= U[0:c0, c0:cend] y[c0:cend]   (adjoint: L[c0:cend, 0:c0]^H)
+                    up.push_back({adjoint ? Pb + (long long)c0 * nf : Pb + c0, nf, c0, w, nullptr, r, nullptr,
+                                  Fr.first, SK_SUB});
                 }
-                if (c0 > 0) {
-                    // rows above the block:  Y[0:c0] -= U[0:c0, c0:cend] Y[c0:cend]
-                    //                 (adjoint: Y[0:c0] -= L[c0:cend, 0:c0]^H Y[c0:cend])
-                    size_t g1 = hg.size();
-                    long long t1 = 0;
-                    for (int f : fl) {
-                        const Front &Fr = sym.fronts[f];
-                        if (Fr.p <= c0) continue;
-                        const int nf = Fr.nf(), cend = std::min(c0 + WS, Fr.p);
-                        cx<T> *Pb = F + Fr.fac_off;
-                        cx<T> *Y = Xp + (long long)Fr.first * ldx;
-                        if (!adjoint)
-                            add_gemm(hg, t1, Pb + c0, nf, Y + (long long)c0 * ldx, ldx, Y, ldx, c0, m, cend - c0);
-                        else
-                            add_gemm(hg, t1, Pb + (long long)c0 * nf, nf, Y + (long long)c0 * ldx, ldx, Y, ldx, c0, m,
-                                     cend - c0, nullptr, nullptr, 1);
-                    }
-                    push_gemm_launch(*sc, hg, g1, t1);
-                }
+                push_products(*sc, hu, std::move(ap), adjoint, Z.p, Y.p, m);
+                push_products(*sc, hu, std::move(up), adjoint, Y.p, Z.p, m);
             }
         }
-        if (sc->step.upload(hs) || sc->zs.alloc((size_t)std::max(maxslots, 1) * KB * MAXRHS)) return nullptr;
-        if (sc->panel.upload(hp) || sc->gemm.upload(hg) || finish_tc(*sc) || finish_ts(*sc)) return nullptr;
+        if (sc->sk.upload(hu) || finish_ts(*sc)) return nullptr;
         Schedule<T> *ret = sc.get();
         ssched[adjoint][m] = std::move(sc);
         return ret;
@@ -737,7 +839,21 @@ public:
             if (!sc.graph) {
                 cudaGraph_t g;
                 WT_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-                for (auto &l : sc.launches) l.fn(st);
+                bool forked = false, behind = true;   // behind: the main branch has moved on since the last fork
+                for (auto &l : sc.launches) {
+                    if (l.side && behind) {
+                        cudaEventRecord(side_ev, st);
+                        cudaStreamWaitEvent(side, side_ev, 0);
+                        forked = true;
+                        behind = false;
+                    }
+                    l.fn(l.side ? side : st);
+                    if (!l.side) behind = true;
+                }
+                if (forked) {
+                    cudaEventRecord(side_ev, side);
+                    cudaStreamWaitEvent(st, side_ev, 0);
+                }
                 WT_CUDA(cudaStreamEndCapture(st, &g));
                 cudaError_t e = cudaGraphInstantiate(&sc.graph, g, 0);
                 cudaGraphDestroy(g);

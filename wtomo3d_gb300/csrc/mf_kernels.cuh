@@ -22,21 +22,13 @@ struct FrontDev {
     long long upd;     // F22 offset in its parity buffer
     long long border;  // offset into the border index array
     int p, b, first, parity;
-    int pan;           // index of the front's first KB panel (tile-inverse store)
+    long long inv;     // offset of the front's first block inverse in the inverse pool
 };
 
 struct PanelTask { int f, k; };
 struct RowTask { int f, k, c0; };
 struct ColTask { int f, k, r0, which; };
 struct EATask { int child, parent; long long row0; };
-// One CTA of a fused substitution step (k_sub_step): panel k of front f.
-// role 0: flush the previous panel's solved rows (kprev >= 0) from the front's
-// scratch slot into X, then store this panel's solved rows in the slot;
-// role 1: update rows [r0, r1) with this panel's solved rows;
-// role 3: as role 0 for a front with no update CTA in this step (its last
-// panel of the block): the solved rows go straight into X.
-struct StepTask { int f, k, r0, r1, role, kprev, slot; };
-
 template <class T>
 struct GemmTask {
     const cx<T> *A;
@@ -152,57 +144,25 @@ __global__ void k_extend_add(const EATask *__restrict__ tasks, int ntasks, long 
 }
 
 // Row order of panel k after its LINPACK-style interchanges: idx[i] is the
-// stored row that lands at position i (the panel kernel stores it per panel
-// in pord; identity when not pivoted).  Threads tid < KB write idx; callers
-// synchronise before reading it.
-__device__ __forceinline__ void panel_rows(const int *__restrict__ pord, int pan, int kb, bool pivoted, int *idx)
+// stored row that lands at position i, from gord, which holds for every pivot
+// position of the new ordering the row that lands there (written by the panel
+// kernel).  Threads tid < KB write idx; callers synchronise before reading it.
+__device__ __forceinline__ void panel_rows(const int *__restrict__ gord, int first, int kb, int *idx)
 {
     const int tid = threadIdx.x;
-    if (tid < KB) idx[tid] = (pivoted && tid < kb) ? pord[(long long)pan * KB + tid] : tid;
+    if (tid < KB) idx[tid] = tid < kb ? gord[first + tid] - first : tid;
 }
 
 // ---------------------------------------------------------------------------
 // panel: LU of the KB x KB diagonal tile with partial pivoting inside the tile
 // ---------------------------------------------------------------------------
-// Columns of L_D^{-1} (thread c < KB) and U_D^{-1} (KB <= c < 2 KB) of the
-// factored kb x kb tile held in S (row stride KB + 1), padded to KB x KB with
-// the identity, stored row-major into Li and Ui.  Scratch: 2 KB columns of
-// KB + 1 elements after the tile.
-template <class T>
-__device__ __forceinline__ void tile_inverse_cols(const cx<T> *S, int kb, cx<T> *Li, cx<T> *Ui, int c)
-{
-    const int LD = KB + 1;
-    const bool up = c >= KB;
-    const int cc = up ? c - KB : c;
-    cx<T> *x = const_cast<cx<T> *>(S) + KB * LD + c * (KB + 1);
-    if (!up) {
-        for (int i = 0; i < KB; i++) {
-            cx<T> s = (i == cc) ? cx<T>(1) : cx<T>(0);
-            if (i < kb && cc < kb)
-                for (int l = cc; l < i; l++) s = s - S[i * LD + l] * x[l];
-            x[i] = s;
-        }
-    } else {
-        for (int i = KB - 1; i >= 0; i--) {
-            cx<T> s = (i == cc) ? cx<T>(1) : cx<T>(0);
-            if (i < kb && cc < kb) {
-                for (int l = i + 1; l <= cc; l++) s = s - S[i * LD + l] * x[l];
-                s = cdiv(s, S[i * LD + i]);
-            }
-            x[i] = s;
-        }
-    }
-    cx<T> *dst = up ? Ui : Li;
-    for (int i = 0; i < KB; i++) dst[i * KB + cc] = x[i];
-}
-
 // The stored row at each position after the tile's interchanges goes to the
-// panel's slot of pord (the row band and the substitution passes read it).
+// positions of gord (the row band and the substitution passes read it).
 template <class T>
 __global__ void __launch_bounds__(256) k_panel(const PanelTask *__restrict__ tasks, const FrontDev *__restrict__ fr,
                                                cx<T> *__restrict__ fac, int *__restrict__ ipiv,
                                                const unsigned long long *__restrict__ amax2, double pivot_rel,
-                                               int *__restrict__ npert, int *__restrict__ pord)
+                                               int *__restrict__ npert, int *__restrict__ gord)
 {
     // static-pivot threshold: pivot_rel * max |a_ij| of the assembled operator
     const T thresh = (T)(pivot_rel * sqrt(__longlong_as_double((long long)*amax2)));
@@ -275,40 +235,7 @@ __global__ void __launch_bounds__(256) k_panel(const PanelTask *__restrict__ tas
         int i = idx / kb, j = idx % kb;
         D[(long long)i * nf + j] = S[i * LD + j];
     }
-    if (tid < KB) pord[(long long)(F.pan + k / KB) * KB + tid] = prow[tid];
-}
-
-// ---------------------------------------------------------------------------
-// Inverses of the unit-lower L_D and upper U_D factors of every factored tile,
-// for the substitution passes of the solves (dense products instead of serial
-// recurrences).  Run once after the factorisation over all panels: a tile is
-// final once its panel step is done (later steps change only rows and columns
-// to its right and below, and row interchanges are LINPACK style), so this
-// work is off the factorisation's chain of dependent panel steps.
-// Thread c < KB: column c of L_D^{-1}; KB <= c < 2 KB: column c - KB of
-// U_D^{-1}.  Padded to KB x KB with the identity.
-// ---------------------------------------------------------------------------
-template <class T>
-__global__ void __launch_bounds__(2 * KB) k_tile_inverse(const PanelTask *__restrict__ tasks,
-                                                         const FrontDev *__restrict__ fr,
-                                                         const cx<T> *__restrict__ fac, cx<T> *__restrict__ inv)
-{
-    extern __shared__ __align__(16) unsigned char smraw[];
-    cx<T> *S = reinterpret_cast<cx<T> *>(smraw);   // KB x (KB+1), then 2 KB scratch columns
-    const int LD = KB + 1;
-    const PanelTask t = tasks[blockIdx.x];
-    const FrontDev F = fr[t.f];
-    const int nf = F.p + F.b, k = t.k, kb = min(KB, F.p - k);
-    const cx<T> *D = fac + F.fac + (long long)k * nf + k;
-    const int tid = threadIdx.x;
-    #pragma unroll 8   // several loads in flight per thread
-    for (int idx = tid; idx < kb * kb; idx += blockDim.x) {
-        const int i = idx / kb, j = idx % kb;
-        S[i * LD + j] = D[(long long)i * nf + j];
-    }
-    __syncthreads();
-    cx<T> *Li = inv + (long long)(F.pan + k / KB) * (2 * KB * KB);
-    tile_inverse_cols<T>(S, kb, Li, Li + KB * KB, tid);
+    if (tid < kb) gord[F.first + k + tid] = F.first + k + prow[tid];
 }
 
 // ---------------------------------------------------------------------------
@@ -317,7 +244,7 @@ __global__ void __launch_bounds__(2 * KB) k_tile_inverse(const PanelTask *__rest
 constexpr int TRW = 128;   // columns per CTA
 template <class T>
 __global__ void __launch_bounds__(TRW) k_trsm_row(const RowTask *__restrict__ tasks, const FrontDev *__restrict__ fr,
-                                                  cx<T> *__restrict__ fac, const int *__restrict__ pord)
+                                                  cx<T> *__restrict__ fac, const int *__restrict__ gord)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T> *L = reinterpret_cast<cx<T> *>(smraw);          // KB x (KB+1)
@@ -334,7 +261,7 @@ __global__ void __launch_bounds__(TRW) k_trsm_row(const RowTask *__restrict__ ta
         int i = q / kb, j = q % kb;
         L[i * (KB + 1) + j] = base[(long long)i * nf + k + j];
     }
-    panel_rows(pord, F.pan + k / KB, kb, true, idx);
+    panel_rows(gord, F.first + k, kb, idx);
     __syncthreads();
     #pragma unroll 8   // several loads in flight per thread
     for (int q = tid; q < kb * nc; q += blockDim.x) {
@@ -478,7 +405,7 @@ __device__ __forceinline__ void load_tile_padded(cx<float> *T, const cx<float> *
 
 template <int UNUSED = 0>
 __global__ void __launch_bounds__(TRW) k_trsm_row_h(const RowTask *__restrict__ tasks, const FrontDev *__restrict__ fr,
-                                                    cx<float> *__restrict__ fac, const int *__restrict__ pord)
+                                                    cx<float> *__restrict__ fac, const int *__restrict__ gord)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<float> *L = reinterpret_cast<cx<float> *>(smraw);   // KB x LDT
@@ -495,7 +422,7 @@ __global__ void __launch_bounds__(TRW) k_trsm_row_h(const RowTask *__restrict__ 
         const int i = q / nc, c = q % nc;
         cp_async_cx(Bt + i * (TRW + 1) + c, base + (long long)i * nf + c0 + c);
     }
-    panel_rows(pord, F.pan + k / KB, kb, true, idx);
+    panel_rows(gord, F.first + k, kb, idx);
     cp_async_wait_all();
     __syncthreads();
     // Row i of the result is kept in the stored slot idx[i] of the row it
@@ -811,229 +738,6 @@ __global__ void __launch_bounds__(256, 2) k_gemm_ts(const GemmTask<T> *__restric
                 cx<T> *p = t.C + (long long)r * t.ldc + c;
                 *p = *p - acc[i][j];
             }
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Fused substitution step: the diagonal-tile product of panel k and the update
-// of the outer block's other rows, in one launch per panel step (the panel
-// steps of a block form a dependent chain; one launch instead of two halves
-// its latency).  Every CTA of a front computes the panel's solved rows
-//   mode 0  Z = L_D^{-1} P y          mode 1  Z = U_D^{-1} y
-//   mode 2  Z = U_D^{-H} y            mode 3  Z = P^T L_D^{-H} y
-// from the panel rows y of X (which no CTA of the launch writes) into shared
-// memory; update CTAs then subtract its contribution from their rows,
-//   mode 0  y_r -= L[r, k:k2] Z       mode 1  y_r -= U[r, k:k2] Z
-//   mode 2  y_r -= U[k:k2, r]^H Z     mode 3  y_r -= L[k:k2, r]^H Z
-// (rows below the panel for the forward modes 0/2, above it for 1/3), and the
-// role-0 CTA leaves Z in the front's scratch slot; the next step's role-0 CTA
-// (or a flush) writes it into X once no CTA reads those rows any more.
-// ---------------------------------------------------------------------------
-constexpr int SUB_RB = 32;   // rows per update CTA
-
-// Shared-memory layout of k_sub_step (complex elements).
-__host__ __device__ constexpr int sub_step_smem_elems()
-{
-    return KB * KB + KB * (MAXRHS + 1) + KB * SUB_RB + SUB_RB * (MAXRHS + 1);
-}
-
-// d += a b and d += conj(a) b as four fused multiply-adds
-template <class T>
-__device__ __forceinline__ void cmac(cx<T> &d, const cx<T> a, const cx<T> b)
-{
-    d.re = fma(a.re, b.re, fma(-a.im, b.im, d.re));
-    d.im = fma(a.re, b.im, fma(a.im, b.re, d.im));
-}
-template <class T>
-__device__ __forceinline__ void cmac_conj(cx<T> &d, const cx<T> a, const cx<T> b)
-{
-    d.re = fma(a.re, b.re, fma(a.im, b.im, d.re));
-    d.im = fma(a.re, b.im, fma(-a.im, b.re, d.im));
-}
-
-// four consecutive complex values from 16-byte-aligned shared memory
-__device__ __forceinline__ void lds4(const cx<float> *p, cx<float> (&a)[4])
-{
-    const float4 u = reinterpret_cast<const float4 *>(p)[0], v = reinterpret_cast<const float4 *>(p)[1];
-    a[0] = cx<float>(u.x, u.y); a[1] = cx<float>(u.z, u.w); a[2] = cx<float>(v.x, v.y); a[3] = cx<float>(v.z, v.w);
-}
-__device__ __forceinline__ void lds4(const cx<double> *p, cx<double> (&a)[4])
-{
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const double2 u = reinterpret_cast<const double2 *>(p)[j];
-        a[j] = cx<double>(u.x, u.y);
-    }
-}
-
-// two consecutive complex values from 16-byte-aligned shared memory
-__device__ __forceinline__ void lds2(const cx<float> *p, cx<float> (&a)[2])
-{
-    const float4 u = reinterpret_cast<const float4 *>(p)[0];
-    a[0] = cx<float>(u.x, u.y); a[1] = cx<float>(u.z, u.w);
-}
-__device__ __forceinline__ void lds2(const cx<double> *p, cx<double> (&a)[2])
-{
-    const double2 u = reinterpret_cast<const double2 *>(p)[0], v = reinterpret_cast<const double2 *>(p)[1];
-    a[0] = cx<double>(u.x, u.y); a[1] = cx<double>(v.x, v.y);
-}
-
-constexpr int SUB_THREADS = 512;   // 16 warps: each thread sums 4 rows of Z and 2 update rows
-template <class T>
-__global__ void __launch_bounds__(SUB_THREADS) k_sub_step(const StepTask *__restrict__ tasks, const FrontDev *__restrict__ fr,
-                                                  const cx<T> *__restrict__ fac, const cx<T> *__restrict__ inv,
-                                                  const int *__restrict__ pord, cx<T> *__restrict__ X, int ldx, int m,
-                                                  int mode, cx<T> *__restrict__ zs)
-{
-    // Launched as a programmatic dependent of the previous step: the next
-    // step may start as soon as every CTA of this one is running; it fetches
-    // what no step writes (task, tile inverse, factor rows, row order) and
-    // then waits for this grid's completion before it touches X or the slots.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    extern __shared__ __align__(16) unsigned char smraw[];
-    // every input is fetched in one batch of asynchronous copies, laid out so
-    // that the four rows a thread sums are adjacent: Ms[l][i] is the mode's
-    // tile-inverse entry (i, l) (conjugated on read for modes 2, 3), As[l][r]
-    // the update CTA's factor entry (r, l) (likewise)
-    cx<T> *Ms = reinterpret_cast<cx<T> *>(smraw);   // KB x KB
-    cx<T> *Ys = Ms + KB * KB;                       // KB x (MAXRHS+1): panel rows as stored, then Z
-    cx<T> *As = Ys + KB * (MAXRHS + 1);             // KB x SUB_RB
-    cx<T> *Yr = As + KB * SUB_RB;                   // SUB_RB x (MAXRHS+1): the update CTA's rows of X
-    __shared__ int idx[KB];
-    const StepTask t = tasks[blockIdx.x];
-    const FrontDev F = fr[t.f];
-    const int tid = threadIdx.x;
-    const int nf = F.p + F.b;
-    const int LY = MAXRHS + 1;
-    cx<T> *Y = X + (long long)F.first * ldx;
-    cx<T> *slot = zs + (long long)t.slot * (KB * MAXRHS);
-    const int k = t.k, kb = min(KB, F.p - k);
-    const cx<T> *Li = inv + (long long)(F.pan + k / KB) * (2 * KB * KB);
-    const cx<T> *Mi = (mode == 0 || mode == 3) ? Li : Li + KB * KB;
-    const bool herm = mode >= 2;
-    const int nr = t.role == 1 ? t.r1 - t.r0 : 0;
-    const cx<T> *P = fac + F.fac;
-    // stored inverse entry q = (a, b): (i, l) = (a, b) transposed into Ms[l][i],
-    // or (l, i) = (a, b) as stored for the conjugate transposes
-    for (int q = tid; q < KB * KB; q += blockDim.x)
-        cp_async_cx(herm ? Ms + q : Ms + (q & (KB - 1)) * KB + (q >> 6), Mi + q);
-    if (nr) {
-        if (mode == 0 || mode == 1) {   // A(r, l) = P[r0 + r][k + l]
-            for (int q = tid; q < nr * KB; q += blockDim.x) {   // (row, column) = (q / KB, q % KB)
-                const int r = q >> 6, l = q & (KB - 1);
-                if (l < kb) cp_async_cx(As + l * SUB_RB + r, P + (long long)(t.r0 + r) * nf + k + l);
-            }
-        } else {                        // A(r, l) = conj(P[k + l][r0 + r])
-            for (int q = tid; q < kb * SUB_RB; q += blockDim.x) {   // (column, row) = (q / SUB_RB, q % SUB_RB)
-                const int l = q / SUB_RB, r = q % SUB_RB;
-                if (r < nr) cp_async_cx(As + l * SUB_RB + r, P + (long long)(k + l) * nf + t.r0 + r);
-            }
-        }
-    }
-    panel_rows(pord, F.pan + k / KB, kb, mode == 0 || mode == 3, idx);
-    // everything below reads or writes rows of X or the slots
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    // (row, column) loops run over MAXRHS columns (a power of two) and skip
-    // those at or beyond m: no integer division per element
-    for (int q = tid; q < kb * MAXRHS; q += blockDim.x) {
-        const int i = q / MAXRHS, c = q % MAXRHS;
-        if (c < m) cp_async_cx(Ys + i * LY + c, Y + (long long)(k + i) * ldx + c);
-    }
-    if (nr) {
-        for (int q = tid; q < nr * MAXRHS; q += blockDim.x) {
-            const int r = q / MAXRHS, c = q % MAXRHS;
-            if (c < m) cp_async_cx(Yr + r * LY + c, Y + (long long)(t.r0 + r) * ldx + c);
-        }
-    }
-    // while the copies fly: the previous panel's solved rows into X (roles
-    // 0 and 3; no CTA of this launch reads those rows)
-    if (t.role != 1 && t.kprev >= 0) {
-        const int kbp = min(KB, F.p - t.kprev);
-        #pragma unroll 8   // several loads in flight per thread
-        for (int q = tid; q < kbp * MAXRHS; q += blockDim.x) {
-            const int i = q / MAXRHS, c = q % MAXRHS;
-            if (c < m) Y[(long long)(t.kprev + i) * ldx + c] = slot[i * MAXRHS + c];
-        }
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    // Z = M y: thread (lane c, warp w) owns rows 4w .. 4w+3 of column c; the
-    // l loop runs outside, so its sums are independent chains (M entries are
-    // warp broadcasts, two 16-byte loads per l for complex64)
-    constexpr int NW = SUB_THREADS / 32, RPT = KB / NW, UPT = SUB_RB / NW;
-    static_assert(RPT == 4 && UPT == 2, "four rows of Z, two update rows per thread");
-    const int c = tid & 31, w = tid >> 5, i0 = RPT * w;
-    cx<T> acc[RPT];
-#pragma unroll
-    for (int j = 0; j < RPT; j++) acc[j] = cx<T>(0);
-    if (c < m) {
-        if (!herm) {
-            for (int l = 0; l < kb; l++) {
-                const cx<T> y = Ys[(mode == 0 ? idx[l] : l) * LY + c];
-                cx<T> a[4];
-                lds4(Ms + l * KB + i0, a);
-#pragma unroll
-                for (int j = 0; j < RPT; j++) cmac(acc[j], a[j], y);
-            }
-        } else {
-            for (int l = 0; l < kb; l++) {
-                const cx<T> y = Ys[l * LY + c];
-                cx<T> a[4];
-                lds4(Ms + l * KB + i0, a);
-#pragma unroll
-                for (int j = 0; j < RPT; j++) cmac_conj(acc[j], a[j], y);
-            }
-        }
-    }
-    __syncthreads();
-    // Z (with the output permutation of mode 3) replaces the panel rows
-    if (c < m) {
-#pragma unroll
-        for (int j = 0; j < RPT; j++) {
-            const int i = i0 + j;
-            if (i < kb) Ys[(mode == 3 ? idx[i] : i) * LY + c] = acc[j];
-        }
-    }
-    __syncthreads();
-    if (t.role == 0 || t.role == 3) {
-        // role 3: the front's last panel of the block, which no other CTA of
-        // this launch reads: solved rows straight into X
-        for (int q = tid; q < kb * MAXRHS; q += blockDim.x) {
-            const int i = q / MAXRHS, cc = q % MAXRHS;
-            if (cc >= m) continue;
-            if (t.role == 0) slot[i * MAXRHS + cc] = Ys[i * LY + cc];
-            else Y[(long long)(k + i) * ldx + cc] = Ys[i * LY + cc];
-        }
-        return;
-    }
-    // update rows 2w, 2w+1 of column c, independent sums as above
-    if (c < m) {
-        const int u0 = UPT * w;
-        cx<T> u[UPT];
-#pragma unroll
-        for (int j = 0; j < UPT; j++) u[j] = cx<T>(0);
-        if (!herm) {
-            for (int l = 0; l < kb; l++) {
-                const cx<T> z = Ys[l * LY + c];
-                cx<T> a[UPT];
-                lds2(As + l * SUB_RB + u0, a);
-#pragma unroll
-                for (int j = 0; j < UPT; j++) cmac(u[j], a[j], z);
-            }
-        } else {
-            for (int l = 0; l < kb; l++) {
-                const cx<T> z = Ys[l * LY + c];
-                cx<T> a[UPT];
-                lds2(As + l * SUB_RB + u0, a);
-#pragma unroll
-                for (int j = 0; j < UPT; j++) cmac_conj(u[j], a[j], z);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < UPT; j++) {
-            const int r = u0 + j;
-            if (r < nr) Y[(long long)(t.r0 + r) * ldx + c] = Yr[r * LY + c] - u[j];
         }
     }
 }

@@ -1,0 +1,451 @@
+// Kernels of the substitution passes: explicit inverses of the diagonal blocks
+// of every front, computed once per factorisation, and the skinny products the
+// passes consist of (block inverse times right-hand sides, and the updates of
+// the rows outside a block).
+//
+// A front's pivot block is cut into diagonal blocks of up to SB columns.  With
+// the inverses of the block's triangular factors at hand, a substitution step
+// over SB unknowns is one product instead of SB / KB dependent ones.  The
+// length of the dependent chain is what bounds a pass on all but the largest
+// grids, not its bytes: a 40^3 pass was 364 dependent 64-wide steps of 18 us,
+// against 0.5 ms to read the factors at the memory rate.
+#pragma once
+#include "mf_kernels.cuh"
+
+namespace wt3d {
+
+// d += a b and d += conj(a) b as four fused multiply-adds
+template <class T>
+__device__ __forceinline__ void cmac(cx<T> &d, const cx<T> a, const cx<T> b)
+{
+    d.re = fma(a.re, b.re, fma(-a.im, b.im, d.re));
+    d.im = fma(a.re, b.im, fma(a.im, b.re, d.im));
+}
+template <class T>
+__device__ __forceinline__ void cmac_conj(cx<T> &d, const cx<T> a, const cx<T> b)
+{
+    d.re = fma(a.re, b.re, fma(a.im, b.im, d.re));
+    d.im = fma(a.re, b.im, fma(-a.im, b.re, d.im));
+}
+
+// ---------------------------------------------------------------------------
+// block inverses
+// ---------------------------------------------------------------------------
+constexpr int SB = 512;   // columns per diagonal block of the substitutions (a multiple of KB)
+
+// Row stride of a block inverse of w columns (even: rows start on 16 bytes).
+__host__ __device__ __forceinline__ int inv_ld(int w) { return (w + 1) & ~1; }
+
+// Entries of all block inverses of a front with p pivots.
+inline long long inv_entries(int p)
+{
+    const int full = p / SB, rest = p % SB;
+    return (long long)full * SB * inv_ld(SB) + (long long)rest * inv_ld(rest);
+}
+
+// The inverse of block c0 of a front is stored packed, row-major: the upper
+// triangle with the diagonal holds U^-1, the strict lower triangle L^-1 (unit
+// diagonal).  L is the block's lower factor with the rows of every KB-wide
+// panel in the order its interchanges leave them in, so that the forward
+// substitution of the block is z = L^-1 y[gord].
+//
+// Diagonal KB x KB tiles first: thread c < KB computes column c of L_D^-1,
+// KB <= c < 2 KB column c - KB of U_D^-1.  A tile is final once its panel step
+// is done (later steps change only rows and columns to its right and below).
+template <class T>
+__global__ void __launch_bounds__(2 * KB) k_tile_inverse(const PanelTask *__restrict__ tasks,
+                                                         const FrontDev *__restrict__ fr,
+                                                         const cx<T> *__restrict__ fac, cx<T> *__restrict__ inv)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    cx<T> *S = reinterpret_cast<cx<T> *>(smraw);   // KB x (KB+1), then 2 KB scratch columns
+    const int LD = KB + 1;
+    const PanelTask t = tasks[blockIdx.x];
+    const FrontDev F = fr[t.f];
+    const int nf = F.p + F.b, k = t.k, kb = min(KB, F.p - k);
+    const cx<T> *D = fac + F.fac + (long long)k * nf + k;
+    const int tid = threadIdx.x;
+    #pragma unroll 8   // several loads in flight per thread
+    for (int idx = tid; idx < kb * kb; idx += blockDim.x) {
+        const int i = idx / kb, j = idx % kb;
+        S[i * LD + j] = D[(long long)i * nf + j];
+    }
+    __syncthreads();
+    const int c0 = k / SB * SB, w = min(SB, F.p - c0), ldw = inv_ld(w), o = k - c0;
+    cx<T> *W = inv + F.inv + (long long)(c0 / SB) * (SB * SB) + (long long)o * ldw + o;
+    const bool up = tid >= KB;
+    const int c = up ? tid - KB : tid;
+    if (c >= kb) return;
+    cx<T> *x = S + KB * LD + tid * LD;
+    if (!up) {
+        x[c] = cx<T>(1);
+        for (int i = c + 1; i < kb; i++) {
+            cx<T> s(0);
+            for (int l = c; l < i; l++) s = s - S[i * LD + l] * x[l];
+            x[i] = s;
+            W[(long long)i * ldw + c] = s;
+        }
+    } else {
+        for (int i = c; i >= 0; i--) {
+            cx<T> s = (i == c) ? cx<T>(1) : cx<T>(0);
+            for (int l = i + 1; l <= c; l++) s = s - S[i * LD + l] * x[l];
+            s = cdiv(s, S[i * LD + i]);
+            x[i] = s;
+            W[(long long)i * ldw + c] = s;
+        }
+    }
+}
+
+// The off-diagonal tiles, by columns: one CTA per 32 columns (h: the first or
+// second half of tile column t) of one triangle of one block.  For L, from the
+// tile below the diagonal down: X_s = -L_ss^-1 sum_{u=t}^{s-1} L_su X_u; for
+// U, from the tile above the diagonal up: X_s = -U_ss^-1 sum_{u>s} U_su X_u.
+// A CTA reads only tiles that it wrote itself, and the diagonal ones.  FP32
+// (FP64) sums as in the substitutions themselves.
+struct InvTask { int f, c0, t, h, upper; };
+constexpr int IV_TH = 128, IV_BK = 16, IV_N = 32;
+
+template <class T>
+__global__ void __launch_bounds__(IV_TH) k_block_inverse(const InvTask *__restrict__ tasks,
+                                                         const FrontDev *__restrict__ fr,
+                                                         const cx<T> *__restrict__ fac, const int *__restrict__ gord,
+                                                         cx<T> *__restrict__ inv)
+{
+    __shared__ cx<T> As[KB][IV_BK + 1];
+    __shared__ cx<T> Bs[IV_BK][IV_N];
+    __shared__ cx<T> Ss[KB][IV_N];
+    __shared__ int rows[KB];
+    const InvTask t = tasks[blockIdx.x];
+    const FrontDev F = fr[t.f];
+    const int nf = F.p + F.b, w = min(SB, F.p - t.c0), ldw = inv_ld(w), nt = (w + KB - 1) / KB;
+    const cx<T> *D = fac + F.fac + (long long)t.c0 * nf + t.c0;   // the block's factors
+    cx<T> *W = inv + F.inv + (long long)(t.c0 / SB) * (SB * SB);
+    const bool up = t.upper != 0;
+    const int col0 = KB * t.t + IV_N * t.h;
+    const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;   // rows ty + 16 i, columns 4 tx + j
+    constexpr int NA = KB * IV_BK / IV_TH, NB = IV_BK * IV_N / IV_TH;
+    cx<T> pa[NA], pb[NB], acc[4][4];
+    for (int s = up ? t.t - 1 : t.t + 1; up ? s >= 0 : s < nt; s += up ? -1 : 1) {
+        const int r0 = KB * s, mr = min(KB, w - r0);
+        const int k0 = up ? KB * (s + 1) : KB * t.t, k1 = up ? min(w, KB * (t.t + 1)) : r0;
+        if (tid < KB) rows[tid] = !up && tid < mr ? gord[F.first + t.c0 + r0 + tid] - F.first - t.c0 : r0 + tid;
+        __syncthreads();   // also: the tile stored last is visible to the whole CTA
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[i][j] = cx<T>(0);
+        // phase 0: S = (factor tiles) X; phase 1: X_s = -(tile inverse) S
+        for (int phase = 0; phase < 2; phase++) {
+            const int ka = phase ? r0 : k0, kz = phase ? r0 + mr : k1;
+            auto load = [&](int kk0) {
+#pragma unroll
+                for (int q = 0; q < NA; q++) {
+                    const int idx = tid + q * IV_TH, i = idx / IV_BK, k = kk0 + idx % IV_BK;
+                    cx<T> v(0);
+                    if (i < mr && k < kz) {
+                        if (!phase) v = D[(long long)rows[i] * nf + k];
+                        else if (up ? k >= r0 + i : k < r0 + i) v = W[(long long)(r0 + i) * ldw + k];
+                        else if (!up && k == r0 + i) v = cx<T>(1);
+                    }
+                    pa[q] = v;
+                }
+                if (!phase) {
+#pragma unroll
+                    for (int q = 0; q < NB; q++) {
+                        const int idx = tid + q * IV_TH, k = kk0 + idx / IV_N, c = col0 + idx % IV_N;
+                        cx<T> v(0);
+                        if (k < kz && c < w) {
+                            if (up ? k <= c : k > c) v = W[(long long)k * ldw + c];
+                            else if (!up && k == c) v = cx<T>(1);
+                        }
+                        pb[q] = v;
+                    }
+                }
+            };
+            load(ka);
+            for (int kk0 = ka; kk0 < kz; kk0 += IV_BK) {
+#pragma unroll
+                for (int q = 0; q < NA; q++) {
+                    const int idx = tid + q * IV_TH;
+                    As[idx / IV_BK][idx % IV_BK] = pa[q];
+                }
+                if (!phase) {
+#pragma unroll
+                    for (int q = 0; q < NB; q++) {
+                        const int idx = tid + q * IV_TH;
+                        Bs[idx / IV_N][idx % IV_N] = pb[q];
+                    }
+                }
+                __syncthreads();
+                if (kk0 + IV_BK < kz) load(kk0 + IV_BK);
+                const cx<T>(*B)[IV_N] = phase ? Ss + (kk0 - r0) : Bs;
+#pragma unroll
+                for (int kk = 0; kk < IV_BK; kk++) {
+                    cx<T> a[4], b[4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) a[i] = As[ty + 16 * i][kk];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) b[j] = B[kk][4 * tx + j];
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+#pragma unroll
+                        for (int j = 0; j < 4; j++) cmac(acc[i][j], a[i], b[j]);
+                }
+                __syncthreads();
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int r = ty + 16 * i, c = col0 + 4 * tx + j;
+                    if (!phase) Ss[r][4 * tx + j] = acc[i][j];
+                    else if (r < mr && c < w) W[(long long)(r0 + r) * ldw + c] = -acc[i][j];
+                    acc[i][j] = cx<T>(0);
+                }
+            __syncthreads();
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// skinny products  out (=, +=, -=) op(A) in  over NC right-hand sides
+// ---------------------------------------------------------------------------
+// One unit per CTA: up to SK_M output rows and up to SK_KMAX input rows of a
+// factor block or a block inverse.  Blocks are cut along K so that every
+// launch has a few units per SM: a single 64 x 512 unit of 32 columns would
+// keep one SM busy for 17 us while the others idle.  Units of one task then
+// add up atomically.
+struct SkUnit {
+    const void *A;     // op = A: tile element (0, 0), rows lda apart; op = A^H: stored row 0, column 0
+    const int *bmap;   // input row of k: bmap[k], or b0 + k
+    const int *cmap;   // output row of i: cmap[i], or c0 + i
+    int b0, c0, lda, M, K;
+    int flags;
+    int d;             // triangles: first k of the unit minus its first row
+};
+enum { SK_LOWER = 1, SK_UPPER = 2, SK_SUB = 4, SK_ATOM = 8 };
+constexpr int SK_M = 64, SK_TH = 128, SK_KMAX = 1024;
+
+// Right-hand-side blocks are stored [row][NC]: NC is the smallest of these that
+// holds the pass's columns, so that one source does not pay for 32.
+inline int sk_columns(int m) { return m <= 1 ? 1 : m <= 4 ? 4 : m <= 8 ? 8 : m <= 16 ? 16 : 32; }
+
+// Stage depth along K, and stages: 40 KB per CTA at 32 columns, five CTAs per
+// SM for complex64.
+template <class T, int NC>
+struct SkCfg {
+    static constexpr int BK = (NC >= 32 ? 16 : 32) / (sizeof(T) / 4);
+    static constexpr int NS = 3;
+    static constexpr int VK = 16 / (int)sizeof(cx<T>);              // complex per 16 bytes
+    static constexpr int lda(bool h) { return h ? SK_M + VK : BK + VK; }
+    static constexpr int a_elems(bool h) { return (h ? BK : SK_M) * lda(h); }
+    static constexpr int b_elems() { return (BK * NC + 1) / 2 * 2; }
+    static constexpr size_t stage(bool h) { return sizeof(cx<T>) * (a_elems(h) + b_elems()); }
+    static constexpr size_t smem(bool h) { return NS * stage(h) + sizeof(int) * (SK_KMAX + SK_M); }
+};
+
+// copy of one complex element that fills the destination with zeros when !ok
+template <class T>
+__device__ __forceinline__ void cp_async_cx_z(cx<T> *dst, const cx<T> *src, bool ok)
+{
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if constexpr (sizeof(cx<T>) == 8)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_16_z(void *dst, const void *src, bool ok)
+{
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
+// 16-byte-aligned shared loads of N consecutive complex values
+template <int N>
+__device__ __forceinline__ void lds_cx(const cx<float> *p, cx<float> (&a)[N])
+{
+    if constexpr (N == 1) {
+        a[0] = *p;
+    } else {
+#pragma unroll
+        for (int j = 0; j < N; j += 2) {
+            const float4 u = reinterpret_cast<const float4 *>(p)[j / 2];
+            a[j] = cx<float>(u.x, u.y);
+            a[j + 1] = cx<float>(u.z, u.w);
+        }
+    }
+}
+template <int N>
+__device__ __forceinline__ void lds_cx(const cx<double> *p, cx<double> (&a)[N])
+{
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        const double2 u = reinterpret_cast<const double2 *>(p)[j];
+        a[j] = cx<double>(u.x, u.y);
+    }
+}
+
+__device__ __forceinline__ void red_add(cx<float> *p, const cx<float> v)
+{
+    atomicAdd(reinterpret_cast<float2 *>(p), make_float2(v.re, v.im));
+}
+__device__ __forceinline__ void red_add(cx<double> *p, const cx<double> v)
+{
+    atomicAdd(&p->re, v.re);
+    atomicAdd(&p->im, v.im);
+}
+
+// 128 threads in KG groups of 16 x TX: a group sums every KG-th k of a stage
+// for the whole 64 x NC tile, 4 rows x CT columns per thread (32 FP32
+// accumulators; narrower blocks have more groups, so that every thread works
+// at any NC).  A and the right-hand sides go through a ring of three
+// asynchronous-copy stages.  Launched as a programmatic dependent of the
+// previous product: the factor entries, which no product writes, are on their
+// way before the wait for it.  One pass, against KB-wide steps and 128 x 32
+// products that computed 32 columns whatever the pass held: 40^3 with 1 column
+// 11.4 -> 2.0 ms, with 32 columns 12.4 -> 4.4 ms (31 TF/s of 73 in the
+// updates), 64x64x48 with 32 columns 31.5 -> 14.1 ms, complex128 16x15x14 with
+// 4 columns 23 -> 1.1 ms.
+template <class T, int NC, bool H>
+__global__ void __launch_bounds__(SK_TH) k_skinny(const SkUnit *__restrict__ units, const cx<T> *__restrict__ in,
+                                                  cx<T> *__restrict__ out)
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    using C = SkCfg<T, NC>;
+    constexpr int BK = C::BK, NS = C::NS, VK = C::VK, LDA = C::lda(H), AE = C::a_elems(H), BE = C::b_elems();
+    constexpr int CT = NC < 4 ? NC : 4, TX = NC / CT, TPG = 16 * TX, KG = SK_TH / TPG;
+    static_assert(KG <= BK / VK && KG * SK_M * NC <= NS * (AE + BE), "groups per stage; the sums fit the ring");
+    extern __shared__ __align__(16) unsigned char smraw[];
+    cx<T> *As = reinterpret_cast<cx<T> *>(smraw), *Bs = As + NS * AE;
+    int *brow = reinterpret_cast<int *>(Bs + NS * BE), *crow = brow + SK_KMAX;
+    const SkUnit u = units[blockIdx.x];
+    const int tid = threadIdx.x, K = u.K, M = u.M;
+    const int g = tid / TPG, tx = tid % TX, ty = (tid % TPG) / TX;
+    const int nst = (K + BK - 1) / BK;
+    const cx<T> *A = reinterpret_cast<const cx<T> *>(u.A);
+    auto load_a = [&](int s) {
+        cx<T> *dst = As + (s % NS) * AE;
+#pragma unroll
+        for (int q = 0; q < SK_M * BK / SK_TH; q++) {
+            const int idx = tid + q * SK_TH;
+            const int i = H ? idx % SK_M : idx / BK, kk = H ? idx / SK_M : idx % BK, k = s * BK + kk;
+            const bool ok = i < M && k < K;
+            const long long o = !ok ? 0 : H ? (long long)k * u.lda + i : (long long)i * u.lda + k;
+            cp_async_cx_z(dst + (H ? kk * LDA + i : i * LDA + kk), A + o, ok);
+        }
+    };
+    auto load_b = [&](int s) {
+        cx<T> *dst = Bs + (s % NS) * BE;
+        if constexpr (sizeof(cx<T>) * NC < 16) {
+            for (int kk = tid; kk < BK; kk += SK_TH) {
+                const int k = s * BK + kk;
+                cp_async_cx_z(dst + kk, in + (k < K ? brow[k] : 0), k < K);
+            }
+        } else {
+            constexpr int CPR = NC / VK;   // 16-byte pieces per row
+#pragma unroll
+            for (int idx = tid; idx < BK * CPR; idx += SK_TH) {
+                const int kk = idx / CPR, c = idx % CPR, k = s * BK + kk;
+                cp_async_16_z(dst + kk * NC + c * VK, in + (k < K ? (long long)brow[k] * NC + c * VK : 0), k < K);
+            }
+        }
+    };
+    for (int s = 0; s < NS - 1; s++)
+        if (s < nst) load_a(s);
+    for (int k = tid; k < K; k += SK_TH) brow[k] = u.bmap ? u.bmap[k] : u.b0 + k;
+    if (tid < M) crow[tid] = u.cmap ? u.cmap[tid] : u.c0 + tid;
+    __syncthreads();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int s = 0; s < NS - 1; s++) {
+        if (s < nst) load_b(s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    cx<T> acc[4][CT];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < CT; j++) acc[i][j] = cx<T>(0);
+    for (int s = 0; s < nst; s++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(NS - 2) : "memory");
+        __syncthreads();   // stage s is there for all; stage s - 1 is no longer read
+        if (s + NS - 1 < nst) {
+            load_a(s + NS - 1);
+            load_b(s + NS - 1);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        cx<T> *Aw = As + (s % NS) * AE;
+        const cx<T> *Bw = Bs + (s % NS) * BE;
+        if (u.flags & (SK_LOWER | SK_UPPER)) {
+            // the other triangle's entries of a stage that the diagonal crosses
+            // become zeros (and ones on the unit diagonal); e: stored column minus
+            // stored row of (row i, k)
+            const int e0 = s * BK + u.d;
+            if (e0 + BK > 0 && e0 - (SK_M - 1) <= 0) {
+                for (int idx = tid; idx < SK_M * BK; idx += SK_TH) {
+                    const int i = H ? idx % SK_M : idx / BK, kk = H ? idx / SK_M : idx % BK;
+                    const int e = H ? i - (e0 + kk) : e0 + kk - i;
+                    cx<T> *p = Aw + (H ? kk * LDA + i : i * LDA + kk);
+                    if (u.flags & SK_UPPER) {
+                        if (e < 0) *p = cx<T>(0);
+                    } else if (e >= 0) {
+                        *p = cx<T>(e == 0 ? T(1) : T(0));
+                    }
+                }
+                __syncthreads();
+            }
+        }
+        if constexpr (!H) {
+#pragma unroll
+            for (int kp = 0; kp < BK / VK; kp += KG) {
+                const int kq = (kp + g) * VK;
+                cx<T> a[4][VK];
+#pragma unroll
+                for (int i = 0; i < 4; i++) lds_cx<VK>(Aw + (ty + 16 * i) * LDA + kq, a[i]);
+#pragma unroll
+                for (int v = 0; v < VK; v++) {
+                    cx<T> b[CT];
+                    lds_cx<CT>(Bw + (kq + v) * NC + tx * CT, b);
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+#pragma unroll
+                        for (int j = 0; j < CT; j++) cmac(acc[i][j], a[i][v], b[j]);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int kp = 0; kp < BK; kp += KG) {
+                const int kq = kp + g;
+                cx<T> a[4], b[CT];
+                lds_cx<4>(Aw + kq * LDA + 4 * ty, a);
+                lds_cx<CT>(Bw + kq * NC + tx * CT, b);
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int j = 0; j < CT; j++) cmac_conj(acc[i][j], a[i], b[j]);
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    // the groups' sums through shared memory, then whole rows of the output
+    cx<T> *red = As;   // KG x SK_M x NC
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int r = H ? 4 * ty + i : ty + 16 * i;
+#pragma unroll
+        for (int j = 0; j < CT; j++) red[(g * SK_M + r) * NC + tx * CT + j] = acc[i][j];
+    }
+    __syncthreads();
+    for (int idx = tid; idx < M * NC; idx += SK_TH) {
+        cx<T> v = red[idx];
+#pragma unroll
+        for (int q = 1; q < KG; q++) v = v + red[q * SK_M * NC + idx];
+        cx<T> *p = out + (long long)crow[idx / NC] * NC + idx % NC;
+        if (u.flags & SK_SUB) v = -v;
+        if (u.flags & SK_ATOM) red_add(p, v);
+        else if (u.flags & SK_SUB) *p = *p + v;
+        else *p = v;
+    }
+}
+
+}  // namespace wt3d
