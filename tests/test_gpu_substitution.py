@@ -40,3 +40,31 @@ def test_widths(dims):
                 # complex64 factors, refined to 1e-11: cond * tol bounds the difference
                 X = getattr(s32, name)(B[:, :k], tol=1e-11, maxit=30)
                 assert np.linalg.norm(X - X64) <= 1e-4 * np.linalg.norm(X64)
+
+
+@pytest.mark.parametrize("k", [1, 3, 8, 11, 32, 35])
+def test_products(k):
+    """A X at every width: FP64 rounding of 81-term sums; an infinity reaches
+    every row that stores an entry for it, zero entries included, as it does in
+    the full product."""
+    import scipy.sparse as sp
+    g = Grid(9, 8, 7, 20.0, pmld=2 * 20.0, fst=1)
+    vp, vs, rho = model.layered_random(9, 8, 7, 20.0, seed=4)
+    ir, jc = wt.pattern(9, 8, 7, base=0)
+    A = sp.csr_matrix((wt.assemble(g, vp, vs, rho, 2 * np.pi), jc, ir), shape=(g.n, g.n))
+    r = np.random.default_rng(k)
+    X = r.standard_normal((g.n, k)) + 1j * r.standard_normal((g.n, k))
+    with wt.Solver(g) as s:
+        s.set_model(vp, vs, rho)
+        s.factor(2 * np.pi)
+        Y = s.apply(X)
+        # at most 162 rounded products and additions per part
+        bound = 200 * np.finfo(float).eps * (abs(A) @ abs(X))
+        assert (abs(Y - A @ X) <= bound).all()
+        hit = 3 * (g.nnodes // 2) + 1
+        X[hit, 0] = np.inf
+        Y = s.apply(X)
+        stored = np.zeros(g.n, bool)
+        stored[np.repeat(np.arange(g.n), np.diff(ir))[jc == hit]] = True
+        np.testing.assert_array_equal(~np.isfinite(Y[:, 0]), stored)
+        assert np.isfinite(Y[:, 1:]).all()

@@ -3,6 +3,7 @@
 // the complex64 multifrontal factorisation.
 #include <atomic>
 #include "engine.cuh"
+#include "refine_kernels.cuh"
 #include "wtomo3d_gpu.h"
 #include <array>
 #include <chrono>
@@ -16,262 +17,6 @@ namespace wt3d {
 
 static thread_local std::string g_err;
 void set_error(const std::string &msg) { g_err = msg; }
-
-// ---------------------------------------------------------------------------
-// FP64 refinement kernels (natural ordering, row-major n x MAXRHS complex128)
-// ---------------------------------------------------------------------------
-__global__ void k_cm_to_rm(long long n, int m, const double2 *__restrict__ cm, double2 *__restrict__ rm)
-{
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    for (int j = 0; j < m; j++) rm[i * MAXRHS + j] = cm[(long long)j * n + i];
-}
-
-__global__ void k_rm_to_cm(long long n, int m, const double2 *__restrict__ rm, double2 *__restrict__ cm)
-{
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    for (int j = 0; j < m; j++) cm[(long long)j * n + i] = rm[i * MAXRHS + j];
-}
-
-__global__ void k_rm_to_cm_neg(long long n, int m, const double2 *__restrict__ rm, double2 *__restrict__ cm)
-{
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    for (int j = 0; j < m; j++) {
-        const double2 v = rm[i * MAXRHS + j];
-        cm[(long long)j * n + i] = make_double2(-v.x, -v.y);
-    }
-}
-
-// R = B - op(A) X (op = A or A^H), per-column squared norms of R into nr and of B into nb.
-// One warp per grid node; lane l holds right-hand sides l, l + 32, ...
-// (NH = MAXRHS / 32 of them).  The node's three rows (u, v, w) are contiguous
-// in the CSR and share one column list, so each column index and each row of
-// X is loaded once for the three rows.
-constexpr int NH = MAXRHS / 32;
-static_assert(MAXRHS % 32 == 0, "k_residual maps right-hand sides to lanes in groups of 32");
-__global__ void __launch_bounds__(256) k_residual(long long n, int m, const int *__restrict__ irptr,
-                                                  const int *__restrict__ jcptr, const double2 *__restrict__ a,
-                                                  const int *__restrict__ tpos, const double2 *__restrict__ X,
-                                                  const double2 *__restrict__ B, double2 *__restrict__ R,
-                                                  double *__restrict__ nr, double *__restrict__ nb, int adjoint)
-{
-    const int lane = threadIdx.x & 31;
-    const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    const long long nnode = n / 3;
-    bool on[NH];
-    double sr[NH], sb[NH];
-#pragma unroll
-    for (int h = 0; h < NH; h++) { on[h] = lane + 32 * h < m; sr[h] = sb[h] = 0; }
-    for (long long g = w0; g < nnode; g += nw) {
-        const long long r0 = 3 * g;
-        const int k0 = irptr[r0];
-        const int len = irptr[r0 + 1] - k0;
-        double2 acc[3][NH];
-#pragma unroll
-        for (int q = 0; q < 3; q++)
-#pragma unroll
-            for (int h = 0; h < NH; h++) acc[q][h] = make_double2(0, 0);
-#pragma unroll 3
-        for (int t = 0; t < len; t++) {
-            const int k = k0 + t;
-            const double2 *xr = X + (long long)jcptr[k] * MAXRHS + lane;
-            double2 x[NH];
-#pragma unroll
-            for (int h = 0; h < NH; h++) x[h] = on[h] ? xr[32 * h] : make_double2(0, 0);
-#pragma unroll
-            for (int q = 0; q < 3; q++) {
-                double2 av;
-                if (adjoint) { av = a[tpos[k + q * len]]; av.y = -av.y; }
-                else av = a[k + q * len];
-#pragma unroll
-                for (int h = 0; h < NH; h++) {
-                    acc[q][h].x = fma(av.x, x[h].x, fma(-av.y, x[h].y, acc[q][h].x));
-                    acc[q][h].y = fma(av.x, x[h].y, fma(av.y, x[h].x, acc[q][h].y));
-                }
-            }
-        }
-#pragma unroll
-        for (int h = 0; h < NH; h++) {
-            if (!on[h]) continue;
-            const int j = lane + 32 * h;
-#pragma unroll
-            for (int q = 0; q < 3; q++) {
-                // B == nullptr: R = op(A) X (the products of the Krylov solver)
-                const double2 b = B ? B[(r0 + q) * MAXRHS + j] : make_double2(0, 0);
-                const double2 r = B ? make_double2(b.x - acc[q][h].x, b.y - acc[q][h].y) : acc[q][h];
-                R[(r0 + q) * MAXRHS + j] = r;
-                sr[h] += r.x * r.x + r.y * r.y;
-                sb[h] += b.x * b.x + b.y * b.y;
-            }
-        }
-    }
-#pragma unroll
-    for (int h = 0; h < NH; h++)
-        if (on[h]) { atomicAdd(&nr[lane + 32 * h], sr[h]); atomicAdd(&nb[lane + 32 * h], sb[h]); }
-}
-
-// The same residual for a general pattern: one warp per row, rows of any
-// length and columns in any order.
-__global__ void __launch_bounds__(256) k_residual_rows(long long n, int m, const int *__restrict__ irptr,
-                                                       const int *__restrict__ jcptr, const double2 *__restrict__ a,
-                                                       const int *__restrict__ tpos, const double2 *__restrict__ X,
-                                                       const double2 *__restrict__ B, double2 *__restrict__ R,
-                                                       double *__restrict__ nr, double *__restrict__ nb, int adjoint)
-{
-    const int lane = threadIdx.x & 31;
-    const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    bool on[NH];
-    double sr[NH], sb[NH];
-#pragma unroll
-    for (int h = 0; h < NH; h++) { on[h] = lane + 32 * h < m; sr[h] = sb[h] = 0; }
-    for (long long r = w0; r < n; r += nw) {
-        double2 acc[NH];
-#pragma unroll
-        for (int h = 0; h < NH; h++) acc[h] = make_double2(0, 0);
-        for (int k = irptr[r]; k < irptr[r + 1]; k++) {
-            const double2 *xr = X + (long long)jcptr[k] * MAXRHS + lane;
-            double2 av;
-            if (adjoint) { av = a[tpos[k]]; av.y = -av.y; }
-            else av = a[k];
-#pragma unroll
-            for (int h = 0; h < NH; h++) {
-                const double2 x = on[h] ? xr[32 * h] : make_double2(0, 0);
-                acc[h].x = fma(av.x, x.x, fma(-av.y, x.y, acc[h].x));
-                acc[h].y = fma(av.x, x.y, fma(av.y, x.x, acc[h].y));
-            }
-        }
-#pragma unroll
-        for (int h = 0; h < NH; h++) {
-            if (!on[h]) continue;
-            const int j = lane + 32 * h;
-            const double2 b = B ? B[r * MAXRHS + j] : make_double2(0, 0);
-            const double2 q = B ? make_double2(b.x - acc[h].x, b.y - acc[h].y) : acc[h];
-            R[r * MAXRHS + j] = q;
-            sr[h] += q.x * q.x + q.y * q.y;
-            sb[h] += b.x * b.x + b.y * b.y;
-        }
-    }
-#pragma unroll
-    for (int h = 0; h < NH; h++)
-        if (on[h]) { atomicAdd(&nr[lane + 32 * h], sr[h]); atomicAdd(&nb[lane + 32 * h], sb[h]); }
-}
-
-// ---- batched Krylov kernels over n x MAXRHS row-major FP64 blocks -------
-// Column c of every block is an independent system; reductions go through
-// per-block partial sums and a second pass, so they do not depend on
-// scheduling.
-constexpr int GM_KMAX = 16;      // longest restart of the flexible GMRES (per-call length gmres_restart())
-constexpr int GM_BLOCKS = 304;   // 2 blocks per SM for the reductions
-
-// part[b][i][c] = sum over the rows of block b of conj(V_i[row, c]) W[row, c], i < nv.
-__global__ void __launch_bounds__(256) k_mdot(long long n, int m, int nv, const double2 *__restrict__ V,
-                                              long long vstride, const double2 *__restrict__ W,
-                                              double2 *__restrict__ part)
-{
-    __shared__ double2 red[8][MAXRHS];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (int i = 0; i < nv; i++) {
-        const double2 *Vi = V + (long long)i * vstride;
-        double2 acc[NH];
-#pragma unroll
-        for (int h = 0; h < NH; h++) acc[h] = make_double2(0, 0);
-        for (long long r = w0; r < n; r += nw) {
-#pragma unroll
-            for (int h = 0; h < NH; h++) {
-                const int c = lane + 32 * h;
-                if (c >= m) continue;
-                const double2 v = Vi[r * MAXRHS + c], w = W[r * MAXRHS + c];
-                acc[h].x = fma(v.x, w.x, fma(v.y, w.y, acc[h].x));
-                acc[h].y = fma(v.x, w.y, fma(-v.y, w.x, acc[h].y));
-            }
-        }
-#pragma unroll
-        for (int h = 0; h < NH; h++) red[warp][lane + 32 * h] = acc[h];
-        __syncthreads();
-        if (threadIdx.x < MAXRHS) {
-            double2 t = make_double2(0, 0);
-            for (int q = 0; q < 8; q++) { t.x += red[q][threadIdx.x].x; t.y += red[q][threadIdx.x].y; }
-            part[((long long)blockIdx.x * (GM_KMAX + 1) + i) * MAXRHS + threadIdx.x] = t;
-        }
-        __syncthreads();
-    }
-}
-
-// h[i][c] = sum_b part[b][i][c]
-__global__ void k_mdot_reduce(int nblocks, int nv, const double2 *__restrict__ part, double2 *__restrict__ h)
-{
-    const int i = blockIdx.x, c = threadIdx.x;
-    if (i >= nv || c >= MAXRHS) return;
-    double2 t = make_double2(0, 0);
-    for (int b = 0; b < nblocks; b++) {
-        const double2 v = part[((long long)b * (GM_KMAX + 1) + i) * MAXRHS + c];
-        t.x += v.x; t.y += v.y;
-    }
-    h[i * MAXRHS + c] = t;
-}
-
-// W[row, c] -= sum_{i < nv} coef[i][c] V_i[row, c]; with part != nullptr also
-// part[b][c] = per-block sum of |W_new[row, c]|^2.
-__global__ void __launch_bounds__(256) k_maxpy(long long n, int m, int nv, const double2 *__restrict__ V,
-                                               long long vstride, const double2 *__restrict__ coef,
-                                               double2 *__restrict__ W, double *__restrict__ part)
-{
-    __shared__ double red[256];
-    const long long tot = n * MAXRHS;
-    const long long stride = (long long)gridDim.x * blockDim.x;   // a multiple of MAXRHS: fixed column per thread
-    const int c = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) % MAXRHS);
-    double2 cf[GM_KMAX + 1];
-#pragma unroll
-    for (int i = 0; i <= GM_KMAX; i++) cf[i] = i < nv ? coef[i * MAXRHS + c] : make_double2(0, 0);
-    double s2 = 0;
-    if (c < m) {
-        for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < tot; q += stride) {
-            double2 w = W[q];
-#pragma unroll
-            for (int i = 0; i <= GM_KMAX; i++) {
-                if (i >= nv) break;
-                const double2 v = V[(long long)i * vstride + q];
-                w.x -= cf[i].x * v.x - cf[i].y * v.y;
-                w.y -= cf[i].x * v.y + cf[i].y * v.x;
-            }
-            W[q] = w;
-            s2 += w.x * w.x + w.y * w.y;
-        }
-    }
-    if (!part) return;
-    red[threadIdx.x] = s2;
-    __syncthreads();
-    if (threadIdx.x < MAXRHS) {
-        double t = 0;
-        for (int q = threadIdx.x; q < 256; q += MAXRHS) t += red[q];
-        part[(long long)blockIdx.x * MAXRHS + threadIdx.x] = t;
-    }
-}
-
-__global__ void k_norm_reduce(int nblocks, const double *__restrict__ part, double *__restrict__ out)
-{
-    const int c = threadIdx.x;
-    if (c >= MAXRHS) return;
-    double t = 0;
-    for (int b = 0; b < nblocks; b++) t += part[(long long)b * MAXRHS + c];
-    out[c] = t;
-}
-
-// W[row, c] *= s[c]
-__global__ void k_colscale(long long n, const double *__restrict__ sc, double2 *__restrict__ W)
-{
-    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n * MAXRHS) return;
-    const double f = sc[q % MAXRHS];
-    W[q].x *= f;
-    W[q].y *= f;
-}
 
 // Spread sources: F[src_col[e] * n + 3 node[e] + comp[e]] += w[e] * sterm[e]
 // (one thread per (source, weight) entry; entries of one source are distinct).
@@ -303,49 +48,6 @@ __global__ void k_get_receivers(long long n, int m, int nrec, const int *__restr
         acc.y += w[e] * u.y;
     }
     out[q] = acc;
-}
-
-// Xs = S R (new ordering, engine precision, rows of nc >= m columns); S the
-// Jacobi scaling of the factor.  Columns m .. nc - 1 and the pass's other two
-// blocks are zeroed.
-template <class T>
-__global__ void k_gather_new(long long n, int m, int nc, const int *__restrict__ perm, const double *__restrict__ s,
-                             const double2 *__restrict__ R, cx<T> *__restrict__ Xs, cx<T> *__restrict__ Zs,
-                             cx<T> *__restrict__ Ys)
-{
-    long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n * nc) return;
-    long long i = q / nc;
-    int j = (int)(q % nc);
-    cx<T> x(0);
-    if (j < m) {
-        const long long o = perm[i];
-        const double2 v = R[o * MAXRHS + j];
-        const double w = s[o];
-        x = cx<T>((T)(v.x * w), (T)(v.y * w));
-    }
-    Xs[q] = x;
-    Zs[q] = cx<T>(0);
-    Ys[q] = cx<T>(0);
-}
-
-// Xn += S Ys (natural ordering, FP64 accumulate).
-template <class T>
-__global__ void k_scatter_add_nat(long long n, int m, int nc, const int *__restrict__ perm,
-                                  const double *__restrict__ s, const cx<T> *__restrict__ Ys,
-                                  double2 *__restrict__ Xn)
-{
-    long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n * nc) return;
-    long long i = q / nc;
-    int j = (int)(q % nc);
-    if (j >= m) return;
-    const cx<T> v = Ys[q];
-    const long long o = perm[i];
-    const double w = s[o];
-    double2 *d = Xn + o * MAXRHS + j;
-    d->x += (double)v.re * w;
-    d->y += (double)v.im * w;
 }
 
 __global__ void k_pw_expand(int nx, int ny, int nz, double dx, int m, const double2 *__restrict__ Uz,
@@ -415,7 +117,7 @@ struct wt3d_solver {
     DevVec<float> vp, vs, rho;
     DevVec<float> qp, qs;                 // 1/Q per node (attenuation), optional
     double freqbase = 0;
-    DevVec<double2> Bn, Xn, Rn, T1;
+    DevVec<double2> Bn, Xn, Rn;
     DevVec<double2> abg, bgda, bgmu;      // background operator and Lame arrays
     DevVec<double> bgro;
     bool have_bg = false;
@@ -423,10 +125,12 @@ struct wt3d_solver {
     DevVec<double> norms;
     DevVec<double> gscr;                  // per-row derivative records of the gradient
     DevVec<double2> batF, batX;           // caller batch buffers (wt3d_batch_buffers)
-    StreamBuf<double2> gmV, gmZ;          // flexible GMRES: Krylov basis, preconditioned basis (per call)
+    StreamBuf<double2> gmV;               // flexible GMRES: Krylov basis and one more block (per call)
+    StreamBuf<char> gmZ;                  // ... preconditioned basis, in the engine's precision
     DevVec<double2> gmH;                  // flexible GMRES: projections
     DevVec<double2> gmPart;
     DevVec<double> gmNorm, gmScale;
+    void *pin = nullptr;                  // SolveHost
     std::unique_ptr<Engine<float>> e32;
     std::unique_ptr<Engine<double>> e64;
     cudaStream_t st = nullptr;
@@ -447,6 +151,7 @@ struct wt3d_solver {
         if (evl) cudaEventDestroy(evl);
         if (st) cudaStreamDestroy(st);
         if (sts) cudaStreamDestroy(sts);
+        if (pin) cudaFreeHost(pin);
     }
 };
 
@@ -484,17 +189,42 @@ int have_gpu()
 }
 
 // R = B - op(A) X (R = op(A) X when B is null), accumulating the squared
-// column norms of R and B into h->norms: node-blocked rows for the grid
-// pattern, one warp per row for a general pattern.
+// column norms of R and B into h->norms: a warp per node of the grid pattern, a
+// warp per row of a general one.
 void residual(const wt3d_solver *h, cudaStream_t st, int m, const double2 *X, const double2 *B, double2 *R,
               bool adjoint)
 {
-    if (h->general)
-        k_residual_rows<<<152 * 8, 256, 0, st>>>(h->n, m, h->irptr.p, h->jcptr.p, h->a.p, h->tpos.p, X, B, R,
-                                                 h->norms.p, h->norms.p + MAXRHS, adjoint ? 1 : 0);
-    else
-        k_residual<<<152 * 8, 256, 0, st>>>(h->n, m, h->irptr.p, h->jcptr.p, h->a.p, h->tpos.p, X, B, R,
-                                            h->norms.p, h->norms.p + MAXRHS, adjoint ? 1 : 0);
+    double *nr = h->norms.p, *nb = h->norms.p + MAXRHS;
+    const int adj = adjoint ? 1 : 0;
+    WT_SWITCH_NC(sk_columns(m),
+        if (h->general)
+            k_residual<NC, 1><<<152 * 8, 256, 0, st>>>(h->n, h->irptr.p, h->jcptr.p, h->a.p, h->tpos.p, X, B, R, nr,
+                                                       nb, adj);
+        else
+            k_residual<NC, 3><<<152 * 8, 256, 0, st>>>(h->n / 3, h->irptr.p, h->jcptr.p, h->a.p, h->tpos.p, X, B, R,
+                                                       nr, nb, adj))
+}
+
+// m columns (column-major, leading dimension n) to a row-major block and back
+void to_rows(const wt3d_solver *h, cudaStream_t st, int m, const double2 *cm, double2 *rm)
+{
+    WT_SWITCH_NC(sk_columns(m), k_cm_to_rm<NC><<<ceil_div(h->n, 32), 256, 0, st>>>(h->n, m, cm, rm))
+}
+void to_columns(const wt3d_solver *h, cudaStream_t st, int m, const double2 *rm, double2 *cm)
+{
+    WT_SWITCH_NC(sk_columns(m), k_rm_to_cm<NC><<<ceil_div(h->n, 32), 256, 0, st>>>(h->n, m, rm, cm))
+}
+
+// Pinned host staging of a solve's small results: the copies stay asynchronous.
+struct SolveHost {
+    double norms[2 * MAXRHS];
+    double2 h1[(GM_KMAX + 1) * MAXRHS], h2[(GM_KMAX + 1) * MAXRHS], coef[(GM_KMAX + 1) * MAXRHS];
+    double wn[MAXRHS], scale[MAXRHS];
+};
+int solve_host_buffer(wt3d_solver *h)
+{
+    if (!h->pin) WT_CUDA(cudaMallocHost(&h->pin, sizeof(SolveHost)));
+    return WT3D_OK;
 }
 
 // Restarted flexible GMRES in FP64, right-preconditioned by the factorisation
@@ -504,7 +234,8 @@ void residual(const wt3d_solver *h, cudaStream_t st, int m, const double2 *X, co
 // Gram-Schmidt applied twice; Givens rotations and the small least-squares
 // problems per column on the host.  The restart length is 8 unless the
 // WT3D_GMRES_RESTART environment variable sets another (1..16); each Arnoldi
-// vector costs 2 blocks of n x 32 complex128 while the call runs.
+// vector costs a block of n x sk_columns(m) complex128 and one in the factors'
+// precision while the call runs.
 static int gmres_restart()
 {
     static const int k = [] {
@@ -520,11 +251,13 @@ int fgmres(wt3d_solver *h, Engine<T> &E, Schedule<T> *sc, int m, bool adjoint, d
            const std::vector<double> &bnorm2, std::vector<double> &rnorm2, double *relres, int &it)
 {
     cudaStream_t st = h->sts;
-    const long long n = h->n, blk = n * MAXRHS;
+    const long long n = h->n;
+    const int nc = sk_columns(m);
+    const long long blk = n * nc;
     const int kr = gmres_restart();
     int rc;
     if (!h->gmH.p) {
-        if ((rc = h->gmH.alloc((size_t)(GM_KMAX + 1) * MAXRHS)) ||
+        if ((rc = h->gmH.alloc((size_t)2 * (GM_KMAX + 1) * MAXRHS)) ||
             (rc = h->gmPart.alloc((size_t)GM_BLOCKS * (GM_KMAX + 1) * MAXRHS)) ||
             (rc = h->gmNorm.alloc(MAXRHS)) || (rc = h->gmScale.alloc(MAXRHS)))
             return rc;
@@ -533,28 +266,27 @@ int fgmres(wt3d_solver *h, Engine<T> &E, Schedule<T> *sc, int m, bool adjoint, d
     // handle's resident memory), in stream order on the handle's solve
     // stream, so that taking and returning them never waits for work of
     // other handles
-    if ((rc = h->gmV.alloc((size_t)blk * (kr + 1), st)) || (rc = h->gmZ.alloc((size_t)blk * kr, st))) return rc;
+    if ((rc = h->gmV.alloc((size_t)blk * (kr + 2), st)) || (rc = h->gmZ.alloc(sizeof(cx<T>) * blk * kr, st))) return rc;
     struct Release {
         wt3d_solver *h;
         ~Release() { h->gmV.release(); h->gmZ.release(); }
     } release{h};
-    double2 *V = h->gmV.p, *Z = h->gmZ.p;
+    double2 *V = h->gmV.p, *Zd = V + blk * (kr + 1);   // Zd: M^-1 v of the current step in FP64
+    cx<T> *Z = reinterpret_cast<cx<T> *>(h->gmZ.p);
+    SolveHost &ph = *static_cast<SolveHost *>(h->pin);
     const int th = 256;
-    const int nc = sk_columns(m);
-    const unsigned nbm = (unsigned)ceil_div(n * nc, th), nbb = (unsigned)ceil_div(blk, th);
+    const unsigned nbb = (unsigned)ceil_div(blk, th);
     typedef std::complex<double> C;
-    std::vector<double> sc_h(MAXRHS);
-    std::vector<double2> hb((kr + 1) * MAXRHS), hb2((kr + 1) * MAXRHS), coef((kr + 1) * MAXRHS);
-    std::vector<double> wn(MAXRHS);
-    auto orth = [&](int nv, double2 *W, std::vector<double2> &out, bool norm) -> int {
-        k_mdot<<<GM_BLOCKS, 256, 0, st>>>(n, m, nv, V, blk, W, h->gmPart.p);
-        k_mdot_reduce<<<nv, MAXRHS, 0, st>>>(GM_BLOCKS, nv, h->gmPart.p, h->gmH.p);
-        k_maxpy<<<GM_BLOCKS, 256, 0, st>>>(n, m, nv, V, blk, h->gmH.p, W, norm ? (double *)h->gmPart.p : nullptr);
-        if (norm) k_norm_reduce<<<1, MAXRHS, 0, st>>>(GM_BLOCKS, (const double *)h->gmPart.p, h->gmNorm.p);
+    double *sc_h = ph.scale;
+    // one Gram-Schmidt sweep of W against V_0 .. V_{nv-1}; projections to out
+    auto orth = [&](int nv, double2 *W, double2 *hd, double2 *out, bool norm) -> int {
+        k_mdot<<<GM_BLOCKS, 256, 0, st>>>(blk, nc, nv, V, W, h->gmPart.p);
+        k_mdot_reduce<<<nv, 256, 0, st>>>(GM_BLOCKS, nc, h->gmPart.p, hd);
+        k_maxpy<<<GM_BLOCKS, 256, 0, st>>>(blk, nc, nv, V, hd, W, norm ? (double *)h->gmPart.p : nullptr);
+        if (norm) k_norm_reduce<<<1, 256, 0, st>>>(GM_BLOCKS, nc, (const double *)h->gmPart.p, h->gmNorm.p);
         WT_CUDA(cudaGetLastError());
-        WT_CUDA(cudaMemcpyAsync(out.data(), h->gmH.p, sizeof(double2) * nv * MAXRHS, cudaMemcpyDeviceToHost, st));
-        if (norm) WT_CUDA(cudaMemcpyAsync(wn.data(), h->gmNorm.p, sizeof(double) * MAXRHS, cudaMemcpyDeviceToHost, st));
-        WT_CUDA(cudaStreamSynchronize(st));
+        WT_CUDA(cudaMemcpyAsync(out, hd, sizeof(double2) * nv * MAXRHS, cudaMemcpyDeviceToHost, st));
+        if (norm) WT_CUDA(cudaMemcpyAsync(ph.wn, h->gmNorm.p, sizeof(double) * MAXRHS, cudaMemcpyDeviceToHost, st));
         return WT3D_OK;
     };
     for (;;) {
@@ -568,9 +300,8 @@ int fgmres(wt3d_solver *h, Engine<T> &E, Schedule<T> *sc, int m, bool adjoint, d
             sc_h[c] = done[c] ? 0.0 : 1.0 / beta[c];
         }
         for (int c = m; c < MAXRHS; c++) sc_h[c] = 0.0;
-        WT_CUDA(cudaMemcpyAsync(V, h->Rn.p, sizeof(double2) * blk, cudaMemcpyDeviceToDevice, st));
-        WT_CUDA(cudaMemcpyAsync(h->gmScale.p, sc_h.data(), sizeof(double) * MAXRHS, cudaMemcpyHostToDevice, st));
-        k_colscale<<<nbb, th, 0, st>>>(n, h->gmScale.p, V);
+        WT_CUDA(cudaMemcpyAsync(h->gmScale.p, sc_h, sizeof(double) * MAXRHS, cudaMemcpyHostToDevice, st));
+        k_colscale<<<nbb, th, 0, st>>>(blk, nc, h->gmScale.p, h->Rn.p, V);
         std::vector<std::vector<C>> H(m, std::vector<C>((kr + 1) * kr, C(0)));
         std::vector<std::vector<C>> g(m, std::vector<C>(kr + 1, C(0))), cs(m, std::vector<C>(kr)),
             sn(m, std::vector<C>(kr));
@@ -581,24 +312,27 @@ int fgmres(wt3d_solver *h, Engine<T> &E, Schedule<T> *sc, int m, bool adjoint, d
             for (int c = 0; c < m; c++) all = all && done[c];
             if (all || it >= maxit) break;
             // z_j = M^-1 v_j
-            double2 *Vj = V + (long long)j * blk, *Zj = Z + (long long)j * blk, *W = V + (long long)(j + 1) * blk;
-            k_gather_new<T><<<nbm, th, 0, st>>>(n, m, nc, h->perm.p, E.scale.p, Vj, E.X.p, E.Z.p, E.Y.p);
+            double2 *Vj = V + (long long)j * blk, *W = V + (long long)(j + 1) * blk;
+            k_gather_new<T><<<nbb, th, 0, st>>>(blk, nc, h->perm.p, E.scale.p, Vj, E.X.p, E.Z.p, E.Y.p);
             if ((rc = E.run(*sc, st))) return rc;
-            WT_CUDA(cudaMemsetAsync(Zj, 0, sizeof(double2) * blk, st));
-            k_scatter_add_nat<T><<<nbm, th, 0, st>>>(n, m, nc, h->perm.p, E.scale.p, E.Y.p, Zj);
+            WT_CUDA(cudaMemcpyAsync(Z + (long long)j * blk, E.Y.p, sizeof(cx<T>) * blk, cudaMemcpyDeviceToDevice, st));
+            k_scatter_nat<T><<<nbb, th, 0, st>>>(blk, nc, h->perm.p, E.scale.p, E.Y.p, Zd, 0);
             // w = op(A) z_j
             WT_CUDA(cudaMemsetAsync(h->norms.p, 0, sizeof(double) * 2 * MAXRHS, st));
-            residual(h, st, m, Zj, nullptr, W, adjoint);
+            residual(h, st, m, Zd, nullptr, W, adjoint);
             h->kernels_solve += sc->kernels() + 11;
-            if ((rc = orth(j + 1, W, hb, false)) || (rc = orth(j + 1, W, hb2, true))) return rc;
+            if ((rc = orth(j + 1, W, h->gmH.p, ph.h1, false)) ||
+                (rc = orth(j + 1, W, h->gmH.p + (GM_KMAX + 1) * MAXRHS, ph.h2, true)))
+                return rc;
+            WT_CUDA(cudaStreamSynchronize(st));
             it++;
             for (int c = 0; c < m; c++) {
                 if (done[c]) { sc_h[c] = 0.0; continue; }
                 std::vector<C> &Hc = H[c];
                 for (int i = 0; i <= j; i++)
-                    Hc[i * kr + j] = C(hb[i * MAXRHS + c].x + hb2[i * MAXRHS + c].x,
-                                         hb[i * MAXRHS + c].y + hb2[i * MAXRHS + c].y);
-                const double hn = sqrt(wn[c]);
+                    Hc[i * kr + j] = C(ph.h1[i * MAXRHS + c].x + ph.h2[i * MAXRHS + c].x,
+                                       ph.h1[i * MAXRHS + c].y + ph.h2[i * MAXRHS + c].y);
+                const double hn = sqrt(ph.wn[c]);
                 // earlier rotations, then a new one zeroing H[j+1][j]
                 for (int i = 0; i < j; i++) {
                     const C a = Hc[i * kr + j], b = Hc[(i + 1) * kr + j];
@@ -619,13 +353,14 @@ int fgmres(wt3d_solver *h, Engine<T> &E, Schedule<T> *sc, int m, bool adjoint, d
                 if (est <= 0.5 * tol || hn <= 1e-300) done[c] = 1;
                 sc_h[c] = done[c] ? 0.0 : 1.0 / hn;
             }
-            WT_CUDA(cudaMemcpyAsync(h->gmScale.p, sc_h.data(), sizeof(double) * MAXRHS, cudaMemcpyHostToDevice, st));
-            k_colscale<<<nbb, th, 0, st>>>(n, h->gmScale.p, W);
+            WT_CUDA(cudaMemcpyAsync(h->gmScale.p, sc_h, sizeof(double) * MAXRHS, cudaMemcpyHostToDevice, st));
+            k_colscale<<<nbb, th, 0, st>>>(blk, nc, h->gmScale.p, W, W);
         }
         // x += Z y, y = R^-1 g per column
         const int jmax = j;
         if (jmax > 0) {
-            std::fill(coef.begin(), coef.end(), make_double2(0, 0));
+            double2 *coef = ph.coef;
+            std::fill(coef, coef + (GM_KMAX + 1) * MAXRHS, make_double2(0, 0));
             for (int c = 0; c < m; c++) {
                 const int L = len[c];
                 std::vector<C> y(L);
@@ -636,15 +371,15 @@ int fgmres(wt3d_solver *h, Engine<T> &E, Schedule<T> *sc, int m, bool adjoint, d
                 }
                 for (int i = 0; i < L; i++) coef[i * MAXRHS + c] = make_double2(-y[i].real(), -y[i].imag());
             }
-            WT_CUDA(cudaMemcpyAsync(h->gmH.p, coef.data(), sizeof(double2) * jmax * MAXRHS, cudaMemcpyHostToDevice, st));
-            k_maxpy<<<GM_BLOCKS, 256, 0, st>>>(n, m, jmax, Z, blk, h->gmH.p, h->Xn.p, nullptr);
+            WT_CUDA(cudaMemcpyAsync(h->gmH.p, coef, sizeof(double2) * jmax * MAXRHS, cudaMemcpyHostToDevice, st));
+            k_zaxpy<T><<<nbb, th, 0, st>>>(blk, nc, jmax, h->perm.p, E.scale.p, Z, h->gmH.p, h->Xn.p);
         }
         // true residual
-        std::vector<double> hn2(2 * MAXRHS);
+        const double *hn2 = ph.norms;
         WT_CUDA(cudaMemsetAsync(h->norms.p, 0, sizeof(double) * 2 * MAXRHS, st));
         residual(h, st, m, h->Xn.p, h->Bn.p, h->Rn.p, adjoint);
         WT_CUDA(cudaGetLastError());
-        WT_CUDA(cudaMemcpyAsync(hn2.data(), h->norms.p, sizeof(double) * 2 * MAXRHS, cudaMemcpyDeviceToHost, st));
+        WT_CUDA(cudaMemcpyAsync(ph.norms, h->norms.p, sizeof(double) * 2 * MAXRHS, cudaMemcpyDeviceToHost, st));
         WT_CUDA(cudaStreamSynchronize(st));
         double worst = 0;
         for (int c = 0; c < m; c++) {
@@ -688,26 +423,28 @@ int refine(wt3d_solver *h, Engine<T> &E, int m, bool adjoint, double tol, int ma
     const long long n = h->n;
     Schedule<T> *sc = E.solve_schedule(m, adjoint);
     if (!sc) return WT3D_ERR_NOMEM;
-    WT_CUDA(cudaMemsetAsync(h->Xn.p, 0, sizeof(double2) * n * MAXRHS, st));
-    // start from R = B
-    WT_CUDA(cudaMemcpyAsync(h->Rn.p, h->Bn.p, sizeof(double2) * n * MAXRHS, cudaMemcpyDeviceToDevice, st));
-    std::vector<double> hn(2 * MAXRHS);
+    if (int e = solve_host_buffer(h)) return e;
+    const double *hn = static_cast<SolveHost *>(h->pin)->norms;
     int it = 0, rc = WT3D_OK;
     // the first pass is a refinement step from x = 0, whose relative residual is 1
     double prev_worst = 1.0;
-    const int th = 256;
-    const int nc = sk_columns(m);
-    const unsigned nb = (unsigned)ceil_div(n * nc, th);
+    const int th = 256, nc = sk_columns(m);
+    const long long blk = n * nc;
+    const unsigned nb = (unsigned)ceil_div(blk, th);
     for (;;) {
-        k_gather_new<T><<<nb, th, 0, st>>>(n, m, nc, h->perm.p, E.scale.p, h->Rn.p, E.X.p, E.Z.p, E.Y.p);
+        // the first pass solves for R = B and stores X, the later ones add to it
+        const bool first = it == 0;
+        k_gather_new<T><<<nb, th, 0, st>>>(blk, nc, h->perm.p, E.scale.p, first ? h->Bn.p : h->Rn.p, E.X.p, E.Z.p,
+                                           E.Y.p);
         rc = E.run(*sc, st);
         if (rc) return rc;
-        h->kernels_solve += sc->kernels() + 3;   // + gather, scatter-add, residual
-        k_scatter_add_nat<T><<<nb, th, 0, st>>>(n, m, nc, h->perm.p, E.scale.p, E.Y.p, h->Xn.p);
+        h->kernels_solve += sc->kernels() + 3;   // + gather, scatter, residual
+        k_scatter_nat<T><<<nb, th, 0, st>>>(blk, nc, h->perm.p, E.scale.p, E.Y.p, h->Xn.p, first ? 0 : 1);
         WT_CUDA(cudaMemsetAsync(h->norms.p, 0, sizeof(double) * 2 * MAXRHS, st));
         residual(h, st, m, h->Xn.p, h->Bn.p, h->Rn.p, adjoint);
         WT_CUDA(cudaGetLastError());
-        WT_CUDA(cudaMemcpyAsync(hn.data(), h->norms.p, sizeof(double) * 2 * MAXRHS, cudaMemcpyDeviceToHost, st));
+        WT_CUDA(cudaMemcpyAsync(static_cast<SolveHost *>(h->pin)->norms, h->norms.p, sizeof(double) * 2 * MAXRHS,
+                                cudaMemcpyDeviceToHost, st));
         WT_CUDA(cudaStreamSynchronize(st));
         double worst = 0;
         for (int j = 0; j < m; j++) {
@@ -719,7 +456,7 @@ int refine(wt3d_solver *h, Engine<T> &E, int m, bool adjoint, double tol, int ma
         if (worst <= tol) break;
         if (it >= maxit) { rc = WT3D_ERR_NOCONV; break; }
         if (worst > refine_switch() * prev_worst) {
-            std::vector<double> bn2(hn.begin() + MAXRHS, hn.begin() + MAXRHS + m), rn2(hn.begin(), hn.begin() + m);
+            std::vector<double> bn2(hn + MAXRHS, hn + MAXRHS + m), rn2(hn, hn + m);
             it++;
             rc = fgmres<T>(h, E, sc, m, adjoint, tol, maxit, bn2, rn2, relres, it);
             break;
@@ -756,7 +493,7 @@ int solve_dev_cm(wt3d_solver *h, int nrhs, const double2 *d_B, double2 *d_X, dou
     cudaEventRecord(h->ev0, h->sts);
     for (int c0 = 0; c0 < nrhs; c0 += MAXRHS) {
         int m = std::min(MAXRHS, nrhs - c0);
-        k_cm_to_rm<<<ceil_div(n, 256), 256, 0, h->sts>>>(n, m, d_B + (long long)c0 * n, h->Bn.p);
+        to_rows(h, h->sts, m, d_B + (long long)c0 * n, h->Bn.p);
         h->kernels_solve += 2;   // layout conversions in and out
         int its = 0, rc;
         if (h->e32) rc = refine<float>(h, *h->e32, m, adjoint, tol, maxit, relres ? relres + c0 : nullptr, &its);
@@ -764,7 +501,7 @@ int solve_dev_cm(wt3d_solver *h, int nrhs, const double2 *d_B, double2 *d_X, dou
         if (rc && rc != WT3D_ERR_NOCONV) return rc;
         if (rc) worst_rc = rc;
         maxits = std::max(maxits, its);
-        k_rm_to_cm<<<ceil_div(n, 256), 256, 0, h->sts>>>(n, m, h->Xn.p, d_X + (long long)c0 * n);
+        to_columns(h, h->sts, m, h->Xn.p, d_X + (long long)c0 * n);
     }
     cudaEventRecord(h->ev1, h->sts);
     WT_CUDA(cudaStreamSynchronize(h->sts));
@@ -841,7 +578,7 @@ double own_bytes(const wt3d_solver *h)
 {
     double b = (double)(h->e32 ? h->e32->device_bytes() : h->e64->device_bytes());
     b += (double)(h->irptr.n + h->jcptr.n + h->tpos.n + h->perm.n + h->vmap.n) * 4;
-    b += (double)(h->a.n + h->da.n + h->mu.n + h->Bn.n + h->Xn.n + h->Rn.n + h->T1.n + h->abg.n + h->bgda.n +
+    b += (double)(h->a.n + h->da.n + h->mu.n + h->Bn.n + h->Xn.n + h->Rn.n + h->abg.n + h->bgda.n +
                   h->bgmu.n + h->batF.n + h->batX.n) * 16;
     b += (double)(h->ro.n + h->bgro.n + h->norms.n + h->gscr.n) * 8 +
          (double)(h->vp.n + h->vs.n + h->rho.n + h->qp.n + h->qs.n) * 4;
@@ -1266,10 +1003,10 @@ int wt3d_rhs_planewave(wt3d_solver *h, const wt3d_layered1d *m, int nsrc, const 
             (rc = dky.upload(ky, h->st)) || (rc = drx.upload(rx, h->st)) || (rc = dry.upload(ry, h->st)))
             return rc;
         k_pw_expand<<<ceil_div((n / 3) * mm, 256), 256, 0, h->st>>>(nx, ny, nz, h->grid.dx, mm, dU.p, dW.p, dkx.p,
-                                                                     dky.p, drx.p, dry.p, h->Rn.p, MAXRHS);
-        k_hetfld<<<152 * 8, 256, 0, h->st>>>(n, mm, h->irptr.p, h->jcptr.p, h->a.p, h->abg.p, h->Rn.p, MAXRHS,
+                                                                     dky.p, drx.p, dry.p, h->Rn.p, sk_columns(mm));
+        k_hetfld<<<152 * 8, 256, 0, h->st>>>(n, mm, h->irptr.p, h->jcptr.p, h->a.p, h->abg.p, h->Rn.p, sk_columns(mm),
                                              (double2 *)d_F + (long long)c0 * n);
-        if (d_U0) k_rm_to_cm<<<ceil_div(n, 256), 256, 0, h->st>>>(n, mm, h->Rn.p, (double2 *)d_U0 + (long long)c0 * n);
+        if (d_U0) to_columns(h, h->st, mm, h->Rn.p, (double2 *)d_U0 + (long long)c0 * n);
         WT_CUDA(cudaGetLastError());
         WT_CUDA(cudaStreamSynchronize(h->st));
     }
@@ -1367,18 +1104,13 @@ int wt3d_apply(wt3d_solver *h, int nrhs, const double _Complex *X, double _Compl
     WT_CUDA(cudaMemcpyAsync(dX.p, X, sizeof(double2) * n * nrhs, cudaMemcpyHostToDevice, h->st));
     for (int c0 = 0; c0 < nrhs; c0 += MAXRHS) {
         int m = std::min(MAXRHS, nrhs - c0);
-        k_cm_to_rm<<<ceil_div(n, 256), 256, 0, h->st>>>(n, m, dX.p + (long long)c0 * n, h->Xn.p);
-        WT_CUDA(cudaMemsetAsync(h->Bn.p, 0, sizeof(double2) * n * MAXRHS, h->st));
-        WT_CUDA(cudaMemsetAsync(h->norms.p, 0, sizeof(double) * 2 * MAXRHS, h->st));
-        // R = 0 - A X
-        residual(h, h->st, m, h->Xn.p, h->Bn.p, h->Rn.p, false);
-        k_rm_to_cm<<<ceil_div(n, 256), 256, 0, h->st>>>(n, m, h->Rn.p, dX.p + (long long)c0 * n);
+        to_rows(h, h->st, m, dX.p + (long long)c0 * n, h->Xn.p);
+        residual(h, h->st, m, h->Xn.p, nullptr, h->Rn.p, false);
+        to_columns(h, h->st, m, h->Rn.p, dX.p + (long long)c0 * n);
     }
-    std::vector<std::complex<double>> tmp((size_t)n * nrhs);
-    WT_CUDA(cudaMemcpyAsync(tmp.data(), dX.p, sizeof(double2) * n * nrhs, cudaMemcpyDeviceToHost, h->st));
+    WT_CUDA(cudaGetLastError());
+    WT_CUDA(cudaMemcpyAsync(Y, dX.p, sizeof(double2) * n * nrhs, cudaMemcpyDeviceToHost, h->st));
     WT_CUDA(cudaStreamSynchronize(h->st));
-    std::complex<double> *Yc = reinterpret_cast<std::complex<double> *>(Y);
-    for (size_t i = 0; i < tmp.size(); i++) Yc[i] = -tmp[i];
     return WT3D_OK;
 }
 
@@ -1390,12 +1122,9 @@ int wt3d_apply_device(wt3d_solver *h, int nrhs, const void *d_X, void *d_Y)
     const long long n = h->n;
     for (int c0 = 0; c0 < nrhs; c0 += MAXRHS) {
         int m = std::min(MAXRHS, nrhs - c0);
-        k_cm_to_rm<<<ceil_div(n, 256), 256, 0, h->st>>>(n, m, (const double2 *)d_X + (long long)c0 * n, h->Xn.p);
-        WT_CUDA(cudaMemsetAsync(h->Bn.p, 0, sizeof(double2) * n * MAXRHS, h->st));
-        WT_CUDA(cudaMemsetAsync(h->norms.p, 0, sizeof(double) * 2 * MAXRHS, h->st));
-        // R = 0 - A X, then Y = -R
-        residual(h, h->st, m, h->Xn.p, h->Bn.p, h->Rn.p, false);
-        k_rm_to_cm_neg<<<ceil_div(n, 256), 256, 0, h->st>>>(n, m, h->Rn.p, (double2 *)d_Y + (long long)c0 * n);
+        to_rows(h, h->st, m, (const double2 *)d_X + (long long)c0 * n, h->Xn.p);
+        residual(h, h->st, m, h->Xn.p, nullptr, h->Rn.p, false);
+        to_columns(h, h->st, m, h->Rn.p, (double2 *)d_Y + (long long)c0 * n);
     }
     WT_CUDA(cudaGetLastError());
     WT_CUDA(cudaStreamSynchronize(h->st));
