@@ -39,8 +39,7 @@ struct Schedule {
         return c;
     }
     DevVec<PanelTask> panel;
-    DevVec<RowTask> row;
-    DevVec<ColTask> col;
+    DevVec<BandTask> band;
     DevVec<GemmTask<T>> gemm;
     DevVec<EATask> ea;
     DevVec<InvTask> inv;                                      // block-inverse columns
@@ -201,18 +200,8 @@ public:
         cudaGetDevice(&dev);
         std::call_once(attr_once[dev & 63], [] {
             size_t sp = sizeof(cx<T>) * (KB * (KB + 1) + 2 * KB * (KB + 1));
-            cudaFuncSetAttribute(k_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp);
             cudaFuncSetAttribute(k_tile_inverse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp);
-            cudaFuncSetAttribute(k_trsm_row<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(cx<T>) * (KB * (KB + 1) + KB * (TRW + 1))));
-            cudaFuncSetAttribute(k_trsm_col<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(cx<T>) * (KB * (KB + 1) + TCR * (KB + 1))));
-            if constexpr (std::is_same<T, float>::value) {
-                cudaFuncSetAttribute(k_trsm_row_h<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)band_row_smem());
-                cudaFuncSetAttribute(k_trsm_col_h<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)band_col_smem());
-            }
+            cudaFuncSetAttribute(k_bands<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BandCfg<T>::smem);
             sk_attr<1>();
             sk_attr<4>();
             sk_attr<8>();
@@ -449,7 +438,7 @@ public:
         const size_t smi = sizeof(cx<T>) * (KB * (KB + 1) + 2 * KB * (KB + 1));
         if (np) {
             sc.launches.push_back({[psc, this, p0, np, smi](cudaStream_t st) {
-                k_tile_inverse<T><<<np, 2 * KB, smi, st>>>(psc->panel.p + p0, fr.p, fac.p, binv.p);
+                k_tile_inverse<T><<<np, 2 * KB, smi, st>>>(psc->panel.p + p0, fr.p, fac.p, gord.p, ipiv.p, binv.p);
             }, LK_PANEL, 0});
             sc.launches.back().side = true;
         }
@@ -487,8 +476,7 @@ public:
     {
         auto sc = std::make_unique<Schedule<T>>();
         std::vector<PanelTask> hp;
-        std::vector<RowTask> hr;
-        std::vector<ColTask> hc;
+        std::vector<BandTask> hb;
         std::vector<GemmTask<T>> hg;
         std::vector<EATask> he;
         std::vector<InvTask> hi;
@@ -555,7 +543,7 @@ public:
             for (int c0 = 0; c0 < maxp; c0 += WB) {
                 const size_t pblk = hp.size();   // first panel of this outer block
                 for (int k = c0; k < std::min(c0 + WB, maxp); k += KB) {
-                    size_t p0 = hp.size(), r0 = hr.size(), cc0 = hc.size(), g0 = hg.size();
+                    size_t p0 = hp.size(), b0 = hb.size(), g0 = hg.size();
                     long long tiles = 0;
                     for (int f : fl) {
                         const Front &Fr = sym.fronts[f];
@@ -563,9 +551,9 @@ public:
                         const int nf = Fr.nf(), kb = std::min(KB, Fr.p - k), k2 = k + kb;
                         const int cend = std::min(c0 + WB, Fr.p);
                         hp.push_back(PanelTask{f, k});
-                        for (int c = k2; c < nf; c += TRW) hr.push_back(RowTask{f, k, c});
-                        for (int r = k2; r < Fr.p; r += TCR) hc.push_back(ColTask{f, k, r, 0});
-                        for (int r = 0; r < Fr.b; r += TCR) hc.push_back(ColTask{f, k, r, 1});
+                        for (int c = k2; c < nf; c += BD_V) hb.push_back(BandTask{f, k, c, 0});
+                        for (int r = k2; r < Fr.p; r += BD_V) hb.push_back(BandTask{f, k, r, 1});
+                        for (int r = 0; r < Fr.b; r += BD_V) hb.push_back(BandTask{f, k, r, 2});
                         cx<T> *Pb = F + Fr.fac_off;
                         cx<T> *Lo = Pb + (long long)Fr.p * nf;
                         // rows inside the outer block, every column right of the panel
@@ -577,27 +565,13 @@ public:
                         add_gemm(hg, tiles, Lo + k, Fr.p, Pb + (long long)k * nf + k2, nf, Lo + k2, Fr.p, Fr.b,
                                  cend - k2, kb);
                     }
-                    int np = (int)(hp.size() - p0), nr = (int)(hr.size() - r0), ncl = (int)(hc.size() - cc0);
-                    size_t smp = sizeof(cx<T>) * (KB * (KB + 1) + 2 * KB * (KB + 1));
-                    size_t smr = sizeof(cx<T>) * (KB * (KB + 1) + KB * (TRW + 1));
-                    size_t smc = sizeof(cx<T>) * (KB * (KB + 1) + TCR * (KB + 1));
-                    sc->launches.push_back({[psc, this, p0, np, smp](cudaStream_t st) {
-                        k_panel<T><<<np, 256, smp, st>>>(psc->panel.p + p0, fr.p, fac.p, ipiv.p, maxabs.p, pivot_rel,
-                                                         npert.p, gord.p);
+                    const int np = (int)(hp.size() - p0), nbd = (int)(hb.size() - b0);
+                    sc->launches.push_back({[psc, this, p0, np](cudaStream_t st) {
+                        k_panel<T><<<np, 256, 0, st>>>(psc->panel.p + p0, fr.p, fac.p, maxabs.p, pivot_rel, npert.p, gord.p);
                     }, LK_PANEL, 0});
-                    if (nr)
-                        sc->launches.push_back({[psc, this, r0, nr, smr](cudaStream_t st) {
-                            if constexpr (std::is_same<T, float>::value)
-                                k_trsm_row_h<0><<<nr, TRW, band_row_smem(), st>>>(psc->row.p + r0, fr.p, fac.p, gord.p);
-                            else
-                                k_trsm_row<T><<<nr, TRW, smr, st>>>(psc->row.p + r0, fr.p, fac.p, gord.p);
-                        }, LK_TRSM, 0});
-                    if (ncl)
-                        sc->launches.push_back({[psc, this, cc0, ncl, smc](cudaStream_t st) {
-                            if constexpr (std::is_same<T, float>::value)
-                                k_trsm_col_h<0><<<ncl, TCR, band_col_smem(), st>>>(psc->col.p + cc0, fr.p, fac.p);
-                            else
-                                k_trsm_col<T><<<ncl, TCR, smc, st>>>(psc->col.p + cc0, fr.p, fac.p);
+                    if (nbd)
+                        sc->launches.push_back({[psc, this, b0, nbd](cudaStream_t st) {
+                            k_bands<T><<<nbd, BD_TH, BandCfg<T>::smem, st>>>(psc->band.p + b0, fr.p, fac.p, gord.p);
                         }, LK_TRSM, 0});
                     push_gemm_launch(*sc, hg, g0, tiles);
                 }
@@ -635,8 +609,7 @@ public:
         }
         int rc;
         if ((rc = sc->panel.upload(hp))) return rc;
-        if ((rc = sc->row.upload(hr))) return rc;
-        if ((rc = sc->col.upload(hc))) return rc;
+        if ((rc = sc->band.upload(hb))) return rc;
         if ((rc = sc->gemm.upload(hg))) return rc;
         if ((rc = sc->ea.upload(he))) return rc;
         if ((rc = sc->inv.upload(hi))) return rc;

@@ -26,8 +26,6 @@ struct FrontDev {
 };
 
 struct PanelTask { int f, k; };
-struct RowTask { int f, k, c0; };
-struct ColTask { int f, k, r0, which; };
 struct EATask { int child, parent; long long row0; };
 template <class T>
 struct GemmTask {
@@ -143,200 +141,152 @@ __global__ void k_extend_add(const EATask *__restrict__ tasks, int ntasks, long 
     }
 }
 
-// Row order of panel k after its LINPACK-style interchanges: idx[i] is the
-// stored row that lands at position i, from gord, which holds for every pivot
-// position of the new ordering the row that lands there (written by the panel
-// kernel).  Threads tid < KB write idx; callers synchronise before reading it.
-__device__ __forceinline__ void panel_rows(const int *__restrict__ gord, int first, int kb, int *idx)
-{
-    const int tid = threadIdx.x;
-    if (tid < KB) idx[tid] = tid < kb ? gord[first + tid] - first : tid;
-}
-
 // ---------------------------------------------------------------------------
 // panel: LU of the KB x KB diagonal tile with partial pivoting inside the tile
 // ---------------------------------------------------------------------------
-// The stored row at each position after the tile's interchanges goes to the
-// positions of gord (the row band and the substitution passes read it).
+// order-preserving unsigned keys of non-negative values, 0 for NaN
+__device__ __forceinline__ unsigned pivot_key(float v) { return v == v ? __float_as_uint(v) : 0u; }
+__device__ __forceinline__ unsigned long long pivot_key(double v)
+{
+    return v == v ? (unsigned long long)__double_as_longlong(v) : 0ull;
+}
+__device__ __forceinline__ unsigned warp_max(unsigned k) { return __reduce_max_sync(0xffffffffu, k); }
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long k)
+{
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(k >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(k >> 32) == hi ? (unsigned)k : 0u);
+    return ((unsigned long long)hi << 32) | lo;
+}
+
+// element i (a run-time index) of four registers
 template <class T>
-__global__ void __launch_bounds__(256) k_panel(const PanelTask *__restrict__ tasks, const FrontDev *__restrict__ fr,
-                                               cx<T> *__restrict__ fac, int *__restrict__ ipiv,
-                                               const unsigned long long *__restrict__ amax2, double pivot_rel,
-                                               int *__restrict__ npert, int *__restrict__ gord)
+__device__ __forceinline__ cx<T> pick(const cx<T> &a0, const cx<T> &a1, const cx<T> &a2, const cx<T> &a3, int i)
+{
+    const cx<T> lo = (i & 1) ? a1 : a0, hi = (i & 1) ? a3 : a2;
+    return (i & 2) ? hi : lo;
+}
+
+// One CTA per tile; a chain of 64 dependent columns, so the latency of a column
+// is what counts.  The tile is held in registers: thread (tx, ty) =
+// (tid / 16, tid % 16) owns rows ty + 16 i and columns tx + 16 c, so that a
+// column's 64 entries sit in one half-warp and its pivot is found by two warp
+// reductions, without a barrier.  Rows stay where they are: a chosen row is
+// marked, the others go on, and rows are stored in the order they were chosen
+// in (gord).  Two barriers per column: the multipliers and the pivot's row
+// number, then the pivot row.  Equal magnitudes: the smallest stored row.
+// With the tile and its row swaps in shared memory a launch of few tiles took
+// 55 - 80 us.  Panels and bands together, 24x22x20: 59 steps 7.3 -> 3.9 ms;
+// 64x64x48: 358 steps 72 -> 54 ms.
+template <class T>
+__global__ void __launch_bounds__(256, 1) k_panel(const PanelTask *__restrict__ tasks,
+                                                  const FrontDev *__restrict__ fr, cx<T> *__restrict__ fac,
+                                                  const unsigned long long *__restrict__ amax2, double pivot_rel,
+                                                  int *__restrict__ npert, int *__restrict__ gord)
 {
     // static-pivot threshold: pivot_rel * max |a_ij| of the assembled operator
     const T thresh = (T)(pivot_rel * sqrt(__longlong_as_double((long long)*amax2)));
-    extern __shared__ __align__(16) unsigned char smraw[];
-    cx<T> *S = reinterpret_cast<cx<T> *>(smraw);   // KB x (KB+1), then 2 KB scratch columns
-    __shared__ int prow[KB];   // stored row at each position, as the interchanges go
+    __shared__ cx<T> lcol[2][KB], urow[KB];
+    __shared__ int s_p[2], pos[KB];
     const PanelTask t = tasks[blockIdx.x];
     const FrontDev F = fr[t.f];
     const int nf = F.p + F.b, k = t.k, kb = min(KB, F.p - k);
-    const int LD = KB + 1;
     cx<T> *D = fac + F.fac + (long long)k * nf + k;
-    const int tid = threadIdx.x;
-    #pragma unroll 8   // several loads in flight per thread
-    for (int idx = tid; idx < kb * kb; idx += blockDim.x) {
-        int i = idx / kb, j = idx % kb;
-        S[i * LD + j] = D[(long long)i * nf + j];
-    }
-    if (tid < KB) prow[tid] = tid;
-    __syncthreads();
-    // Column j: warp 0 finds the pivot, swaps the two rows, applies the
-    // static-pivot threshold and scales the column below the diagonal (one
-    // block barrier); then all threads update the trailing block, thread
-    // (tid / 16, tid % 16) taking every 16th row and column (a second one).
-    const int ty = tid >> 4, tx = tid & 15;
-    for (int j = 0; j < kb; j++) {
-        if (tid < 32) {
-            T best = -1; int bi = j;
-            for (int i = j + tid; i < kb; i += 32) {
-                T v = cabs2(S[i * LD + j]);
-                if (v > best) { best = v; bi = i; }
-            }
-            for (int o = 16; o > 0; o >>= 1) {   // every lane ends with the same (best, bi)
-                T ov = __shfl_xor_sync(0xffffffffu, best, o);
-                int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-            }
-            const int pv = bi;
-            if (pv != j)
-                for (int c = tid; c < kb; c += 32) {
-                    cx<T> a = S[j * LD + c];
-                    S[j * LD + c] = S[pv * LD + c];
-                    S[pv * LD + c] = a;
+    const int tid = threadIdx.x, tx = tid >> 4, ty = tid & 15, warp = tid >> 5, lane = tid & 31;
+    cx<T> a[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int r = ty + 16 * i, q = tx + 16 * c;
+            a[i][c] = (r < kb && q < kb) ? D[(long long)r * nf + q] : cx<T>(0);
+        }
+    unsigned used = 0;   // bit i: row ty + 16 i has been chosen, or is none of the tile's
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        if (ty + 16 * i >= kb) used |= 1u << i;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        for (int jj = 0; jj < 16; jj++) {
+            const int j = 16 * c + jj, buf = j & 1;
+            if (j >= kb) break;
+            if (warp == jj >> 1) {
+                const bool mine = (lane >> 4) == (jj & 1);   // the half-warp that holds column j
+                decltype(pivot_key(T(0))) key = 0, ki[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    ki[i] = pivot_key(cabs2(a[i][c]));
+                    if (!((used >> i) & 1u) && ki[i] > key) key = ki[i];
                 }
-            __syncwarp();
-            if (tid == 0) {
-                ipiv[F.first + k + j] = k + pv;
-                const int a = prow[j];
-                prow[j] = prow[pv];
-                prow[pv] = a;
-                cx<T> d = S[j * LD + j];
-                T m2 = cabs2(d);
+                if (!mine) key = 0;
+                const auto best = warp_max(key);
+                int row = KB;
+#pragma unroll
+                for (int i = 3; i >= 0; i--)
+                    if (mine && !((used >> i) & 1u) && ki[i] == best) row = ty + 16 * i;
+                const int p = (int)__reduce_min_sync(0xffffffffu, (unsigned)row);
+                const int src = (p & 15) + 16 * (jj & 1);
+                cx<T> d = pick(a[0][c], a[1][c], a[2][c], a[3][c], p >> 4);
+                d.re = __shfl_sync(0xffffffffu, d.re, src);
+                d.im = __shfl_sync(0xffffffffu, d.im, src);
+                const T m2 = cabs2(d);
                 if (!(m2 >= thresh * thresh)) {   // also catches NaN
-                    T m = sqrt(m2);
-                    S[j * LD + j] = (m > 0 && m == m) ? d * (thresh / m) : cx<T>(thresh);
-                    atomicAdd(npert, 1);
+                    const T m = sqrt(m2);
+                    d = (m > 0 && m == m) ? d * (thresh / m) : cx<T>(thresh);
+                    if (lane == src) atomicAdd(npert, 1);
+                }
+                const cx<T> inv = cdiv(cx<T>(1), d);
+                if (mine) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const int r = ty + 16 * i;
+                        if (r == p) a[i][c] = d;
+                        else if (!((used >> i) & 1u)) {
+                            a[i][c] = a[i][c] * inv;
+                            lcol[buf][r] = a[i][c];
+                        }
+                    }
+                    if (lane == src) {
+                        s_p[buf] = p;
+                        pos[p] = j;
+                    }
                 }
             }
-            __syncwarp();
-            const cx<T> inv = cdiv(cx<T>(1), S[j * LD + j]);
-            for (int i = j + 1 + tid; i < kb; i += 32) S[i * LD + j] = S[i * LD + j] * inv;
-        }
-        __syncthreads();
-        for (int i = j + 1 + ty; i < kb; i += 16) {
-            const cx<T> l = S[i * LD + j];
-            for (int c = j + 1 + tx; c < kb; c += 16) S[i * LD + c] = S[i * LD + c] - l * S[j * LD + c];
-        }
-        __syncthreads();
-    }
-    for (int idx = tid; idx < kb * kb; idx += blockDim.x) {
-        int i = idx / kb, j = idx % kb;
-        D[(long long)i * nf + j] = S[i * LD + j];
-    }
-    if (tid < kb) gord[F.first + k + tid] = F.first + k + prow[tid];
-}
-
-// ---------------------------------------------------------------------------
-// row band right of the panel: swap rows, then L_D^{-1} (unit lower)
-// ---------------------------------------------------------------------------
-constexpr int TRW = 128;   // columns per CTA
-template <class T>
-__global__ void __launch_bounds__(TRW) k_trsm_row(const RowTask *__restrict__ tasks, const FrontDev *__restrict__ fr,
-                                                  cx<T> *__restrict__ fac, const int *__restrict__ gord)
-{
-    extern __shared__ __align__(16) unsigned char smraw[];
-    cx<T> *L = reinterpret_cast<cx<T> *>(smraw);          // KB x (KB+1)
-    cx<T> *Bt = L + KB * (KB + 1);                       // KB x (TRW+1)
-    __shared__ int idx[KB];
-    const RowTask t = tasks[blockIdx.x];
-    const FrontDev F = fr[t.f];
-    const int nf = F.p + F.b, k = t.k, kb = min(KB, F.p - k);
-    const int c0 = t.c0, nc = min(TRW, nf - c0);
-    const int tid = threadIdx.x;
-    cx<T> *base = fac + F.fac + (long long)k * nf;
-    #pragma unroll 8   // several loads in flight per thread
-    for (int q = tid; q < kb * kb; q += blockDim.x) {
-        int i = q / kb, j = q % kb;
-        L[i * (KB + 1) + j] = base[(long long)i * nf + k + j];
-    }
-    panel_rows(gord, F.first + k, kb, idx);
-    __syncthreads();
-    #pragma unroll 8   // several loads in flight per thread
-    for (int q = tid; q < kb * nc; q += blockDim.x) {
-        int i = q / nc, c = q % nc;
-        Bt[i * (TRW + 1) + c] = base[(long long)idx[i] * nf + c0 + c];
-    }
-    __syncthreads();
-    if (tid < nc) {
-        for (int i = 1; i < kb; i++) {
-            cx<T> s = Bt[i * (TRW + 1) + tid];
-            for (int l = 0; l < i; l++) s = s - L[i * (KB + 1) + l] * Bt[l * (TRW + 1) + tid];
-            Bt[i * (TRW + 1) + tid] = s;
+            __syncthreads();
+            const int p = s_p[buf];
+            if ((p & 15) == ty) {
+                const int i = p >> 4;
+#pragma unroll
+                for (int q = c; q < 4; q++) urow[tx + 16 * q] = pick(a[0][q], a[1][q], a[2][q], a[3][q], i);
+                used |= 1u << i;
+            }
+            __syncthreads();
+            cx<T> l[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (!((used >> i) & 1u)) l[i] = lcol[buf][ty + 16 * i];
+#pragma unroll
+            for (int q = c; q < 4; q++) {
+                if (q == c && tx <= jj) continue;
+                const cx<T> u = urow[tx + 16 * q];
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (!((used >> i) & 1u)) {
+                        a[i][q].re = fma(-l[i].re, u.re, fma(l[i].im, u.im, a[i][q].re));
+                        a[i][q].im = fma(-l[i].re, u.im, fma(-l[i].im, u.re, a[i][q].im));
+                    }
+            }
         }
     }
     __syncthreads();
-    for (int q = tid; q < kb * nc; q += blockDim.x) {
-        int i = q / nc, c = q % nc;
-        base[(long long)i * nf + c0 + c] = Bt[i * (TRW + 1) + c];
-    }
-}
-
-// ---------------------------------------------------------------------------
-// column band below the panel: X <- X U_D^{-1}
-// ---------------------------------------------------------------------------
-constexpr int TCR = 128;   // rows per CTA
-template <class T>
-__global__ void __launch_bounds__(TCR) k_trsm_col(const ColTask *__restrict__ tasks, const FrontDev *__restrict__ fr,
-                                                  cx<T> *__restrict__ fac)
-{
-    extern __shared__ __align__(16) unsigned char smraw[];
-    cx<T> *U = reinterpret_cast<cx<T> *>(smraw);          // KB x (KB+1)
-    cx<T> *Xs = U + KB * (KB + 1);                        // TCR x (KB+1)
-    __shared__ cx<T> invd[KB];
-    const ColTask t = tasks[blockIdx.x];
-    const FrontDev F = fr[t.f];
-    const int nf = F.p + F.b, k = t.k, kb = min(KB, F.p - k);
-    const int tid = threadIdx.x;
-    const cx<T> *D = fac + F.fac + (long long)k * nf + k;
-    #pragma unroll 8   // several loads in flight per thread
-    for (int q = tid; q < kb * kb; q += blockDim.x) {
-        int i = q / kb, j = q % kb;
-        U[i * (KB + 1) + j] = D[(long long)i * nf + j];
-    }
-    cx<T> *xb;
-    long long ld;
-    int nr;
-    if (t.which == 0) {
-        xb = fac + F.fac + (long long)t.r0 * nf + k;
-        ld = nf;
-        nr = min(TCR, F.p - t.r0);
-    } else {
-        xb = fac + F.fac + (long long)F.p * nf + (long long)t.r0 * F.p + k;
-        ld = F.p;
-        nr = min(TCR, F.b - t.r0);
-    }
-    #pragma unroll 8   // several loads in flight per thread
-    for (int q = tid; q < nr * kb; q += blockDim.x) {
-        int r = q / kb, j = q % kb;
-        Xs[r * (KB + 1) + j] = xb[(long long)r * ld + j];
-    }
-    __syncthreads();
-    for (int j = tid; j < kb; j += blockDim.x) invd[j] = cdiv(cx<T>(1), U[j * (KB + 1) + j]);
-    __syncthreads();
-    if (tid < nr) {
-        cx<T> *x = Xs + tid * (KB + 1);
-        for (int j = 0; j < kb; j++) {
-            cx<T> s = x[j];
-            for (int l = 0; l < j; l++) s = s - x[l] * U[l * (KB + 1) + j];
-            x[j] = s * invd[j];
-        }
-    }
-    __syncthreads();
-    for (int q = tid; q < nr * kb; q += blockDim.x) {
-        int r = q / kb, j = q % kb;
-        xb[(long long)r * ld + j] = Xs[r * (KB + 1) + j];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int r = ty + 16 * i;
+        if (r >= kb) continue;
+        const int o = pos[r];
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            if (tx + 16 * c < kb) D[(long long)o * nf + tx + 16 * c] = a[i][c];
+        if (tx == 0) gord[F.first + k + o] = F.first + k + r;
     }
 }
 
@@ -356,194 +306,160 @@ __device__ __forceinline__ void cp_async_wait_all()
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
 }
 
-// ---------------------------------------------------------------------------
-// complex64 band solves by substitution, one column (row band) or one row
-// (column band) per thread, in eight groups of eight unknowns.  For group G
-// the thread solves its eight unknowns in registers with the diagonal 8 x 8
-// block of the tile, writes them back to its own column (row) in shared
-// memory, and then subtracts their multiples from every later group H, one
-// 8 x 8 block of the tile at a time (the tile's rows are read as 16-byte
-// broadcasts).  The loops over G and H are not unrolled, so the kernel's code
-// stays small: fully unrolled, the 2,016 multiply-adds of a 64-vector are
-// some 12k instructions per thread, and the warps then wait on instruction
-// fetch (ncu: 1.7 cycles per issue stalled on no_instruction, 24 % issue
-// activity).  The tile is padded with the identity beyond kb (a last,
-// narrower panel).
-// ---------------------------------------------------------------------------
-constexpr int TG = 8;                       // unknowns per group
-constexpr int LDT = KB + 2;                 // tile row stride: 16-byte-aligned rows
-__host__ __device__ constexpr size_t band_row_smem() { return sizeof(cx<float>) * (KB * LDT + KB * (TRW + 1)); }
-__host__ __device__ constexpr size_t band_col_smem() { return sizeof(cx<float>) * (KB * LDT + TCR * (KB + 1)); }
-
-__device__ __forceinline__ void cfms(cx<float> &d, const cx<float> a, const cx<float> b)   // d -= a b
+template <class T>
+__device__ __forceinline__ void cfms(cx<T> &d, const cx<T> a, const cx<T> b)   // d -= a b
 {
-    d.re = fmaf(-a.re, b.re, fmaf(a.im, b.im, d.re));
-    d.im = fmaf(-a.re, b.im, fmaf(-a.im, b.re, d.im));
+    d.re = fma(-a.re, b.re, fma(a.im, b.im, d.re));
+    d.im = fma(-a.re, b.im, fma(-a.im, b.re, d.im));
 }
 
-// eight consecutive complex values of a 16-byte-aligned shared-memory row
-__device__ __forceinline__ void lds8(const cx<float> *p, cx<float> (&a)[TG])
+// 16-byte-aligned shared loads of N consecutive complex values
+template <int N>
+__device__ __forceinline__ void lds_cx(const cx<float> *p, cx<float> (&a)[N])
+{
+    if constexpr (N == 1) {
+        a[0] = *p;
+    } else {
+#pragma unroll
+        for (int j = 0; j < N; j += 2) {
+            const float4 u = reinterpret_cast<const float4 *>(p)[j / 2];
+            a[j] = cx<float>(u.x, u.y);
+            a[j + 1] = cx<float>(u.z, u.w);
+        }
+    }
+}
+template <int N>
+__device__ __forceinline__ void lds_cx(const cx<double> *p, cx<double> (&a)[N])
 {
 #pragma unroll
-    for (int j = 0; j < TG; j += 2) {
-        const float4 u = reinterpret_cast<const float4 *>(p)[j / 2];
-        a[j] = cx<float>(u.x, u.y);
-        a[j + 1] = cx<float>(u.z, u.w);
+    for (int j = 0; j < N; j++) {
+        const double2 u = reinterpret_cast<const double2 *>(p)[j];
+        a[j] = cx<double>(u.x, u.y);
     }
 }
 
-// the KB x KB diagonal tile into shared memory (row stride LDT), identity
-// beyond kb
-__device__ __forceinline__ void load_tile_padded(cx<float> *T, const cx<float> *D, long long nf, int kb)
-{
-    for (int q = threadIdx.x; q < KB * KB; q += blockDim.x) {
-        const int i = q / KB, j = q % KB;
-        if (i < kb && j < kb) cp_async_cx(T + i * LDT + j, D + (long long)i * nf + j);
-        else T[i * LDT + j] = cx<float>(i == j ? 1.f : 0.f, 0.f);
-    }
-}
+// ---------------------------------------------------------------------------
+// bands of a panel: the rows right of it, B <- L_D^{-1} P B, and the columns
+// below it, X <- X U_D^{-1}, by substitution, in one launch (they do not depend
+// on one another).  Both are solves with a lower triangle T, vector by vector:
+// T = L_D (unit) for a column of the row band, T = U_D^T for a row of the column
+// band.  Four threads share a vector, in groups of TG unknowns: each of them
+// solves the group's diagonal block (redundantly, in registers) and subtracts
+// its multiples from every fourth row below, so that the dependent chain of a
+// vector is a third of one thread's.  A launch of the small and middle levels
+// has few vectors and is bound by that chain: 27 us each for the two launches
+// with one thread per vector.  The loops over groups are not unrolled: the
+// kernel's code stays in the instruction cache.  The tile is padded with the
+// identity beyond kb (a last, narrower panel).
+// ---------------------------------------------------------------------------
+struct BandTask { int f, k, c0, which; };   // which: 0 columns right, 1 pivot rows below, 2 border rows; c0: the first
+constexpr int BD_V = 32, BD_TH = 4 * BD_V;  // vectors and threads per CTA
+template <class T>
+struct BandCfg {
+    static constexpr int TG = sizeof(T) == 4 ? 8 : 4;       // unknowns per group
+    static constexpr int LDT = KB + 16 / (int)sizeof(cx<T>);   // tile rows on 16 bytes, four rows on different banks
+    static constexpr int LDX = sizeof(T) == 4 ? BD_V + 4 : BD_V + 2;
+    static constexpr size_t smem = sizeof(cx<T>) * (KB * LDT + KB * LDX);
+};
 
-template <int UNUSED = 0>
-__global__ void __launch_bounds__(TRW) k_trsm_row_h(const RowTask *__restrict__ tasks, const FrontDev *__restrict__ fr,
-                                                    cx<float> *__restrict__ fac, const int *__restrict__ gord)
+template <class T>
+__global__ void __launch_bounds__(BD_TH) k_bands(const BandTask *__restrict__ tasks, const FrontDev *__restrict__ fr,
+                                                 cx<T> *__restrict__ fac, const int *__restrict__ gord)
 {
+    using C = BandCfg<T>;
+    constexpr int TG = C::TG, LDT = C::LDT, LDX = C::LDX;
     extern __shared__ __align__(16) unsigned char smraw[];
-    cx<float> *L = reinterpret_cast<cx<float> *>(smraw);   // KB x LDT
-    cx<float> *Bt = L + KB * LDT;                         // KB x (TRW+1): band rows as stored
+    cx<T> *Tm = reinterpret_cast<cx<T> *>(smraw);   // KB x LDT
+    cx<T> *X = Tm + KB * LDT;                       // KB x LDX: unknown i of vector v
     __shared__ int idx[KB];
-    const RowTask t = tasks[blockIdx.x];
+    __shared__ cx<T> invd[KB];
+    const BandTask t = tasks[blockIdx.x];
     const FrontDev F = fr[t.f];
     const int nf = F.p + F.b, k = t.k, kb = min(KB, F.p - k);
-    const int c0 = t.c0, nc = min(TRW, nf - c0);
     const int tid = threadIdx.x;
-    cx<float> *base = fac + F.fac + (long long)k * nf;
-    load_tile_padded(L, base + k, nf, kb);
-    for (int q = tid; q < kb * nc; q += blockDim.x) {
-        const int i = q / nc, c = q % nc;
-        cp_async_cx(Bt + i * (TRW + 1) + c, base + (long long)i * nf + c0 + c);
+    const bool row = t.which == 0;
+    const cx<T> *D = fac + F.fac + (long long)k * nf + k;
+    for (int q = tid; q < KB * KB; q += BD_TH) {
+        const int i = q / KB, j = q % KB;   // tile entry (i, j) as stored
+        cx<T> *dst = row ? Tm + i * LDT + j : Tm + j * LDT + i;
+        if (i < kb && j < kb) cp_async_cx(dst, D + (long long)i * nf + j);
+        else *dst = cx<T>(i == j ? T(1) : T(0));
     }
-    panel_rows(gord, F.first + k, kb, idx);
+    cx<T> *xb;     // unknown i of vector v at xb + i * si + v * sv
+    long long si, sv;
+    int nv;
+    if (row) {
+        xb = fac + F.fac + (long long)k * nf + t.c0;
+        si = nf;
+        sv = 1;
+        nv = min(BD_V, nf - t.c0);
+        if (tid < KB) idx[tid] = tid < kb ? gord[F.first + k + tid] - F.first - k : 0;
+        __syncthreads();
+        for (int q = tid; q < KB * BD_V; q += BD_TH) {
+            const int i = q / BD_V, v = q % BD_V;
+            if (i < kb && v < nv) cp_async_cx(X + i * LDX + v, xb + idx[i] * si + v);
+            else X[i * LDX + v] = cx<T>(0);
+        }
+    } else {
+        if (t.which == 1) {
+            xb = fac + F.fac + (long long)t.c0 * nf + k;
+            sv = nf;
+            nv = min(BD_V, F.p - t.c0);
+        } else {
+            xb = fac + F.fac + (long long)F.p * nf + (long long)t.c0 * F.p + k;
+            sv = F.p;
+            nv = min(BD_V, F.b - t.c0);
+        }
+        si = 1;
+        for (int q = tid; q < KB * BD_V; q += BD_TH) {
+            const int i = q % KB, v = q / KB;
+            if (i < kb && v < nv) cp_async_cx(X + i * LDX + v, xb + v * sv + i);
+            else X[i * LDX + v] = cx<T>(0);
+        }
+    }
     cp_async_wait_all();
     __syncthreads();
-    // Row i of the result is kept in the stored slot idx[i] of the row it
-    // came from: the slots of rows not yet read stay untouched.  Unknowns at
-    // or beyond kb are zero and stay zero (identity padding).
-    if (tid < nc) {
-        cx<float> *col = Bt + tid;
-        const int ng = (kb + TG - 1) / TG;
+    if (tid < KB) invd[tid] = row ? cx<T>(1) : cdiv(cx<T>(1), Tm[tid * LDT + tid]);
+    __syncthreads();
+    const int v = tid >> 2, q4 = tid & 3;
+    const int ng = (kb + TG - 1) / TG;
+    cx<T> *x = X + v;
 #pragma unroll 1
-        for (int G = 0; G < ng; G++) {
-            cx<float> b[TG];
+    for (int G = 0; G < ng; G++) {
+        cx<T> b[TG];
 #pragma unroll
-            for (int i = 0; i < TG; i++) b[i] = TG * G + i < kb ? col[idx[TG * G + i] * (TRW + 1)] : cx<float>(0.f, 0.f);
+        for (int i = 0; i < TG; i++) b[i] = x[(TG * G + i) * LDX];
 #pragma unroll
-            for (int i = 1; i < TG; i++) {
-                cx<float> lr[TG];
-                lds8(L + (TG * G + i) * LDT + TG * G, lr);
+        for (int i = 0; i < TG; i++) {
+            if (i > 0) {
+                cx<T> lr[TG];
+                lds_cx<TG>(Tm + (TG * G + i) * LDT + TG * G, lr);
 #pragma unroll
                 for (int l = 0; l < i; l++) cfms(b[i], lr[l], b[l]);
             }
+            if (!row) b[i] = b[i] * invd[TG * G + i];
+        }
+        __syncwarp();   // the four threads have read the group
 #pragma unroll
-            for (int i = 0; i < TG; i++)
-                if (TG * G + i < kb) col[idx[TG * G + i] * (TRW + 1)] = b[i];
+        for (int i = 0; i < TG; i++)
+            if ((i & 3) == q4) x[(TG * G + i) * LDX] = b[i];
 #pragma unroll 1
-            for (int H = G + 1; H < ng; H++) {
+        for (int H = TG * (G + 1) + q4; H < TG * ng; H += TG) {
 #pragma unroll
-                for (int i = 0; i < TG; i++) {
-                    const int row = TG * H + i;
-                    if (row < kb) {
-                        cx<float> lr[TG];
-                        lds8(L + row * LDT + TG * G, lr);
-                        cx<float> c = col[idx[row] * (TRW + 1)];
+            for (int i = 0; i < TG; i += 4) {
+                cx<T> lr[TG], c = x[(H + i) * LDX];
+                lds_cx<TG>(Tm + (H + i) * LDT + TG * G, lr);
 #pragma unroll
-                        for (int l = 0; l < TG; l++) cfms(c, lr[l], b[l]);
-                        col[idx[row] * (TRW + 1)] = c;
-                    }
-                }
+                for (int l = 0; l < TG; l++) cfms(c, lr[l], b[l]);
+                x[(H + i) * LDX] = c;
             }
         }
+        __syncwarp();
     }
     __syncthreads();
-    for (int q = tid; q < kb * nc; q += blockDim.x) {
-        const int i = q / nc, c = q % nc;
-        base[(long long)i * nf + c0 + c] = Bt[idx[i] * (TRW + 1) + c];
-    }
-}
-
-template <int UNUSED = 0>
-__global__ void __launch_bounds__(TCR) k_trsm_col_h(const ColTask *__restrict__ tasks, const FrontDev *__restrict__ fr,
-                                                    cx<float> *__restrict__ fac)
-{
-    extern __shared__ __align__(16) unsigned char smraw[];
-    cx<float> *U = reinterpret_cast<cx<float> *>(smraw);   // KB x LDT
-    cx<float> *Xs = U + KB * LDT;                         // TCR x (KB+1)
-    __shared__ cx<float> invd[KB];
-    const ColTask t = tasks[blockIdx.x];
-    const FrontDev F = fr[t.f];
-    const int nf = F.p + F.b, k = t.k, kb = min(KB, F.p - k);
-    const int tid = threadIdx.x;
-    load_tile_padded(U, fac + F.fac + (long long)k * nf + k, nf, kb);
-    cx<float> *xb;
-    long long ld;
-    int nr;
-    if (t.which == 0) {
-        xb = fac + F.fac + (long long)t.r0 * nf + k;
-        ld = nf;
-        nr = min(TCR, F.p - t.r0);
-    } else {
-        xb = fac + F.fac + (long long)F.p * nf + (long long)t.r0 * F.p + k;
-        ld = F.p;
-        nr = min(TCR, F.b - t.r0);
-    }
-    for (int q = tid; q < nr * kb; q += blockDim.x) {
-        const int r = q / kb, j = q % kb;
-        cp_async_cx(Xs + r * (KB + 1) + j, xb + (long long)r * ld + j);
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    for (int j = tid; j < KB; j += blockDim.x) invd[j] = cdiv(cx<float>(1.f, 0.f), U[j * LDT + j]);
-    __syncthreads();
-    if (tid < nr) {
-        cx<float> *row = Xs + tid * (KB + 1);
-        const int ng = (kb + TG - 1) / TG;
-#pragma unroll 1
-        for (int G = 0; G < ng; G++) {
-            cx<float> x[TG];
-#pragma unroll
-            for (int j = 0; j < TG; j++) x[j] = TG * G + j < kb ? row[TG * G + j] : cx<float>(0.f, 0.f);
-#pragma unroll
-            for (int j = 0; j < TG; j++) {
-                x[j] = x[j] * invd[TG * G + j];
-                cx<float> ur[TG];
-                lds8(U + (TG * G + j) * LDT + TG * G, ur);
-#pragma unroll
-                for (int j2 = j + 1; j2 < TG; j2++) cfms(x[j2], x[j], ur[j2]);
-            }
-#pragma unroll
-            for (int j = 0; j < TG; j++)
-                if (TG * G + j < kb) row[TG * G + j] = x[j];
-#pragma unroll 1
-            for (int H = G + 1; H < ng; H++) {
-                cx<float> y[TG];
-#pragma unroll
-                for (int j = 0; j < TG; j++) y[j] = TG * H + j < kb ? row[TG * H + j] : cx<float>(0.f, 0.f);
-#pragma unroll
-                for (int l = 0; l < TG; l++) {
-                    cx<float> ur[TG];
-                    lds8(U + (TG * G + l) * LDT + TG * H, ur);
-#pragma unroll
-                    for (int j = 0; j < TG; j++) cfms(y[j], x[l], ur[j]);
-                }
-#pragma unroll
-                for (int j = 0; j < TG; j++)
-                    if (TG * H + j < kb) row[TG * H + j] = y[j];
-            }
-        }
-    }
-    __syncthreads();
-    for (int q = tid; q < nr * kb; q += blockDim.x) {
-        const int r = q / kb, j = q % kb;
-        xb[(long long)r * ld + j] = Xs[r * (KB + 1) + j];
+    for (int q = tid; q < KB * BD_V; q += BD_TH) {
+        const int i = row ? q / BD_V : q % KB, w = row ? q % BD_V : q / KB;
+        if (i < kb && w < nv) xb[i * si + w * sv] = X[i * LDX + w];
     }
 }
 

@@ -55,7 +55,8 @@ inline long long inv_entries(int p)
 template <class T>
 __global__ void __launch_bounds__(2 * KB) k_tile_inverse(const PanelTask *__restrict__ tasks,
                                                          const FrontDev *__restrict__ fr,
-                                                         const cx<T> *__restrict__ fac, cx<T> *__restrict__ inv)
+                                                         const cx<T> *__restrict__ fac, const int *__restrict__ gord,
+                                                         int *__restrict__ ipiv, cx<T> *__restrict__ inv)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T> *S = reinterpret_cast<cx<T> *>(smraw);   // KB x (KB+1), then 2 KB scratch columns
@@ -70,7 +71,18 @@ __global__ void __launch_bounds__(2 * KB) k_tile_inverse(const PanelTask *__rest
         const int i = idx / kb, j = idx % kb;
         S[i * LD + j] = D[(long long)i * nf + j];
     }
+    // the tile's row order as a sequence of interchanges (checks read it): at
+    // step j the row that ends at position j is at position s[j]
+    __shared__ int at[KB], where[KB];
+    if (tid < KB) at[tid] = where[tid] = tid;
     __syncthreads();
+    if (tid == 0)
+        for (int j = 0; j < kb; j++) {
+            const int r = gord[F.first + k + j] - F.first - k, q = where[r], o = at[j];
+            ipiv[F.first + k + j] = k + q;
+            at[q] = o;
+            where[o] = q;
+        }
     const int c0 = k / SB * SB, w = min(SB, F.p - c0), ldw = inv_ld(w), o = k - c0;
     cx<T> *W = inv + F.inv + (long long)(c0 / SB) * (SB * SB) + (long long)o * ldw + o;
     const bool up = tid >= KB;
@@ -258,31 +270,6 @@ __device__ __forceinline__ void cp_async_16_z(void *dst, const void *src, bool o
 {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
-}
-
-// 16-byte-aligned shared loads of N consecutive complex values
-template <int N>
-__device__ __forceinline__ void lds_cx(const cx<float> *p, cx<float> (&a)[N])
-{
-    if constexpr (N == 1) {
-        a[0] = *p;
-    } else {
-#pragma unroll
-        for (int j = 0; j < N; j += 2) {
-            const float4 u = reinterpret_cast<const float4 *>(p)[j / 2];
-            a[j] = cx<float>(u.x, u.y);
-            a[j + 1] = cx<float>(u.z, u.w);
-        }
-    }
-}
-template <int N>
-__device__ __forceinline__ void lds_cx(const cx<double> *p, cx<double> (&a)[N])
-{
-#pragma unroll
-    for (int j = 0; j < N; j++) {
-        const double2 u = reinterpret_cast<const double2 *>(p)[j];
-        a[j] = cx<double>(u.x, u.y);
-    }
 }
 
 __device__ __forceinline__ void red_add(cx<float> *p, const cx<float> v)
