@@ -41,6 +41,9 @@ struct Schedule {
     DevVec<PanelTask> panel;
     DevVec<BandTask> band;
     DevVec<GemmTask<T>> gemm;
+    DevVec<GemmUnit> unit;                                    // their tiles
+    std::vector<GemmTask<T>> hgemm;                           // host copies while the schedule is built
+    std::vector<GemmUnit> hunit;
     DevVec<EATask> ea;
     DevVec<InvTask> inv;                                      // block-inverse columns
     DevVec<SkUnit> sk;                                        // units of the substitution products
@@ -92,6 +95,8 @@ public:
     // products of at least this many factor entries go to the tall-skinny
     // tensor-core kernel
     static constexpr double TS_MIN_ENTRIES = 4e6;
+    // flops from which a factorisation's update goes to the tensor-core kernel
+    static constexpr double TC_MIN_FLOPS = 1e9;
     // units a launch of k_skinny is cut into, and the shortest K of a unit
     static constexpr int SK_SLOTS = 152 * 4, SK_KMIN = 64;
     // outer block width of the two-level LU (WT3D_WB: a multiple of KB, 512 by default)
@@ -199,8 +204,8 @@ public:
         int dev = 0;
         cudaGetDevice(&dev);
         std::call_once(attr_once[dev & 63], [] {
-            size_t sp = sizeof(cx<T>) * (KB * (KB + 1) + 2 * KB * (KB + 1));
-            cudaFuncSetAttribute(k_tile_inverse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp);
+            cudaFuncSetAttribute(k_tile_inverse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)BandCfg<T>::smem);
             cudaFuncSetAttribute(k_bands<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BandCfg<T>::smem);
             sk_attr<1>();
             sk_attr<4>();
@@ -259,18 +264,13 @@ public:
     }
 
     // ---------------------------------------------------------------------
-    static void add_gemm(std::vector<GemmTask<T>> &v, long long &tiles, const cx<T> *A, int lda, const cx<T> *B,
-                         int ldb, cx<T> *C, int ldc, int M, int N, int K, const int *brow = nullptr,
-                         const int *crow = nullptr, int conjA = 0)
+    static void add_gemm(std::vector<GemmTask<T>> &v, const cx<T> *A, int lda, const cx<T> *B, int ldb, cx<T> *C,
+                         int ldc, int M, int N, int K)
     {
         if (M <= 0 || N <= 0 || K <= 0) return;
         GemmTask<T> g{};
-        g.A = A; g.B = B; g.C = C; g.brow = brow; g.crow = crow;
+        g.A = A; g.B = B; g.C = C;
         g.lda = lda; g.ldb = ldb; g.ldc = ldc; g.M = M; g.N = N; g.K = K;
-        g.tiles_n = (N + GBN - 1) / GBN;
-        g.tile0 = tiles;
-        g.conjA = conjA;
-        tiles += (long long)((M + GBM - 1) / GBM) * g.tiles_n;
         v.push_back(g);
     }
 
@@ -279,90 +279,53 @@ public:
         return ((double)g.M * g.K + (double)g.K * g.N + 2.0 * g.M * g.N) * sizeof(cx<T>);
     }
 
-    // Appends the launches for GEMM tasks [b, end) of `all`: tasks the
-    // tensor-core kernel takes (complex64 path) go to a tcgen05 launch, the
-    // rest to the SIMT kernel with tile numbering rebased to the launch.
-    void push_gemm_launch(Schedule<T> &sc, std::vector<GemmTask<T>> &all, size_t b, long long /*tiles*/)
+    // Appends the launches of the GEMM tasks v (and empties it): tasks the
+    // tensor-core kernel takes (complex64) go to a tcgen05 launch, the rest to the
+    // SIMT kernel.  A tensor-core launch comes with two operand-split launches
+    // before it, 45 us for the three at the least; below TC_MIN_FLOPS the SIMT
+    // kernel is done sooner.
+    void push_gemm_launch(Schedule<T> &sc, std::vector<GemmTask<T>> &v)
     {
-        if (all.size() == b) return;
         std::vector<GemmTask<T>> simt;
+        Schedule<T> *psc = &sc;
         if constexpr (std::is_same<T, float>::value) {
             std::vector<GemmTask<float>> tcv;
-            for (size_t i = b; i < all.size(); i++) {
-                if (use_tc && tc_eligible(all[i])) tcv.push_back(all[i]);
-                else simt.push_back(all[i]);
+            double fl = 0, by = 0;
+            for (const auto &g : v) {
+                if (use_tc && tc_eligible(g)) {
+                    tcv.push_back(g);
+                    fl += 8.0 * g.M * (double)g.N * g.K;
+                    by += gemm_bytes(g);
+                } else {
+                    simt.push_back(g);
+                }
             }
-            if (!tcv.empty()) {
-                double fl = 0, by = 0;
-                for (auto &g : tcv) { fl += 8.0 * g.M * (double)g.N * g.K; by += gemm_bytes(g); }
+            if (fl < TC_MIN_FLOPS) {
+                simt = v;
+            } else {
                 const int idx = (int)sc.tc_pending.size();
                 sc.tc_pending.push_back(std::move(tcv));
-                Schedule<T> *psc = &sc;
                 sc.launches.push_back({[psc, idx](cudaStream_t st) { tc_split(*psc->tc[idx], st); }, LK_SPLIT, 0});
                 sc.launches.push_back({[psc, idx, this](cudaStream_t st) { tc_mma(*psc->tc[idx], tc_err.p, st); },
                                        LK_TCGEMM, fl, by});
             }
         } else {
-            simt.assign(all.begin() + b, all.end());
+            simt = v;
         }
-        all.resize(b);
+        v.clear();
         if (simt.empty()) return;
-        // tasks with at most 32 columns go to the tall-skinny kernel
-        std::vector<GemmTask<T>> narrow, wide;
-        for (auto &g : simt) (g.N <= TSBN ? narrow : wide).push_back(g);
-        Schedule<T> *psc = &sc;
-        if (!narrow.empty()) {
-            // split-K: tasks whose K exceeds a chunk sized for ~8 CTAs per SM
-            // over the whole launch are cut into K-chunks that subtract their
-            // partial products atomically
-            double work = 0;
-            for (auto &g : narrow) work += (double)((g.M + TSBM - 1) / TSBM) * g.K;
-            const int kchunk = std::max(256, (int)((work / (8.0 * 152) + TSBK - 1) / TSBK) * TSBK);
-            std::vector<GemmTask<T>> split;
-            for (auto &g : narrow) {
-                if (g.K <= kchunk + kchunk / 2) { split.push_back(g); continue; }
-                for (int k0 = 0; k0 < g.K; k0 += kchunk) {
-                    GemmTask<T> c = g;
-                    c.K = std::min(kchunk, g.K - k0);
-                    c.A = g.conjA ? g.A + (long long)k0 * g.lda : g.A + k0;
-                    if (g.brow) c.brow = g.brow + k0;
-                    else c.B = g.B + (long long)k0 * g.ldb;
-                    c.atom = 1;
-                    split.push_back(c);
-                }
-            }
-            narrow.swap(split);
-            const size_t b0 = all.size();
-            long long tiles = 0;
-            double fl = 0, by = 0;
-            for (auto &g : narrow) {
-                g.tile0 = tiles;
-                tiles += (g.M + TSBM - 1) / TSBM;
-                fl += 8.0 * g.M * (double)g.N * g.K;
-                by += gemm_bytes(g);
-                all.push_back(g);
-            }
-            const int nt = (int)narrow.size();
-            sc.launches.push_back({[psc, b0, nt, tiles](cudaStream_t st) {
-                k_gemm_ts<T><<<(unsigned)tiles, 256, 0, st>>>(psc->gemm.p + b0, nt);
-            }, LK_GEMM, fl, by});
+        double fl = 0, by = 0;
+        for (const auto &g : simt) {
+            fl += 8.0 * g.M * (double)g.N * g.K;
+            by += gemm_bytes(g);
         }
-        if (!wide.empty()) {
-            const size_t b0 = all.size();
-            long long tiles = 0;
-            double fl = 0, by = 0;
-            for (auto &g : wide) {
-                g.tile0 = tiles;
-                tiles += (long long)((g.M + GBM - 1) / GBM) * g.tiles_n;
-                fl += 8.0 * g.M * (double)g.N * g.K;
-                by += gemm_bytes(g);
-                all.push_back(g);
-            }
-            const int nt = (int)wide.size();
-            sc.launches.push_back({[psc, b0, nt, tiles](cudaStream_t st) {
-                k_gemm<T><<<(unsigned)tiles, 256, 0, st>>>(psc->gemm.p + b0, nt);
-            }, LK_GEMM, fl, by});
-        }
+        const size_t u0 = sc.hunit.size();
+        gemm_units(simt, (int)sc.hgemm.size(), sc.hunit);
+        sc.hgemm.insert(sc.hgemm.end(), simt.begin(), simt.end());
+        const unsigned nu = (unsigned)(sc.hunit.size() - u0);
+        sc.launches.push_back({[psc, u0, nu](cudaStream_t st) {
+            k_gemm<T><<<nu, GemmCfg<T>::TH, 0, st>>>(psc->gemm.p, psc->unit.p + u0);
+        }, LK_GEMM, fl, by});
     }
 
     // Allocates a solve schedule's own B~ workspace (sized for its largest
@@ -435,10 +398,9 @@ public:
     {
         Schedule<T> *psc = &sc;
         const int np = (int)(hp.size() - p0);
-        const size_t smi = sizeof(cx<T>) * (KB * (KB + 1) + 2 * KB * (KB + 1));
         if (np) {
-            sc.launches.push_back({[psc, this, p0, np, smi](cudaStream_t st) {
-                k_tile_inverse<T><<<np, 2 * KB, smi, st>>>(psc->panel.p + p0, fr.p, fac.p, gord.p, ipiv.p, binv.p);
+            sc.launches.push_back({[psc, this, p0, np](cudaStream_t st) {
+                k_tile_inverse<T><<<4 * np, BD_TH, BandCfg<T>::smem, st>>>(psc->panel.p + p0, fr.p, fac.p, gord.p, ipiv.p, binv.p);
             }, LK_PANEL, 0});
             sc.launches.back().side = true;
         }
@@ -533,18 +495,24 @@ public:
             }
             // Two-level blocked partial LU, level-synchronous over fronts.
             // Inner KB-wide panels: panel LU, row band (all columns right of
-            // the panel), column band (all rows below), and rank-KB updates
-            // confined to the rows or the columns of the current WB-wide outer
-            // block.  Once an outer block is done, the rows and columns below
-            // and right of it receive one rank-WB update, so most of the
-            // elimination runs as K = WB GEMMs on the tensor cores.
+            // the panel), column band (all rows below), and updates confined to
+            // the rows or the columns of the current WB-wide outer block, by
+            // recursive halving: after 1, 2, 4 .. panels the rows and columns of
+            // as many next panels receive one update of rank 64, 128, 256 ..
+            // (a rank-64 update of the whole rest after every panel moves the
+            // outer block's rows and columns 28 times instead of 12).  Once an
+            // outer block is done, the rows and columns below and right of it
+            // receive one rank-WB update, so most of the elimination runs as
+            // K = WB GEMMs on the tensor cores.
             int maxp = 0;
             for (int f : fl) maxp = std::max(maxp, sym.fronts[f].p);
             for (int c0 = 0; c0 < maxp; c0 += WB) {
                 const size_t pblk = hp.size();   // first panel of this outer block
                 for (int k = c0; k < std::min(c0 + WB, maxp); k += KB) {
-                    size_t p0 = hp.size(), b0 = hb.size(), g0 = hg.size();
-                    long long tiles = 0;
+                    const size_t p0 = hp.size(), b0 = hb.size();
+                    // panels the next update covers: the largest power of two that
+                    // divides the number of panels done in this outer block
+                    const int done = (k - c0) / KB + 1, s = done & -done;
                     for (int f : fl) {
                         const Front &Fr = sym.fronts[f];
                         if (Fr.p <= k) continue;
@@ -554,16 +522,17 @@ public:
                         for (int c = k2; c < nf; c += BD_V) hb.push_back(BandTask{f, k, c, 0});
                         for (int r = k2; r < Fr.p; r += BD_V) hb.push_back(BandTask{f, k, r, 1});
                         for (int r = 0; r < Fr.b; r += BD_V) hb.push_back(BandTask{f, k, r, 2});
+                        if (k2 >= cend) continue;
                         cx<T> *Pb = F + Fr.fac_off;
                         cx<T> *Lo = Pb + (long long)Fr.p * nf;
-                        // rows inside the outer block, every column right of the panel
-                        add_gemm(hg, tiles, Pb + (long long)k2 * nf + k, nf, Pb + (long long)k * nf + k2, nf,
-                                 Pb + (long long)k2 * nf + k2, nf, cend - k2, nf - k2, kb);
-                        // rows below the outer block, columns inside it
-                        add_gemm(hg, tiles, Pb + (long long)cend * nf + k, nf, Pb + (long long)k * nf + k2, nf,
-                                 Pb + (long long)cend * nf + k2, nf, Fr.p - cend, cend - k2, kb);
-                        add_gemm(hg, tiles, Lo + k, Fr.p, Pb + (long long)k * nf + k2, nf, Lo + k2, Fr.p, Fr.b,
-                                 cend - k2, kb);
+                        const int ks = k2 - s * KB, t1 = std::min(k2 + s * KB, cend), w = k2 - ks;
+                        // the rows of the next s panels, every column right of them
+                        add_gemm(hg, Pb + (long long)k2 * nf + ks, nf, Pb + (long long)ks * nf + k2, nf,
+                                 Pb + (long long)k2 * nf + k2, nf, t1 - k2, nf - k2, w);
+                        // their columns, the rows below
+                        add_gemm(hg, Pb + (long long)t1 * nf + ks, nf, Pb + (long long)ks * nf + k2, nf,
+                                 Pb + (long long)t1 * nf + k2, nf, Fr.p - t1, t1 - k2, w);
+                        add_gemm(hg, Lo + ks, Fr.p, Pb + (long long)ks * nf + k2, nf, Lo + k2, Fr.p, Fr.b, t1 - k2, w);
                     }
                     const int np = (int)(hp.size() - p0), nbd = (int)(hb.size() - b0);
                     sc->launches.push_back({[psc, this, p0, np](cudaStream_t st) {
@@ -573,44 +542,42 @@ public:
                         sc->launches.push_back({[psc, this, b0, nbd](cudaStream_t st) {
                             k_bands<T><<<nbd, BD_TH, BandCfg<T>::smem, st>>>(psc->band.p + b0, fr.p, fac.p, gord.p);
                         }, LK_TRSM, 0});
-                    push_gemm_launch(*sc, hg, g0, tiles);
+                    push_gemm_launch(*sc, hg);
                 }
                 push_inverses(*sc, fl, hp, pblk, hi, c0, std::min(c0 + WB, maxp));
                 // rank-WB update of everything below and right of the outer block
-                size_t g0 = hg.size();
-                long long tiles = 0;
                 for (int f : fl) {
                     const Front &Fr = sym.fronts[f];
                     if (Fr.p <= c0) continue;
                     const int nf = Fr.nf(), cend = std::min(c0 + WB, Fr.p), w = cend - c0;
                     cx<T> *Pb = F + Fr.fac_off;
                     cx<T> *Lo = Pb + (long long)Fr.p * nf;
-                    add_gemm(hg, tiles, Pb + (long long)cend * nf + c0, nf, Pb + (long long)c0 * nf + cend, nf,
+                    add_gemm(hg, Pb + (long long)cend * nf + c0, nf, Pb + (long long)c0 * nf + cend, nf,
                              Pb + (long long)cend * nf + cend, nf, Fr.p - cend, nf - cend, w);
-                    add_gemm(hg, tiles, Lo + c0, Fr.p, Pb + (long long)c0 * nf + cend, nf, Lo + cend, Fr.p, Fr.b,
+                    add_gemm(hg, Lo + c0, Fr.p, Pb + (long long)c0 * nf + cend, nf, Lo + cend, Fr.p, Fr.b,
                              Fr.p - cend, w);
                 }
-                push_gemm_launch(*sc, hg, g0, tiles);
+                push_gemm_launch(*sc, hg);
             }
             // Schur complement F22 -= L21 U12 (K = p)
             {
-                size_t g0 = hg.size();
-                long long tiles = 0;
                 for (int f : fl) {
                     const Front &Fr = sym.fronts[f];
                     if (Fr.b == 0) continue;
                     const int nf = Fr.nf();
                     cx<T> *Pb = F + Fr.fac_off;
                     cx<T> *Lo = Pb + (long long)Fr.p * nf;
-                    add_gemm(hg, tiles, Lo, Fr.p, Pb + Fr.p, nf, U[L & 1] + Fr.upd_off, Fr.b, Fr.b, Fr.b, Fr.p);
+                    add_gemm(hg, Lo, Fr.p, Pb + Fr.p, nf, U[L & 1] + Fr.upd_off, Fr.b, Fr.b, Fr.b, Fr.p);
                 }
-                push_gemm_launch(*sc, hg, g0, tiles);
+                push_gemm_launch(*sc, hg);
             }
         }
         int rc;
         if ((rc = sc->panel.upload(hp))) return rc;
         if ((rc = sc->band.upload(hb))) return rc;
-        if ((rc = sc->gemm.upload(hg))) return rc;
+        if ((rc = sc->gemm.upload(sc->hgemm)) || (rc = sc->unit.upload(sc->hunit))) return rc;
+        sc->hgemm.clear();
+        sc->hunit.clear();
         if ((rc = sc->ea.upload(he))) return rc;
         if ((rc = sc->inv.upload(hi))) return rc;
         if ((rc = finish_tc(*sc))) return rc;

@@ -11,6 +11,8 @@
 // block by block.
 #pragma once
 #include "common.cuh"
+#include <algorithm>
+#include <vector>
 
 namespace wt3d {
 
@@ -35,10 +37,7 @@ struct GemmTask {
     const int *brow;   // optional row gather for B
     const int *crow;   // optional row scatter for C (atomic)
     int lda, ldb, ldc, M, N, K;
-    int tiles_n;
-    long long tile0;
     int conjA;         // use conj(A^T): A is read as its conjugate transpose
-    int atom;          // C -= A B with atomics (a K-chunk of a split task)
 };
 
 template <class T>
@@ -46,18 +45,6 @@ __device__ __forceinline__ void atomic_sub(cx<T> *p, cx<T> v)
 {
     atomicAdd(&p->re, -v.re);
     atomicAdd(&p->im, -v.im);
-}
-
-template <class Task>
-__device__ __forceinline__ int find_task(const Task *tasks, int ntasks, long long key)
-{
-    int lo = 0, hi = ntasks - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (tasks[mid].tile0 <= key) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
 }
 
 // ---------------------------------------------------------------------------
@@ -362,12 +349,55 @@ struct BandCfg {
     static constexpr size_t smem = sizeof(cx<T>) * (KB * LDT + KB * LDX);
 };
 
+// T x = b for the BD_V vectors of X (b on entry, zero before group first / TG);
+// unit: T's diagonal is one, otherwise invd holds its inverse.
+template <class T>
+__device__ __forceinline__ void band_solve(const cx<T> *Tm, cx<T> *X, const cx<T> *invd, bool unit, int first, int kb)
+{
+    constexpr int TG = BandCfg<T>::TG, LDT = BandCfg<T>::LDT, LDX = BandCfg<T>::LDX;
+    const int v = threadIdx.x >> 2, q4 = threadIdx.x & 3;
+    const int ng = (kb + TG - 1) / TG;
+    cx<T> *x = X + v;
+#pragma unroll 1
+    for (int G = first / TG; G < ng; G++) {
+        cx<T> b[TG];
+#pragma unroll
+        for (int i = 0; i < TG; i++) b[i] = x[(TG * G + i) * LDX];
+#pragma unroll
+        for (int i = 0; i < TG; i++) {
+            if (i > 0) {
+                cx<T> lr[TG];
+                lds_cx<TG>(Tm + (TG * G + i) * LDT + TG * G, lr);
+#pragma unroll
+                for (int l = 0; l < i; l++) cfms(b[i], lr[l], b[l]);
+            }
+            if (!unit) b[i] = b[i] * invd[TG * G + i];
+        }
+        __syncwarp();   // the four threads have read the group
+#pragma unroll
+        for (int i = 0; i < TG; i++)
+            if ((i & 3) == q4) x[(TG * G + i) * LDX] = b[i];
+#pragma unroll 1
+        for (int H = TG * (G + 1) + q4; H < TG * ng; H += TG) {
+#pragma unroll
+            for (int i = 0; i < TG; i += 4) {
+                cx<T> lr[TG], c = x[(H + i) * LDX];
+                lds_cx<TG>(Tm + (H + i) * LDT + TG * G, lr);
+#pragma unroll
+                for (int l = 0; l < TG; l++) cfms(c, lr[l], b[l]);
+                x[(H + i) * LDX] = c;
+            }
+        }
+        __syncwarp();
+    }
+}
+
 template <class T>
 __global__ void __launch_bounds__(BD_TH) k_bands(const BandTask *__restrict__ tasks, const FrontDev *__restrict__ fr,
                                                  cx<T> *__restrict__ fac, const int *__restrict__ gord)
 {
     using C = BandCfg<T>;
-    constexpr int TG = C::TG, LDT = C::LDT, LDX = C::LDX;
+    constexpr int LDT = C::LDT, LDX = C::LDX;
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T> *Tm = reinterpret_cast<cx<T> *>(smraw);   // KB x LDT
     cx<T> *X = Tm + KB * LDT;                       // KB x LDX: unknown i of vector v
@@ -421,41 +451,7 @@ __global__ void __launch_bounds__(BD_TH) k_bands(const BandTask *__restrict__ ta
     __syncthreads();
     if (tid < KB) invd[tid] = row ? cx<T>(1) : cdiv(cx<T>(1), Tm[tid * LDT + tid]);
     __syncthreads();
-    const int v = tid >> 2, q4 = tid & 3;
-    const int ng = (kb + TG - 1) / TG;
-    cx<T> *x = X + v;
-#pragma unroll 1
-    for (int G = 0; G < ng; G++) {
-        cx<T> b[TG];
-#pragma unroll
-        for (int i = 0; i < TG; i++) b[i] = x[(TG * G + i) * LDX];
-#pragma unroll
-        for (int i = 0; i < TG; i++) {
-            if (i > 0) {
-                cx<T> lr[TG];
-                lds_cx<TG>(Tm + (TG * G + i) * LDT + TG * G, lr);
-#pragma unroll
-                for (int l = 0; l < i; l++) cfms(b[i], lr[l], b[l]);
-            }
-            if (!row) b[i] = b[i] * invd[TG * G + i];
-        }
-        __syncwarp();   // the four threads have read the group
-#pragma unroll
-        for (int i = 0; i < TG; i++)
-            if ((i & 3) == q4) x[(TG * G + i) * LDX] = b[i];
-#pragma unroll 1
-        for (int H = TG * (G + 1) + q4; H < TG * ng; H += TG) {
-#pragma unroll
-            for (int i = 0; i < TG; i += 4) {
-                cx<T> lr[TG], c = x[(H + i) * LDX];
-                lds_cx<TG>(Tm + (H + i) * LDT + TG * G, lr);
-#pragma unroll
-                for (int l = 0; l < TG; l++) cfms(c, lr[l], b[l]);
-                x[(H + i) * LDX] = c;
-            }
-        }
-        __syncwarp();
-    }
+    band_solve<T>(Tm, X, invd, row, 0, kb);
     __syncthreads();
     for (int q = tid; q < KB * BD_V; q += BD_TH) {
         const int i = row ? q / BD_V : q % KB, w = row ? q % BD_V : q / KB;
@@ -464,197 +460,127 @@ __global__ void __launch_bounds__(BD_TH) k_bands(const BandTask *__restrict__ ta
 }
 
 // ---------------------------------------------------------------------------
-// SIMT complex GEMM  C -= op(A) * B  (64x64 tiles, 4x4 per thread)
+// SIMT complex GEMM  C -= A B: the products that are too small for the
+// tensor-core kernel and its operand split, and all complex128 ones
 // ---------------------------------------------------------------------------
-constexpr int GBM = 64, GBN = 64, GBK = 16;
+// One CTA per unit: a BM x 32 tile of C (4 x 4 per thread) and a range of K.
+// Operands go through a ring of three asynchronous-copy stages; the tile of C,
+// which does not depend on the product, is loaded first.  Complex64 tiles are 64
+// rows high (73 TF/s FP32 peak; the unpipelined 64 x 64 kernel reached 4 - 11).
+// Complex128 tiles are 32 rows high: the FP64 pipe (2 FMA per cycle and SM) is
+// the bound, and smaller tiles fill the last wave (a 630 x 630 x 600 update is
+// 100 tiles of 64 x 64 on 152 SMs, but 400 of 32 x 32).
+struct GemmUnit { int task, m0, n0, k0, k1, atom; };
 template <class T>
-__global__ void __launch_bounds__(256) k_gemm(const GemmTask<T> *__restrict__ tasks, int ntasks)
+struct GemmCfg {
+    static constexpr int BM = sizeof(T) == 4 ? 64 : 32, BN = 32;
+    static constexpr int BK = sizeof(T) == 4 ? 16 : 8, NS = 3;
+    static constexpr int TH = (BM / 4) * (BN / 4), VK = 16 / (int)sizeof(cx<T>), LDA = BK + VK;
+};
+
+template <class T>
+__device__ __forceinline__ void cp_async_cx_z(cx<T> *dst, const cx<T> *src, bool ok)   // zeros when !ok
 {
-    __shared__ cx<T> As[GBK][GBM + 1];
-    __shared__ cx<T> Bs[GBK][GBN];
-    const int ti = find_task(tasks, ntasks, (long long)blockIdx.x);
-    const GemmTask<T> t = tasks[ti];
-    const long long lt = (long long)blockIdx.x - t.tile0;
-    const int m0 = (int)(lt / t.tiles_n) * GBM, n0 = (int)(lt % t.tiles_n) * GBN;
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    cx<T> acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = cx<T>(0);
-    for (int k0 = 0; k0 < t.K; k0 += GBK) {
-        if (!t.conjA) {
-#pragma unroll
-            for (int q = 0; q < (GBM * GBK) / 256; q++) {
-                int idx = tid + q * 256;
-                int i = idx / GBK, kk = idx % GBK;
-                int r = m0 + i, c = k0 + kk;
-                As[kk][i] = (r < t.M && c < t.K) ? t.A[(long long)r * t.lda + c] : cx<T>(0);
-            }
-        } else {
-            // op(A)[r][c] = conj(A[c][r])
-#pragma unroll
-            for (int q = 0; q < (GBM * GBK) / 256; q++) {
-                int idx = tid + q * 256;
-                int kk = idx / GBM, i = idx % GBM;
-                int r = m0 + i, c = k0 + kk;
-                As[kk][i] = (r < t.M && c < t.K) ? conj(t.A[(long long)c * t.lda + r]) : cx<T>(0);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < (GBK * GBN) / 256; q++) {
-            int idx = tid + q * 256;
-            int kk = idx / GBN, j = idx % GBN;
-            int r = k0 + kk, c = n0 + j;
-            cx<T> v(0);
-            if (r < t.K && c < t.N) {
-                long long row = t.brow ? (long long)t.brow[r] : (long long)r;
-                v = t.B[row * t.ldb + c];
-            }
-            Bs[kk][j] = v;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < GBK; kk++) {
-            cx<T> a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    acc[i][j].re = fma(a[i].re, b[j].re, fma(-a[i].im, b[j].im, acc[i][j].re));
-                    acc[i][j].im = fma(a[i].re, b[j].im, fma(a[i].im, b[j].re, acc[i][j].im));
-                }
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        int r = m0 + ty + 16 * i;
-        if (r >= t.M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            int c = n0 + tx + 16 * j;
-            if (c >= t.N) continue;
-            if (t.crow) {
-                atomic_sub(t.C + (long long)t.crow[r] * t.ldc + c, acc[i][j]);
-            } else {
-                cx<T> *p = t.C + (long long)r * t.ldc + c;
-                *p = *p - acc[i][j];
-            }
-        }
-    }
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if constexpr (sizeof(cx<T>) == 8)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
 
-// ---------------------------------------------------------------------------
-// Tall-skinny SIMT complex GEMM  C -= op(A) * B  for N <= 32 (the right-hand
-// side blocks of the substitution passes): 128 x 32 tiles, 4 x 4 complex
-// outputs per thread, every A element read once per tile.
-// ---------------------------------------------------------------------------
-constexpr int TSBM = 128, TSBN = 32, TSBK = 16;   // TSBK: K granularity of split-K chunks
-template <class T> struct TsCfg { static constexpr int BK = sizeof(T) == 4 ? 32 : 16; };
-
-// 128 x 32 tile per CTA of 256 threads; thread (tx, ty) owns rows 4ty..4ty+3
-// and columns 4tx..4tx+3 (16 complex accumulators).  The K loop stages
-// BK-deep slices of A (transposed in shared memory) and B, prefetching the
-// next slice into registers while the current one is consumed.
 template <class T>
-__global__ void __launch_bounds__(256, 2) k_gemm_ts(const GemmTask<T> *__restrict__ tasks, int ntasks)
+__global__ void __launch_bounds__(GemmCfg<T>::TH) k_gemm(const GemmTask<T> *__restrict__ tasks,
+                                                         const GemmUnit *__restrict__ units)
 {
-    constexpr int BK = TsCfg<T>::BK;
-    constexpr int AP = TSBM + 1;                       // padded row of the A^T slice
-    constexpr int NA = TSBM * BK / 256, NB = BK * TSBN / 256;
-    __shared__ cx<T> As[BK][AP];
-    __shared__ cx<T> Bs[BK][TSBN];
-    const int ti = find_task(tasks, ntasks, (long long)blockIdx.x);
-    const GemmTask<T> t = tasks[ti];
-    const int m0 = (int)((long long)blockIdx.x - t.tile0) * TSBM;
-    const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
-    cx<T> acc[4][4];
+    using C = GemmCfg<T>;
+    constexpr int BM = C::BM, BN = C::BN, BK = C::BK, NS = C::NS, TH = C::TH, VK = C::VK, LDA = C::LDA;
+    __shared__ __align__(16) cx<T> As[NS][BM * LDA];
+    __shared__ __align__(16) cx<T> Bs[NS][BK * BN];
+    const GemmUnit u = units[blockIdx.x];
+    const GemmTask<T> t = tasks[u.task];
+    const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;   // rows ty + (BM / 4) i, columns 4 tx + j
+    const int M = t.M - u.m0, N = t.N - u.n0, K = u.k1 - u.k0, nst = (K + BK - 1) / BK;
+    const cx<T> *A = t.A + (long long)u.m0 * t.lda + u.k0, *B = t.B + (long long)u.k0 * t.ldb + u.n0;
+    auto load = [&](int s) {
+        cx<T> *da = As[s % NS], *db = Bs[s % NS];
+#pragma unroll
+        for (int q = 0; q < BM * BK / TH; q++) {
+            const int idx = tid + q * TH, i = idx / BK, kk = idx % BK, k = s * BK + kk;
+            const bool ok = i < M && k < K;
+            cp_async_cx_z(da + i * LDA + kk, A + (ok ? (long long)i * t.lda + k : 0), ok);
+        }
+#pragma unroll
+        for (int q = 0; q < BK * BN / TH; q++) {
+            const int idx = tid + q * TH, kk = idx / BN, j = idx % BN, k = s * BK + kk;
+            const bool ok = j < N && k < K;
+            cp_async_cx_z(db + idx, B + (ok ? (long long)k * t.ldb + j : 0), ok);
+        }
+    };
+    for (int s = 0; s < NS - 1; s++) {
+        if (s < nst) load(s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    cx<T> *Cp = t.C + (long long)u.m0 * t.ldc + u.n0;
+    cx<T> acc[4][4];   // C minus the products so far
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = cx<T>(0);
-    cx<T> pa[NA], pb[NB];
-    // A slice element q of this thread: non-conjugate A is read along K
-    // (row-contiguous), the conjugate transpose along M.
-    auto load = [&](int k0) {
-#pragma unroll
-        for (int q = 0; q < NA; q++) {
-            const int idx = tid + q * 256;
-            int i, kk;
-            if (!t.conjA) { i = idx / BK; kk = idx % BK; }
-            else { kk = idx / TSBM; i = idx % TSBM; }
-            const int r = m0 + i, c = k0 + kk;
-            cx<T> v(0);
-            if (r < t.M && c < t.K) v = t.conjA ? conj(t.A[(long long)c * t.lda + r]) : t.A[(long long)r * t.lda + c];
-            pa[q] = v;
-        }
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-            const int idx = tid + q * 256;
-            const int kk = idx / TSBN, j = idx % TSBN;
-            const int r = k0 + kk;
-            cx<T> v(0);
-            if (r < t.K && j < t.N) v = t.B[(t.brow ? (long long)t.brow[r] : (long long)r) * t.ldb + j];
-            pb[q] = v;
-        }
-    };
-    auto store = [&]() {
-#pragma unroll
-        for (int q = 0; q < NA; q++) {
-            const int idx = tid + q * 256;
-            int i, kk;
-            if (!t.conjA) { i = idx / BK; kk = idx % BK; }
-            else { kk = idx / TSBM; i = idx % TSBM; }
-            As[kk][i] = pa[q];
-        }
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-            const int idx = tid + q * 256;
-            Bs[idx / TSBN][idx % TSBN] = pb[q];
-        }
-    };
-    load(0);
-    for (int k0 = 0; k0 < t.K; k0 += BK) {
-        store();
-        __syncthreads();
-        if (k0 + BK < t.K) load(k0 + BK);
-#pragma unroll
-        for (int kk = 0; kk < BK; kk++) {
-            cx<T> a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][4 * ty + i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[kk][4 * tx + j];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    acc[i][j].re = fma(a[i].re, b[j].re, fma(-a[i].im, b[j].im, acc[i][j].re));
-                    acc[i][j].im = fma(a[i].re, b[j].im, fma(a[i].im, b[j].re, acc[i][j].im));
-                }
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int r = m0 + 4 * ty + i;
-        if (r >= t.M) continue;
-#pragma unroll
         for (int j = 0; j < 4; j++) {
-            const int c = 4 * tx + j;
-            if (c >= t.N) continue;
-            if (t.crow) atomic_sub(t.C + (long long)t.crow[r] * t.ldc + c, acc[i][j]);
-            else if (t.atom) atomic_sub(t.C + (long long)r * t.ldc + c, acc[i][j]);
-            else {
-                cx<T> *p = t.C + (long long)r * t.ldc + c;
-                *p = *p - acc[i][j];
+            const int r = ty + BM / 4 * i, c = 4 * tx + j;
+            acc[i][j] = (!u.atom && r < M && c < N) ? Cp[(long long)r * t.ldc + c] : cx<T>(0);
+        }
+    for (int s = 0; s < nst; s++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(NS - 2) : "memory");
+        __syncthreads();   // stage s is there for all; stage s - 1 is no longer read
+        if (s + NS - 1 < nst) load(s + NS - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const cx<T> *Aw = As[s % NS], *Bw = Bs[s % NS];
+#pragma unroll
+        for (int kq = 0; kq < BK; kq += VK) {
+            cx<T> a[4][VK];
+#pragma unroll
+            for (int i = 0; i < 4; i++) lds_cx<VK>(Aw + (ty + BM / 4 * i) * LDA + kq, a[i]);
+#pragma unroll
+            for (int v = 0; v < VK; v++) {
+                cx<T> b[4];
+                lds_cx<4>(Bw + (kq + v) * BN + 4 * tx, b);
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) cfms(acc[i][j], a[i][v], b[j]);
             }
         }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int r = ty + BM / 4 * i, c = 4 * tx + j;
+            if (r >= M || c >= N) continue;
+            cx<T> *p = Cp + (long long)r * t.ldc + c;
+            if (u.atom) atomic_sub(p, -acc[i][j]);
+            else *p = acc[i][j];
+        }
+}
+
+// The units of tasks v, numbered from `first` in the launch's task array.  A
+// launch with fewer tiles than half the SMs is also cut along K.
+template <class T>
+void gemm_units(const std::vector<GemmTask<T>> &v, int first, std::vector<GemmUnit> &out)
+{
+    using C = GemmCfg<T>;
+    long long tiles = 0;
+    for (const auto &g : v) tiles += (long long)((g.M + C::BM - 1) / C::BM) * ((g.N + C::BN - 1) / C::BN);
+    const int cut = tiles > 0 && tiles < 76 ? (int)(152 / tiles) : 1;
+    for (size_t i = 0; i < v.size(); i++) {
+        const auto &g = v[i];
+        const int n = std::max(1, std::min(cut, g.K / 64));
+        const int len = ((g.K + n - 1) / n + C::BK - 1) / C::BK * C::BK;
+        for (int m0 = 0; m0 < g.M; m0 += C::BM)
+            for (int n0 = 0; n0 < g.N; n0 += C::BN)
+                for (int k0 = 0; k0 < g.K; k0 += len)
+                    out.push_back(GemmUnit{first + (int)i, m0, n0, k0, std::min(g.K, k0 + len), len < g.K ? 1 : 0});
     }
 }
 

@@ -665,8 +665,8 @@ int tc_init()
 // tall-skinny tensor-core kernel of the solves (path = 3; path = 4 with a row
 // gather of B and a row scatter of C; path = 5 with C -= A^H B for A given as
 // the K x M block, lda >= M); paths 3 and 4 stream A by TMA when it is
-// 16-byte aligned with an even stride.  wt3d_bench_gemm also times path 2,
-// the tall-skinny SIMT kernel, path 3, and path 6 (path 3 with A always
+// 16-byte aligned with an even stride.  wt3d_bench_gemm also times path 2
+// (path 0 with N <= 32), path 3, and path 6 (path 3 with A always
 // copied by the loader warps).
 // ---------------------------------------------------------------------------
 using namespace wt3d;
@@ -690,12 +690,11 @@ extern "C" int wt3d_debug_gemm(int path, int M, int N, int K, const void *A, int
     WT_CUDA(cudaMemcpy(dC.p, C, sizeof(cx<float>) * M * ldc, cudaMemcpyHostToDevice));
     GemmTask<float> g{};
     g.A = dA.p; g.B = dB.p; g.C = dC.p; g.lda = lda; g.ldb = ldb; g.ldc = ldc; g.M = M; g.N = N; g.K = K;
-    g.tiles_n = (N + GBN - 1) / GBN;
-    g.tile0 = 0;
     DevVec<int> err;
     if ((rc = err.alloc(1))) return rc;
     WT_CUDA(cudaMemset(err.p, 0, sizeof(int)));
     DevVec<int> drow, dcol;
+    DevVec<GemmUnit> du;
     if (path == 1) {
         if ((rc = tc_init())) return rc;
         DevVec<float> ws;
@@ -728,8 +727,10 @@ extern "C" int wt3d_debug_gemm(int path, int M, int N, int K, const void *A, int
         DevVec<GemmTask<float>> dt;
         std::vector<GemmTask<float>> v{g};
         if ((rc = dt.upload(v))) return rc;
-        long long tiles = (long long)((M + GBM - 1) / GBM) * g.tiles_n;
-        k_gemm<float><<<(unsigned)tiles, 256>>>(dt.p, 1);
+        std::vector<GemmUnit> hu;
+        gemm_units(v, 0, hu);
+        if ((rc = du.upload(hu))) return rc;
+        k_gemm<float><<<(unsigned)hu.size(), GemmCfg<float>::TH>>>(dt.p, du.p);
     }
     WT_CUDA(cudaGetLastError());
     WT_CUDA(cudaDeviceSynchronize());
@@ -761,7 +762,6 @@ extern "C" int wt3d_bench_gemm(int path, int M, int N, int K, int iters, double 
     k_fill<<<ceil_div((long long)M * N, 256), 256>>>(dC.p, (long long)M * N, 3);
     GemmTask<float> g{};
     g.A = dA.p; g.B = dB.p; g.C = dC.p; g.lda = K; g.ldb = N; g.ldc = N; g.M = M; g.N = N; g.K = K;
-    g.tiles_n = (N + GBN - 1) / GBN;
     DevVec<int> err;
     if ((rc = err.alloc(1))) return rc;
     WT_CUDA(cudaMemset(err.p, 0, sizeof(int)));
@@ -769,6 +769,8 @@ extern "C" int wt3d_bench_gemm(int path, int M, int N, int K, int iters, double 
     TcLaunch L;
     TsLaunch LT;
     DevVec<GemmTask<float>> dt;
+    std::vector<GemmUnit> hu;
+    DevVec<GemmUnit> du;
     if (path == 1) {
         if ((rc = tc_init()) || (rc = ws.alloc(tc_workspace_floats(&g, 1))) || (rc = tc_build_launch(L, &g, 1, ws.p)))
             return rc;
@@ -782,19 +784,17 @@ extern "C" int wt3d_bench_gemm(int path, int M, int N, int K, int iters, double 
         ts_expand(LT, 0);
     } else {
         std::vector<GemmTask<float>> v{g};
-        if ((rc = dt.upload(v))) return rc;
+        gemm_units(v, 0, hu);
+        if ((rc = dt.upload(v)) || (rc = du.upload(hu))) return rc;
     }
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    const long long tiles = (long long)((M + GBM - 1) / GBM) * g.tiles_n;
-    const long long ts_tiles = (M + TSBM - 1) / TSBM;   // path 2: tall-skinny kernel (N <= 32)
-    if (path == 2 && N > TSBN) { set_error("wt3d_bench_gemm: path 2 needs N <= 32"); return WT3D_ERR_ARG; }
+    if (path == 2 && N > 32) { set_error("wt3d_bench_gemm: path 2 needs N <= 32"); return WT3D_ERR_ARG; }
     auto launch = [&]() {
         if (path == 1) tc_mma(L, err.p, 0);
         else if (path == 3 || path == 6) ts_mma(LT, err.p, 0);
-        else if (path == 2) k_gemm_ts<float><<<(unsigned)ts_tiles, 256>>>(dt.p, 1);
-        else k_gemm<float><<<(unsigned)tiles, 256>>>(dt.p, 1);
+        else k_gemm<float><<<(unsigned)hu.size(), GemmCfg<float>::TH>>>(dt.p, du.p);
     };
     for (int w = 0; w < 2; w++) launch();   // warm-up
     cudaEventRecord(e0);

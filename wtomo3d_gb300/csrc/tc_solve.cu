@@ -594,7 +594,7 @@ int ts_build_launch(TsLaunch &L, const GemmTask<float> *g, int n, float *ws, boo
         t.Kr = (int)ts_kr(t.K);
         t.kchunk = kchunk;
         t.nkc = (t.K + kchunk - 1) / kchunk;
-        t.atom = (t.crow || t.nkc > 1 || g[i].atom) ? 1 : 0;
+        t.atom = (t.crow || t.nkc > 1) ? 1 : 0;
         t.bhi = ws + off; off += (long long)TS_NR * t.Kr;
         t.blo = ws + off; off += (long long)TS_NR * t.Kr;
         t.unit0 = units;
