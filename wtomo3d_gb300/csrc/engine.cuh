@@ -95,6 +95,8 @@ public:
     // products of at least this many factor entries go to the tall-skinny
     // tensor-core kernel
     static constexpr double TS_MIN_ENTRIES = 4e6;
+    // vectors of a band launch from which four threads take two
+    static constexpr long long BAND_TWO = 152 * 4 * 32;
     // flops from which a factorisation's update goes to the tensor-core kernel
     static constexpr double TC_MIN_FLOPS = 1e9;
     // units a launch of k_skinny is cut into, and the shortest K of a unit
@@ -205,8 +207,12 @@ public:
         cudaGetDevice(&dev);
         std::call_once(attr_once[dev & 63], [] {
             cudaFuncSetAttribute(k_tile_inverse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)BandCfg<T>::smem);
-            cudaFuncSetAttribute(k_bands<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BandCfg<T>::smem);
+                                 (int)BandCfg<T, 1>::smem);
+            cudaFuncSetAttribute(k_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)panel_smem<T>());
+            cudaFuncSetAttribute(k_bands<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)BandCfg<T, 1>::smem);
+            cudaFuncSetAttribute(k_bands<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)BandCfg<T, 2>::smem);
             sk_attr<1>();
             sk_attr<4>();
             sk_attr<8>();
@@ -400,7 +406,7 @@ public:
         const int np = (int)(hp.size() - p0);
         if (np) {
             sc.launches.push_back({[psc, this, p0, np](cudaStream_t st) {
-                k_tile_inverse<T><<<4 * np, BD_TH, BandCfg<T>::smem, st>>>(psc->panel.p + p0, fr.p, fac.p, gord.p, ipiv.p, binv.p);
+                k_tile_inverse<T><<<4 * np, BD_TH, BandCfg<T, 1>::smem, st>>>(psc->panel.p + p0, fr.p, fac.p, gord.p, ipiv.p, binv.p);
             }, LK_PANEL, 0});
             sc.launches.back().side = true;
         }
@@ -513,15 +519,22 @@ public:
                     // panels the next update covers: the largest power of two that
                     // divides the number of panels done in this outer block
                     const int done = (k - c0) / KB + 1, s = done & -done;
+                    // band vectors of the step: two per four threads if they fill the chip
+                    long long nvec = 0;
+                    for (int f : fl)
+                        if (sym.fronts[f].p > k)
+                            nvec += 2LL * std::max(0, sym.fronts[f].p - k - KB) + 2LL * sym.fronts[f].b;
+                    const bool two = nvec >= BAND_TWO;
+                    const int bv = two ? BandCfg<T, 2>::V : BandCfg<T, 1>::V;
                     for (int f : fl) {
                         const Front &Fr = sym.fronts[f];
                         if (Fr.p <= k) continue;
                         const int nf = Fr.nf(), kb = std::min(KB, Fr.p - k), k2 = k + kb;
                         const int cend = std::min(c0 + WB, Fr.p);
                         hp.push_back(PanelTask{f, k});
-                        for (int c = k2; c < nf; c += BD_V) hb.push_back(BandTask{f, k, c, 0});
-                        for (int r = k2; r < Fr.p; r += BD_V) hb.push_back(BandTask{f, k, r, 1});
-                        for (int r = 0; r < Fr.b; r += BD_V) hb.push_back(BandTask{f, k, r, 2});
+                        for (int c = k2; c < nf; c += bv) hb.push_back(BandTask{f, k, c, 0});
+                        for (int r = k2; r < Fr.p; r += bv) hb.push_back(BandTask{f, k, r, 1});
+                        for (int r = 0; r < Fr.b; r += bv) hb.push_back(BandTask{f, k, r, 2});
                         if (k2 >= cend) continue;
                         cx<T> *Pb = F + Fr.fac_off;
                         cx<T> *Lo = Pb + (long long)Fr.p * nf;
@@ -536,11 +549,16 @@ public:
                     }
                     const int np = (int)(hp.size() - p0), nbd = (int)(hb.size() - b0);
                     sc->launches.push_back({[psc, this, p0, np](cudaStream_t st) {
-                        k_panel<T><<<np, 256, 0, st>>>(psc->panel.p + p0, fr.p, fac.p, maxabs.p, pivot_rel, npert.p, gord.p);
+                        k_panel<T><<<np, 256, panel_smem<T>(), st>>>(psc->panel.p + p0, fr.p, fac.p, maxabs.p, pivot_rel, npert.p, gord.p);
                     }, LK_PANEL, 0});
                     if (nbd)
-                        sc->launches.push_back({[psc, this, b0, nbd](cudaStream_t st) {
-                            k_bands<T><<<nbd, BD_TH, BandCfg<T>::smem, st>>>(psc->band.p + b0, fr.p, fac.p, gord.p);
+                        sc->launches.push_back({[psc, this, b0, nbd, two](cudaStream_t st) {
+                            if (two)
+                                k_bands<T, 2><<<nbd, BD_TH, BandCfg<T, 2>::smem, st>>>(psc->band.p + b0, fr.p, fac.p,
+                                                                                       gord.p);
+                            else
+                                k_bands<T, 1><<<nbd, BD_TH, BandCfg<T, 1>::smem, st>>>(psc->band.p + b0, fr.p, fac.p,
+                                                                                       gord.p);
                         }, LK_TRSM, 0});
                     push_gemm_launch(*sc, hg);
                 }

@@ -145,138 +145,6 @@ __device__ __forceinline__ unsigned long long warp_max(unsigned long long k)
     return ((unsigned long long)hi << 32) | lo;
 }
 
-// element i (a run-time index) of four registers
-template <class T>
-__device__ __forceinline__ cx<T> pick(const cx<T> &a0, const cx<T> &a1, const cx<T> &a2, const cx<T> &a3, int i)
-{
-    const cx<T> lo = (i & 1) ? a1 : a0, hi = (i & 1) ? a3 : a2;
-    return (i & 2) ? hi : lo;
-}
-
-// One CTA per tile; a chain of 64 dependent columns, so the latency of a column
-// is what counts.  The tile is held in registers: thread (tx, ty) =
-// (tid / 16, tid % 16) owns rows ty + 16 i and columns tx + 16 c, so that a
-// column's 64 entries sit in one half-warp and its pivot is found by two warp
-// reductions, without a barrier.  Rows stay where they are: a chosen row is
-// marked, the others go on, and rows are stored in the order they were chosen
-// in (gord).  Two barriers per column: the multipliers and the pivot's row
-// number, then the pivot row.  Equal magnitudes: the smallest stored row.
-// With the tile and its row swaps in shared memory a launch of few tiles took
-// 55 - 80 us.  Panels and bands together, 24x22x20: 59 steps 7.3 -> 3.9 ms;
-// 64x64x48: 358 steps 72 -> 54 ms.
-template <class T>
-__global__ void __launch_bounds__(256, 1) k_panel(const PanelTask *__restrict__ tasks,
-                                                  const FrontDev *__restrict__ fr, cx<T> *__restrict__ fac,
-                                                  const unsigned long long *__restrict__ amax2, double pivot_rel,
-                                                  int *__restrict__ npert, int *__restrict__ gord)
-{
-    // static-pivot threshold: pivot_rel * max |a_ij| of the assembled operator
-    const T thresh = (T)(pivot_rel * sqrt(__longlong_as_double((long long)*amax2)));
-    __shared__ cx<T> lcol[2][KB], urow[KB];
-    __shared__ int s_p[2], pos[KB];
-    const PanelTask t = tasks[blockIdx.x];
-    const FrontDev F = fr[t.f];
-    const int nf = F.p + F.b, k = t.k, kb = min(KB, F.p - k);
-    cx<T> *D = fac + F.fac + (long long)k * nf + k;
-    const int tid = threadIdx.x, tx = tid >> 4, ty = tid & 15, warp = tid >> 5, lane = tid & 31;
-    cx<T> a[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const int r = ty + 16 * i, q = tx + 16 * c;
-            a[i][c] = (r < kb && q < kb) ? D[(long long)r * nf + q] : cx<T>(0);
-        }
-    unsigned used = 0;   // bit i: row ty + 16 i has been chosen, or is none of the tile's
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-        if (ty + 16 * i >= kb) used |= 1u << i;
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        for (int jj = 0; jj < 16; jj++) {
-            const int j = 16 * c + jj, buf = j & 1;
-            if (j >= kb) break;
-            if (warp == jj >> 1) {
-                const bool mine = (lane >> 4) == (jj & 1);   // the half-warp that holds column j
-                decltype(pivot_key(T(0))) key = 0, ki[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    ki[i] = pivot_key(cabs2(a[i][c]));
-                    if (!((used >> i) & 1u) && ki[i] > key) key = ki[i];
-                }
-                if (!mine) key = 0;
-                const auto best = warp_max(key);
-                int row = KB;
-#pragma unroll
-                for (int i = 3; i >= 0; i--)
-                    if (mine && !((used >> i) & 1u) && ki[i] == best) row = ty + 16 * i;
-                const int p = (int)__reduce_min_sync(0xffffffffu, (unsigned)row);
-                const int src = (p & 15) + 16 * (jj & 1);
-                cx<T> d = pick(a[0][c], a[1][c], a[2][c], a[3][c], p >> 4);
-                d.re = __shfl_sync(0xffffffffu, d.re, src);
-                d.im = __shfl_sync(0xffffffffu, d.im, src);
-                const T m2 = cabs2(d);
-                if (!(m2 >= thresh * thresh)) {   // also catches NaN
-                    const T m = sqrt(m2);
-                    d = (m > 0 && m == m) ? d * (thresh / m) : cx<T>(thresh);
-                    if (lane == src) atomicAdd(npert, 1);
-                }
-                const cx<T> inv = cdiv(cx<T>(1), d);
-                if (mine) {
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const int r = ty + 16 * i;
-                        if (r == p) a[i][c] = d;
-                        else if (!((used >> i) & 1u)) {
-                            a[i][c] = a[i][c] * inv;
-                            lcol[buf][r] = a[i][c];
-                        }
-                    }
-                    if (lane == src) {
-                        s_p[buf] = p;
-                        pos[p] = j;
-                    }
-                }
-            }
-            __syncthreads();
-            const int p = s_p[buf];
-            if ((p & 15) == ty) {
-                const int i = p >> 4;
-#pragma unroll
-                for (int q = c; q < 4; q++) urow[tx + 16 * q] = pick(a[0][q], a[1][q], a[2][q], a[3][q], i);
-                used |= 1u << i;
-            }
-            __syncthreads();
-            cx<T> l[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-                if (!((used >> i) & 1u)) l[i] = lcol[buf][ty + 16 * i];
-#pragma unroll
-            for (int q = c; q < 4; q++) {
-                if (q == c && tx <= jj) continue;
-                const cx<T> u = urow[tx + 16 * q];
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-                    if (!((used >> i) & 1u)) {
-                        a[i][q].re = fma(-l[i].re, u.re, fma(l[i].im, u.im, a[i][q].re));
-                        a[i][q].im = fma(-l[i].re, u.im, fma(-l[i].im, u.re, a[i][q].im));
-                    }
-            }
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int r = ty + 16 * i;
-        if (r >= kb) continue;
-        const int o = pos[r];
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-            if (tx + 16 * c < kb) D[(long long)o * nf + tx + 16 * c] = a[i][c];
-        if (tx == 0) gord[F.first + k + o] = F.first + k + r;
-    }
-}
-
 // Asynchronous global -> shared copy of one complex element (8 or 16 bytes,
 // naturally aligned), and the wait for all of a thread's copies.
 template <class T>
@@ -325,6 +193,202 @@ __device__ __forceinline__ void lds_cx(const cx<double> *p, cx<double> (&a)[N])
     }
 }
 
+// 1 / d for |d|^2 = m2 between 1e-30 and 1e30: conj(d) times a hardware
+// approximation of 1 / m2, then one step of Newton's iteration z (2 - d z), which
+// leaves it more accurate than the scaled division, without its branches
+// (a panel takes 26 us with it, 34 us with cdiv).
+__device__ __forceinline__ cx<float> cinv_fast(const cx<float> d, float m2)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(m2));
+    const cx<float> z(d.re * r, -d.im * r);
+    const cx<float> e(fmaf(-d.re, z.re, fmaf(d.im, z.im, 1.f)), -fmaf(d.re, z.im, d.im * z.re));
+    return cx<float>(fmaf(z.re, e.re, fmaf(-z.im, e.im, z.re)), fmaf(z.re, e.im, fmaf(z.im, e.re, z.im)));
+}
+__device__ __forceinline__ cx<double> cinv_fast(const cx<double> d, double) { return cdiv(cx<double>(1), d); }
+
+// PG columns of a panel in one warp, which holds two rows per lane (rows lane and
+// lane + 32; used: chosen before).  piv[jj] is the row that column jj chose.
+// FAST: straight-line code, so that the next column's pivot search overlaps the
+// update of the columns behind it; it returns false, with nothing to keep, when a
+// pivot is below the threshold or its square near overflow or underflow, and the
+// other form (branches for those cases, and for a narrower last group) has to do
+// the group.
+template <class T, int PG, bool FAST>
+__device__ __forceinline__ bool panel_group(cx<T> (&x0)[PG], cx<T> (&x1)[PG], bool &used0, bool &used1, int nc,
+                                            T thresh, int lane, int (&piv)[PG], int &npert)
+{
+    constexpr T big = sizeof(T) == 4 ? T(1e30) : T(1e250);
+    bool good = true;
+#pragma unroll
+    for (int jj = 0; jj < PG; jj++) {
+        if (!FAST && jj >= nc) break;
+        const auto k0 = pivot_key(cabs2(x0[jj])), k1 = pivot_key(cabs2(x1[jj]));
+        auto key = used0 ? decltype(k0)(0) : k0;
+        if (!used1 && k1 > key) key = k1;
+        const auto best = warp_max(key);
+        const unsigned b0 = __ballot_sync(0xffffffffu, !used0 && k0 == best);
+        const unsigned b1 = __ballot_sync(0xffffffffu, !used1 && k1 == best);
+        const bool up = b0 == 0;   // the pivot is in rows 32 - 63
+        const int src = __ffs(up ? b1 : b0) - 1;
+        cx<T> u[PG];               // the pivot row
+#pragma unroll
+        for (int c = jj; c < PG; c++) {
+            const cx<T> v(up ? x1[c].re : x0[c].re, up ? x1[c].im : x0[c].im);
+            u[c] = cx<T>(__shfl_sync(0xffffffffu, v.re, src), __shfl_sync(0xffffffffu, v.im, src));
+        }
+        piv[jj] = src + (up ? 32 : 0);
+        used0 |= lane == src && !up;
+        used1 |= lane == src && up;
+        cx<T> d = u[jj], inv;
+        T m2 = cabs2(d);
+        if constexpr (FAST) {
+            good = good && m2 >= thresh * thresh && m2 < big && m2 > T(1) / big;
+            inv = cinv_fast(d, m2);
+        } else {
+            if (!(m2 >= thresh * thresh)) {   // also catches NaN
+                const T m = sqrt(m2);
+                d = (m > 0 && m == m) ? d * (thresh / m) : cx<T>(thresh);
+                npert++;
+                if (lane == src) {
+                    if (up) x1[jj] = d;
+                    else x0[jj] = d;
+                }
+            }
+            inv = cdiv(cx<T>(1), d);
+        }
+        // multipliers; zero for chosen rows, which stay as they are
+        const cx<T> l0 = used0 ? cx<T>(0) : x0[jj] * inv, l1 = used1 ? cx<T>(0) : x1[jj] * inv;
+        if (!used0) x0[jj] = l0;
+        if (!used1) x1[jj] = l1;
+#pragma unroll
+        for (int c = jj + 1; c < PG; c++) {
+            cfms(x0[c], l0, u[c]);
+            cfms(x1[c], l1, u[c]);
+        }
+    }
+    return good;
+}
+
+// One CTA per tile: a chain of 64 dependent columns, so the latency of a column
+// is what counts.  The columns are taken in groups of PG: warp 0 holds the
+// group's 64 rows in registers, finds every pivot with a warp reduction and
+// broadcasts the pivot row with shuffles - no barrier inside a group; then all
+// threads update the columns to the right with the group's PG rank-one products
+// at once.  Rows stay where they are: a chosen row is marked, and rows are stored
+// in the order they were chosen in (gord).  Equal magnitudes: the smallest stored
+// row.  A launch of few tiles took 55 - 80 us with the tile and its row swaps in
+// shared memory, 42 us with the tile in the registers of 256 threads and two
+// barriers per column, and takes 26 us.
+constexpr int PG = 8;
+constexpr int PLD = KB + 2;   // row stride: 16-byte-aligned rows
+template <class T> constexpr size_t panel_smem() { return sizeof(cx<T>) * KB * PLD; }
+
+template <class T>
+__global__ void __launch_bounds__(256, 1) k_panel(const PanelTask *__restrict__ tasks,
+                                                  const FrontDev *__restrict__ fr, cx<T> *__restrict__ fac,
+                                                  const unsigned long long *__restrict__ amax2, double pivot_rel,
+                                                  int *__restrict__ npert, int *__restrict__ gord)
+{
+    // static-pivot threshold: pivot_rel * max |a_ij| of the assembled operator
+    const T thresh = (T)(pivot_rel * sqrt(__longlong_as_double((long long)*amax2)));
+    extern __shared__ __align__(16) unsigned char smraw[];
+    cx<T> *S = reinterpret_cast<cx<T> *>(smraw);   // KB x PLD
+    __shared__ int spiv[2][PG], pos[KB];           // two sets: a group's is read while the next is found
+    __shared__ unsigned s_used[2];                 // rows chosen so far: bits of rows 0-31, 32-63
+    const PanelTask t = tasks[blockIdx.x];
+    const FrontDev F = fr[t.f];
+    const int nf = F.p + F.b, k = t.k, kb = min(KB, F.p - k);
+    cx<T> *D = fac + F.fac + (long long)k * nf + k;
+    const int tid = threadIdx.x, lane = tid & 31;
+    for (int q = tid; q < KB * KB; q += 256) {
+        const int i = q / KB, j = q % KB;
+        if (i < kb && j < kb) cp_async_cx(S + i * PLD + j, D + (long long)i * nf + j);
+        else S[i * PLD + j] = cx<T>(0);
+    }
+    bool used0 = lane >= kb, used1 = lane + 32 >= kb;   // warp 0: this lane's rows lane and lane + 32
+    cp_async_wait_all();
+    __syncthreads();
+    const int ng = (kb + PG - 1) / PG;
+    for (int G = 0; G < ng; G++) {
+        const int j0 = PG * G;
+        int *piv = spiv[G & 1];
+        if (tid < 32) {
+            const bool w0 = !used0, w1 = !used1;   // rows this group may change
+            cx<T> x0[PG], x1[PG];
+            int pv[PG], np = 0;
+            auto fetch = [&]() {
+#pragma unroll
+                for (int c = 0; c < PG; c++) x0[c] = x1[c] = cx<T>(0);
+                if (w0) lds_cx<PG>(S + lane * PLD + j0, x0);
+                if (w1) lds_cx<PG>(S + (lane + 32) * PLD + j0, x1);
+            };
+            fetch();
+            const int nc = min(PG, kb - j0);
+            if (nc < PG || !panel_group<T, PG, true>(x0, x1, used0, used1, nc, thresh, lane, pv, np)) {
+                used0 = !w0;
+                used1 = !w1;
+                fetch();
+                panel_group<T, PG, false>(x0, x1, used0, used1, nc, thresh, lane, pv, np);
+                if (lane == 0 && np) atomicAdd(npert, np);
+            }
+            if (lane == 0) {
+#pragma unroll
+                for (int jj = 0; jj < PG; jj++)
+                    if (jj < nc) {
+                        piv[jj] = pv[jj];
+                        pos[pv[jj]] = j0 + jj;
+                    }
+            }
+#pragma unroll
+            for (int c = 0; c < PG; c++) {
+                if (w0) S[lane * PLD + j0 + c] = x0[c];
+                if (w1) S[(lane + 32) * PLD + j0 + c] = x1[c];
+            }
+            const unsigned m0 = __ballot_sync(0xffffffffu, used0), m1 = __ballot_sync(0xffffffffu, used1);
+            if (lane == 0) { s_used[0] = m0; s_used[1] = m1; }
+        }
+        __syncthreads();
+        if (G + 1 == ng) break;
+        // columns right of the group (all PG pivots exist: kb > j0 + PG): thread
+        // (column, quarter of the rows)
+        const int c = tid & (KB - 1), r0 = (tid >> 6) * (KB / 4);
+        const bool on = c >= j0 + PG && c < kb;
+        cx<T> u[PG];
+        if (on) {
+#pragma unroll
+            for (int q = 0; q < PG; q++) {
+                const cx<T> *row = S + piv[q] * PLD;
+                u[q] = row[c];
+#pragma unroll
+                for (int l = 0; l < q; l++) cfms(u[q], row[j0 + l], u[l]);
+            }
+            const unsigned used = s_used[r0 >> 5] >> (r0 & 31);
+#pragma unroll 2
+            for (int i = 0; i < KB / 4; i++) {
+                if ((used >> i) & 1u) continue;
+                cx<T> *row = S + (r0 + i) * PLD, a = row[c], l[PG];
+                lds_cx<PG>(row + j0, l);
+#pragma unroll
+                for (int q = 0; q < PG; q++) cfms(a, l[q], u[q]);
+                row[c] = a;
+            }
+        }
+        __syncthreads();
+        // the pivot rows' part of U: nobody reads it before the tile is stored
+        if (on && r0 == 0) {
+#pragma unroll
+            for (int q = 0; q < PG; q++) S[piv[q] * PLD + c] = u[q];
+        }
+    }
+    __syncthreads();
+    for (int q = tid; q < kb * KB; q += 256) {
+        const int i = q / KB, j = q % KB;
+        if (j < kb) D[(long long)pos[i] * nf + j] = S[i * PLD + j];
+    }
+    if (tid < kb) gord[F.first + k + pos[tid]] = F.first + k + tid;
+}
+
 // ---------------------------------------------------------------------------
 // bands of a panel: the rows right of it, B <- L_D^{-1} P B, and the columns
 // below it, X <- X U_D^{-1}, by substitution, in one launch (they do not depend
@@ -340,63 +404,83 @@ __device__ __forceinline__ void lds_cx(const cx<double> *p, cx<double> (&a)[N])
 // identity beyond kb (a last, narrower panel).
 // ---------------------------------------------------------------------------
 struct BandTask { int f, k, c0, which; };   // which: 0 columns right, 1 pivot rows below, 2 border rows; c0: the first
-constexpr int BD_V = 32, BD_TH = 4 * BD_V;  // vectors and threads per CTA
-template <class T>
+// NV vectors per four threads: with two, a row of the tile is read from shared
+// memory once for both; a launch of many vectors is bound by those reads, one of
+// few by the chain, which is shorter with one.
+constexpr int BD_TH = 128;
+template <class T, int NV>
 struct BandCfg {
+    static constexpr int V = BD_TH / 4 * NV;                // vectors per CTA
     static constexpr int TG = sizeof(T) == 4 ? 8 : 4;       // unknowns per group
     static constexpr int LDT = KB + 16 / (int)sizeof(cx<T>);   // tile rows on 16 bytes, four rows on different banks
-    static constexpr int LDX = sizeof(T) == 4 ? BD_V + 4 : BD_V + 2;
+    static constexpr int LDX = V + (sizeof(T) == 4 ? 4 : 2);
     static constexpr size_t smem = sizeof(cx<T>) * (KB * LDT + KB * LDX);
 };
 
-// T x = b for the BD_V vectors of X (b on entry, zero before group first / TG);
-// unit: T's diagonal is one, otherwise invd holds its inverse.
-template <class T>
+// T x = b for the vectors of X (b on entry, zero before group first / TG); unit:
+// T's diagonal is one, otherwise invd holds its inverse.  Vector e of a quad is
+// vector quad + 32 e.
+template <class T, int NV>
 __device__ __forceinline__ void band_solve(const cx<T> *Tm, cx<T> *X, const cx<T> *invd, bool unit, int first, int kb)
 {
-    constexpr int TG = BandCfg<T>::TG, LDT = BandCfg<T>::LDT, LDX = BandCfg<T>::LDX;
-    const int v = threadIdx.x >> 2, q4 = threadIdx.x & 3;
-    const int ng = (kb + TG - 1) / TG;
-    cx<T> *x = X + v;
+    using C = BandCfg<T, NV>;
+    constexpr int TG = C::TG, LDT = C::LDT, LDX = C::LDX;
+    const int q4 = threadIdx.x & 3, ng = (kb + TG - 1) / TG;
+    cx<T> *x = X + (threadIdx.x >> 2);
 #pragma unroll 1
     for (int G = first / TG; G < ng; G++) {
-        cx<T> b[TG];
+        cx<T> b[NV][TG];
 #pragma unroll
-        for (int i = 0; i < TG; i++) b[i] = x[(TG * G + i) * LDX];
+        for (int e = 0; e < NV; e++)
+#pragma unroll
+            for (int i = 0; i < TG; i++) b[e][i] = x[(TG * G + i) * LDX + 32 * e];
 #pragma unroll
         for (int i = 0; i < TG; i++) {
             if (i > 0) {
                 cx<T> lr[TG];
                 lds_cx<TG>(Tm + (TG * G + i) * LDT + TG * G, lr);
 #pragma unroll
-                for (int l = 0; l < i; l++) cfms(b[i], lr[l], b[l]);
+                for (int e = 0; e < NV; e++)
+#pragma unroll
+                    for (int l = 0; l < i; l++) cfms(b[e][i], lr[l], b[e][l]);
             }
-            if (!unit) b[i] = b[i] * invd[TG * G + i];
+            if (!unit) {
+                const cx<T> d = invd[TG * G + i];
+#pragma unroll
+                for (int e = 0; e < NV; e++) b[e][i] = b[e][i] * d;
+            }
         }
         __syncwarp();   // the four threads have read the group
 #pragma unroll
-        for (int i = 0; i < TG; i++)
-            if ((i & 3) == q4) x[(TG * G + i) * LDX] = b[i];
+        for (int e = 0; e < NV; e++)
+#pragma unroll
+            for (int i = 0; i < TG; i++)
+                if ((i & 3) == q4) x[(TG * G + i) * LDX + 32 * e] = b[e][i];
 #pragma unroll 1
         for (int H = TG * (G + 1) + q4; H < TG * ng; H += TG) {
 #pragma unroll
             for (int i = 0; i < TG; i += 4) {
-                cx<T> lr[TG], c = x[(H + i) * LDX];
+                cx<T> lr[TG], c[NV];
+#pragma unroll
+                for (int e = 0; e < NV; e++) c[e] = x[(H + i) * LDX + 32 * e];
                 lds_cx<TG>(Tm + (H + i) * LDT + TG * G, lr);
 #pragma unroll
-                for (int l = 0; l < TG; l++) cfms(c, lr[l], b[l]);
-                x[(H + i) * LDX] = c;
+                for (int l = 0; l < TG; l++)
+#pragma unroll
+                    for (int e = 0; e < NV; e++) cfms(c[e], lr[l], b[e][l]);
+#pragma unroll
+                for (int e = 0; e < NV; e++) x[(H + i) * LDX + 32 * e] = c[e];
             }
         }
         __syncwarp();
     }
 }
 
-template <class T>
+template <class T, int NV>
 __global__ void __launch_bounds__(BD_TH) k_bands(const BandTask *__restrict__ tasks, const FrontDev *__restrict__ fr,
                                                  cx<T> *__restrict__ fac, const int *__restrict__ gord)
 {
-    using C = BandCfg<T>;
+    using C = BandCfg<T, NV>;
     constexpr int LDT = C::LDT, LDX = C::LDX;
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T> *Tm = reinterpret_cast<cx<T> *>(smraw);   // KB x LDT
@@ -422,11 +506,11 @@ __global__ void __launch_bounds__(BD_TH) k_bands(const BandTask *__restrict__ ta
         xb = fac + F.fac + (long long)k * nf + t.c0;
         si = nf;
         sv = 1;
-        nv = min(BD_V, nf - t.c0);
+        nv = min(C::V, nf - t.c0);
         if (tid < KB) idx[tid] = tid < kb ? gord[F.first + k + tid] - F.first - k : 0;
         __syncthreads();
-        for (int q = tid; q < KB * BD_V; q += BD_TH) {
-            const int i = q / BD_V, v = q % BD_V;
+        for (int q = tid; q < KB * C::V; q += BD_TH) {
+            const int i = q / C::V, v = q % C::V;
             if (i < kb && v < nv) cp_async_cx(X + i * LDX + v, xb + idx[i] * si + v);
             else X[i * LDX + v] = cx<T>(0);
         }
@@ -434,14 +518,14 @@ __global__ void __launch_bounds__(BD_TH) k_bands(const BandTask *__restrict__ ta
         if (t.which == 1) {
             xb = fac + F.fac + (long long)t.c0 * nf + k;
             sv = nf;
-            nv = min(BD_V, F.p - t.c0);
+            nv = min(C::V, F.p - t.c0);
         } else {
             xb = fac + F.fac + (long long)F.p * nf + (long long)t.c0 * F.p + k;
             sv = F.p;
-            nv = min(BD_V, F.b - t.c0);
+            nv = min(C::V, F.b - t.c0);
         }
         si = 1;
-        for (int q = tid; q < KB * BD_V; q += BD_TH) {
+        for (int q = tid; q < KB * C::V; q += BD_TH) {
             const int i = q % KB, v = q / KB;
             if (i < kb && v < nv) cp_async_cx(X + i * LDX + v, xb + v * sv + i);
             else X[i * LDX + v] = cx<T>(0);
@@ -451,10 +535,10 @@ __global__ void __launch_bounds__(BD_TH) k_bands(const BandTask *__restrict__ ta
     __syncthreads();
     if (tid < KB) invd[tid] = row ? cx<T>(1) : cdiv(cx<T>(1), Tm[tid * LDT + tid]);
     __syncthreads();
-    band_solve<T>(Tm, X, invd, row, 0, kb);
+    band_solve<T, NV>(Tm, X, invd, row, 0, kb);
     __syncthreads();
-    for (int q = tid; q < KB * BD_V; q += BD_TH) {
-        const int i = row ? q / BD_V : q % KB, w = row ? q % BD_V : q / KB;
+    for (int q = tid; q < KB * C::V; q += BD_TH) {
+        const int i = row ? q / C::V : q % KB, w = row ? q % C::V : q / KB;
         if (i < kb && w < nv) xb[i * si + w * sv] = X[i * LDX + w];
     }
 }

@@ -61,14 +61,14 @@ __global__ void __launch_bounds__(BD_TH) k_tile_inverse(const PanelTask *__restr
                                                         const cx<T> *__restrict__ fac, const int *__restrict__ gord,
                                                         int *__restrict__ ipiv, cx<T> *__restrict__ inv)
 {
-    using C = BandCfg<T>;
+    using C = BandCfg<T, 1>;
     constexpr int LDT = C::LDT, LDX = C::LDX;
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T> *Tm = reinterpret_cast<cx<T> *>(smraw);
     cx<T> *X = Tm + KB * LDT;
     __shared__ cx<T> invd[KB];
     const PanelTask t = tasks[blockIdx.x >> 2];
-    const int part = blockIdx.x & 3, v0 = BD_V * (part & 1);
+    const int part = blockIdx.x & 3, v0 = C::V * (part & 1);
     const bool row = part < 2;
     const FrontDev F = fr[t.f];
     const int nf = F.p + F.b, k = t.k, kb = min(KB, F.p - k);
@@ -95,20 +95,20 @@ __global__ void __launch_bounds__(BD_TH) k_tile_inverse(const PanelTask *__restr
         if (i < kb && j < kb) cp_async_cx(dst, D + (long long)i * nf + j);
         else *dst = cx<T>(i == j ? T(1) : T(0));
     }
-    for (int q = tid; q < KB * BD_V; q += BD_TH) {
-        const int i = q / BD_V, v = q % BD_V;
+    for (int q = tid; q < KB * C::V; q += BD_TH) {
+        const int i = q / C::V, v = q % C::V;
         X[i * LDX + v] = cx<T>(i == v0 + v ? T(1) : T(0));
     }
     cp_async_wait_all();
     __syncthreads();
     if (tid < KB) invd[tid] = row ? cx<T>(1) : cdiv(cx<T>(1), Tm[tid * LDT + tid]);
     __syncthreads();
-    band_solve<T>(Tm, X, invd, row, v0, kb);
+    band_solve<T, 1>(Tm, X, invd, row, v0, kb);
     __syncthreads();
     const int c0 = k / SB * SB, w = min(SB, F.p - c0), ldw = inv_ld(w), o = k - c0;
     cx<T> *W = inv + F.inv + (long long)(c0 / SB) * (SB * SB) + (long long)o * ldw + o;
-    for (int q = tid; q < KB * BD_V; q += BD_TH) {
-        const int i = row ? q / BD_V : q % KB, v = row ? q % BD_V : q / KB, e = v0 + v;
+    for (int q = tid; q < KB * C::V; q += BD_TH) {
+        const int i = row ? q / C::V : q % KB, v = row ? q % C::V : q / KB, e = v0 + v;
         if (i >= kb || e >= kb) continue;
         if (row) { if (i > e) W[(long long)i * ldw + e] = X[i * LDX + v]; }
         else if (i >= e) W[(long long)e * ldw + i] = X[i * LDX + v];
