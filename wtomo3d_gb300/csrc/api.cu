@@ -18,6 +18,45 @@ namespace wt3d {
 static thread_local std::string g_err;
 void set_error(const std::string &msg) { g_err = msg; }
 
+// One pool per device, made at its first use and kept for the process; empty
+// between handles.  A stream takes memory that another has released only where
+// that release has completed: no stream is made to wait for another's work.
+static std::mutex g_pool_mu;
+static std::map<int, cudaMemPool_t> g_pools;
+static std::atomic<int> g_handles{0};
+
+cudaMemPool_t scratch_pool()
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    auto it = g_pools.find(dev);
+    if (it != g_pools.end()) return it->second;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+        cudaGetLastError();
+        pool = nullptr;
+    } else {
+        unsigned long long keep = SCRATCH_KEEP;
+        int off = 0;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &off);
+    }
+    g_pools[dev] = pool;
+    return pool;
+}
+
+void scratch_trim()
+{
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    for (auto &kv : g_pools)
+        if (kv.second) cudaMemPoolTrimTo(kv.second, 0);
+}
+
 // Spread sources: F[src_col[e] * n + 3 node[e] + comp[e]] += w[e] * sterm[e]
 // (one thread per (source, weight) entry; entries of one source are distinct).
 __global__ void k_put_sources(long long n, long long ne, const int *__restrict__ col, const long long *__restrict__ node,
@@ -140,6 +179,7 @@ struct wt3d_solver {
     bool have_model = false, have_values = false, have_factor = false;
     long long kernels_solve = 0;
     wt3d_stats stats{};
+    wt3d_solver() { g_handles.fetch_add(1); }
     ~wt3d_solver()
     {
         if (st) cudaStreamSynchronize(st);
@@ -152,6 +192,7 @@ struct wt3d_solver {
         if (st) cudaStreamDestroy(st);
         if (sts) cudaStreamDestroy(sts);
         if (pin) cudaFreeHost(pin);
+        if (g_handles.fetch_sub(1) == 1) scratch_trim();
     }
 };
 
@@ -634,17 +675,11 @@ int wt3d_assemble_device(const wt3d_grid *g, const float *d_vp, const float *d_v
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
     long long nn = (long long)g->nx * g->ny * g->nz;
-    void *da = nullptr, *mu = nullptr;
-    double *ro = nullptr;
-    WT_CUDA(cudaMallocAsync(&da, sizeof(double2) * nn, st));
-    WT_CUDA(cudaMallocAsync(&mu, sizeof(double2) * nn, st));
-    WT_CUDA(cudaMallocAsync(&ro, sizeof(double) * nn, st));
-    rc = device_lame(nn, d_vp, d_vs, d_rho, da, mu, ro, st);
-    if (!rc) rc = device_assemble(*g, da, mu, ro, omega_re, omega_im, d_irptr, d_a, st);
-    cudaFreeAsync(da, st);
-    cudaFreeAsync(mu, st);
-    cudaFreeAsync(ro, st);
-    return rc;
+    StreamBuf<double2> da, mu;
+    StreamBuf<double> ro;
+    if ((rc = da.alloc(nn, st)) || (rc = mu.alloc(nn, st)) || (rc = ro.alloc(nn, st))) return rc;
+    if ((rc = device_lame(nn, d_vp, d_vs, d_rho, da.p, mu.p, ro.p, st))) return rc;
+    return device_assemble(*g, da.p, mu.p, ro.p, omega_re, omega_im, d_irptr, d_a, st);
 }
 
 int wt3d_assemble(const wt3d_grid *g, const float *vp, const float *vs, const float *rho, double omega_re,
@@ -1181,16 +1216,19 @@ int wt3d_misfit_gradient(wt3d_solver *h, int nsrc, const void *d_F, const void *
     for (int r = 0; r < nrec; r++)
         if (rec_node[r] < 0 || rec_node[r] >= nn) { set_error("wt3d_misfit_gradient: receiver node out of range"); return WT3D_ERR_ARG; }
     const long long nd = (long long)nsrc * nrec * 3;
-    DevVec<double2> X, S, Lm, dd, dp, dr;
-    DevVec<long long> drec;
-    DevVec<double> dg;
+    // taken and released in the order of h->st; the solves on h->sts start after
+    // the synchronisation below and are done when they return
+    StreamBuf<double2> X, S, Lm, dd, dp, dr;
+    StreamBuf<long long> drec;
+    StreamBuf<double> dg;
     int rc;
-    if ((rc = X.alloc((size_t)n * nsrc)) || (rc = S.alloc((size_t)n * nsrc)) || (rc = Lm.alloc((size_t)n * nsrc)) ||
-        (rc = dd.alloc(nd)) || (rc = dp.alloc(nd)) || (rc = dr.alloc(nd)) || (rc = drec.alloc(nrec)) ||
-        (rc = dg.alloc(3 * nn)))
+    if ((rc = X.alloc((size_t)n * nsrc, h->st)) || (rc = S.alloc((size_t)n * nsrc, h->st)) ||
+        (rc = Lm.alloc((size_t)n * nsrc, h->st)) || (rc = dd.alloc(nd, h->st)) || (rc = dp.alloc(nd, h->st)) ||
+        (rc = dr.alloc(nd, h->st)) || (rc = drec.alloc(nrec, h->st)) || (rc = dg.alloc(3 * nn, h->st)))
         return rc;
     WT_CUDA(cudaMemcpyAsync(drec.p, rec_node, sizeof(long long) * nrec, cudaMemcpyHostToDevice, h->st));
     WT_CUDA(cudaMemcpyAsync(dd.p, dobs, sizeof(double2) * nd, cudaMemcpyHostToDevice, h->st));
+    WT_CUDA(cudaStreamSynchronize(h->st));
     // forward wavefields; the total field adds the background u0
     int rcf = solve_dev_cm(h, nsrc, (const double2 *)d_F, X.p, tol, maxit, nullptr, nullptr, false);
     if (rcf && rcf != WT3D_ERR_NOCONV) return rcf;
@@ -1208,7 +1246,8 @@ int wt3d_misfit_gradient(wt3d_solver *h, int nsrc, const void *d_F, const void *
     int rca = solve_dev_cm(h, nsrc, S.p, Lm.p, tol, maxit, nullptr, nullptr, true);
     if (rca && rca != WT3D_ERR_NOCONV) return rca;
     if ((rc = wt3d_gradient_contract(h, nsrc, X.p, Lm.p, dg.p))) return rc;
-    WT_CUDA(cudaMemcpy(grad, dg.p, sizeof(double) * 3 * nn, cudaMemcpyDeviceToHost));
+    WT_CUDA(cudaMemcpyAsync(grad, dg.p, sizeof(double) * 3 * nn, cudaMemcpyDeviceToHost, h->st));
+    WT_CUDA(cudaStreamSynchronize(h->st));
     return rcf ? rcf : rca;
 }
 
@@ -1259,13 +1298,13 @@ int wt3d_rhs_sources(wt3d_solver *h, int nsrc, const double *xyz, const int *com
         const std::complex<double> v = sterm ? reinterpret_cast<const std::complex<double> *>(sterm)[j] : 1.0;
         st[j] = make_double2(v.real(), v.imag());
     }
-    DevVec<int> dcol, dcmp;
-    DevVec<long long> dnd;
-    DevVec<double> dw;
-    DevVec<double2> dst;
+    StreamBuf<int> dcol, dcmp;
+    StreamBuf<long long> dnd;
+    StreamBuf<double> dw;
+    StreamBuf<double2> dst;
     int rc;
-    if ((rc = dcol.upload(col)) || (rc = dcmp.upload(cmp)) || (rc = dnd.upload(nd)) || (rc = dw.upload(w)) ||
-        (rc = dst.upload(st)))
+    if ((rc = dcol.upload(col, h->st)) || (rc = dcmp.upload(cmp, h->st)) || (rc = dnd.upload(nd, h->st)) ||
+        (rc = dw.upload(w, h->st)) || (rc = dst.upload(st, h->st)))
         return rc;
     WT_CUDA(cudaMemsetAsync(d_F, 0, sizeof(double2) * n * nsrc, h->st));
     const long long ne = (long long)col.size();
@@ -1294,13 +1333,15 @@ int wt3d_sample_receivers(wt3d_solver *h, int nrhs, const void *d_U, int nrec, c
         w.insert(w.end(), b.begin(), b.end());
         start.push_back((int)nd.size());
     }
-    DevVec<int> dstart;
-    DevVec<long long> dnd;
-    DevVec<double> dw;
-    DevVec<double2> dout;
+    StreamBuf<int> dstart;
+    StreamBuf<long long> dnd;
+    StreamBuf<double> dw;
+    StreamBuf<double2> dout;
     const long long tot = (long long)nrhs * nrec * 3;
     int rc;
-    if ((rc = dstart.upload(start)) || (rc = dnd.upload(nd)) || (rc = dw.upload(w)) || (rc = dout.alloc(tot))) return rc;
+    if ((rc = dstart.upload(start, h->st)) || (rc = dnd.upload(nd, h->st)) || (rc = dw.upload(w, h->st)) ||
+        (rc = dout.alloc(tot, h->st)))
+        return rc;
     k_get_receivers<<<ceil_div(tot, 256), 256, 0, h->st>>>(h->n, nrhs, nrec, dstart.p, dnd.p, dw.p,
                                                             (const double2 *)d_U, dout.p);
     WT_CUDA(cudaGetLastError());
