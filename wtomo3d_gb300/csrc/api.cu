@@ -273,17 +273,23 @@ int solve_host_buffer(wt3d_solver *h)
 // the current iterate, h->Rn = B - op(A) Xn and bnorm2/rnorm2 the squared
 // column norms of B and R; on exit Xn is the new iterate.  Classical
 // Gram-Schmidt applied twice; Givens rotations and the small least-squares
-// problems per column on the host.  The restart length is 8 unless the
-// WT3D_GMRES_RESTART environment variable sets another (1..16); each Arnoldi
-// vector costs a block of n x sk_columns(m) complex128 and one in the factors'
-// precision while the call runs.
-static int gmres_restart()
+// problems per column on the host.  The restart length is the longest, up to
+// GM_KMAX, whose bases take no more than GM_BYTES per row: 10 for 32 columns of
+// complex64 factors, 16 for up to 16 columns (WT3D_GMRES_RESTART sets another,
+// 1..16).  Every restart forgets what the basis has learnt of the few slow
+// modes: 64^3 at 1 Hz, 4 adjoint columns, took 19 to 27 passes with a restart of
+// 8 and 15 with one of 16.
+constexpr long long GM_BYTES = 272 * 32;
+static int gmres_restart(int nc, size_t zsize)
 {
-    static const int k = [] {
+    static const int env = [] {
         const char *e = getenv("WT3D_GMRES_RESTART");
-        const int v = e ? atoi(e) : 8;
-        return v < 1 ? 1 : (v > GM_KMAX ? GM_KMAX : v);
+        const int v = e ? atoi(e) : 0;
+        return !e ? 0 : v < 1 ? 1 : (v > GM_KMAX ? GM_KMAX : v);
     }();
+    if (env) return env;
+    int k = 8;
+    while (k < GM_KMAX && nc * ((k + 3) * 16LL + (k + 1) * (long long)zsize) <= GM_BYTES) k++;
     return k;
 }
 
@@ -295,7 +301,7 @@ int fgmres(wt3d_solver *h, Engine<T> &E, Schedule<T> *sc, int m, bool adjoint, d
     const long long n = h->n;
     const int nc = sk_columns(m);
     const long long blk = n * nc;
-    const int kr = gmres_restart();
+    const int kr = gmres_restart(nc, sizeof(cx<T>));
     int rc;
     if (!h->gmH.p) {
         if ((rc = h->gmH.alloc((size_t)2 * (GM_KMAX + 1) * MAXRHS)) ||

@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(256) k_residual(long long ngroups, const int *
 // Column c of every block is an independent system; reductions go through
 // per-block partial sums and a second pass, so they do not depend on
 // scheduling.  Grid strides are multiples of nc: a thread stays in its column.
-constexpr int GM_KMAX = 16;      // longest restart of the flexible GMRES (per-call length gmres_restart())
+constexpr int GM_KMAX = 16;      // longest restart of the flexible GMRES (per-call length: gmres_restart())
 constexpr int GM_BLOCKS = 304;   // 2 blocks per SM for the reductions
 constexpr int GM_CHUNK = 4;      // basis vectors per sweep over W
 
