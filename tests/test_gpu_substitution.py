@@ -68,3 +68,25 @@ def test_products(k):
         stored[np.repeat(np.arange(g.n), np.diff(ir))[jc == hit]] = True
         np.testing.assert_array_equal(~np.isfinite(Y[:, 0]), stored)
         assert np.isfinite(Y[:, 1:]).all()
+
+
+@pytest.mark.parametrize("k", [8, 17, 33])
+def test_incident_field_sources(k):
+    """(A_bg - A) u0 by digit products (8 and more sources) against the same
+    sources one to three at a time, by the FP64 sum: 162-term sums in both, so
+    200 eps of the largest entry of a column."""
+    dims = (13, 11, 18)
+    g = Grid(*dims, 20.0, pmld=3 * 20.0, fst=1)
+    ain, baz = np.radians(np.linspace(1.0, 29.0, k)), np.radians(np.linspace(0.0, 350.0, k))
+    lay = wt.Layered1D(*model.layered1d(dims[2], 20.0))
+    with wt.Solver(g) as s:
+        s.set_model(*model.layered_random(*dims, 20.0, seed=5))
+        s.set_background(*model.layered(*dims))
+        s.factor(2 * np.pi * 1.5)
+        F, U = s.rhs_planewave(lay, ain, baz)
+        for c in range(0, k, 3):
+            f, u = s.rhs_planewave(lay, ain[c:c + 3], baz[c:c + 3])
+            np.testing.assert_array_equal(U[:, c:c + 3], u)
+            # the sums' terms: |A_bg - A| |u0| <= 81 * 4e8 * |u0|, F itself 1e5 times less
+            scale = 81 * 4e8 * np.abs(u).max(axis=0)
+            assert (np.abs(F[:, c:c + 3] - f) <= 200 * np.finfo(float).eps * scale).all()

@@ -3,7 +3,7 @@
 // the complex64 multifrontal factorisation.
 #include <atomic>
 #include "engine.cuh"
-#include "refine_kernels.cuh"
+#include "exact_product.cuh"
 #include "wtomo3d_gpu.h"
 #include <array>
 #include <chrono>
@@ -170,6 +170,9 @@ struct wt3d_solver {
     DevVec<double2> gmPart;
     DevVec<double> gmNorm, gmScale;
     void *pin = nullptr;                  // SolveHost
+    StreamBuf<ulonglong2> epA;            // the operator's digits (product_prepare), per call
+    StreamBuf<int> epE;                   // ... exponents of its rows, its columns, blocks of nodes
+    ProductOp epOp{};
     std::unique_ptr<Engine<float>> e32;
     std::unique_ptr<Engine<double>> e64;
     cudaStream_t st = nullptr;
@@ -229,15 +232,69 @@ int have_gpu()
     return WT3D_OK;
 }
 
+// Digits of op(A) (abg - A with abg != nullptr) for the tensor-core products of a
+// call with up to m columns, until product_done.  Grid operators and 8 or more
+// columns only: with fewer the FP64 kernel is as fast (0.5 ms for one column of
+// 48^3, 0.9 for four), and without the memory it does the work too.
+struct ProductDone {
+    wt3d_solver *h;
+    ~ProductDone() { h->epA.release(); h->epE.release(); }
+};
+int product_prepare(wt3d_solver *h, cudaStream_t st, int m, bool adjoint, const double2 *abg)
+{
+    if (h->general || sk_columns(std::min(m, MAXRHS)) < 8) return WT3D_OK;
+    static std::once_flag once[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::call_once(once[dev & 63], [] {
+        cudaFuncSetAttribute(k_product_tc<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EP_SMEM);
+        cudaFuncSetAttribute(k_product_tc<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EP_SMEM);
+        cudaFuncSetAttribute(k_product_tc<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EP_SMEM);
+    });
+    const long long tiles =
+        (long long)ceil_div(h->grid.nx, EP_T) * ceil_div(h->grid.ny, EP_T) * ceil_div(h->grid.nz, EP_T);
+    if (h->epA.alloc((size_t)h->n * EP_SLOTS, st) || h->epE.alloc(2 * (size_t)h->n + tiles, st)) {
+        h->epA.release();
+        h->epE.release();
+        return WT3D_OK;
+    }
+    h->epOp = ProductOp{h->irptr.p, h->jcptr.p, h->tpos.p, h->a.p, abg, adjoint ? 1 : 0};
+    int *pe = h->epE.p + h->n, *bmax = pe + h->n;
+    k_column_exponents<<<ceil_div(h->n * 32, 256), 256, 0, st>>>(h->n, h->epOp, pe);
+    k_block_exponents<<<ceil_div(tiles * 32, 256), 256, 0, st>>>(h->grid.nx, h->grid.ny, h->grid.nz, pe, bmax);
+    k_operator_digits<<<ceil_div(h->n / 3 * 32, 256), 256, 0, st>>>(h->grid.nx, h->grid.ny, h->grid.nz, h->epOp, pe,
+                                                                     bmax, h->epA.p, h->epE.p);
+    WT_CUDA(cudaGetLastError());
+    return WT3D_OK;
+}
+
+template <int NC>
+void product_tc(const wt3d_solver *h, cudaStream_t st, const double2 *X, const double2 *B, double2 *R, double *nr,
+                double *nb)
+{
+    const wt3d_grid &g = h->grid;
+    const unsigned grid = (unsigned)((long long)ceil_div(g.nx, EP_T) * ceil_div(g.ny, EP_T) * ceil_div(g.nz, EP_T) *
+                                     ceil_div(NC, EP_COLS));
+    k_product_tc<NC><<<grid, EP_THREADS, EP_SMEM, st>>>(g.nx, g.ny, g.nz, h->epOp, h->epA.p, h->epE.p,
+                                                        h->epE.p + h->n, X, B, R, nr, nb);
+}
+
 // R = B - op(A) X (R = op(A) X when B is null), accumulating the squared
-// column norms of R and B into h->norms: a warp per node of the grid pattern, a
-// warp per row of a general one.
+// column norms of R and B into h->norms: on the tensor cores where the call has
+// prepared them, else a warp per node of the grid pattern or per row of a general
+// one.
 void residual(const wt3d_solver *h, cudaStream_t st, int m, const double2 *X, const double2 *B, double2 *R,
               bool adjoint)
 {
     double *nr = h->norms.p, *nb = h->norms.p + MAXRHS;
-    const int adj = adjoint ? 1 : 0;
-    WT_SWITCH_NC(sk_columns(m),
+    const int adj = adjoint ? 1 : 0, nc = sk_columns(m);
+    if (h->epA.p && nc >= 8) {
+        if (nc == 8) product_tc<8>(h, st, X, B, R, nr, nb);
+        else if (nc == 16) product_tc<16>(h, st, X, B, R, nr, nb);
+        else product_tc<32>(h, st, X, B, R, nr, nb);
+        return;
+    }
+    WT_SWITCH_NC(nc,
         if (h->general)
             k_residual<NC, 1><<<152 * 8, 256, 0, st>>>(h->n, h->irptr.p, h->jcptr.p, h->a.p, h->tpos.p, X, B, R, nr,
                                                        nb, adj);
@@ -538,6 +595,8 @@ int solve_dev_cm(wt3d_solver *h, int nrhs, const double2 *d_B, double2 *d_X, dou
     int worst_rc = WT3D_OK, maxits = 0;
     h->kernels_solve = 0;
     cudaEventRecord(h->ev0, h->sts);
+    if (int rc = product_prepare(h, h->sts, nrhs, adjoint, nullptr)) return rc;
+    ProductDone done{h};
     for (int c0 = 0; c0 < nrhs; c0 += MAXRHS) {
         int m = std::min(MAXRHS, nrhs - c0);
         to_rows(h, h->sts, m, d_B + (long long)c0 * n, h->Bn.p);
@@ -1016,6 +1075,8 @@ int wt3d_rhs_planewave(wt3d_solver *h, const wt3d_layered1d *m, int nsrc, const 
                               h->st)))
         return rc;
     const int nl = m->nl;
+    if ((rc = product_prepare(h, h->st, nsrc, false, h->abg.p))) return rc;
+    ProductDone done{h};
     for (int c0 = 0; c0 < nsrc; c0 += MAXRHS) {
         const int mm = std::min(MAXRHS, nsrc - c0);
         std::vector<std::complex<double>> Uz((size_t)mm * nz), Wz((size_t)mm * nz);
@@ -1043,10 +1104,15 @@ int wt3d_rhs_planewave(wt3d_solver *h, const wt3d_layered1d *m, int nsrc, const 
         if ((rc = dU.upload(hu, h->st)) || (rc = dW.upload(hw, h->st)) || (rc = dkx.upload(kx, h->st)) ||
             (rc = dky.upload(ky, h->st)) || (rc = drx.upload(rx, h->st)) || (rc = dry.upload(ry, h->st)))
             return rc;
-        k_pw_expand<<<ceil_div((n / 3) * mm, 256), 256, 0, h->st>>>(nx, ny, nz, h->grid.dx, mm, dU.p, dW.p, dkx.p,
+        k_pw_expand<<<ceil_div((n / 3) * sk_columns(mm), 256), 256, 0, h->st>>>(nx, ny, nz, h->grid.dx, mm, dU.p, dW.p, dkx.p,
                                                                      dky.p, drx.p, dry.p, h->Rn.p, sk_columns(mm));
-        k_hetfld<<<152 * 8, 256, 0, h->st>>>(n, mm, h->irptr.p, h->jcptr.p, h->a.p, h->abg.p, h->Rn.p, sk_columns(mm),
-                                             (double2 *)d_F + (long long)c0 * n);
+        if (h->epA.p && sk_columns(mm) >= 8) {
+            residual(h, h->st, mm, h->Rn.p, nullptr, h->Xn.p, false);
+            to_columns(h, h->st, mm, h->Xn.p, (double2 *)d_F + (long long)c0 * n);
+        } else {
+            k_hetfld<<<152 * 8, 256, 0, h->st>>>(n, mm, h->irptr.p, h->jcptr.p, h->a.p, h->abg.p, h->Rn.p,
+                                                 sk_columns(mm), (double2 *)d_F + (long long)c0 * n);
+        }
         if (d_U0) to_columns(h, h->st, mm, h->Rn.p, (double2 *)d_U0 + (long long)c0 * n);
         WT_CUDA(cudaGetLastError());
         WT_CUDA(cudaStreamSynchronize(h->st));
@@ -1141,7 +1207,8 @@ int wt3d_apply(wt3d_solver *h, int nrhs, const double _Complex *X, double _Compl
     const long long n = h->n;
     StreamBuf<double2> dX;   // per-call, in stream order (see StreamBuf)
     int rc = dX.alloc((size_t)n * nrhs, h->st);
-    if (rc) return rc;
+    if (rc || (rc = product_prepare(h, h->st, nrhs, false, nullptr))) return rc;
+    ProductDone done{h};
     WT_CUDA(cudaMemcpyAsync(dX.p, X, sizeof(double2) * n * nrhs, cudaMemcpyHostToDevice, h->st));
     for (int c0 = 0; c0 < nrhs; c0 += MAXRHS) {
         int m = std::min(MAXRHS, nrhs - c0);
@@ -1161,6 +1228,8 @@ int wt3d_apply_device(wt3d_solver *h, int nrhs, const void *d_X, void *d_Y)
     if (int rc0 = after_legacy(h, h->st)) return rc0;
     if (!h->have_values) { set_error("no operator"); return WT3D_ERR_STATE; }
     const long long n = h->n;
+    if (int rc = product_prepare(h, h->st, nrhs, false, nullptr)) return rc;
+    ProductDone done{h};
     for (int c0 = 0; c0 < nrhs; c0 += MAXRHS) {
         int m = std::min(MAXRHS, nrhs - c0);
         to_rows(h, h->st, m, (const double2 *)d_X + (long long)c0 * n, h->Xn.p);

@@ -100,7 +100,7 @@ public:
     // flops from which a factorisation's update goes to the tensor-core kernel
     static constexpr double TC_MIN_FLOPS = 1e9;
     // units a launch of k_skinny is cut into, and the shortest K of a unit
-    static constexpr int SK_SLOTS = 152 * 4, SK_KMIN = 64;
+    static constexpr int SK_SLOTS = 152 * 8, SK_KMIN = 64;
     // outer block width of the two-level LU (WT3D_WB: a multiple of KB, 512 by default)
     const int WB = [] {
         const char *e = getenv("WT3D_WB");

@@ -1,0 +1,421 @@
+// Products of the grid's operator with 8 to 32 complex128 right-hand sides, on
+// the tensor cores, to FP64 accuracy or better.
+//
+// The FP64 pipe (2 FMA per cycle and SM) bounds the residual r = b - A x: 8.8 ms
+// for 32 columns of 64x64x48, a third of a refinement step, where reading the
+// operator takes 0.1 ms.  Here every operand is an integer of 62 bits and sign
+// times a power of two (per row of A; per column and 6 x 6 x 6 block of nodes of
+// X, so that a quiet region is not held to the scale of a source elsewhere), cut
+// into eight signed digits of 8 bits.  Before that the columns of A are brought to
+// a largest entry in [1, 2) by powers of two, and the rows of X multiplied by
+// them: Dirichlet rows carry a unit diagonal next to stiffness entries of 1e8, and
+// in a conjugate-transpose solve their unknowns are 1e8 times the others.  A product of two digits is an integer of
+// at most 2^14; the sums of 162 products over up to seven digit pairs of equal
+// weight stay below 2^24, so FP16 tensor-core products with FP32 accumulation are
+// exact (the error-free splitting of Ozaki, Ogita, Oishi and Rump, 2012).  The 43
+// digit pairs down to weight 2^-64 of the leading one are summed; what is left
+// out is of the order of 2^-65 of the largest |a| |x| of a row's block, against
+// 2^-53 per operation of an FP64 sum.  The integers are added in 64 bits and
+// rounded once.
+//
+// The integers' unit is set by the largest |a| of a row times the largest |x| of
+// the block, so a row all of whose products are far smaller than that would lose
+// bits: such rows (at the outer corners of the absorbing layers, where the operator
+// falls off by orders of magnitude within a block; 0.2 % of the rows at 40^3) take
+// the plain FP64 sum, and so do rows and columns with an infinity or a NaN.  Rows
+// with one entry (Dirichlet rows) are one FP64 product.
+//
+// Errors against extended precision, 2-norm over the product, 13x12x11: random
+// fields 4.7e-17 (FP64 kernel 1.6e-16), wave fields 4.3e-17 (1.4e-15).  32 columns
+// of 64x64x48 in 3.5 ms instead of 8.8; the digits of the operator, 0.6 ms, are
+// made once per call.
+#pragma once
+#include "refine_kernels.cuh"
+#include <cuda_fp16.h>
+
+namespace wt3d {
+
+constexpr int EP_SLOTS = 88;      // complex entries per row: 27 neighbours x 3, padded to 11 steps of 8
+constexpr int EP_T = 4, EP_H = EP_T + 2;   // nodes of a block and of its halo per axis
+constexpr int EP_COLS = 16;       // columns per CTA (the M of the tensor-core shape)
+constexpr int EP_ES = EP_COLS + 2;   // row of one entry in shared memory (16-byte units; four entries on different banks)
+constexpr int EP_THREADS = 512;
+constexpr int EP_ENTRIES = EP_H * EP_H * EP_H * 3;
+constexpr size_t EP_SMEM = (size_t)EP_ENTRIES * EP_ES * 16;
+constexpr unsigned long long EP_BIAS = 0x8080808080808080ull;   // digit + 128 in every byte
+constexpr int EP_BAD = 1 << 20;   // exponent of rows and columns with infinities or NaNs
+constexpr int EP_NONE = -(1 << 20);   // ... of all zeros
+constexpr int EP_SINGLE = 1 << 21;   // ... of rows with one entry: plus its position in the row
+constexpr int EP_LOSS = 8;        // bits a row may lose: the error stays at that of an FP64 sum
+
+// The operator of a product: A, A^H, or B - A (the sources of an incident field).
+struct ProductOp {
+    const int *irptr, *jcptr, *tpos;
+    const double2 *a, *b;         // b: with b != nullptr the operator is b - a
+    int adjoint;
+    __device__ __forceinline__ double2 at(long long k) const
+    {
+        if (b) {
+            const double2 u = b[k], v = a[k];
+            return make_double2(u.x - v.x, u.y - v.y);
+        }
+        if (adjoint) {
+            const double2 v = a[tpos[k]];
+            return make_double2(v.x, -v.y);
+        }
+        return a[k];
+    }
+};
+
+// exponent field of v, EP_NONE for zero
+__device__ __forceinline__ int ep_exponent(double v)
+{
+    const int e = (__double2hiint(v) >> 20) & 0x7ff;
+    return e == 0x7ff ? EP_BAD : zero_bits(v) ? EP_NONE : max(e, 1);
+}
+__device__ __forceinline__ int ep_exponent(double2 v) { return max(ep_exponent(v.x), ep_exponent(v.y)); }
+
+// v 2^(s + 62 - (E - 1022)) rounded to an integer, plus the digits' bias; E the
+// largest of the exponents + s of v's row or column, so that the integer is below
+// 2^62
+__device__ __forceinline__ unsigned long long ep_quantise(double v, int s, int E)
+{
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+    const int e = (int)(bits >> 52) & 0x7ff;
+    unsigned long long m = bits & 0xfffffffffffffull;
+    if (e) m |= 0x10000000000000ull;
+    const int sh = 9 - (E - (max(e, 1) + s));
+    unsigned long long q = sh >= 0 ? m << min(sh, 9) : sh > -60 ? (m + (1ull << (-sh - 1))) >> -sh : 0ull;
+    if ((long long)bits < 0) q = 0ull - q;
+    return q + EP_BIAS;
+}
+
+// pe[j]: exponent of column j of the operator (1023, that is no scaling, for a
+// column of zeros or with infinities or NaNs): a warp per row of its transpose
+__global__ void __launch_bounds__(256) k_column_exponents(long long n, ProductOp op, int *__restrict__ pe)
+{
+    const long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (r >= n) return;
+    int E = EP_NONE;
+    for (int k = op.irptr[r] + lane; k < op.irptr[r + 1]; k += 32) {
+        const int j = op.adjoint ? k : op.tpos[k];   // entry (column r) of A, of A^H: row r of A
+        double2 v = op.a[j];
+        if (op.b) { const double2 u = op.b[j]; v = make_double2(u.x - v.x, u.y - v.y); }
+        E = max(E, ep_exponent(v));
+    }
+    E = __reduce_max_sync(0xffffffffu, E);
+    if (lane == 0) pe[r] = E == EP_NONE || E == EP_BAD ? 1023 : E;
+}
+
+// digit i (0: the most significant) of a biased pair as two FP16 values (re, im):
+// bytes 0x64xx are 1024 + xx; mul (1, 1) or (1, -1) and add -1152 mul give the digits
+__device__ __forceinline__ uint32_t ep_digit(const ulonglong2 &q, int i, __half2 mul, __half2 add)
+{
+    const uint32_t wr = i < 4 ? (uint32_t)(q.x >> 32) : (uint32_t)q.x, wi = i < 4 ? (uint32_t)(q.y >> 32) : (uint32_t)q.y;
+    const int b = 3 - (i & 3);
+    uint32_t t = __byte_perm(wr, wi, b | (b << 4) | ((4 + b) << 8) | ((4 + b) << 12));
+    t = (t & 0x00ff00ffu) | 0x64006400u;
+    const __half2 h = __hfma2(*reinterpret_cast<__half2 *>(&t), mul, add);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+
+// bmax[tile]: largest column exponent in the tile's block with halo: a warp per tile
+__global__ void __launch_bounds__(256) k_block_exponents(int nx, int ny, int nz, const int *__restrict__ pe,
+                                                         int *__restrict__ bmax)
+{
+    const int tz = (nz + EP_T - 1) / EP_T, tx = (nx + EP_T - 1) / EP_T, ty = (ny + EP_T - 1) / EP_T;
+    const long long b = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (b >= (long long)tz * tx * ty) return;
+    const int bz = (int)(b % tz) * EP_T, bx = (int)((b / tz) % tx) * EP_T, by = (int)(b / ((long long)tz * tx)) * EP_T;
+    int E = 0;
+    for (int e = threadIdx.x & 31; e < EP_ENTRIES; e += 32) {
+        const int h = e / 3, z = bz + h % EP_H - 1, x = bx + (h / EP_H) % EP_H - 1, y = by + h / (EP_H * EP_H) - 1;
+        if (z < 0 || z >= nz || x < 0 || x >= nx || y < 0 || y >= ny) continue;
+        E = max(E, pe[3 * (z + (long long)nz * (x + (long long)nx * y)) + e % 3]);
+    }
+    E = __reduce_max_sync(0xffffffffu, E);
+    if ((threadIdx.x & 31) == 0) bmax[b] = E;
+}
+
+// Rows of the operator as digits: a warp per node; row q of node g holds its 27
+// neighbours (dy, dx, dz) x 3 components at aq[(3 g + q) EP_SLOTS ..], zeros where
+// there is no neighbour, and the row's exponent in aexp.
+__global__ void __launch_bounds__(256) k_operator_digits(int nx, int ny, int nz, ProductOp op,
+                                                         const int *__restrict__ pe, const int *__restrict__ bmax,
+                                                         ulonglong2 *__restrict__ aq,
+                                                         int *__restrict__ aexp)
+{
+    const long long nn = (long long)nx * ny * nz;
+    const long long g = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (g >= nn) return;
+    const int iz = (int)(g % nz), ix = (int)((g / nz) % nx), iy = (int)(g / ((long long)nz * nx));
+    const int z0 = max(iz - 1, 0), z1 = min(iz + 1, nz - 1), x0 = max(ix - 1, 0), x1 = min(ix + 1, nx - 1),
+              y0 = max(iy - 1, 0);
+    const int y1 = min(iy + 1, ny - 1);
+    const long long k0 = op.irptr[3 * g];
+    const int len = op.irptr[3 * g + 1] - (int)k0;
+    const int bm = bmax[iz / EP_T + (long long)((nz + EP_T - 1) / EP_T) * (ix / EP_T + (long long)((nx + EP_T - 1) / EP_T) * (iy / EP_T))];
+    int pos[3], sc[3];   // the lane's slots lane + 32 j: position in the row, -1 for none; column scaling
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        const int s = lane + 32 * j, nb = s / 3, c = s % 3;
+        const int y = iy + nb / 9 - 1, x = ix + (nb / 3) % 3 - 1, z = iz + nb % 3 - 1;
+        pos[j] = (s < 81 && y >= y0 && y <= y1 && x >= x0 && x <= x1 && z >= z0 && z <= z1)
+                     ? (((y - y0) * (x1 - x0 + 1) + (x - x0)) * (z1 - z0 + 1) + (z - z0)) * 3 + c
+                     : -1;
+        sc[j] = pos[j] >= 0 ? 1023 - pe[op.jcptr[k0 + pos[j]]] : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        double2 v[3];
+        int E = EP_NONE, S = EP_NONE, cnt = 0, at = -1;   // largest exponent scaled, as it is; nonzero entries
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            v[j] = pos[j] >= 0 ? op.at(k0 + (long long)q * len + pos[j]) : make_double2(0, 0);
+            const int e = ep_exponent(v[j]);
+            E = max(E, e == EP_BAD ? e : e + sc[j]);
+            S = max(S, e);
+            if (e != EP_NONE) {
+                cnt++;
+                at = pos[j];
+            }
+        }
+        E = __reduce_max_sync(0xffffffffu, E);
+        S = __reduce_max_sync(0xffffffffu, S);
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        at = __reduce_max_sync(0xffffffffu, at);
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const int s = lane + 32 * j;
+            if (s < EP_SLOTS)
+                aq[(3 * g + q) * EP_SLOTS + s] = make_ulonglong2(ep_quantise(v[j].x, sc[j], E), ep_quantise(v[j].y, sc[j], E));
+        }
+        if (lane == 0)
+            aexp[3 * g + q] = E >= EP_BAD || E < EP_NONE / 2 ? E
+                              : cnt == 1 ? EP_SINGLE + at
+                              : E + bm - S - 1023 > EP_LOSS ? EP_BAD : E;
+    }
+}
+
+__device__ __forceinline__ void ep_mma(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2])
+{
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// an integer of magnitude below 2^51 as a double
+__device__ __forceinline__ double ep_double(long long v)
+{
+    return __longlong_as_double(v + 0x4338000000000000ll) - 6755399441055744.0;
+}
+
+// R = B - A X, with the column norms of R and B added to nr and nb as k_residual
+// does it; with B null R = A X, no norms.  One CTA per 4 x 4 x 4 nodes and
+// 16 columns: the block's X with its halo goes into shared memory as biased integers; then a
+// warp per node (four in turn) runs the node's three rows as the N = 8 side (re and
+// im of each row, two unused) and the columns as the M = 16 side of
+// m16n8k16 products, 8 entries per step, making the digits of both sides in
+// registers.
+template <int NC>
+__global__ void __launch_bounds__(EP_THREADS, 1)
+    k_product_tc(int nx, int ny, int nz, ProductOp op, const ulonglong2 *__restrict__ aq, const int *__restrict__ aexp,
+                 const int *__restrict__ pe, const double2 *__restrict__ X, const double2 *__restrict__ B, double2 *__restrict__ R,
+                 double *__restrict__ nr, double *__restrict__ nb)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    ulonglong2 *Xq = reinterpret_cast<ulonglong2 *>(smraw);   // EP_ENTRIES x EP_ES
+    __shared__ int cexp[EP_COLS], off[EP_SLOTS];
+    __shared__ double red[2][EP_THREADS / 32][EP_COLS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tz = (nz + EP_T - 1) / EP_T, tx = (nx + EP_T - 1) / EP_T;
+    // the column groups of a tile follow one another: the second finds A in L2
+    constexpr int NG = (NC + EP_COLS - 1) / EP_COLS;
+    const long long tile = blockIdx.x / NG;
+    const int bz = (int)(tile % tz) * EP_T, bx = (int)((tile / tz) % tx) * EP_T,
+              by = (int)(tile / ((long long)tz * tx)) * EP_T;
+    const int c0 = EP_COLS * (int)(blockIdx.x % NG);
+    // the tile's operator rows are read one step ahead of their use, which does not
+    // cover DRAM: on their way to L2 while X is loaded (runs of 4 nodes along z)
+    for (int q = tid; q < EP_T * EP_T * (EP_T * 3 * EP_SLOTS * 16 / 128); q += EP_THREADS) {
+        constexpr int LINES = EP_T * 3 * EP_SLOTS * 16 / 128;
+        const int ix = bx + (q / LINES) % EP_T, iy = by + q / (LINES * EP_T);
+        const long long node = bz + (long long)nz * (ix + (long long)nx * iy);
+        const long long off = (3 * node * EP_SLOTS) * 16 + (long long)(q % LINES) * 128;
+        if (ix < nx && iy < ny && off < 3LL * nx * ny * nz * EP_SLOTS * 16)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char *>(aq) + off));
+    }
+    if (tid < EP_COLS) cexp[tid] = EP_NONE;
+    if (tid < EP_SLOTS) {
+        const int s = min(tid, 80), k = s / 3;
+        off[tid] = ((k % 3 + EP_H * ((k / 3) % 3 + EP_H * (k / 9))) * 3 + s % 3) * EP_ES;
+    }
+    __syncthreads();
+    // X with halo, as stored; the columns' exponents
+    {
+        const int c = tid % EP_COLS;
+        const bool col = c0 + c < NC;
+        int E = EP_NONE;
+        auto row_of = [&](int e) -> long long {   // entry's row of X, -1 outside the grid
+            const int h = e / 3;
+            const int z = bz + h % EP_H - 1, x = bx + (h / EP_H) % EP_H - 1, y = by + h / (EP_H * EP_H) - 1;
+            if (z < 0 || z >= nz || x < 0 || x >= nx || y < 0 || y >= ny) return -1;
+            return 3 * (z + (long long)nz * (x + (long long)nx * y)) + e % 3;
+        };
+#pragma unroll 4
+        for (int e = tid / EP_COLS; e < EP_ENTRIES; e += EP_THREADS / EP_COLS) {
+            const long long r = row_of(e);
+            double2 v = make_double2(0, 0);
+            if (col && r >= 0) {
+                v = X[r * NC + c0 + c];
+                const int x = ep_exponent(v);
+                E = max(E, x == EP_BAD ? x : x + pe[r] - 1023);
+            }
+            Xq[e * EP_ES + c] = make_ulonglong2((unsigned long long)__double_as_longlong(v.x),
+                                                (unsigned long long)__double_as_longlong(v.y));
+        }
+        atomicMax(&cexp[c], E);
+        __syncthreads();
+        E = cexp[c];
+        for (int e = tid / EP_COLS; e < EP_ENTRIES; e += EP_THREADS / EP_COLS) {
+            const long long r = row_of(e);
+            const int s = r >= 0 ? pe[r] - 1023 : 0;
+            const ulonglong2 v = Xq[e * EP_ES + c];
+            Xq[e * EP_ES + c] = make_ulonglong2(ep_quantise(__longlong_as_double((long long)v.x), s, E),
+                                                ep_quantise(__longlong_as_double((long long)v.y), s, E));
+        }
+    }
+    __syncthreads();
+    const int g = lane >> 2, t = lane & 3;   // fragment coordinates
+    // this lane's operand of A: row q = g / 2, (ar, -ai) for its real part, (ai, ar)
+    // for its imaginary part; g = 6, 7 are the unused ones
+    const int qa = g >> 1;
+    const bool part = g & 1, live = g < 6;
+    const __half2 one = __floats2half2_rn(1.f, 1.f), one_off = __floats2half2_rn(-1152.f, -1152.f);
+    const __half2 amul = part ? one : __floats2half2_rn(1.f, -1.f);
+    const __half2 aadd = part ? one_off : __floats2half2_rn(-1152.f, 1152.f);
+    double sr[2] = {0, 0}, sb[2] = {0, 0};
+    for (int ln = warp; ln < EP_T * EP_T * EP_T; ln += EP_THREADS / 32) {
+        const int lz = ln % EP_T, lx = (ln / EP_T) % EP_T, ly = ln / (EP_T * EP_T);
+        const int iz = bz + lz, ix = bx + lx, iy = by + ly;
+        if (iz >= nz || ix >= nx || iy >= ny) continue;
+        const long long node = iz + (long long)nz * (ix + (long long)nx * iy);
+        const ulonglong2 *ar = aq + (3 * node + (live ? qa : 0)) * EP_SLOTS + t;
+        const ulonglong2 *xb = Xq + (size_t)((lz + EP_H * (lx + EP_H * ly)) * 3) * EP_ES + g;
+        float acc[11][4];   // digit pairs of weight 0 .. 6, 7 and 8 (two halves each: sums below 2^24)
+#pragma unroll
+        for (int s = 0; s < 11; s++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[s][j] = 0.f;
+        ulonglong2 p0 = ar[0], p1 = ar[4];
+#pragma unroll 1
+        for (int st = 0; st < EP_SLOTS / 8; st++) {
+            ulonglong2 a0 = p0, a1 = p1;
+            if (st + 1 < EP_SLOTS / 8) { p0 = ar[8 * st + 8]; p1 = ar[8 * st + 12]; }
+            if (part) { a0 = make_ulonglong2(a0.y, a0.x); a1 = make_ulonglong2(a1.y, a1.x); }
+            const ulonglong2 *e0 = xb + off[8 * st + t], *e1 = xb + off[8 * st + 4 + t];
+            const ulonglong2 x0 = e0[0], x1 = e0[8], x2 = e1[0], x3 = e1[8];
+            uint32_t ad[8][2];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                ad[j][0] = live ? ep_digit(a0, j, amul, aadd) : 0u;
+                ad[j][1] = live ? ep_digit(a1, j, amul, aadd) : 0u;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                uint32_t xd[4];
+                xd[0] = ep_digit(x0, i, one, one_off);
+                xd[1] = ep_digit(x1, i, one, one_off);
+                xd[2] = ep_digit(x2, i, one, one_off);
+                xd[3] = ep_digit(x3, i, one, one_off);
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (i + j < 9) ep_mma(acc[i + j < 7 ? i + j : 2 * (i + j) - 7 + (i < 4 ? 0 : 1)], xd, ad[j]);
+            }
+        }
+        if (t < 3) {
+            // entries (column g or g + 8, row q = t): re and im
+            const long long row = 3 * node + t;
+            const int Ea = aexp[row];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int cl = g + 8 * h, c = c0 + cl;
+                if (c >= NC) continue;
+                const int Ex = cexp[cl];
+                double2 v;
+                if (Ex != EP_BAD && Ea >= EP_SINGLE) {
+                    const long long k = op.irptr[row] + (Ea - EP_SINGLE);
+                    const double2 av = op.at(k), x = X[(long long)op.jcptr[k] * NC + c];
+                    v = make_double2(fma(av.x, x.x, -av.y * x.y), fma(av.x, x.y, av.y * x.x));
+                } else if (Ea != EP_BAD && Ex != EP_BAD) {
+                    double w[2];
+#pragma unroll
+                    for (int p = 0; p < 2; p++) {
+                        long long hi = 0, lo = 0;
+#pragma unroll
+                        for (int s = 0; s < 4; s++) hi = hi * 256 + __float2int_rn(acc[s][2 * h + p]);
+#pragma unroll
+                        for (int s = 4; s < 7; s++) lo = lo * 256 + __float2int_rn(acc[s][2 * h + p]);
+                        lo = lo * 256 + __float2int_rn(acc[7][2 * h + p]) + __float2int_rn(acc[8][2 * h + p]);
+                        // weight 8: rounded to the unit of lo, 2^-68 of the leading product
+                        lo += (__float2int_rn(acc[9][2 * h + p]) + __float2int_rn(acc[10][2 * h + p]) + 128) >> 8;
+                        w[p] = fma(ep_double(hi), 4294967296.0, ep_double(lo));
+                    }
+                    // unit of the integers: 2^56 from the digits, 2^(E - 1022 - 62) of each side
+                    if (Ea == EP_NONE || Ex == EP_NONE) {
+                        v = make_double2(0, 0);
+                    } else {
+                        const int e = Ea + Ex - 2 * (1022 + 62) + 56;
+                        if (e > -900 && e < 900) {
+                            const double f = __hiloint2double((e + 1023) << 20, 0);
+                            v = make_double2(w[0] * f, w[1] * f);
+                        } else {
+                            v = make_double2(scalbn(w[0], e), scalbn(w[1], e));
+                        }
+                    }
+                } else {
+                    v = make_double2(0, 0);
+                    const long long k0 = op.irptr[row];
+                    const int len = op.irptr[row + 1] - (int)k0;
+#pragma unroll 4
+                    for (int k = 0; k < len; k++) {
+                        const double2 av = op.at(k0 + k), x = X[(long long)op.jcptr[k0 + k] * NC + c];
+                        v.x = fma(av.x, x.x, fma(-av.y, x.y, v.x));
+                        v.y = fma(av.x, x.y, fma(av.y, x.x, v.y));
+                    }
+                }
+                const double2 b = B ? B[row * NC + c] : make_double2(0, 0);
+                const double2 r = B ? make_double2(b.x - v.x, b.y - v.y) : v;
+                R[row * NC + c] = r;
+                if (B) {
+                    sr[h] = fma(r.x, r.x, fma(r.y, r.y, sr[h]));
+                    sb[h] = fma(b.x, b.x, fma(b.y, b.y, sb[h]));
+                }
+            }
+        }
+    }
+    if (!B) return;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            sr[h] += __shfl_xor_sync(0xffffffffu, sr[h], o);
+            sb[h] += __shfl_xor_sync(0xffffffffu, sb[h], o);
+        }
+        if (t == 0) {
+            red[0][warp][g + 8 * h] = sr[h];
+            red[1][warp][g + 8 * h] = sb[h];
+        }
+    }
+    __syncthreads();
+    if (tid < 2 * EP_COLS) {
+        const int h = tid / EP_COLS, c = tid % EP_COLS;
+        double s = 0;
+        for (int w = 0; w < EP_THREADS / 32; w++) s += red[h][w][c];
+        if (c0 + c < NC) atomicAdd((h ? nb : nr) + c0 + c, s);
+    }
+}
+
+}  // namespace wt3d

@@ -171,7 +171,8 @@ int haskgrn_host(const wt3d_layered1d &M, double omega, double ain, int s_wave, 
     return WT3D_OK;
 }
 
-// u0 on the grid for m sources; U0 row-major n x ld (complex128).
+// u0 on the grid for m sources; U0 row-major n x ld (complex128), zeros in columns
+// m .. ld - 1.
 __global__ void k_pw_expand(int nx, int ny, int nz, double dx, int m, const double2 *__restrict__ Uz,
                             const double2 *__restrict__ Wz, const double *__restrict__ kx,
                             const double *__restrict__ ky, const double *__restrict__ rx,
@@ -179,9 +180,13 @@ __global__ void k_pw_expand(int nx, int ny, int nz, double dx, int m, const doub
 {
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long nn = (long long)nx * ny * nz;
-    if (q >= nn * m) return;
-    const long long g = q / m;
-    const int j = (int)(q % m);
+    if (q >= nn * ld) return;
+    const long long g = q / ld;
+    const int j = (int)(q % ld);
+    if (j >= m) {
+        for (int c = 0; c < 3; c++) U0[(3 * g + c) * ld + j] = make_double2(0, 0);
+        return;
+    }
     const int iz = (int)(g % nz), ix = (int)((g / nz) % nx), iy = (int)(g / ((long long)nz * nx));
     const double ph = kx[j] * (ix * dx) + ky[j] * (iy * dx);
     double s, c;
