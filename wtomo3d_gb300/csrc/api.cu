@@ -669,9 +669,13 @@ void handle_bytes(const Symbolic &S, long long nnz, int prec, double *out)
 {
     const double n = (double)S.n, nn = n / 3, sz = prec == WT3D_PREC_MIXED ? 8.0 : 16.0;
     long long ninv = 0;
-    for (const Front &F : S.fronts) ninv += inv_entries(F.p);
+    double epos = 0;   // positions of the children's borders in their parents
+    for (const Front &F : S.fronts) {
+        ninv += prec == WT3D_PREC_MIXED ? inv_entries<float>(F.p) : inv_entries<double>(F.p);
+        for (int s = 0; s < F.nchild; s++) epos += F.nf();
+    }
     const double engine = (double)S.fac_total * sz + 3 * n * MAXRHS * sz + (double)ninv * sz + 2 * n * 4 +
-                          (double)(S.border.size() + S.rel.size()) * 4 + (double)S.fronts.size() * sizeof(FrontDev) +
+                          (double)S.border.size() * 4 + epos * 4 + (double)S.fronts.size() * sizeof(FrontDev) +
                           (double)nnz * 8 + n * 8;
     const double api = (n + 1) * 4 + (double)nnz * (4 + 16 + 4) + n * 4 + 3 * n * MAXRHS * 16 + nn * (12 + 32 + 8);
     out[0] = engine + api;
@@ -1791,6 +1795,43 @@ extern "C" int wt3d_debug_fetch(wt3d_solver *h, int what, void *out, long long c
     } else {
         return WT3D_ERR_ARG;
     }
+    return WT3D_OK;
+}
+
+// One product of the substitution passes on host complex64 arrays, as its kernel
+// computes it: out (M x nc) = op(A) in (K x nc), op(A) = A (M x K) or, with herm,
+// A^H (A K x M), rows lda apart; tri 1 or 2: A is a packed block inverse (M = K) and
+// its lower (unit) or upper triangle is meant.  K is cut into units of chunk rows.
+extern "C" int wt3d_debug_skinny(int herm, int tri, int M, int K, int nc, int chunk, const void *A, int lda,
+                                 const void *in, void *out)
+{
+    if (nc != sk_columns(nc) || chunk < 32 || chunk % 32 || chunk > SK_KMAX || (tri && M != K)) return WT3D_ERR_ARG;
+    const size_t na = (size_t)(herm ? K : M) * lda;
+    DevVec<cx<float>> dA, dB, dC;
+    DevVec<SkUnit> du;
+    int rc;
+    if ((rc = dA.alloc(na)) || (rc = dB.alloc((size_t)K * nc)) || (rc = dC.alloc((size_t)M * nc))) return rc;
+    WT_CUDA(cudaMemcpy(dA.p, A, sizeof(cx<float>) * na, cudaMemcpyHostToDevice));
+    WT_CUDA(cudaMemcpy(dB.p, in, sizeof(cx<float>) * K * nc, cudaMemcpyHostToDevice));
+    WT_CUDA(cudaMemset(dC.p, 0, sizeof(cx<float>) * M * nc));
+    std::vector<SkUnit> hu;
+    for (int r0 = 0; r0 < M; r0 += SK_M) {
+        int k0 = 0, k1 = K;
+        if (tri) ((tri == 1) != (herm != 0) ? k1 : k0) = (tri == 1) != (herm != 0) ? std::min(K, r0 + SK_M) : r0;
+        for (int k = k0; k < k1; k += chunk) {
+            SkUnit u{};
+            u.A = herm ? dA.p + (size_t)k * lda + r0 : dA.p + (size_t)r0 * lda + k;
+            u.b0 = k; u.c0 = r0; u.lda = lda; u.M = std::min(SK_M, M - r0); u.K = std::min(chunk, k1 - k);
+            u.flags = (tri == 1 ? SK_LOWER : tri == 2 ? SK_UPPER : 0) | (k1 - k0 > chunk ? SK_ATOM : 0);
+            u.d = k - r0;
+            hu.push_back(u);
+        }
+    }
+    if ((rc = du.upload(hu))) return rc;
+    Engine<float>::sk_attributes();
+    Engine<float>::sk_launch(nc, herm != 0, du.p, (int)hu.size(), dB.p, dC.p, 0);
+    WT_CUDA(cudaGetLastError());
+    WT_CUDA(cudaMemcpy(out, dC.p, sizeof(cx<float>) * M * nc, cudaMemcpyDeviceToHost));
     return WT3D_OK;
 }
 

@@ -45,6 +45,7 @@ struct Schedule {
     std::vector<GemmTask<T>> hgemm;                           // host copies while the schedule is built
     std::vector<GemmUnit> hunit;
     DevVec<EATask> ea;
+    DevVec<EAUnit> eau;
     DevVec<InvTask> inv;                                      // block-inverse columns
     DevVec<SkUnit> sk;                                        // units of the substitution products
     std::vector<std::vector<GemmTask<float>>> tc_pending;   // tensor-core task lists, built after allocation
@@ -84,7 +85,7 @@ public:
     std::shared_ptr<FactorWorkspace<T>> ws;
     DevVec<int> ipiv, border;
     DevVec<int> gord;   // per pivot position (new ordering): the row that the interchanges leave there
-    DevVec<int> rel;
+    DevVec<int> eapos;   // per child: border index of every row of the parent front, -1 for none (k_extend_add)
     DevVec<FrontDev> fr;
     std::vector<FrontDev> hfr;
     DevVec<long long> map;
@@ -99,6 +100,7 @@ public:
     static constexpr long long BAND_TWO = 152 * 4 * 32;
     // flops from which a factorisation's update goes to the tensor-core kernel
     static constexpr double TC_MIN_FLOPS = 1e9;
+    static constexpr int SBW = SB<T>;   // columns per diagonal block of the substitutions
     // units a launch of k_skinny is cut into, and the shortest K of a unit
     static constexpr int SK_SLOTS = 152 * 8, SK_KMIN = 64;
     // outer block width of the two-level LU (WT3D_WB: a multiple of KB, 512 by default)
@@ -129,7 +131,7 @@ public:
         size_t sw = 0;   // the solve schedules' tall-skinny workspaces
         for (const auto &m : ssched)
             for (const auto &kv : m) sw += kv.second->tsws.n * sizeof(float);
-        return (fac.n + X.n + Z.n + Y.n + binv.n) * sizeof(cx<T>) + (ipiv.n + border.n + rel.n + gord.n) * 4 +
+        return (fac.n + X.n + Z.n + Y.n + binv.n) * sizeof(cx<T>) + (ipiv.n + border.n + eapos.n + gord.n) * 4 +
                fr.n * sizeof(FrontDev) +
                map.n * 8 + scale.n * 8 + own_tcws.n * sizeof(float) + sw;
     }
@@ -172,7 +174,6 @@ public:
         if ((rc = X.alloc(nx)) || (rc = Z.alloc(nx)) || (rc = Y.alloc(nx))) return rc;
         if ((rc = ipiv.alloc(sym.n))) return rc;
         if ((rc = border.upload(sym.border))) return rc;
-        if ((rc = rel.upload(sym.rel))) return rc;
         if ((rc = map.upload(hmap))) return rc;
         if ((rc = npert.alloc(1))) return rc;
         if ((rc = maxabs.alloc(1))) return rc;
@@ -186,7 +187,7 @@ public:
         for (size_t f = 0; f < h.size(); f++) {
             const Front &F = sym.fronts[f];
             h[f].inv = ninv;
-            ninv += inv_entries(F.p);
+            ninv += inv_entries<T>(F.p);
             h[f].fac = F.fac_off;
             h[f].upd = F.upd_off;
             h[f].border = F.border_off;
@@ -213,11 +214,7 @@ public:
                                  (int)BandCfg<T, 1>::smem);
             cudaFuncSetAttribute(k_bands<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)BandCfg<T, 2>::smem);
-            sk_attr<1>();
-            sk_attr<4>();
-            sk_attr<8>();
-            sk_attr<16>();
-            sk_attr<32>();
+            sk_attributes();
         });
         return build_factor_schedule();
     }
@@ -230,6 +227,14 @@ public:
         if (side) cudaStreamDestroy(side);
     }
 
+    static void sk_attributes()
+    {
+        sk_attr<1>();
+        sk_attr<4>();
+        sk_attr<8>();
+        sk_attr<16>();
+        sk_attr<32>();
+    }
     template <int NC>
     static void sk_attr()
     {
@@ -413,8 +418,8 @@ public:
         const size_t i0 = hi.size();
         for (int f : fl) {
             const int p = S->fronts[f].p;
-            for (int c0 = 0; c0 < p; c0 += SB) {
-                const int end = std::min(c0 + SB, p), w = end - c0, nt = (w + KB - 1) / KB;
+            for (int c0 = 0; c0 < p; c0 += SBW) {
+                const int end = std::min(c0 + SBW, p), w = end - c0, nt = (w + KB - 1) / KB;
                 if (end - 1 < k0 || end - 1 >= k1) continue;
                 for (int up = 0; up < 2; up++)
                     for (int t = 0; t < nt; t++) {
@@ -427,7 +432,7 @@ public:
         // longest chains first
         std::stable_sort(hi.begin() + i0, hi.end(), [this](const InvTask &a, const InvTask &b) {
             auto len = [this](const InvTask &x) {
-                return x.upper ? x.t : (std::min(SB, S->fronts[x.f].p - x.c0) + KB - 1) / KB - 1 - x.t;
+                return x.upper ? x.t : (std::min(SBW, S->fronts[x.f].p - x.c0) + KB - 1) / KB - 1 - x.t;
             };
             return len(a) > len(b);
         });
@@ -447,6 +452,8 @@ public:
         std::vector<BandTask> hb;
         std::vector<GemmTask<T>> hg;
         std::vector<EATask> he;
+        std::vector<EAUnit> heu;
+        std::vector<int> hpos;
         std::vector<InvTask> hi;
         Schedule<T> *psc = sc.get();
         const Symbolic &sym = *S;
@@ -471,33 +478,32 @@ public:
         const int nlev = (int)sym.levels.size();
         for (int L = nlev - 1; L >= 0; L--) {
             const std::vector<int> &fl = sym.levels[L];
-            // zero this level's update region
-            long long usz = 0;
-            for (int f : fl) usz += (long long)sym.fronts[f].b * sym.fronts[f].b;
-            if (usz > 0) {
-                cx<T> *up = U[L & 1];
-                size_t bytes = usz * sizeof(cx<T>);
-                sc->launches.push_back({[up, bytes](cudaStream_t st) { cudaMemsetAsync(up, 0, bytes, st); }, LK_MEMSET, 0});
-            }
-            // extend-add, one child slot at a time (siblings overlap in the parent)
-            for (int slot = 0; slot < 2; slot++) {
-                size_t b0 = he.size();
-                long long rows = 0;
+            // what the children left, into the factor pool and this level's update
+            // region (all of it: zeros where no child contributes)
+            {
+                const size_t u0 = heu.size();
                 for (int f : fl) {
                     const Front &P = sym.fronts[f];
-                    if (P.nchild <= slot) continue;
-                    int c = P.child[slot];
-                    if (sym.fronts[c].b == 0) continue;
-                    he.push_back(EATask{c, f, rows});
-                    rows += sym.fronts[c].b;
+                    EATask t{f, -1, -1, 0, 0};
+                    for (int s = 0; s < P.nchild; s++) {
+                        const Front &C = sym.fronts[P.child[s]];
+                        if (C.b == 0) continue;
+                        const size_t o = hpos.size();
+                        hpos.resize(o + P.nf(), -1);
+                        for (int i = 0; i < C.b; i++) hpos[o + sym.rel[C.border_off + i]] = i;
+                        (t.child0 < 0 ? t.child0 : t.child1) = P.child[s];
+                        (t.child1 < 0 ? t.pos0 : t.pos1) = (long long)o;
+                    }
+                    const int first = t.child0 < 0 ? P.p : 0;   // a leaf only has zeros to write
+                    for (int r = first; r < P.nf(); r += EA_ROWS) heu.push_back(EAUnit{(int)he.size(), r});
+                    he.push_back(t);
                 }
-                if (he.size() > b0) {
-                    int nt = (int)(he.size() - b0);
-                    sc->launches.push_back({[psc, this, b0, nt, rows](cudaStream_t st) {
-                        k_extend_add<T><<<ceil_div(rows * 32, 256), 256, 0, st>>>(
-                            psc->ea.p + b0, nt, rows, fr.p, rel.p, fac.p, ws->upd0.p, ws->upd1.p);
+                const unsigned nu = (unsigned)(heu.size() - u0);
+                if (nu)
+                    sc->launches.push_back({[psc, this, u0, nu](cudaStream_t st) {
+                        k_extend_add<T><<<nu, 32 * EA_ROWS, 0, st>>>(psc->ea.p, psc->eau.p + u0, fr.p, eapos.p, fac.p,
+                                                                     ws->upd0.p, ws->upd1.p);
                     }, LK_EXTEND_ADD, 0});
-                }
             }
             // Two-level blocked partial LU, level-synchronous over fronts.
             // Inner KB-wide panels: panel LU, row band (all columns right of
@@ -596,7 +602,7 @@ public:
         if ((rc = sc->gemm.upload(sc->hgemm)) || (rc = sc->unit.upload(sc->hunit))) return rc;
         sc->hgemm.clear();
         sc->hunit.clear();
-        if ((rc = sc->ea.upload(he))) return rc;
+        if ((rc = sc->ea.upload(he)) || (rc = sc->eau.upload(heu)) || (rc = eapos.upload(hpos))) return rc;
         if ((rc = sc->inv.upload(hi))) return rc;
         if ((rc = finish_tc(*sc))) return rc;
         fsched = std::move(sc);
@@ -698,7 +704,7 @@ public:
     }
 
     // Solve schedule for m right-hand sides: X (sources, new ordering) to Y.
-    // Every level of a sweep walks the SB-wide diagonal blocks of its fronts: the
+    // Every level of a sweep walks the SBW-wide diagonal blocks of its fronts: the
     // block inverse gives the block's unknowns, then the rows outside the block
     // are updated with them.
     Schedule<T> *solve_schedule(int m, bool adjoint)
@@ -710,19 +716,19 @@ public:
         const Symbolic &sym = *S;
         const int nlev = (int)sym.levels.size();
         auto block = [&](int f, int c0) {   // the packed inverse of block c0
-            return binv.p + hfr[f].inv + (long long)(c0 / SB) * SB * SB;
+            return binv.p + hfr[f].inv + (long long)(c0 / SBW) * SBW * SBW;
         };
         // ---- forward sweep: leaves to root ----
         for (int L = nlev - 1; L >= 0; L--) {
             const std::vector<int> &fl = sym.levels[L];
             int maxp = 0;
             for (int f : fl) maxp = std::max(maxp, sym.fronts[f].p);
-            for (int c0 = 0; c0 < maxp; c0 += SB) {
+            for (int c0 = 0; c0 < maxp; c0 += SBW) {
                 std::vector<Product> ap, up;
                 for (int f : fl) {
                     const Front &Fr = sym.fronts[f];
                     if (Fr.p <= c0) continue;
-                    const int nf = Fr.nf(), cend = std::min(c0 + SB, Fr.p), w = cend - c0, r = Fr.first + c0;
+                    const int nf = Fr.nf(), cend = std::min(c0 + SBW, Fr.p), w = cend - c0, r = Fr.first + c0;
                     const cx<T> *Pb = fac.p + Fr.fac_off;
                     const cx<T> *W = block(f, c0);
                     if (!adjoint) ap.push_back({W, inv_ld(w), w, w, gord.p + r, 0, nullptr, r, SK_LOWER});
@@ -764,12 +770,12 @@ public:
                               border.p + Fr.border_off, 0, nullptr, Fr.first, SK_SUB});
             }
             push_products(*sc, hu, std::move(bo), adjoint, Y.p, Z.p, m);
-            for (int c0 = (maxp - 1) / SB * SB; c0 >= 0; c0 -= SB) {
+            for (int c0 = (maxp - 1) / SBW * SBW; c0 >= 0; c0 -= SBW) {
                 std::vector<Product> ap, up;
                 for (int f : fl) {
                     const Front &Fr = sym.fronts[f];
                     if (Fr.p <= c0) continue;
-                    const int nf = Fr.nf(), w = std::min(c0 + SB, Fr.p) - c0, r = Fr.first + c0;
+                    const int nf = Fr.nf(), w = std::min(c0 + SBW, Fr.p) - c0, r = Fr.first + c0;
                     const cx<T> *Pb = fac.p + Fr.fac_off;
                     const cx<T> *W = block(f, c0);
                     if (!adjoint) ap.push_back({W, inv_ld(w), w, w, nullptr, r, nullptr, r, SK_UPPER});

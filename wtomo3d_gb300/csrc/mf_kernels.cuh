@@ -28,7 +28,8 @@ struct FrontDev {
 };
 
 struct PanelTask { int f, k; };
-struct EATask { int child, parent; long long row0; };
+struct EATask { int front, child0, child1; long long pos0, pos1; };   // children -1: none
+struct EAUnit { int task, row0; };
 template <class T>
 struct GemmTask {
     const cx<T> *A;
@@ -92,39 +93,63 @@ static __global__ void k_maxabs(long long n, const double2 *__restrict__ a, unsi
 }
 
 // ---------------------------------------------------------------------------
-// extend-add: child update matrix into the parent front (one warp per row)
+// extend-add: the children's update matrices into a front, gathered by the front's
+// rows (one warp per row)
 // ---------------------------------------------------------------------------
+// Bound by memory traffic.  Each entry of the front's own update block F22 is
+// written once, as the sum of what its children have there (pos: the front's row or
+// column of each child's border, inverted; -1 where the child has none); adding one
+// child after the other into a zeroed block read and wrote it twice more and took
+// two launches and a memset per level (64x64x48: 30 ms of a factorisation).
+constexpr int EA_ROWS = 8;   // rows per CTA
 template <class T>
-__global__ void k_extend_add(const EATask *__restrict__ tasks, int ntasks, long long nrows,
-                             const FrontDev *__restrict__ fr, const int *__restrict__ rel, cx<T> *__restrict__ fac,
-                             cx<T> *__restrict__ upd0, cx<T> *__restrict__ upd1)
+__global__ void __launch_bounds__(32 * EA_ROWS) k_extend_add(const EATask *__restrict__ tasks,
+                                                             const EAUnit *__restrict__ units,
+                                                             const FrontDev *__restrict__ fr,
+                                                             const int *__restrict__ pos, cx<T> *__restrict__ fac,
+                                                             cx<T> *__restrict__ upd0, cx<T> *__restrict__ upd1)
 {
-    long long gr = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    if (gr >= nrows) return;
-    int lo = 0, hi = ntasks - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (tasks[mid].row0 <= gr) lo = mid;
-        else hi = mid - 1;
+    const EAUnit u = units[blockIdx.x];
+    const EATask t = tasks[u.task];
+    const FrontDev P = fr[t.front];
+    const int nf = P.p + P.b, R = u.row0 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (R >= nf) return;
+    const int *m0 = pos + t.pos0, *m1 = pos + t.pos1;
+    const int i0 = t.child0 >= 0 ? m0[R] : -1, i1 = t.child1 >= 0 ? m1[R] : -1;
+    if (i0 < 0 && i1 < 0 && R < P.p) return;
+    const cx<T> *s0 = nullptr, *s1 = nullptr;   // the children's rows
+    if (i0 >= 0) {
+        const FrontDev C = fr[t.child0];
+        s0 = (C.parity ? upd1 : upd0) + C.upd + (long long)i0 * C.b;
     }
-    const EATask t = tasks[lo];
-    const FrontDev C = fr[t.child], P = fr[t.parent];
-    const int i = (int)(gr - t.row0);
-    const int *rl = rel + C.border;   // rel shares the border indexing
-    const cx<T> *src = (C.parity ? upd1 : upd0) + C.upd + (long long)i * C.b;
-    const int R = rl[i];
-    const int nfP = P.p + P.b;
-    cx<T> *pf = fac + P.fac;
-    cx<T> *p22 = (P.parity ? upd1 : upd0) + P.upd;
-    for (int j = lane; j < C.b; j += 32) {
-        const int Cc = rl[j];
-        cx<T> v = src[j];
-        cx<T> *dst;
-        if (R < P.p) dst = pf + (long long)R * nfP + Cc;
-        else if (Cc < P.p) dst = pf + (long long)P.p * nfP + (long long)(R - P.p) * P.p + Cc;
-        else dst = p22 + (long long)(R - P.p) * P.b + (Cc - P.p);
-        *dst = *dst + v;
+    if (i1 >= 0) {
+        const FrontDev C = fr[t.child1];
+        s1 = (C.parity ? upd1 : upd0) + C.upd + (long long)i1 * C.b;
+    }
+    auto sum = [&](int c, bool &any) {
+        const int j0 = s0 ? m0[c] : -1, j1 = s1 ? m1[c] : -1;
+        any = j0 >= 0 || j1 >= 0;
+        cx<T> v = j0 >= 0 ? s0[j0] : cx<T>(0);
+        if (j1 >= 0) v = v + s1[j1];
+        return v;
+    };
+    // the factor part: columns of the pivot rows, pivot columns of the border rows
+    cx<T> *row = fac + P.fac + (R < P.p ? (long long)R * nf : (long long)P.p * nf + (long long)(R - P.p) * P.p);
+    const int w = R < P.p ? nf : P.p;
+    if (s0 || s1) {
+#pragma unroll 4
+        for (int c = lane; c < w; c += 32) {
+            bool any;
+            const cx<T> v = sum(c, any);
+            if (any) row[c] = row[c] + v;
+        }
+    }
+    if (R < P.p) return;
+    cx<T> *p22 = (P.parity ? upd1 : upd0) + P.upd + (long long)(R - P.p) * P.b;
+#pragma unroll 4
+    for (int c = lane; c < P.b; c += 32) {
+        bool any;
+        p22[c] = sum(P.p + c, any);
     }
 }
 

@@ -31,16 +31,22 @@ __device__ __forceinline__ void cmac_conj(cx<T> &d, const cx<T> a, const cx<T> b
 // ---------------------------------------------------------------------------
 // block inverses
 // ---------------------------------------------------------------------------
-constexpr int SB = 512;   // columns per diagonal block of the substitutions (a multiple of KB)
+// Columns per diagonal block of the substitutions (a multiple of KB).  Longer blocks
+// make shorter chains; their inverses cost more.  complex64: 128, 256 and 512 give
+// passes of 14.5, 11.9 and 11.0 ms on 48^3 with 32 columns.  complex128: the inverses
+// are bound by the FP64 pipe, and those of 512 took 10 ms of the 41 ms of kernel
+// time of a 16x15x14 factorisation.
+template <class T> constexpr int SB = sizeof(T) == 4 ? 512 : 256;
 
 // Row stride of a block inverse of w columns (even: rows start on 16 bytes).
 __host__ __device__ __forceinline__ int inv_ld(int w) { return (w + 1) & ~1; }
 
 // Entries of all block inverses of a front with p pivots.
+template <class T>
 inline long long inv_entries(int p)
 {
-    const int full = p / SB, rest = p % SB;
-    return (long long)full * SB * inv_ld(SB) + (long long)rest * inv_ld(rest);
+    const int full = p / SB<T>, rest = p % SB<T>;
+    return (long long)full * SB<T> * inv_ld(SB<T>) + (long long)rest * inv_ld(rest);
 }
 
 // The inverse of block c0 of a front is stored packed, row-major: the upper
@@ -105,8 +111,8 @@ __global__ void __launch_bounds__(BD_TH) k_tile_inverse(const PanelTask *__restr
     __syncthreads();
     band_solve<T, 1>(Tm, X, invd, row, v0, kb);
     __syncthreads();
-    const int c0 = k / SB * SB, w = min(SB, F.p - c0), ldw = inv_ld(w), o = k - c0;
-    cx<T> *W = inv + F.inv + (long long)(c0 / SB) * (SB * SB) + (long long)o * ldw + o;
+    const int c0 = k / SB<T> * SB<T>, w = min(SB<T>, F.p - c0), ldw = inv_ld(w), o = k - c0;
+    cx<T> *W = inv + F.inv + (long long)(c0 / SB<T>) * (SB<T> * SB<T>) + (long long)o * ldw + o;
     for (int q = tid; q < KB * C::V; q += BD_TH) {
         const int i = row ? q / C::V : q % KB, v = row ? q % C::V : q / KB, e = v0 + v;
         if (i >= kb || e >= kb) continue;
@@ -136,9 +142,9 @@ __global__ void __launch_bounds__(IV_TH) k_block_inverse(const InvTask *__restri
     __shared__ int rows[KB];
     const InvTask t = tasks[blockIdx.x];
     const FrontDev F = fr[t.f];
-    const int nf = F.p + F.b, w = min(SB, F.p - t.c0), ldw = inv_ld(w), nt = (w + KB - 1) / KB;
+    const int nf = F.p + F.b, w = min(SB<T>, F.p - t.c0), ldw = inv_ld(w), nt = (w + KB - 1) / KB;
     const cx<T> *D = fac + F.fac + (long long)t.c0 * nf + t.c0;   // the block's factors
-    cx<T> *W = inv + F.inv + (long long)(t.c0 / SB) * (SB * SB);
+    cx<T> *W = inv + F.inv + (long long)(t.c0 / SB<T>) * (SB<T> * SB<T>);
     const bool up = t.upper != 0;
     const int col0 = KB * t.t + IV_N * t.h;
     const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;   // rows ty + 16 i, columns 4 tx + j
@@ -249,8 +255,7 @@ constexpr int SK_M = 64, SK_TH = 128, SK_KMAX = 1024;
 // holds the pass's columns, so that one source does not pay for 32.
 inline int sk_columns(int m) { return m <= 1 ? 1 : m <= 4 ? 4 : m <= 8 ? 8 : m <= 16 ? 16 : 32; }
 
-// Stage depth along K, and stages: 40 KB per CTA at 32 columns, five CTAs per
-// SM for complex64.
+// Stage depth along K, and stages: 40 KB per CTA at 32 columns.
 template <class T, int NC>
 struct SkCfg {
     static constexpr int BK = (NC >= 32 ? 16 : 32) / (sizeof(T) / 4);

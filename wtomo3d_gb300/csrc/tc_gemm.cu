@@ -206,59 +206,66 @@ __global__ void k_split_a_f16_rows(const TcTask *__restrict__ tasks, int ntasks,
     }
 }
 
-__global__ void __launch_bounds__(256) k_split_b_f16_cols(const TcTask *__restrict__ tasks, int ntasks,
-                                                          long long total_groups)
+// 1024 threads: a launch has few column groups on the small and middle levels (38
+// for 1200 columns), and the time of a group is its passes over K, 32 rows each
+// (34 us on average with 8 rows per pass on 24x22x20).
+__global__ void __launch_bounds__(1024) k_split_b_f16_cols(const TcTask *__restrict__ tasks, int ntasks,
+                                                           long long total_groups)
 {
-    __shared__ float2 tile[32][33];
-    __shared__ float red[8][33];
+    __shared__ float2 tile[2][32][33];
+    __shared__ float red[32][33];
     const long long q = blockIdx.x;
     const int ti = block_task(tasks, ntasks, q, q, &TcTask::b_col0);
     if (q >= total_groups) return;
     const TcTask &t = tasks[ti];
     const int j0 = (int)(q - t.b_col0) * 32;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;   // 32 x 8
-    const int jx = j0 + tx;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;   // 32 x 32
+    const int jx = j0 + tx, K = t.K, N = t.N, ldb = t.ldb;
+    const cx<float> *B = t.B;
     float m = 0.f;
-    if (jx < t.N)
-        for (int k = ty; k < t.K; k += 8) {
-            const cx<float> v = t.B[(long long)k * t.ldb + jx];
+    if (jx < N) {
+#pragma unroll 4
+        for (int k = ty; k < K; k += 32) {
+            const cx<float> v = B[(long long)k * ldb + jx];
             m = fmaxf(m, fmaxf(fabsf(v.re), fabsf(v.im)));
         }
+    }
     red[ty][tx] = m;
     __syncthreads();
     if (ty == 0) {
-        for (int y = 1; y < 8; y++) m = fmaxf(m, red[y][tx]);
+        for (int y = 1; y < 32; y++) m = fmaxf(m, red[y][tx]);
         red[0][tx] = f16_scale(__float_as_uint(m));
-        if (jx < t.N) t.sb[jx] = 1.f / red[0][tx];
+        if (jx < N) t.sb[jx] = 1.f / red[0][tx];
     }
     __syncthreads();
     __half2 *bh = reinterpret_cast<__half2 *>(t.bhi), *bl = reinterpret_cast<__half2 *>(t.blo);
-    for (int k0 = 0; k0 < t.Kr / 2; k0 += 32) {
-        for (int kk = ty; kk < 32; kk += 8) {
-            const int k = k0 + kk;
-            cx<float> v(0.f, 0.f);
-            if (k < t.K && jx < t.N) v = t.B[(long long)k * t.ldb + jx];
-            tile[kk][tx] = make_float2(v.re, v.im);
-        }
+    const float sc = red[0][ty];   // column j0 + ty, which this warp writes
+    const int j = j0 + ty;
+    const long long o0 = ((long long)(2 * j) * t.Kr) >> 1, o1 = o0 + (t.Kr >> 1);
+    auto fetch = [&](int k) {
+        cx<float> v(0.f, 0.f);
+        if (k < K && jx < N) v = B[(long long)k * ldb + jx];
+        return make_float2(v.re, v.im);
+    };
+    const int kr = t.Kr / 2;
+    float2 next = fetch(ty);
+    for (int k0 = 0; k0 < kr; k0 += 32) {
+        float2(*tl)[33] = tile[(k0 >> 5) & 1];
+        tl[ty][tx] = next;
+        if (k0 + 32 < kr) next = fetch(k0 + 32 + ty);
         __syncthreads();
-        for (int jj = ty; jj < 32; jj += 8) {
-            const int j = j0 + jj;
-            if (j < t.N) {
-                const float sc = red[0][jj];
-                const float br = tile[tx][jj].x * sc, bi = tile[tx][jj].y * sc;
-                const int k = k0 + tx;
-                __half rh, rl, ih, il, nih, nil;
-                split_f16(br, rh, rl);
-                split_f16(bi, ih, il);
-                split_f16(-bi, nih, nil);
-                const long long o0 = ((long long)(2 * j) * t.Kr + 2 * k) >> 1, o1 = o0 + (t.Kr >> 1);
-                bh[o0] = __halves2half2(rh, nih);
-                bl[o0] = __halves2half2(rl, nil);
-                bh[o1] = __halves2half2(ih, rh);
-                bl[o1] = __halves2half2(il, rl);
-            }
+        if (j < N) {
+            const float br = tl[tx][ty].x * sc, bi = tl[tx][ty].y * sc;
+            const int k = k0 + tx;
+            __half rh, rl, ih, il, nih, nil;
+            split_f16(br, rh, rl);
+            split_f16(bi, ih, il);
+            split_f16(-bi, nih, nil);
+            bh[o0 + k] = __halves2half2(rh, nih);
+            bl[o0 + k] = __halves2half2(rl, nil);
+            bh[o1 + k] = __halves2half2(ih, rh);
+            bl[o1 + k] = __halves2half2(il, rl);
         }
-        __syncthreads();
     }
 }
 
@@ -614,7 +621,7 @@ void tc_split(const TcLaunch &L, cudaStream_t st)
     if (L.ntasks == 0) return;
     if (L.f16) {
         k_split_a_f16_rows<<<ceil_div(L.a_rows * 32, 256), 256, 0, st>>>(L.tasks.p, L.ntasks, L.a_rows);
-        k_split_b_f16_cols<<<(unsigned)L.b_cols, 256, 0, st>>>(L.tasks.p, L.ntasks, L.b_cols);
+        k_split_b_f16_cols<<<(unsigned)L.b_cols, 1024, 0, st>>>(L.tasks.p, L.ntasks, L.b_cols);
         return;
     }
     k_split_a<<<ceil_div(L.a_work, 256), 256, 0, st>>>(L.tasks.p, L.ntasks, L.a_work);
