@@ -1829,7 +1829,8 @@ extern "C" int wt3d_debug_skinny(int herm, int tri, int M, int K, int nc, int ch
     }
     if ((rc = du.upload(hu))) return rc;
     Engine<float>::sk_attributes();
-    Engine<float>::sk_launch(nc, herm != 0, du.p, (int)hu.size(), dB.p, dC.p, 0);
+    if (sk_tensor(nc, chunk)) sk_tensor_launch(nc, herm != 0, du.p, (int)hu.size(), dB.p, dC.p, 0);
+    else Engine<float>::sk_launch(nc, herm != 0, du.p, (int)hu.size(), dB.p, dC.p, 0);
     WT_CUDA(cudaGetLastError());
     WT_CUDA(cudaMemcpy(out, dC.p, sizeof(cx<float>) * M * nc, cudaMemcpyDeviceToHost));
     return WT3D_OK;

@@ -50,10 +50,6 @@ struct Schedule {
     DevVec<SkUnit> sk;                                        // units of the substitution products
     std::vector<std::vector<GemmTask<float>>> tc_pending;   // tensor-core task lists, built after allocation
     std::vector<std::unique_ptr<TcLaunch>> tc;
-    std::vector<std::vector<GemmTask<float>>> ts_pending;   // tall-skinny tensor-core task lists (solves)
-    std::vector<char> ts_tma;                                 // ... whose A is streamed by TMA
-    std::vector<std::unique_ptr<TsLaunch>> ts;
-    DevVec<float> tsws;                                       // their expanded right-hand sides
     cudaGraphExec_t graph = nullptr;
     ~Schedule()
     {
@@ -93,9 +89,6 @@ public:
     DevVec<unsigned long long> maxabs;
     std::unique_ptr<Schedule<T>> fsched;
     std::map<int, std::unique_ptr<Schedule<T>>> ssched[2];   // [adjoint][m]
-    // products of at least this many factor entries go to the tall-skinny
-    // tensor-core kernel
-    static constexpr double TS_MIN_ENTRIES = 4e6;
     // vectors of a band launch from which four threads take two
     static constexpr long long BAND_TWO = 152 * 4 * 32;
     // flops from which a factorisation's update goes to the tensor-core kernel
@@ -117,7 +110,7 @@ public:
     double pivot_rel = 1e-20;
     // tcgen05 path for complex64 front updates (WT3D_TC=0 selects the SIMT kernel)
     bool use_tc = std::is_same<T, float>::value && !(getenv("WT3D_TC") && getenv("WT3D_TC")[0] == '0');
-    // tcgen05 path for the large blocks of complex64 substitution passes (WT3D_TS=0: SIMT)
+    // tensor cores for the products of complex64 substitution passes (WT3D_TS=0: FP32 pipe)
     bool use_ts = std::is_same<T, float>::value && !(getenv("WT3D_TS") && getenv("WT3D_TS")[0] == '0');
     DevVec<float> own_tcws;   // private split workspace, only if the shared one is too small
     DevVec<int> tc_err;                                 // barrier-timeout flag of the tensor-core kernel
@@ -128,12 +121,9 @@ public:
     // device bytes this engine holds on its own (the shared workspace excluded)
     size_t device_bytes() const
     {
-        size_t sw = 0;   // the solve schedules' tall-skinny workspaces
-        for (const auto &m : ssched)
-            for (const auto &kv : m) sw += kv.second->tsws.n * sizeof(float);
         return (fac.n + X.n + Z.n + Y.n + binv.n) * sizeof(cx<T>) + (ipiv.n + border.n + eapos.n + gord.n) * 4 +
                fr.n * sizeof(FrontDev) +
-               map.n * 8 + scale.n * 8 + own_tcws.n * sizeof(float) + sw;
+               map.n * 8 + scale.n * 8 + own_tcws.n * sizeof(float);
     }
 
     // Reads (and clears) the barrier-timeout flag of the tensor-core kernels;
@@ -181,7 +171,6 @@ public:
         if ((rc = tc_err.alloc(1))) return rc;
         WT_CUDA(cudaMemset(tc_err.p, 0, sizeof(int)));
         if (use_tc && (rc = tc_init())) return rc;
-        if (use_ts && (rc = ts_init())) return rc;
         std::vector<FrontDev> h(sym.fronts.size());
         long long ninv = 0;
         for (size_t f = 0; f < h.size(); f++) {
@@ -337,28 +326,6 @@ public:
         sc.launches.push_back({[psc, u0, nu](cudaStream_t st) {
             k_gemm<T><<<nu, GemmCfg<T>::TH, 0, st>>>(psc->gemm.p, psc->unit.p + u0);
         }, LK_GEMM, fl, by});
-    }
-
-    // Allocates a solve schedule's own B~ workspace (sized for its largest
-    // tall-skinny launch; launches run one after another) and builds the
-    // tensor maps of its tall-skinny tensor-core launches.
-    int finish_ts(Schedule<T> &sc)
-    {
-        if constexpr (std::is_same<T, float>::value) {
-            long long need = 0;
-            for (auto &v : sc.ts_pending) need = std::max(need, ts_workspace_floats(v.data(), (int)v.size()));
-            if (need == 0) return WT3D_OK;
-            int rc;
-            if ((rc = sc.tsws.alloc(need))) return rc;
-            sc.ts.clear();
-            for (size_t i = 0; i < sc.ts_pending.size(); i++) {
-                auto &v = sc.ts_pending[i];
-                sc.ts.emplace_back(new TsLaunch());
-                if ((rc = ts_build_launch(*sc.ts.back(), v.data(), (int)v.size(), sc.tsws.p, sc.ts_tma[i] != 0)))
-                    return rc;
-            }
-        }
-        return WT3D_OK;
     }
 
     // Allocates the shared tensor-core workspace and builds the tensor maps of
@@ -627,34 +594,6 @@ public:
     {
         const int nc = sk_columns(m);
         Schedule<T> *psc = &sc;
-        if constexpr (std::is_same<T, float>::value) {
-            // large blocks go to the tall-skinny tensor-core kernel: those that TMA
-            // can address (16-byte aligned, even stride) and the rest, one launch each
-            std::vector<GemmTask<float>> tsv[2];
-            std::vector<Product> rest;
-            for (const Product &q : v) {
-                GemmTask<float> g{};
-                g.A = q.A; g.lda = q.lda; g.M = q.M; g.K = q.K; g.N = m; g.conjA = herm;
-                g.B = in + (q.bmap ? 0 : (long long)q.b0 * nc); g.brow = q.bmap; g.ldb = nc;
-                g.C = out + (q.cmap ? 0 : (long long)q.c0 * nc); g.crow = q.cmap; g.ldc = nc;
-                const bool tri = (q.flags & (SK_LOWER | SK_UPPER)) != 0;
-                if (use_ts && !tri && nc >= 8 && (double)q.M * q.K >= TS_MIN_ENTRIES && ts_eligible(g))
-                    tsv[ts_tma_ok(g) ? 1 : 0].push_back(g);
-                else rest.push_back(q);
-            }
-            v.swap(rest);
-            for (int tma = 0; tma < 2; tma++) {
-                if (tsv[tma].empty()) continue;
-                double fl = 0, by = 0;
-                for (auto &g : tsv[tma]) { fl += 8.0 * g.M * (double)g.N * g.K; by += gemm_bytes(g); }
-                const int idx = (int)sc.ts_pending.size();
-                sc.ts_pending.push_back(std::move(tsv[tma]));
-                sc.ts_tma.push_back((char)tma);
-                sc.launches.push_back({[psc, idx](cudaStream_t st) { ts_expand(*psc->ts[idx], st); }, LK_SPLIT, 0});
-                sc.launches.push_back({[psc, idx, this](cudaStream_t st) { ts_mma(*psc->ts[idx], tc_err.p, st); },
-                                       LK_TCGEMM, fl, by});
-            }
-        }
         if (v.empty()) return;
         // K range of the 64 rows from r0: all of it, or the triangle's part
         auto range = [&](const Product &q, int r0, int &k0, int &k1) {
@@ -698,9 +637,17 @@ public:
             }
         const int nu = (int)(hu.size() - u0);
         const bool tri = (v[0].flags & (SK_LOWER | SK_UPPER)) != 0;
+        const double by = fl / m * sizeof(cx<T>) / 8;
+        if constexpr (std::is_same<T, float>::value)
+            if (use_ts && sk_tensor(nc, chunk)) {
+                sc.launches.push_back({[psc, u0, nu, nc, herm, in, out](cudaStream_t st) {
+                    sk_tensor_launch(nc, herm, psc->sk.p + u0, nu, in, out, st);
+                }, tri ? LK_SUBSTEP : LK_TCGEMM, fl, by});
+                return;
+            }
         sc.launches.push_back({[psc, u0, nu, nc, herm, in, out](cudaStream_t st) {
             sk_launch(nc, herm, psc->sk.p + u0, nu, in, out, st);
-        }, tri ? LK_SUBSTEP : LK_GEMM, fl, fl / m * sizeof(cx<T>) / 8});
+        }, tri ? LK_SUBSTEP : LK_GEMM, fl, by});
     }
 
     // Solve schedule for m right-hand sides: X (sources, new ordering) to Y.
@@ -789,7 +736,7 @@ public:
                 push_products(*sc, hu, std::move(up), adjoint, Y.p, Z.p, m);
             }
         }
-        if (sc->sk.upload(hu) || finish_ts(*sc)) return nullptr;
+        if (sc->sk.upload(hu)) return nullptr;
         Schedule<T> *ret = sc.get();
         ssched[adjoint][m] = std::move(sc);
         return ret;

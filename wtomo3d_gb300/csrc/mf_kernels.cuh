@@ -35,10 +35,7 @@ struct GemmTask {
     const cx<T> *A;
     const cx<T> *B;
     cx<T> *C;
-    const int *brow;   // optional row gather for B
-    const int *crow;   // optional row scatter for C (atomic)
     int lda, ldb, ldc, M, N, K;
-    int conjA;         // use conj(A^T): A is read as its conjugate transpose
 };
 
 template <class T>

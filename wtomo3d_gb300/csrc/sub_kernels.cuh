@@ -14,6 +14,12 @@
 
 namespace wt3d {
 
+// Start of a kernel that is launched as a programmatic dependent of the one before
+// it: the next kernel may be set up from here on; after the wait everything before
+// this kernel is complete and visible.
+__device__ __forceinline__ void chain_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // d += a b and d += conj(a) b as four fused multiply-adds
 template <class T>
 __device__ __forceinline__ void cmac(cx<T> &d, const cx<T> a, const cx<T> b)
@@ -255,6 +261,14 @@ constexpr int SK_M = 64, SK_TH = 128, SK_KMAX = 1024;
 // holds the pass's columns, so that one source does not pay for 32.
 inline int sk_columns(int m) { return m <= 1 ? 1 : m <= 4 ? 4 : m <= 8 ? 8 : m <= 16 ? 16 : 32; }
 
+// Products that go to the tensor cores (skinny_tc.cu), by width and K per unit.  At 8
+// columns a launch of units shorter than 128 k is faster on the FP32 pipe: a pass of
+// 24x22x20 takes 0.55 ms with it, 0.65 ms on the tensor cores; one of 64x64x48 8.7 ms
+// and 6.5 ms.  At 16 and 32 columns the tensor cores win at every size measured
+// (33x31x29 with 16: 1.50 and 1.13 ms).
+inline bool sk_tensor(int nc, int chunk) { return nc > 8 || (nc == 8 && chunk >= 128); }
+void sk_tensor_launch(int nc, bool herm, const SkUnit *u, int n, const cx<float> *in, cx<float> *out, cudaStream_t st);
+
 // Stage depth along K, and stages: 40 KB per CTA at 32 columns.
 template <class T, int NC>
 struct SkCfg {
@@ -292,14 +306,13 @@ __device__ __forceinline__ void red_add(cx<double> *p, const cx<double> v)
 // previous product: the factor entries, which no product writes, are on their
 // way before the wait for it.  One pass, against KB-wide steps and 128 x 32
 // products that computed 32 columns whatever the pass held: 40^3 with 1 column
-// 11.4 -> 2.0 ms, with 32 columns 12.4 -> 4.4 ms (31 TF/s of 73 in the
-// updates), 64x64x48 with 32 columns 31.5 -> 14.1 ms, complex128 16x15x14 with
-// 4 columns 23 -> 1.1 ms.
+// 11.4 -> 2.0 ms, with 32 columns 12.4 -> 4.4 ms (2.8 ms on the tensor cores),
+// complex128 16x15x14 with 4 columns 23 -> 1.1 ms.
 template <class T, int NC, bool H>
 __global__ void __launch_bounds__(SK_TH) k_skinny(const SkUnit *__restrict__ units, const cx<T> *__restrict__ in,
                                                   cx<T> *__restrict__ out)
 {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    chain_start();
     using C = SkCfg<T, NC>;
     constexpr int BK = C::BK, NS = C::NS, VK = C::VK, LDA = C::lda(H), AE = C::a_elems(H), BE = C::b_elems();
     constexpr int CT = NC < 4 ? NC : 4, TX = NC / CT, TPG = 16 * TX, KG = SK_TH / TPG;
@@ -344,7 +357,7 @@ __global__ void __launch_bounds__(SK_TH) k_skinny(const SkUnit *__restrict__ uni
     for (int k = tid; k < K; k += SK_TH) brow[k] = u.bmap ? u.bmap[k] : u.b0 + k;
     if (tid < M) crow[tid] = u.cmap ? u.cmap[tid] : u.c0 + tid;
     __syncthreads();
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    chain_wait();
     for (int s = 0; s < NS - 1; s++) {
         if (s < nst) load_b(s);
         asm volatile("cp.async.commit_group;" ::: "memory");

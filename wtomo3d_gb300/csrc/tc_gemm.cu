@@ -40,6 +40,7 @@
 #include <cuda_fp16.h>
 #include <cudaTypedefs.h>
 #include "tc_gemm.h"
+#include "sub_kernels.cuh"
 #include "tc_ptx.cuh"
 #include <atomic>
 #include <cstring>
@@ -539,7 +540,7 @@ bool tc_eligible(const GemmTask<float> &g)
 {
     // large enough that the tensor-core tile (128 x 128 complex) is not mostly
     // padding; the narrow right-hand-side blocks of the solves stay on SIMT
-    return !g.brow && !g.crow && !g.conjA && g.M >= 64 && g.N >= 96 && g.K >= 32;
+    return g.M >= 64 && g.N >= 96 && g.K >= 32;
 }
 
 // f16 mode unless WT3D_TC_F16=0 (then the TF32 split)
@@ -684,6 +685,23 @@ extern "C" int wt3d_set_sm_reserve(int n)
     return WT3D_OK;
 }
 
+// Units of C -= op(A) B for the substitutions' products.
+static void skinny_units(const cx<float> *A, int lda, int M, int K, bool herm, const int *bmap, const int *cmap,
+                         bool atom, std::vector<SkUnit> &hu)
+{
+    constexpr int chunk = 512;
+    for (int r0 = 0; r0 < M; r0 += SK_M)
+        for (int k = 0; k < K; k += chunk) {
+            SkUnit u{};
+            u.A = herm ? A + (size_t)k * lda + r0 : A + (size_t)r0 * lda + k;
+            u.bmap = bmap ? bmap + k : nullptr;
+            u.cmap = cmap ? cmap + r0 : nullptr;
+            u.b0 = k; u.c0 = r0; u.lda = lda; u.M = std::min(SK_M, M - r0); u.K = std::min(chunk, K - k);
+            u.flags = SK_SUB | (atom || K > chunk ? SK_ATOM : 0);
+            hu.push_back(u);
+        }
+}
+
 extern "C" int wt3d_debug_gemm(int path, int M, int N, int K, const void *A, int lda, const void *B, int ldb, void *C,
                                int ldc)
 {
@@ -711,25 +729,31 @@ extern "C" int wt3d_debug_gemm(int path, int M, int N, int K, const void *A, int
         tc_split(L, 0);
         tc_mma(L, err.p, 0);
     } else if (path >= 3 && path <= 5) {
-        // tall-skinny tensor-core kernel; path 4 gathers B rows K-1-k and
-        // scatters C rows M-1-r (atomic epilogue); path 5 uses A^H
+        // the substitutions' tensor-core products; path 4 gathers B rows K-1-k and
+        // scatters C rows M-1-r (atomic sums); path 5 uses A^H
         if (N > 32) { set_error("wt3d_debug_gemm: paths 3 to 5 need N <= 32"); return WT3D_ERR_ARG; }
-        g.conjA = path == 5 ? 1 : 0;
+        const int nc = std::max(8, sk_columns(N));
+        std::vector<cx<float>> in((size_t)K * nc, cx<float>(0)), out((size_t)M * nc, cx<float>(0));
+        const cx<float> *hB = (const cx<float> *)B;
+        cx<float> *hC = (cx<float> *)C;
+        for (int k = 0; k < K; k++) std::copy(hB + (size_t)k * ldb, hB + (size_t)k * ldb + N, &in[(size_t)k * nc]);
+        for (int r = 0; r < M; r++) std::copy(hC + (size_t)r * ldc, hC + (size_t)r * ldc + N, &out[(size_t)r * nc]);
         if (path == 4) {
             std::vector<int> br(K), cr(M);
             for (int k = 0; k < K; k++) br[k] = K - 1 - k;
             for (int r = 0; r < M; r++) cr[r] = M - 1 - r;
             if ((rc = drow.upload(br)) || (rc = dcol.upload(cr))) return rc;
-            g.brow = drow.p;
-            g.crow = dcol.p;
         }
-        if ((rc = ts_init())) return rc;
-        DevVec<float> ws;
-        if ((rc = ws.alloc(ts_workspace_floats(&g, 1)))) return rc;
-        TsLaunch L;
-        if ((rc = ts_build_launch(L, &g, 1, ws.p, ts_tma_ok(g)))) return rc;
-        ts_expand(L, 0);
-        ts_mma(L, err.p, 0);
+        DevVec<cx<float>> din, dout;
+        DevVec<SkUnit> dsk;
+        std::vector<SkUnit> hu;
+        skinny_units(dA.p, lda, M, K, path == 5, drow.p, dcol.p, path == 4, hu);
+        if ((rc = din.upload(in)) || (rc = dout.upload(out)) || (rc = dsk.upload(hu))) return rc;
+        sk_tensor_launch(nc, path == 5, dsk.p, (int)hu.size(), din.p, dout.p, 0);
+        WT_CUDA(cudaGetLastError());
+        WT_CUDA(cudaMemcpy(out.data(), dout.p, sizeof(cx<float>) * out.size(), cudaMemcpyDeviceToHost));
+        for (int r = 0; r < M; r++) std::copy(&out[(size_t)r * nc], &out[(size_t)r * nc] + N, hC + (size_t)r * ldc);
+        return WT3D_OK;
     } else {
         DevVec<GemmTask<float>> dt;
         std::vector<GemmTask<float>> v{g};
@@ -774,7 +798,10 @@ extern "C" int wt3d_bench_gemm(int path, int M, int N, int K, int iters, double 
     WT_CUDA(cudaMemset(err.p, 0, sizeof(int)));
     DevVec<float> ws;
     TcLaunch L;
-    TsLaunch LT;
+    DevVec<cx<float>> din, dout;
+    DevVec<SkUnit> dsk;
+    std::vector<SkUnit> hsk;
+    const int nc = std::max(8, sk_columns(std::min(N, 32)));
     DevVec<GemmTask<float>> dt;
     std::vector<GemmUnit> hu;
     DevVec<GemmUnit> du;
@@ -784,11 +811,10 @@ extern "C" int wt3d_bench_gemm(int path, int M, int N, int K, int iters, double 
         tc_split(L, 0);
     } else if (path == 3 || path == 6) {
         if (N > 32) { set_error("wt3d_bench_gemm: paths 3 and 6 need N <= 32"); return WT3D_ERR_ARG; }
-        const bool tma = path == 3 && ts_tma_ok(g);
-        if ((rc = ts_init()) || (rc = ws.alloc(ts_workspace_floats(&g, 1))) ||
-            (rc = ts_build_launch(LT, &g, 1, ws.p, tma)))
-            return rc;
-        ts_expand(LT, 0);
+        skinny_units(dA.p, K, M, K, false, nullptr, nullptr, false, hsk);
+        if ((rc = din.alloc((size_t)K * nc)) || (rc = dout.alloc((size_t)M * nc)) || (rc = dsk.upload(hsk))) return rc;
+        k_fill<<<ceil_div((long long)K * nc, 256), 256>>>(din.p, (long long)K * nc, 2);
+        WT_CUDA(cudaMemset(dout.p, 0, sizeof(cx<float>) * M * nc));
     } else {
         std::vector<GemmTask<float>> v{g};
         gemm_units(v, 0, hu);
@@ -800,7 +826,7 @@ extern "C" int wt3d_bench_gemm(int path, int M, int N, int K, int iters, double 
     if (path == 2 && N > 32) { set_error("wt3d_bench_gemm: path 2 needs N <= 32"); return WT3D_ERR_ARG; }
     auto launch = [&]() {
         if (path == 1) tc_mma(L, err.p, 0);
-        else if (path == 3 || path == 6) ts_mma(LT, err.p, 0);
+        else if (path == 3 || path == 6) sk_tensor_launch(nc, false, dsk.p, (int)hsk.size(), din.p, dout.p, 0);
         else k_gemm<float><<<(unsigned)hu.size(), GemmCfg<float>::TH>>>(dt.p, du.p);
     };
     for (int w = 0; w < 2; w++) launch();   // warm-up
