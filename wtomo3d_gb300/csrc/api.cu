@@ -170,7 +170,7 @@ struct wt3d_solver {
     DevVec<double2> gmPart;
     DevVec<double> gmNorm, gmScale;
     void *pin = nullptr;                  // SolveHost
-    StreamBuf<ulonglong2> epA;            // the operator's digits (product_prepare), per call
+    StreamBuf<uint4> epA;            // the operator's digits (product_prepare), per call
     StreamBuf<int> epE;                   // ... exponents of its rows, its columns, blocks of nodes
     ProductOp epOp{};
     std::unique_ptr<Engine<float>> e32;
