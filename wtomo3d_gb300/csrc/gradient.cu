@@ -89,7 +89,7 @@ __device__ __forceinline__ double re_dot9(const cx<double> *b, const cx<double> 
 {
     double s = 0;
 #pragma unroll
-    for (int k = 0; k < 9; k++) s += b[k].re * G[k].re - b[k].im * G[k].im;
+    for (int k = 0; k < 9; k++) s = fma(b[k].re, G[k].re, fma(-b[k].im, G[k].im, s));
     return s;
 }
 
@@ -112,7 +112,11 @@ __device__ __forceinline__ void outer_sum(const double2 *__restrict__ U, const d
 #pragma unroll
         for (int a = 0; a < 3; a++)
 #pragma unroll
-            for (int b = 0; b < 3; b++) G[3 * a + b] = G[3 * a + b] + l[a] * u[b];
+            for (int b = 0; b < 3; b++) {
+                cx<double> &g = G[3 * a + b];
+                g.re = fma(l[a].re, u[b].re, fma(-l[a].im, u[b].im, g.re));
+                g.im = fma(l[a].re, u[b].im, fma(l[a].im, u[b].re, g.im));
+            }
     }
 }
 
@@ -156,14 +160,43 @@ __device__ __forceinline__ void axis_factor_d(int idx, int n, int ipml, double d
 }
 
 // ---------------------------------------------------------------------------
-// pass 0: cell-mean, density and weight derivatives of each row
+// pass 0: cell-mean, density, weight and vpreal derivatives of each row
 // ---------------------------------------------------------------------------
+// What the vpreal derivative of a row inside the PML needs: the derivatives of the
+// stretch (stencil rows) or of r1 along x and y (rows of the free surface).
+struct VpTerms {
+    bool on;
+    Stretch<double> fd;
+    cx<double> dr1x, dr1y;
+    double acc;
+};
+
+template <int S>
+__device__ __forceinline__ void vp_slot(int region, const NodeCoefs<double> &c, double dxo8, const cx<double> *G,
+                                        VpTerms &vt)
+{
+    cx<double> b[9];
+    if (region == REG_STENCIL) {
+        stencil_block<S, double>(c, vt.fd, 0.0, 0.0, 0.0, cx<double>(0), b);   // linear in the stretch
+        vt.acc += re_dot9(b, G);
+    } else if constexpr (S == 2 || S == 20 || S == 8 || S == 26 || S == 13) {   // the others: zero blocks
+        // TPFREE blocks are affine in (r1x, r1y)
+        cx<double> b0[9], bx[9], by[9];
+        tpfree_block<S, double>(c, cx<double>(0), cx<double>(0), dxo8, b0);
+        tpfree_block<S, double>(c, cx<double>(1), cx<double>(0), dxo8, bx);
+        tpfree_block<S, double>(c, cx<double>(0), cx<double>(1), dxo8, by);
+#pragma unroll
+        for (int k = 0; k < 9; k++) b[k] = vt.dr1x * (bx[k] - b0[k]) + vt.dr1y * (by[k] - b0[k]);
+        vt.acc += re_dot9(b, G);
+    }
+}
+
 template <int S>
 __device__ __forceinline__ void rows_slot(int region, unsigned mask, const Stretch<double> &f, cx<double> r1x,
                                           cx<double> r1y, double dxo8, const NodeCoefs<double> &c, cx<double> om2,
                                           double m2, double m3, double m4, const double2 *U, const double2 *L,
                                           long long ld, int m, long long n, int nz, int nx, double *du, double *dd,
-                                          double *dwm, double *D, long long nn)
+                                          double *dwm, VpTerms &vt, double *D, long long nn)
 {
     if (!((mask >> S) & 1u)) {
         D[(long long)(GD_RO + S) * nn + n] = 0.0;
@@ -173,6 +206,7 @@ __device__ __forceinline__ void rows_slot(int region, unsigned mask, const Stret
     const long long nb = n + dz + (long long)nz * (dxo + (long long)nx * dy);
     cx<double> G[9];
     outer_sum(U, L, ld, m, n, nb, G);
+    if (vt.on) vp_slot<S>(region, c, dxo8, G, vt);
     constexpr unsigned cm = slot_cells(S);
 #pragma unroll
     for (int q = 1; q <= 8; q++) {
@@ -213,13 +247,20 @@ __device__ __forceinline__ void rows_all(std::integer_sequence<int, Ss...>, int 
                                          const Stretch<double> &f, cx<double> r1x, cx<double> r1y, double dxo8,
                                          const NodeCoefs<double> &c, cx<double> om2, double m2, double m3, double m4,
                                          const double2 *U, const double2 *L, long long ld, int m, long long n, int nz,
-                                         int nx, double *du, double *dd, double *dwm, double *D, long long nn)
+                                         int nx, double *du, double *dd, double *dwm, VpTerms &vt, double *D, long long nn)
 {
-    (rows_slot<Ss>(region, mask, f, r1x, r1y, dxo8, c, om2, m2, m3, m4, U, L, ld, m, n, nz, nx, du, dd, dwm, D, nn),
+    (rows_slot<Ss>(region, mask, f, r1x, r1y, dxo8, c, om2, m2, m3, m4, U, L, ld, m, n, nz, nx, du, dd, dwm, vt, D, nn),
      ...);
 }
 
-__global__ void __launch_bounds__(128) k_grad_rows(AsmParams p, const cx<double> *__restrict__ da,
+// Bound by the FP64 pipe (two multiply-adds per cycle and SM): 36 per slot and
+// source.  One warp per CTA, so that a grid of a few hundred warps is spread evenly
+// over the SMs; the vpreal derivative shares the row's sums G, although that makes
+// the compiler spill.  32x32x24 with 16 sources: 1.29 ms; CTAs of 128, six operations
+// per product and a second kernel with the same sums for vpreal took 2.30 + 1.89 ms.
+constexpr int GR_TH = 32;
+
+__global__ void __launch_bounds__(GR_TH) k_grad_rows(AsmParams p, const cx<double> *__restrict__ da,
                                                    const cx<double> *__restrict__ mu, const double *__restrict__ ro,
                                                    int m, long long ld, const double2 *__restrict__ U,
                                                    const double2 *__restrict__ L, double *__restrict__ D)
@@ -234,7 +275,7 @@ __global__ void __launch_bounds__(128) k_grad_rows(AsmParams p, const cx<double>
     int region, zidx;
     node_region(p, iz, ix, iy, region, zidx, mask);
     if (region == REG_FIXED) {
-        for (int k = 0; k < GD_VP; k++) D[(long long)k * nn + n] = 0.0;
+        for (int k = 0; k < GD_N; k++) D[(long long)k * nn + n] = 0.0;
         return;
     }
     NodeCoefs<double> c;
@@ -254,6 +295,32 @@ __global__ void __launch_bounds__(128) k_grad_rows(AsmParams p, const cx<double>
         axis_factor<double>(iy + 1, p.ny, p.ipml, p.dx, p.pmld, p.pmlf, c.vpreal, eyeom, r1y, r2);
         dxo8 = 1.0 / (p.dx * 8.0);
     }
+    const int jx = ix + 1, jy = iy + 1;
+    VpTerms vt;
+    vt.acc = 0.0;
+    vt.on = jx <= p.ipml || p.nx - jx + 1 <= p.ipml || jy <= p.ipml || p.ny - jy + 1 <= p.ipml ||
+            (zidx > 0 && (zidx <= p.ipml || p.nz - zidx + 1 <= p.ipml));
+    if (vt.on) {
+        const cx<double> eyeom = cx<double>(0.0, -1.0) * om;
+        cx<double> s1x, s1y, s1z, d1z, d2x, d2y, d2z;
+        axis_factor_d(jx, p.nx, p.ipml, p.dx, p.pmld, p.pmlf, c.vpreal, eyeom, s1x, vt.dr1x, d2x);
+        axis_factor_d(jy, p.ny, p.ipml, p.dx, p.pmld, p.pmlf, c.vpreal, eyeom, s1y, vt.dr1y, d2y);
+        if (region == REG_STENCIL) {
+            axis_factor_d(zidx, p.nz, p.ipml, p.dx, p.pmld, p.pmlf, c.vpreal, eyeom, s1z, d1z, d2z);
+            // derivative of build_stretch's scaled combinations
+            const double dxx = p.dx * p.dx;
+            const cx<double> d1x = vt.dr1x, d1y = vt.dr1y;
+            vt.fd.X2 = (2.0 * s1x * d1x) / (8.0 * dxx);
+            vt.fd.Y2 = (2.0 * s1y * d1y) / (8.0 * dxx);
+            vt.fd.Z2 = (2.0 * s1z * d1z) / (8.0 * dxx);
+            vt.fd.XY = (d1x * s1y + s1x * d1y) / (16.0 * dxx);
+            vt.fd.XZ = (d1x * s1z + s1x * d1z) / (16.0 * dxx);
+            vt.fd.YZ = (d1y * s1z + s1y * d1z) / (16.0 * dxx);
+            vt.fd.rx = d2x / (8.0 * p.dx);
+            vt.fd.ry = d2y / (8.0 * p.dx);
+            vt.fd.rz = d2z / (8.0 * p.dx);
+        }
+    }
     double du[8], dd[8], dwm[4];
 #pragma unroll
     for (int k = 0; k < 8; k++) du[k] = dd[k] = 0.0;
@@ -261,7 +328,7 @@ __global__ void __launch_bounds__(128) k_grad_rows(AsmParams p, const cx<double>
     for (int k = 0; k < 4; k++) dwm[k] = 0.0;
     // dwm index: 0 = wm1 (centre), 1 = wm2 (faces), 2 = wm3 (edges), 3 = wm4 (corners)
     rows_all(std::make_integer_sequence<int, 27>{}, region, mask, f, r1x, r1y, dxo8, c, om2, m2, m3, m4, U, L, ld,
-             m, n, p.nz, p.nx, du, dd, dwm, D, nn);
+             m, n, p.nz, p.nx, du, dd, dwm, vt, D, nn);
     // a free surface on top zeroes the upper cell means (setcoefs3d.f:177-192):
     // they no longer depend on the model
     if (p.fst && iz == 0) {
@@ -281,101 +348,11 @@ __global__ void __launch_bounds__(128) k_grad_rows(AsmParams p, const cx<double>
         dxr = dwm[0] * dw[0] + dwm[1] * dw[1] + dwm[2] * dw[2] + dwm[3] * dw[3];
     }
     D[(long long)GD_X * nn + n] = dxr;
+    D[(long long)GD_VP * nn + n] = vt.acc;
 }
 
 // ---------------------------------------------------------------------------
-// pass 1: vpreal derivative of the PML rows
-// ---------------------------------------------------------------------------
-template <int S>
-__device__ __forceinline__ void vp_slot(int region, unsigned mask, const NodeCoefs<double> &c,
-                                        const Stretch<double> &fd, cx<double> dr1x, cx<double> dr1y, double dxo8,
-                                        const double2 *U, const double2 *L, long long ld, int m, long long n, int nz,
-                                        int nx, double &acc)
-{
-    if (!((mask >> S) & 1u)) return;
-    constexpr int dy = S / 9 - 1, dxo = (S / 3) % 3 - 1, dz = S % 3 - 1;
-    const long long nb = n + dz + (long long)nz * (dxo + (long long)nx * dy);
-    cx<double> G[9], b[9];
-    if (region == REG_STENCIL) {
-        outer_sum(U, L, ld, m, n, nb, G);
-        stencil_block<S, double>(c, fd, 0.0, 0.0, 0.0, cx<double>(0), b);   // linear in the stretch
-        acc += re_dot9(b, G);
-    } else {
-        if constexpr (S != 2 && S != 20 && S != 8 && S != 26 && S != 13) return;   // zero TPFREE blocks
-        outer_sum(U, L, ld, m, n, nb, G);
-        // TPFREE blocks are affine in (r1x, r1y)
-        cx<double> b0[9], bx[9], by[9];
-        tpfree_block<S, double>(c, cx<double>(0), cx<double>(0), dxo8, b0);
-        tpfree_block<S, double>(c, cx<double>(1), cx<double>(0), dxo8, bx);
-        tpfree_block<S, double>(c, cx<double>(0), cx<double>(1), dxo8, by);
-#pragma unroll
-        for (int k = 0; k < 9; k++) b[k] = dr1x * (bx[k] - b0[k]) + dr1y * (by[k] - b0[k]);
-        acc += re_dot9(b, G);
-    }
-}
-
-template <int... Ss>
-__device__ __forceinline__ void vp_all(std::integer_sequence<int, Ss...>, int region, unsigned mask,
-                                       const NodeCoefs<double> &c, const Stretch<double> &fd, cx<double> dr1x,
-                                       cx<double> dr1y, double dxo8, const double2 *U, const double2 *L, long long ld,
-                                       int m, long long n, int nz, int nx, double &acc)
-{
-    (vp_slot<Ss>(region, mask, c, fd, dr1x, dr1y, dxo8, U, L, ld, m, n, nz, nx, acc), ...);
-}
-
-__global__ void __launch_bounds__(128) k_grad_vpreal(AsmParams p, const cx<double> *__restrict__ da,
-                                                     const cx<double> *__restrict__ mu,
-                                                     const double *__restrict__ ro, int m, long long ld,
-                                                     const double2 *__restrict__ U, const double2 *__restrict__ L,
-                                                     double *__restrict__ D)
-{
-    const long long nn = (long long)p.nx * p.ny * p.nz;
-    const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= nn) return;
-    const int iz = (int)(n % p.nz);
-    const int ix = (int)((n / p.nz) % p.nx);
-    const int iy = (int)(n / ((long long)p.nz * p.nx));
-    unsigned mask;
-    int region, zidx;
-    node_region(p, iz, ix, iy, region, zidx, mask);
-    double acc = 0.0;
-    const int jx = ix + 1, jy = iy + 1;
-    const bool in_pml = jx <= p.ipml || p.nx - jx + 1 <= p.ipml || jy <= p.ipml || p.ny - jy + 1 <= p.ipml ||
-                        (zidx > 0 && (zidx <= p.ipml || p.nz - zidx + 1 <= p.ipml));
-    if (region != REG_FIXED && in_pml) {
-        NodeCoefs<double> c;
-        gather_coefs<double>(da, mu, ro, p.nx, p.ny, p.nz, iz, ix, iy, p.fst != 0, c);
-        const cx<double> om(p.om_re, p.om_im);
-        const cx<double> eyeom = cx<double>(0.0, -1.0) * om;
-        cx<double> r1x, r1y, r1z, d1x, d1y, d1z, d2x, d2y, d2z;
-        axis_factor_d(jx, p.nx, p.ipml, p.dx, p.pmld, p.pmlf, c.vpreal, eyeom, r1x, d1x, d2x);
-        axis_factor_d(jy, p.ny, p.ipml, p.dx, p.pmld, p.pmlf, c.vpreal, eyeom, r1y, d1y, d2y);
-        Stretch<double> fd;
-        double dxo8 = 0;
-        if (region == REG_STENCIL) {
-            axis_factor_d(zidx, p.nz, p.ipml, p.dx, p.pmld, p.pmlf, c.vpreal, eyeom, r1z, d1z, d2z);
-            // derivative of build_stretch's scaled combinations
-            const double dxx = p.dx * p.dx;
-            fd.X2 = (2.0 * r1x * d1x) / (8.0 * dxx);
-            fd.Y2 = (2.0 * r1y * d1y) / (8.0 * dxx);
-            fd.Z2 = (2.0 * r1z * d1z) / (8.0 * dxx);
-            fd.XY = (d1x * r1y + r1x * d1y) / (16.0 * dxx);
-            fd.XZ = (d1x * r1z + r1x * d1z) / (16.0 * dxx);
-            fd.YZ = (d1y * r1z + r1y * d1z) / (16.0 * dxx);
-            fd.rx = d2x / (8.0 * p.dx);
-            fd.ry = d2y / (8.0 * p.dx);
-            fd.rz = d2z / (8.0 * p.dx);
-        } else {
-            dxo8 = 1.0 / (p.dx * 8.0);
-        }
-        vp_all(std::make_integer_sequence<int, 27>{}, region, mask, c, fd, d1x, d1y, dxo8, U, L, ld, m, n, p.nz,
-               p.nx, acc);
-    }
-    D[(long long)GD_VP * nn + n] = acc;
-}
-
-// ---------------------------------------------------------------------------
-// pass 2: gather per node and chain rule to (Vp, Vs, rho)
+// pass 1: gather per node and chain rule to (Vp, Vs, rho)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_grad_nodes(int nx, int ny, int nz, const cx<double> *__restrict__ da,
                                                     const cx<double> *__restrict__ mu,
@@ -477,8 +454,7 @@ int device_gradient(const wt3d_grid &g, const void *d_da, const void *d_mu, cons
     const auto *mu = (const cx<double> *)d_mu;
     const auto *U = (const double2 *)d_U;
     const auto *L = (const double2 *)d_L;
-    k_grad_rows<<<ceil_div(nn, 128), 128, 0, st>>>(p, da, mu, d_ro, m, ld, U, L, d_D);
-    k_grad_vpreal<<<ceil_div(nn, 128), 128, 0, st>>>(p, da, mu, d_ro, m, ld, U, L, d_D);
+    k_grad_rows<<<ceil_div(nn, GR_TH), GR_TH, 0, st>>>(p, da, mu, d_ro, m, ld, U, L, d_D);
     k_grad_nodes<<<ceil_div(nn, 256), 256, 0, st>>>(g.nx, g.ny, g.nz, da, mu, d_ro, d_vp, d_vs, d_rho, d_D, d_grad);
     WT_CUDA(cudaGetLastError());
     return WT3D_OK;
