@@ -215,19 +215,31 @@ __device__ __forceinline__ void lds_cx(const cx<double> *p, cx<double> (&a)[N])
     }
 }
 
-// 1 / d for |d|^2 = m2 between 1e-30 and 1e30: conj(d) times a hardware
-// approximation of 1 / m2, then one step of Newton's iteration z (2 - d z), which
-// leaves it more accurate than the scaled division, without its branches
-// (a panel takes 26 us with it, 34 us with cdiv).
-__device__ __forceinline__ cx<float> cinv_fast(const cx<float> d, float m2)
+// 1 / d for |d|^2 = m2 far from overflow and underflow (panel_group's bounds): conj(d)
+// times a hardware approximation of 1 / m2 (with one Newton step for its 20 bits in
+// FP64), then one step of Newton's iteration z (2 - d z), which leaves it more
+// accurate than the scaled division, without its branches and divisions (a panel
+// takes 26 us with it, 34 us with cdiv).
+__device__ __forceinline__ float rcp_approx(float x)
 {
     float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(m2));
-    const cx<float> z(d.re * r, -d.im * r);
-    const cx<float> e(fmaf(-d.re, z.re, fmaf(d.im, z.im, 1.f)), -fmaf(d.re, z.im, d.im * z.re));
-    return cx<float>(fmaf(z.re, e.re, fmaf(-z.im, e.im, z.re)), fmaf(z.re, e.im, fmaf(z.im, e.re, z.im)));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
-__device__ __forceinline__ cx<double> cinv_fast(const cx<double> d, double) { return cdiv(cx<double>(1), d); }
+__device__ __forceinline__ double rcp_approx(double x)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    return fma(r, fma(-x, r, 1.0), r);
+}
+template <class T>
+__device__ __forceinline__ cx<T> cinv_fast(const cx<T> d, T m2)
+{
+    const T r = rcp_approx(m2);
+    const cx<T> z(d.re * r, -d.im * r);
+    const cx<T> e(fma(-d.re, z.re, fma(d.im, z.im, T(1))), -fma(d.re, z.im, d.im * z.re));
+    return cx<T>(fma(z.re, e.re, fma(-z.im, e.im, z.re)), fma(z.re, e.im, fma(z.im, e.re, z.im)));
+}
 
 // PG columns of a panel in one warp, which holds two rows per lane (rows lane and
 // lane + 32; used: chosen before).  piv[jj] is the row that column jj chose.
@@ -302,7 +314,10 @@ __device__ __forceinline__ bool panel_group(cx<T> (&x0)[PG], cx<T> (&x1)[PG], bo
 // row.  A launch of few tiles took 55 - 80 us with the tile and its row swaps in
 // shared memory, 42 us with the tile in the registers of 256 threads and two
 // barriers per column, and takes 26 us.
-constexpr int PG = 8;
+// Columns per group.  complex128: warp 0 has a quarter of the SM's FP64 rate and is
+// what bounds the panel, so narrower groups leave more of the work to all warps (348 us
+// with groups of 8 and scaled divisions, 237 us with groups of 4).
+template <class T> constexpr int panel_group_cols = sizeof(T) == 4 ? 8 : 4;
 constexpr int PLD = KB + 2;   // row stride: 16-byte-aligned rows
 template <class T> constexpr size_t panel_smem() { return sizeof(cx<T>) * KB * PLD; }
 
@@ -316,6 +331,7 @@ __global__ void __launch_bounds__(256, 1) k_panel(const PanelTask *__restrict__ 
     const T thresh = (T)(pivot_rel * sqrt(__longlong_as_double((long long)*amax2)));
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T> *S = reinterpret_cast<cx<T> *>(smraw);   // KB x PLD
+    constexpr int PG = panel_group_cols<T>;
     __shared__ int spiv[2][PG], pos[KB];           // two sets: a group's is read while the next is found
     __shared__ unsigned s_used[2];                 // rows chosen so far: bits of rows 0-31, 32-63
     const PanelTask t = tasks[blockIdx.x];
