@@ -316,8 +316,8 @@ __device__ __forceinline__ bool panel_group(cx<T> (&x0)[PG], cx<T> (&x1)[PG], bo
 // barriers per column, and takes 26 us.
 // Columns per group.  complex128: warp 0 has a quarter of the SM's FP64 rate and is
 // what bounds the panel, so narrower groups leave more of the work to all warps (348 us
-// with groups of 8 and scaled divisions, 237 us with groups of 4).
-template <class T> constexpr int panel_group_cols = sizeof(T) == 4 ? 8 : 4;
+// with groups of 8 and scaled divisions, 237 us with groups of 4, 217 us with 2).
+template <class T> constexpr int panel_group_cols = sizeof(T) == 4 ? 8 : 2;
 constexpr int PLD = KB + 2;   // row stride: 16-byte-aligned rows
 template <class T> constexpr size_t panel_smem() { return sizeof(cx<T>) * KB * PLD; }
 
