@@ -1732,6 +1732,8 @@ extern "C" int wt3d_profile_solve(wt3d_solver *h, int m, double *out)
         rc = h->e64->profile_schedule(*sc, h->st, out);
     }
     if (rc) return rc;
+    ProductDone done{h};
+    if ((rc = product_prepare(h, h->st, m, false, nullptr))) return rc;
     cudaEventRecord(h->ev0, h->st);
     residual(h, h->st, m, h->Xn.p, h->Bn.p, h->Rn.p, false);
     cudaEventRecord(h->ev1, h->st);
