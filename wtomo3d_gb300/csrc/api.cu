@@ -1803,7 +1803,8 @@ extern "C" int wt3d_debug_fetch(wt3d_solver *h, int what, void *out, long long c
 // One product of the substitution passes on host complex64 arrays, as its kernel
 // computes it: out (M x nc) = op(A) in (K x nc), op(A) = A (M x K) or, with herm,
 // A^H (A K x M), rows lda apart; tri 1 or 2: A is a packed block inverse (M = K) and
-// its lower (unit) or upper triangle is meant.  K is cut into units of chunk rows.
+// its lower (unit) or upper triangle is meant.  K is cut into units of chunk rows;
+// one column with units of more than 64 rows goes to the kernel of large grids.
 extern "C" int wt3d_debug_skinny(int herm, int tri, int M, int K, int nc, int chunk, const void *A, int lda,
                                  const void *in, void *out)
 {
@@ -1832,7 +1833,7 @@ extern "C" int wt3d_debug_skinny(int herm, int tri, int M, int K, int nc, int ch
     if ((rc = du.upload(hu))) return rc;
     Engine<float>::sk_attributes();
     if (sk_tensor(nc, chunk)) sk_tensor_launch(nc, herm != 0, du.p, (int)hu.size(), dB.p, dC.p, 0);
-    else Engine<float>::sk_launch(nc, herm != 0, du.p, (int)hu.size(), dB.p, dC.p, 0);
+    else Engine<float>::sk_launch(nc, nc == 1 && chunk > 64, herm != 0, du.p, (int)hu.size(), dB.p, dC.p, 0);
     WT_CUDA(cudaGetLastError());
     WT_CUDA(cudaMemcpy(out, dC.p, sizeof(cx<float>) * M * nc, cudaMemcpyDeviceToHost));
     return WT3D_OK;

@@ -96,6 +96,13 @@ public:
     static constexpr int SBW = SB<T>;   // columns per diagonal block of the substitutions
     // units a launch of k_skinny is cut into, and the shortest K of a unit
     static constexpr int SK_SLOTS = 152 * 8, SK_KMIN = 64;
+    // factor entries from which the products of a pass over one column are k_gemv's (all of
+    // A^H are).  One kernel for a whole pass: launches of two that need different splits
+    // of L1 and shared memory wait for each other's SMs, and choosing by launch lost 10 %.
+    // Milliseconds per pass, k_skinny and k_gemv: 14x12x13 0.158 and 0.169, 20^3 0.268 and
+    // 0.279, 29x27x25 (1.2e8 entries) 0.50 and 0.47, 40^3 1.54 and 1.29, 64x64x48 5.4 and
+    // 4.2; A^H: 14x12x13 0.111 and 0.109, 20^3 0.27 and 0.20, 64x64x48 5.7 and 4.0.
+    static constexpr double GEMV_MIN_ENTRIES = 8e7;
     // outer block width of the two-level LU (WT3D_WB: a multiple of KB, 512 by default)
     const int WB = [] {
         const char *e = getenv("WT3D_WB");
@@ -233,29 +240,35 @@ public:
                              (int)SkCfg<T, NC>::smem(true));
     }
 
-    template <int NC, bool H>
-    static void sk_launch_t(const SkUnit *u, int n, const cx<T> *in, cx<T> *out, cudaStream_t st)
+    // a launch as programmatic dependent of the product before it
+    template <class Kernel>
+    static void sk_chain(Kernel k, size_t smem, const SkUnit *u, int n, const cx<T> *in, cx<T> *out, cudaStream_t st)
     {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)n);
         cfg.blockDim = dim3(SK_TH);
-        cfg.dynamicSmemBytes = SkCfg<T, NC>::smem(H);
+        cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
         cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see k_skinny
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, k_skinny<T, NC, H>, u, in, out);
+        cudaLaunchKernelEx(&cfg, k, u, in, out);
     }
     template <int NC>
     static void sk_launch_n(bool herm, const SkUnit *u, int n, const cx<T> *in, cx<T> *out, cudaStream_t st)
     {
-        if (herm) sk_launch_t<NC, true>(u, n, in, out, st);
-        else sk_launch_t<NC, false>(u, n, in, out, st);
+        if (herm) sk_chain(k_skinny<T, NC, true>, SkCfg<T, NC>::smem(true), u, n, in, out, st);
+        else sk_chain(k_skinny<T, NC, false>, SkCfg<T, NC>::smem(false), u, n, in, out, st);
     }
-    static void sk_launch(int nc, bool herm, const SkUnit *u, int n, const cx<T> *in, cx<T> *out, cudaStream_t st)
+    static void sk_launch(int nc, bool gemv, bool herm, const SkUnit *u, int n, const cx<T> *in, cx<T> *out,
+                          cudaStream_t st)
     {
+        if (gemv) {
+            sk_chain(herm ? k_gemv<T, true> : k_gemv<T, false>, 0, u, n, in, out, st);
+            return;
+        }
         if (nc == 1) sk_launch_n<1>(herm, u, n, in, out, st);
         else if (nc == 4) sk_launch_n<4>(herm, u, n, in, out, st);
         else if (nc == 8) sk_launch_n<8>(herm, u, n, in, out, st);
@@ -645,8 +658,9 @@ public:
                 }, tri ? LK_SUBSTEP : LK_TCGEMM, fl, by});
                 return;
             }
-        sc.launches.push_back({[psc, u0, nu, nc, herm, in, out](cudaStream_t st) {
-            sk_launch(nc, herm, psc->sk.p + u0, nu, in, out, st);
+        const bool gemv = nc == 1 && (herm || (double)fac.n >= GEMV_MIN_ENTRIES);
+        sc.launches.push_back({[psc, u0, nu, nc, gemv, herm, in, out](cudaStream_t st) {
+            sk_launch(nc, gemv, herm, psc->sk.p + u0, nu, in, out, st);
         }, tri ? LK_SUBSTEP : LK_GEMM, fl, by});
     }
 

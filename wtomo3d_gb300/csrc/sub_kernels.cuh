@@ -450,4 +450,148 @@ __global__ void __launch_bounds__(SK_TH) k_skinny(const SkUnit *__restrict__ uni
     }
 }
 
+// The products with one column, except forward passes of small grids.  Bound by
+// reading A, once, so entries go from memory to registers without a stop in shared
+// memory: as stored, a warp reads eight rows at a time, 32 neighbouring k each; of
+// A^H, a warp reads whole stored rows, a lane per output row.  The loads are a tile
+// ahead, the first two before the wait.  The large launches read 5.4 - 6 TB/s,
+// 3.3 - 3.7 with the ring of k_skinny.
+template <class T> __device__ __forceinline__ cx<T> ldg_cx(const cx<T> *p)
+{
+    if constexpr (sizeof(T) == 4) {
+        const float2 v = __ldg(reinterpret_cast<const float2 *>(p));
+        return cx<T>(v.x, v.y);
+    } else {
+        const double2 v = __ldg(reinterpret_cast<const double2 *>(p));
+        return cx<T>(v.x, v.y);
+    }
+}
+template <class T> __device__ __forceinline__ cx<T> ldcg_cx(const cx<T> *p)   // through L2
+{
+    if constexpr (sizeof(T) == 4) {
+        const float2 v = __ldcg(reinterpret_cast<const float2 *>(p));
+        return cx<T>(v.x, v.y);
+    } else {
+        const double2 v = __ldcg(reinterpret_cast<const double2 *>(p));
+        return cx<T>(v.x, v.y);
+    }
+}
+
+template <class T, bool H>
+__global__ void __launch_bounds__(SK_TH) k_gemv(const SkUnit *__restrict__ units, const cx<T> *__restrict__ in,
+                                                cx<T> *__restrict__ out)
+{
+    chain_start();
+    // a warp's tile of entries: R rows x U times 32 k; of A^H U k x 64 rows
+    constexpr int W = SK_TH / 32, R = H ? 2 : 8, U = (H ? 8 : 2) / ((int)sizeof(T) / 4);
+    __shared__ cx<T> x[SK_KMAX], red[H ? W : 1][H ? SK_M : 1];
+    const SkUnit u = units[blockIdx.x];
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, K = u.K, M = u.M;
+    const cx<T> *A = reinterpret_cast<const cx<T> *>(u.A);
+    // a tile of the warp: its rows' group and its step along k
+    struct Tile { int group, step; };
+    const int nk = H ? (K + U * W - 1) / (U * W) : (K + 32 * U - 1) / (32 * U);
+    const int ng = H ? 1 : max(0, (M - R * w + R * W - 1) / (R * W));
+    auto next = [&](Tile n) { return n.step + 1 < nk ? Tile{n.group, n.step + 1} : Tile{n.group + 1, 0}; };
+    auto row_of = [&](Tile n, int r) { return H ? lane + 32 * r : R * (w + W * n.group) + r; };
+    auto k_of = [&](Tile n, int j) { return H ? (n.step * U + j) * W + w : (n.step * U + j) * 32 + lane; };
+    auto load = [&](Tile n, cx<T>(&a)[U][R]) {
+        if (n.group >= ng) return;
+#pragma unroll
+        for (int j = 0; j < U; j++)
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int k = k_of(n, j), i = row_of(n, r);
+                a[j][r] = k < K && i < M ? ldg_cx(A + (H ? (long long)k * u.lda + i : (long long)i * u.lda + k))
+                                         : cx<T>(0);
+            }
+    };
+    cx<T> a[U][R], b[U][R], s[R];
+    Tile at{0, 0}, ahead = next(at);   // K >= 1
+    load(at, a);
+    load(ahead, b);
+    int row[SK_KMAX / SK_TH];   // of the input
+#pragma unroll
+    for (int j = 0; j < SK_KMAX / SK_TH; j++) {
+        const int k = tid + j * SK_TH;
+        row[j] = k >= K ? 0 : u.bmap ? u.bmap[k] : u.b0 + k;
+    }
+    chain_wait();
+#pragma unroll
+    for (int j = 0; j < SK_KMAX / SK_TH; j++)
+        if (tid + j * SK_TH < K) x[tid + j * SK_TH] = ldcg_cx(in + row[j]);
+    __syncthreads();
+    const bool cut = (u.flags & (SK_LOWER | SK_UPPER)) != 0;
+    auto store = [&](int i, cx<T> v) {
+        cx<T> *p = out + (u.cmap ? u.cmap[i] : u.c0 + i);
+        if (u.flags & SK_SUB) v = -v;
+        if (u.flags & SK_ATOM) red_add(p, v);
+        else if (u.flags & SK_SUB) *p = *p + v;
+        else *p = v;
+    };
+#pragma unroll
+    for (int r = 0; r < R; r++) s[r] = cx<T>(0);
+    auto sum = [&](Tile n, cx<T>(&a)[U][R]) {
+#pragma unroll
+        for (int j = 0; j < U; j++) {
+            const int k = k_of(n, j);
+            const cx<T> xk = k < K ? x[k] : cx<T>(0);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                cx<T> v = a[j][r];
+                if (cut) {   // the other triangle, as in k_skinny
+                    const int e = H ? row_of(n, r) - (k + u.d) : k + u.d - row_of(n, r);
+                    if ((u.flags & SK_UPPER) && e < 0) v = cx<T>(0);
+                    if ((u.flags & SK_LOWER) && e >= 0) v = cx<T>(e == 0 ? T(1) : T(0));
+                }
+                if constexpr (H) cmac_conj(s[r], v, xk);
+                else cmac(s[r], v, xk);
+            }
+        }
+        if constexpr (!H) {
+            if (n.step != nk - 1) return;
+            // the lanes' sums: halves of the 2 R values are exchanged, so that after
+            // four steps a pair of lanes holds one value
+            T v[2 * R];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                v[2 * r] = s[r].re;
+                v[2 * r + 1] = s[r].im;
+                s[r] = cx<T>(0);
+            }
+#pragma unroll
+            for (int h = R, o = 16; h >= 1; h /= 2, o /= 2)
+#pragma unroll
+                for (int i = 0; i < h; i++) {
+                    const T send = lane & o ? v[i] : v[i + h], keep = lane & o ? v[i + h] : v[i];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            const T re = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+            const T im = __shfl_down_sync(0xffffffffu, re, 2);
+            const int i = row_of(n, lane >> 2);
+            if (lane % 4 == 0 && i < M) store(i, cx<T>(re, im));
+        }
+    };
+    while (at.group < ng) {
+        sum(at, a);
+        at = next(ahead);
+        load(at, a);
+        if (ahead.group >= ng) break;
+        sum(ahead, b);
+        ahead = next(at);
+        load(ahead, b);
+    }
+    if constexpr (H) {
+        red[w][lane] = s[0];
+        red[w][lane + 32] = s[1];
+        __syncthreads();
+        if (tid < M) {
+            cx<T> v = red[0][tid];
+#pragma unroll
+            for (int q = 1; q < W; q++) v = v + red[q][tid];
+            store(tid, v);
+        }
+    }
+}
+
 }  // namespace wt3d
