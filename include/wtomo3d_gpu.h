@@ -384,7 +384,7 @@ int wt3d_profile_launches(wt3d_solver *h, int which, int m, double *out, int cap
 int wt3d_debug_fetch(wt3d_solver *h, int what, void *out, long long count);
 
 /* One complex64 GEMM C -= A B on host row-major arrays through the tensor-core
- * kernel (path 1), the SIMT kernel (path 0) or the tall-skinny tensor-core
+ * kernel (path 1), the SIMT kernel (path 0) or the tensor-core
  * kernel of the substitution passes (path 3, N <= 32; path 4 also gathers B
  * rows K-1-k and scatters C rows M-1-r; path 5 computes C -= A^H B with A
  * given as the K x M block, lda >= M); for checks of the kernels. */

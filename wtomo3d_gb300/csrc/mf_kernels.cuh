@@ -6,9 +6,8 @@
 // factor pool; the Schur/update block F22 (b x b) lives in one of two
 // level-parity update buffers.  Factorisation is right-looking blocked LU on
 // the first p columns with KB-wide panels and partial pivoting restricted to
-// the diagonal KB x KB tile; row interchanges are LINPACK style (applied to
-// the columns right of the panel only), so the forward solve applies them
-// block by block.
+// the diagonal KB x KB tile; a panel's row order (gord) applies to the columns
+// right of the panel only, and the substitutions' block inverses take it in.
 #pragma once
 #include "common.cuh"
 #include <algorithm>

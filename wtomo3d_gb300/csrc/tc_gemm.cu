@@ -670,12 +670,10 @@ int tc_init()
 // ---------------------------------------------------------------------------
 // C ABI check entry: one GEMM C -= A B on host complex64 arrays (row-major),
 // through the tensor-core path (path = 1), the SIMT path (path = 0) or the
-// tall-skinny tensor-core kernel of the solves (path = 3; path = 4 with a row
-// gather of B and a row scatter of C; path = 5 with C -= A^H B for A given as
-// the K x M block, lda >= M); paths 3 and 4 stream A by TMA when it is
-// 16-byte aligned with an even stride.  wt3d_bench_gemm also times path 2
-// (path 0 with N <= 32), path 3, and path 6 (path 3 with A always
-// copied by the loader warps).
+// substitutions' tensor-core kernel (path = 3; path = 4 with a row gather of B and
+// a row scatter of C; path = 5 with C -= A^H B for A given as the K x M block,
+// lda >= M).  wt3d_bench_gemm also takes path 2 (path 0 with N <= 32) and path 6
+// (path 3).
 // ---------------------------------------------------------------------------
 using namespace wt3d;
 extern "C" int wt3d_set_sm_reserve(int n)
