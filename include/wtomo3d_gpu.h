@@ -383,6 +383,10 @@ int wt3d_profile_launches(wt3d_solver *h, int which, int m, double *out, int cap
  * complex entries of the handle's precision; 1: pivot indices). */
 int wt3d_debug_fetch(wt3d_solver *h, int what, void *out, long long count);
 
+/* Y = op(A) X (op = A, or A^H with adjoint) on host complex128 arrays,
+ * column-major n x nrhs, by the product that the refinement uses; for checks. */
+int wt3d_debug_product(wt3d_solver *h, int adjoint, int nrhs, const void *X, void *Y);
+
 /* One complex64 GEMM C -= A B on host row-major arrays through the tensor-core
  * kernel (path 1), the SIMT kernel (path 0) or the tensor-core
  * kernel of the substitution passes (path 3, N <= 32; path 4 also gathers B

@@ -170,8 +170,8 @@ struct wt3d_solver {
     DevVec<double2> gmPart;
     DevVec<double> gmNorm, gmScale;
     void *pin = nullptr;                  // SolveHost
-    StreamBuf<uint4> epA;            // the operator's digits (product_prepare), per call
-    StreamBuf<int> epE;                   // ... exponents of its rows, its columns, blocks of nodes
+    StreamBuf<uint4> epA;                 // the operator's digits, then their bytes `below` (product_prepare), per call
+    StreamBuf<int> epE;                   // ... exponents of its rows, its columns; tasks of k_product_rest
     ProductOp epOp{};
     std::unique_ptr<Engine<float>> e32;
     std::unique_ptr<Engine<double>> e64;
@@ -240,6 +240,10 @@ struct ProductDone {
     wt3d_solver *h;
     ~ProductDone() { h->epA.release(); h->epE.release(); }
 };
+unsigned char *digits_below(const wt3d_solver *h)
+{
+    return reinterpret_cast<unsigned char *>(h->epA.p + (size_t)h->n * EP_SLOTS);
+}
 int product_prepare(wt3d_solver *h, cudaStream_t st, int m, bool adjoint, const double2 *abg)
 {
     if (h->general || sk_columns(std::min(m, MAXRHS)) < 8) return WT3D_OK;
@@ -251,22 +255,23 @@ int product_prepare(wt3d_solver *h, cudaStream_t st, int m, bool adjoint, const 
         cudaFuncSetAttribute(k_product_tc<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EP_SMEM);
         cudaFuncSetAttribute(k_product_tc<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EP_SMEM);
     });
-    const long long tiles =
-        (long long)ceil_div(h->grid.nx, EP_T) * ceil_div(h->grid.ny, EP_T) * ceil_div(h->grid.nz, EP_T);
-    if (h->epA.alloc((size_t)h->n * EP_SLOTS, st) || h->epE.alloc(2 * (size_t)h->n + tiles, st)) {
+    if (h->epA.alloc((size_t)h->n * (EP_SLOTS + (EP_SLOTS + 15) / 16), st) || h->epE.alloc(6 * (size_t)h->n + 2, st)) {
         h->epA.release();
         h->epE.release();
         return WT3D_OK;
     }
     h->epOp = ProductOp{h->irptr.p, h->jcptr.p, h->tpos.p, h->a.p, abg, adjoint ? 1 : 0};
-    int *pe = h->epE.p + h->n, *bmax = pe + h->n;
+    int *pe = h->epE.p + h->n;
     k_column_exponents<<<ceil_div(h->n * 32, 256), 256, 0, st>>>(h->n, h->epOp, pe);
-    k_block_exponents<<<ceil_div(tiles * 32, 256), 256, 0, st>>>(h->grid.nx, h->grid.ny, h->grid.nz, pe, bmax);
     k_operator_digits<<<ceil_div(h->n / 3 * 32, 256), 256, 0, st>>>(h->grid.nx, h->grid.ny, h->grid.nz, h->epOp, pe,
-                                                                     bmax, h->epA.p, h->epE.p);
+                                                                     h->epA.p, digits_below(h), h->epE.p);
     WT_CUDA(cudaGetLastError());
     return WT3D_OK;
 }
+
+// Kernels of a product: the tensor-core one and its rest where the call has prepared
+// the digits, else one.
+int product_kernels(const wt3d_solver *h, int nc) { return h->epA.p && nc >= 8 ? 2 : 1; }
 
 template <int NC>
 void product_tc(const wt3d_solver *h, cudaStream_t st, const double2 *X, const double2 *B, double2 *R, double *nr,
@@ -275,8 +280,11 @@ void product_tc(const wt3d_solver *h, cudaStream_t st, const double2 *X, const d
     const wt3d_grid &g = h->grid;
     const unsigned grid = (unsigned)((long long)ceil_div(g.nx, EP_T) * ceil_div(g.ny, EP_T) * ceil_div(g.nz, EP_T) *
                                      ceil_div(NC, EP_COLS));
-    k_product_tc<NC><<<grid, EP_THREADS, EP_SMEM, st>>>(g.nx, g.ny, g.nz, h->epOp, h->epA.p, h->epE.p,
-                                                        h->epE.p + h->n, X, B, R, nr, nb);
+    unsigned *rest = reinterpret_cast<unsigned *>(h->epE.p + 2 * h->n);
+    cudaMemsetAsync(rest, 0, sizeof(unsigned), st);
+    k_product_tc<NC><<<grid, EP_THREADS, EP_SMEM, st>>>(g.nx, g.ny, g.nz, h->epOp, h->epA.p, digits_below(h),
+                                                        h->epE.p, h->epE.p + h->n, X, B, R, nr, nb, rest);
+    k_product_rest<NC><<<EP_REST_BLOCKS, EP_REST_TH, 0, st>>>(h->epOp, X, B, R, nr, nb, rest);
 }
 
 // R = B - op(A) X (R = op(A) X when B is null), accumulating the squared
@@ -288,7 +296,7 @@ void residual(const wt3d_solver *h, cudaStream_t st, int m, const double2 *X, co
 {
     double *nr = h->norms.p, *nb = h->norms.p + MAXRHS;
     const int adj = adjoint ? 1 : 0, nc = sk_columns(m);
-    if (h->epA.p && nc >= 8) {
+    if (product_kernels(h, nc) == 2) {
         if (nc == 8) product_tc<8>(h, st, X, B, R, nr, nb);
         else if (nc == 16) product_tc<16>(h, st, X, B, R, nr, nb);
         else product_tc<32>(h, st, X, B, R, nr, nb);
@@ -424,7 +432,7 @@ int fgmres(wt3d_solver *h, Engine<T> &E, Schedule<T> *sc, int m, bool adjoint, d
             // w = op(A) z_j
             WT_CUDA(cudaMemsetAsync(h->norms.p, 0, sizeof(double) * 2 * MAXRHS, st));
             residual(h, st, m, Zd, nullptr, W, adjoint);
-            h->kernels_solve += sc->kernels() + 11;
+            h->kernels_solve += sc->kernels() + 10 + product_kernels(h, nc);
             if ((rc = orth(j + 1, W, h->gmH.p, ph.h1, false)) ||
                 (rc = orth(j + 1, W, h->gmH.p + (GM_KMAX + 1) * MAXRHS, ph.h2, true)))
                 return rc;
@@ -542,7 +550,7 @@ int refine(wt3d_solver *h, Engine<T> &E, int m, bool adjoint, double tol, int ma
                                            E.Y.p);
         rc = E.run(*sc, st);
         if (rc) return rc;
-        h->kernels_solve += sc->kernels() + 3;   // + gather, scatter, residual
+        h->kernels_solve += sc->kernels() + 2 + product_kernels(h, nc);   // + gather, scatter
         k_scatter_nat<T><<<nb, th, 0, st>>>(blk, nc, h->perm.p, E.scale.p, E.Y.p, h->Xn.p, first ? 0 : 1);
         WT_CUDA(cudaMemsetAsync(h->norms.p, 0, sizeof(double) * 2 * MAXRHS, st));
         residual(h, st, m, h->Xn.p, h->Bn.p, h->Rn.p, adjoint);
@@ -1797,6 +1805,29 @@ extern "C" int wt3d_debug_fetch(wt3d_solver *h, int what, void *out, long long c
     } else {
         return WT3D_ERR_ARG;
     }
+    return WT3D_OK;
+}
+
+// Y = op(A) X, host complex128 arrays (column-major), as the solves form it.
+extern "C" int wt3d_debug_product(wt3d_solver *h, int adjoint, int nrhs, const void *X, void *Y)
+{
+    if (!h || !X || !Y || nrhs < 1) return WT3D_ERR_ARG;
+    if (!h->have_values) { set_error("no operator"); return WT3D_ERR_STATE; }
+    const size_t bytes = sizeof(double2) * h->n * nrhs;
+    DevVec<double2> d;
+    if (int rc = d.alloc((size_t)h->n * nrhs)) return rc;
+    WT_CUDA(cudaMemcpy(d.p, X, bytes, cudaMemcpyHostToDevice));
+    if (int rc = product_prepare(h, h->st, nrhs, adjoint != 0, nullptr)) return rc;
+    ProductDone done{h};
+    for (int c0 = 0; c0 < nrhs; c0 += MAXRHS) {
+        const int m = std::min(MAXRHS, nrhs - c0);
+        to_rows(h, h->st, m, d.p + (size_t)c0 * h->n, h->Xn.p);
+        residual(h, h->st, m, h->Xn.p, nullptr, h->Rn.p, adjoint != 0);
+        to_columns(h, h->st, m, h->Rn.p, d.p + (size_t)c0 * h->n);
+    }
+    WT_CUDA(cudaGetLastError());
+    WT_CUDA(cudaStreamSynchronize(h->st));
+    WT_CUDA(cudaMemcpy(Y, d.p, bytes, cudaMemcpyDeviceToHost));
     return WT3D_OK;
 }
 
