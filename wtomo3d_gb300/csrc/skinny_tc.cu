@@ -3,39 +3,38 @@
 //
 // On the FP32 pipe these products are bound by its 73 TF/s (36 - 39 TF/s
 // reached: at 32 columns a factor entry costs 128 multiply-adds for its 8 bytes).
-// mma.sync in FP16 does 604 TF/s here, so that three products of split operands are
-// not the bound.  The split keeps FP32: every operand is hi + lo with two 11-bit
-// halves, scaled to FP16's range by a power of two of its own row of A or column of
-// B in every chunk of 16 k, so that the split is exact to 2^-24 of an operand and an
-// entry 2^-16 of its row's largest still has both halves in normal range.
-// hi hi + hi lo + lo hi of a k16 step is summed by the tensor cores, whose additions
-// truncate, and only then added to FP32 sums with rounded operations: longer sums in
-// the tensor cores had an error of 1.4e-5 at K = 1024, against 1.8e-7 here and
-// 4.0e-7 (8 columns) to 8.2e-7 (32) with FP32 multiply-adds.  The operands come
+// mma.sync in BF16 does 604 TF/s here, so that six products of split operands are
+// not the bound.  Every operand is h + m + l of 8 bits each, all 24 bits of FP32 and
+// (BF16 has FP32's exponents) whatever the magnitudes of the entries beside it; an
+// entry of A below 2^-110 is held to 2^-134, and one of X likewise against its column's
+// largest of 16 k, as the columns are scaled by powers of two.  Two halves in FP16
+// with three products take 2/3 to 3/4 of the time of a pass, but hold 22 bits, and
+// fewer of an entry below 2^-16 of the largest of its row or column in 16 k.
+// l h + h l + m m + m h + h m + h h of a k16 step is summed by the tensor cores, whose
+// additions truncate, and only then added to FP32 sums with rounded operations: the
+// error is 1.6e-7 at K = 1024 and 6e-8 at K = 32 (Gaussian entries), with FP32
+// multiply-adds 4.0e-7 (8 columns) to 8.2e-7 (32) and 8e-8.  The operands come
 // from tables through plain copies: a tcgen05 kernel that expanded B to real form in
 // memory and kept its sums in tensor memory reached 63 TF/s on the largest blocks.
 //
-// A pass of 64x64x48 with 32, 16, 8 columns: 14.2, 10.9, 8.7 ms with FP32 products
-// and that kernel, 9.0, 6.7, 6.5 ms with these; 48^3 with 32: 7.9 and 4.9 ms.  Bound
-// now by no single unit: 24576 x 1024 entries and 32 columns have shared memory 51 %,
-// the issue slots 36 % and the tensor pipe 34 % busy (1.3 waves of CTAs, four warps per
-// scheduler); with 8 columns the large launches read 3.7 TB/s.
-#include <cuda_fp16.h>
+// A pass of 64x64x48 with 32, 16, 8 columns: 15.4, 10.5, 7.1 ms with FP32 products,
+// 12.4, 8.0, 6.6 ms with these; 48^3 with 32: 8.2 and 6.7 ms.
+#include <cuda_bf16.h>
 #include "sub_kernels.cuh"
 
 namespace wt3d {
 
-__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
         "{%0, %1, %2, %3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ void mma_f16_0(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+__device__ __forceinline__ void mma_bf16_0(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
                  "{%10, %10, %10, %10};"
                  : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
@@ -66,38 +65,44 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
     return d;
 }
 
-// (re, im) scaled by s = hi + lo, each a pair of FP16 (re in the low half)
-__device__ __forceinline__ void split_pair(float2 v, float s, uint32_t &hi, uint32_t &lo)
+// (re, im) = h + m + l, each a pair of BF16 (re in the low half): 8 + 8 + 8 bits
+__device__ __forceinline__ uint32_t bf16_pair(float2 v)
 {
-    v = mul2(v, make_float2(s, s));
-    const __half2 h = __floats2half2_rn(v.x, v.y);
-    v = fma2(__half22float2(h), make_float2(-1.f, -1.f), v);
-    const __half2 l = __floats2half2_rn(v.x, v.y);
-    hi = *reinterpret_cast<const uint32_t *>(&h);
-    lo = *reinterpret_cast<const uint32_t *>(&l);
+    const __nv_bfloat162 b = __floats2bfloat162_rn(v.x, v.y);
+    return *reinterpret_cast<const uint32_t *>(&b);
+}
+__device__ __forceinline__ float2 minus_bf16(float2 v, uint32_t b)
+{
+    return fma2(make_float2(__uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u)), make_float2(-1.f, -1.f), v);
+}
+__device__ __forceinline__ void split_pair(float2 v, uint32_t &h, uint32_t &m, uint32_t &l)
+{
+    h = bf16_pair(v);
+    v = minus_bf16(v, h);
+    m = bf16_pair(v);
+    l = bf16_pair(minus_bf16(v, m));
 }
 
-// Powers of two that take a largest magnitude m to [2^14, 2^15), and back.  Infinity
-// and NaN stay what they are; what is below 2^-112 is scaled by 2^126.
+// Powers of two that take a largest magnitude m to [1, 2) ([2, 4) at the upper end of
+// the range), and back
 __device__ __forceinline__ void split_scale(float m, float &s, float &inv)
 {
-    const int e = max((int)(__float_as_uint(m) >> 23), 15);
-    s = __uint_as_float((unsigned)(268 - e) << 23);
-    inv = __uint_as_float((unsigned)(e - 14) << 23);
+    const int e = min(max((int)(__float_as_uint(m) >> 23), 1), 253);
+    s = __uint_as_float((unsigned)(254 - e) << 23);
+    inv = __uint_as_float((unsigned)e << 23);
 }
 
 __device__ __forceinline__ float max_abs(float m, float2 v) { return fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))); }
 
 // The units and their semantics are k_skinny's.  Four warps of 16 rows x NC
 // columns.  A complex entry is one 32-bit register of an A fragment - the pair
-// (re, im) along K; a warp splits each entry of its rows once and forms from it the
-// pairs whose products with (xr, xi) are the real and the imaginary part.  B is split
-// once per CTA, into shared memory in fragment order (two buffers, one barrier per
+// (re, im) along K, which a warp splits once; the pairs of B whose products with it are
+// the real and the imaginary part are formed in registers.  B is split once per CTA, into shared memory in fragment order (two buffers, one barrier per
 // chunk; loads one chunk ahead).  A comes through a ring per warp: fragments loaded
 // straight from the matrix touch eight rows with every load, and those loads, not the
 // tensor cores, were the bound.
 // Units of fewer than st_kmin k are summed with FP32 multiply-adds: a chunk's
-// truncated additions have an error of 9.7e-8 whatever its length.
+// truncated additions have an error of 6e-8 whatever its length.
 constexpr int ST_KC = 16;   // complex k of a chunk: two k16 steps of the tensor cores
 __host__ __device__ constexpr int st_kmin(int nc) { return nc == 8 ? 64 : 32; }
 constexpr int ST_NS = 3;    // stages of a warp's ring
@@ -113,7 +118,8 @@ __global__ void __launch_bounds__(SK_TH, 4) k_skinny_tc(const SkUnit *__restrict
     constexpr int CW = NC / 4;              // columns a warp splits
     constexpr int KMIN = st_kmin(NC);
     __shared__ __align__(16) float2 Aw[SK_TH / 32][ST_NS][16 * ST_LD];   // a ring per warp
-    __shared__ uint4 Bf[2][KMIN * NC / 4 > 2 * NT * 32 ? KMIN * NC / 4 : 2 * NT * 32];
+    __shared__ uint4 Bf[2][KMIN * NC / 4 > 2 * NT * 32 ? KMIN * NC / 4 : 2 * NT * 32];   // h, m
+    __shared__ uint2 Bl[2][2 * NT * 32];                                                 // l
     __shared__ float2 sb[2][NC / 2];
     __shared__ int brow[SK_KMAX], crow[SK_M];
     const SkUnit u = units[blockIdx.x];
@@ -228,9 +234,14 @@ __global__ void __launch_bounds__(SK_TH, 4) k_skinny_tc(const SkUnit *__restrict
 #pragma unroll
             for (int j = 0; j < XV; j++) {
                 uint4 v;
-                split_pair(x[2 * j], sc, v.x, v.z);
-                split_pair(x[2 * j + 1], sc, v.y, v.w);
-                if (xw) Bf[buf][((xs + j) * NT + (xc >> 3)) * 32 + 4 * (xc & 7) + q] = v;
+                uint2 l;
+                split_pair(mul2(x[2 * j], make_float2(sc, sc)), v.x, v.z, l.x);
+                split_pair(mul2(x[2 * j + 1], make_float2(sc, sc)), v.y, v.w, l.y);
+                const int at = ((xs + j) * NT + (xc >> 3)) * 32 + 4 * (xc & 7) + q;
+                if (xw) {
+                    Bf[buf][at] = v;
+                    Bl[buf][at] = l;
+                }
             }
         }
         if (s + 1 < nst) load_x(s + 1);
@@ -268,58 +279,42 @@ __global__ void __launch_bounds__(SK_TH, 4) k_skinny_tc(const SkUnit *__restrict
                 }
             }
         }
-        float m0 = 0.f, m1 = 0.f, s0, s1, i0, i1;
+        uint32_t ah[2][4], am[2][4], al[2][4];   // [k16 step]
 #pragma unroll
-        for (int h = 0; h < 4; h++) {
-            m0 = max_abs(m0, a[2 * h]);
-            m1 = max_abs(m1, a[2 * h + 1]);
-        }
-#pragma unroll
-        for (int o = 1; o <= 2; o *= 2) {
-            m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
-            m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-        }
-        split_scale(m0, s0, i0);
-        split_scale(m1, s1, i1);
-        // [re, im][k16 step]: (ar, -ai) and (ai, ar); for A^H (ar, ai) and (-ai, ar)
-        uint32_t ah[2][2][4], al[2][2][4];
-#pragma unroll
-        for (int h = 0; h < 8; h++) {
-            uint32_t vh, vl;
-            split_pair(a[h], h & 1 ? s1 : s0, vh, vl);
-            constexpr uint32_t NR = H ? 0u : 0x80000000u, NI = H ? 0x8000u : 0u;
-            ah[0][h >> 2][h & 3] = vh ^ NR;
-            al[0][h >> 2][h & 3] = vl ^ NR;
-            ah[1][h >> 2][h & 3] = __byte_perm(vh, 0, 0x1032) ^ NI;
-            al[1][h >> 2][h & 3] = __byte_perm(vl, 0, 0x1032) ^ NI;
-        }
+        for (int h = 0; h < 8; h++) split_pair(a[h], ah[h >> 2][h & 3], am[h >> 2][h & 3], al[h >> 2][h & 3]);
 #pragma unroll
         for (int t = 0; t < NT; t++) {
-            uint4 b[2];
             float d[2][2][4];   // [re, im][k16 step]: four independent chains
 #pragma unroll
-            for (int e = 0; e < 2; e++) b[e] = Bf[buf][(e * NT + t) * 32 + lane];
-            // the small products first
+            for (int e = 0; e < 2; e++) {
+                const uint4 f = Bf[buf][(e * NT + t) * 32 + lane];
+                const uint2 f2 = Bl[buf][(e * NT + t) * 32 + lane];
 #pragma unroll
-            for (int p = 0; p < 3; p++)
-#pragma unroll
-                for (int c = 0; c < 2; c++)
-#pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        if (p == 0) mma_f16_0(d[c][e], al[c][e], b[e].x, b[e].y);
-                        else if (p == 1) mma_f16(d[c][e], ah[c][e], b[e].z, b[e].w);
-                        else mma_f16(d[c][e], ah[c][e], b[e].x, b[e].y);
-                    }
+                for (int c = 0; c < 2; c++) {
+                    // (xr, -xi) and (xi, xr); for A^H (xr, xi) and (xi, -xr)
+                    auto form = [&](uint32_t v) {
+                        if (c == 0) return H ? v : v ^ 0x80000000u;
+                        const uint32_t r = __byte_perm(v, 0, 0x1032);
+                        return H ? r ^ 0x80000000u : r;
+                    };
+                    const uint32_t h0 = form(f.x), h1 = form(f.y), m0 = form(f.z), m1 = form(f.w), l0 = form(f2.x),
+                                   l1 = form(f2.y);
+                    // the small products first
+                    mma_bf16_0(d[c][e], al[e], h0, h1);
+                    mma_bf16(d[c][e], ah[e], l0, l1);
+                    mma_bf16(d[c][e], am[e], m0, m1);
+                    mma_bf16(d[c][e], am[e], h0, h1);
+                    mma_bf16(d[c][e], ah[e], m0, m1);
+                    mma_bf16(d[c][e], ah[e], h0, h1);
+                }
+            }
             const float2 sx = sb[buf][4 * t + q];
 #pragma unroll
             for (int c = 0; c < 2; c++)
 #pragma unroll
                 for (int r = 0; r < 2; r++) {
-                    // one factor after the other: their product may be below FP32's range
                     const float(&d0)[4] = d[c][0], (&d1)[4] = d[c][1];
-                    const float i = r ? i1 : i0;
-                    float2 v = add2(make_float2(d0[2 * r], d0[2 * r + 1]), make_float2(d1[2 * r], d1[2 * r + 1]));
-                    v = mul2(v, make_float2(i, i));
+                    const float2 v = add2(make_float2(d0[2 * r], d0[2 * r + 1]), make_float2(d1[2 * r], d1[2 * r + 1]));
                     acc[t][c][r] = fma2(v, sx, acc[t][c][r]);
                 }
         }

@@ -263,9 +263,10 @@ inline int sk_columns(int m) { return m <= 1 ? 1 : m <= 4 ? 4 : m <= 8 ? 8 : m <
 
 // Products that go to the tensor cores (skinny_tc.cu), by width and K per unit.  At 8
 // columns a launch of units shorter than 128 k is faster on the FP32 pipe: a pass of
-// 24x22x20 takes 0.55 ms with it, 0.65 ms on the tensor cores; one of 64x64x48 8.7 ms
-// and 6.5 ms.  At 16 and 32 columns the tensor cores win at every size measured
-// (33x31x29 with 16: 1.50 and 1.13 ms).
+// 24x22x20 took 0.55 ms with it, 0.65 ms on the tensor cores; one of 64x64x48 takes 7.1
+// and 6.6 ms.  At 16 and 32 columns the tensor cores win at every size measured, FP32 and
+// they in ms per pass: 24x22x20 0.68 and 0.58, 0.86 and 0.75; 40^3 3.2 and 2.5, 4.4 and
+// 3.7; 64x64x48 10.5 and 8.0, 15.4 and 12.4.
 inline bool sk_tensor(int nc, int chunk) { return nc > 8 || (nc == 8 && chunk >= 128); }
 void sk_tensor_launch(int nc, bool herm, const SkUnit *u, int n, const cx<float> *in, cx<float> *out, cudaStream_t st);
 
@@ -306,7 +307,7 @@ __device__ __forceinline__ void red_add(cx<double> *p, const cx<double> v)
 // previous product: the factor entries, which no product writes, are on their
 // way before the wait for it.  One pass, against KB-wide steps and 128 x 32
 // products that computed 32 columns whatever the pass held: 40^3 with 1 column
-// 11.4 -> 2.0 ms, with 32 columns 12.4 -> 4.4 ms (2.8 ms on the tensor cores),
+// 11.4 -> 2.0 ms, with 32 columns 12.4 -> 4.4 ms (3.7 ms on the tensor cores),
 // complex128 16x15x14 with 4 columns 23 -> 1.1 ms.
 template <class T, int NC, bool H>
 __global__ void __launch_bounds__(SK_TH) k_skinny(const SkUnit *__restrict__ units, const cx<T> *__restrict__ in,
