@@ -93,16 +93,20 @@ def make_stream(n_requests, rate_hz, seed, grids=((48, 48, 48), (64, 64, 64), (9
 class Server:
     """Continuous-batching scheduler over a factorisation cache.
 
-    While the cache is thrashing - the factorisations that a new key would evict
-    were in use less than `thrash_s` ago - the key's requests are held for up to
-    `hold_s` before it is admitted, so that others for the same key can join and
-    share its factorisation.  A cache that is not under pressure never holds.
-    Small grids make this worth it: a 24x22x18 factorisation is opened in 11 ms
-    and solved with in 4, so requests for one key 26 ms apart no longer met in a
-    batch, and every one of 18 requests at 40 Hz over 12 keys had its own."""
+    With `hold_s` above 0, and only then: while the cache is thrashing - the
+    factorisations that a new key would evict were in use less than `thrash_s`
+    ago - the key, and the keys that came after it, wait for up to `hold_s` from
+    its first request on, so that other requests for it can join and share its
+    factorisation.  It trades latency for factorisations, so it is the caller's
+    choice: a 24x22x18 factorisation is opened in 11 ms and solved with in 4, and
+    18 requests at 40 Hz over 12 keys, those of one key 26 ms apart and more, took
+    one factorisation each."""
 
-    def __init__(self, backend, budget_bytes=120e9, max_batch=64, workers=4, hold_s=0.04, thrash_s=0.1):
-        self.hold_s, self.thrash_s = float(hold_s), float(thrash_s)
+    HOLD_S, THRASH_S = 0.0, 0.1               # where the caller gives none
+
+    def __init__(self, backend, budget_bytes=120e9, max_batch=64, workers=4, hold_s=None, thrash_s=None):
+        self.hold_s = float(self.HOLD_S if hold_s is None else hold_s)
+        self.thrash_s = float(self.THRASH_S if thrash_s is None else thrash_s)
         self.held = {}                        # key -> time of its first request waiting for admission
         self.backend = backend
         self.budget = float(budget_bytes)
