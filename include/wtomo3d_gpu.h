@@ -383,6 +383,12 @@ int wt3d_profile_launches(wt3d_solver *h, int which, int m, double *out, int cap
  * complex entries of the handle's precision; 1: pivot indices). */
 int wt3d_debug_fetch(wt3d_solver *h, int what, void *out, long long count);
 
+/* The nth device allocation that the calling thread makes from here on for
+ * handles and calls fails, once, as for lack of memory (0: none); for checks of
+ * what then happens.  Returns what was left of the number before: 0 once that
+ * allocation has come. */
+int wt3d_debug_fail_alloc(int nth);
+
 /* Y = op(A) X (op = A, or A^H with adjoint) on host complex128 arrays,
  * column-major n x nrhs, by the product that the refinement uses; for checks. */
 int wt3d_debug_product(wt3d_solver *h, int adjoint, int nrhs, const void *X, void *Y);

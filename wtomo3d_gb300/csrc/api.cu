@@ -18,6 +18,9 @@ namespace wt3d {
 static thread_local std::string g_err;
 void set_error(const std::string &msg) { g_err = msg; }
 
+static thread_local int g_fail_alloc = 0;   // allocations until the one that fails, 0 for none
+bool alloc_is_to_fail() { return g_fail_alloc > 0 && --g_fail_alloc == 0; }
+
 // One pool per device, made at its first use and kept for the process; empty
 // between handles.  A stream takes memory that another has released only where
 // that release has completed: no stream is made to wait for another's work.
@@ -378,7 +381,19 @@ int fgmres(wt3d_solver *h, Engine<T> &E, Schedule<T> *sc, int m, bool adjoint, d
     // handle's resident memory), in stream order on the handle's solve
     // stream, so that taking and returning them never waits for work of
     // other handles
-    if ((rc = h->gmV.alloc((size_t)blk * (kr + 2), st)) || (rc = h->gmZ.alloc(sizeof(cx<T>) * blk * kr, st))) return rc;
+    auto bases = [&]() -> int {
+        int e = h->gmV.alloc((size_t)blk * (kr + 2), st);
+        return e ? e : h->gmZ.alloc(sizeof(cx<T>) * blk * kr, st);
+    };
+    if ((rc = bases()) && h->epA.p) {
+        // the operator's digits are a convenience, the bases are not: what is left of
+        // the call uses the FP64 kernel
+        h->gmV.release();
+        h->epA.release();
+        h->epE.release();
+        rc = bases();
+    }
+    if (rc) { h->gmV.release(); return rc; }
     struct Release {
         wt3d_solver *h;
         ~Release() { h->gmV.release(); h->gmZ.release(); }
@@ -1806,6 +1821,16 @@ extern "C" int wt3d_debug_fetch(wt3d_solver *h, int what, void *out, long long c
         return WT3D_ERR_ARG;
     }
     return WT3D_OK;
+}
+
+// The nth device allocation from here on that the calling thread makes for handles and
+// calls fails, once, as for lack of memory; 0: none.  Returns what was left of the
+// number before, 0 once that allocation has come.
+extern "C" int wt3d_debug_fail_alloc(int nth)
+{
+    const int left = g_fail_alloc;
+    g_fail_alloc = nth;
+    return left;
 }
 
 // Y = op(A) X, host complex128 arrays (column-major), as the solves form it.

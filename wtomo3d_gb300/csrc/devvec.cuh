@@ -13,6 +13,15 @@ constexpr unsigned long long SCRATCH_KEEP = 16ull << 30;
 cudaMemPool_t scratch_pool();
 void scratch_trim();
 
+// For checks (wt3d_debug_fail_alloc): whether this allocation of the calling thread is
+// the one that is to fail as for lack of memory.
+bool alloc_is_to_fail();
+inline int no_memory(const char *call, size_t bytes, const char *why)
+{
+    set_error(std::string(call) + "(" + std::to_string(bytes) + " B): " + why);
+    return WT3D_ERR_NOMEM;
+}
+
 template <class T>
 struct DevVec {
     T *p = nullptr;
@@ -21,6 +30,7 @@ struct DevVec {
     {
         free();
         if (count == 0) return WT3D_OK;
+        if (alloc_is_to_fail()) return no_memory("cudaMalloc", count * sizeof(T), "failed for a check");
         cudaError_t e = cudaMalloc(&p, count * sizeof(T));
         if (e == cudaErrorMemoryAllocation) {   // what the scratch pool keeps may be enough
             cudaGetLastError();
@@ -30,8 +40,7 @@ struct DevVec {
         if (e != cudaSuccess) {
             cudaGetLastError();   // an allocation failure is not sticky: clear it for later checks
             p = nullptr;
-            set_error(std::string("cudaMalloc(") + std::to_string(count * sizeof(T)) + " B): " + cudaGetErrorString(e));
-            return WT3D_ERR_NOMEM;
+            return no_memory("cudaMalloc", count * sizeof(T), cudaGetErrorString(e));
         }
         n = count;
         return WT3D_OK;
@@ -75,15 +84,14 @@ struct StreamBuf {
         release();
         st = s;
         if (count == 0) return WT3D_OK;
+        if (alloc_is_to_fail()) return no_memory("cudaMallocAsync", count * sizeof(T), "failed for a check");
         cudaMemPool_t pool = scratch_pool();
         cudaError_t e = pool ? cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), count * sizeof(T), pool, s)
                              : cudaMallocAsync(reinterpret_cast<void **>(&p), count * sizeof(T), s);
         if (e != cudaSuccess) {
             cudaGetLastError();
             p = nullptr;
-            set_error(std::string("cudaMallocAsync(") + std::to_string(count * sizeof(T)) +
-                      " B): " + cudaGetErrorString(e));
-            return WT3D_ERR_NOMEM;
+            return no_memory("cudaMallocAsync", count * sizeof(T), cudaGetErrorString(e));
         }
         n = count;
         return WT3D_OK;
