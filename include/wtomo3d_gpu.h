@@ -389,6 +389,9 @@ int wt3d_debug_fetch(wt3d_solver *h, int what, void *out, long long count);
  * allocation has come. */
 int wt3d_debug_fail_alloc(int nth);
 
+/* 1 if nothing is running or queued on the handle's streams, else 0. */
+int wt3d_debug_idle(wt3d_solver *h);
+
 /* Y = op(A) X (op = A, or A^H with adjoint) on host complex128 arrays,
  * column-major n x nrhs, by the product that the refinement uses; for checks. */
 int wt3d_debug_product(wt3d_solver *h, int adjoint, int nrhs, const void *X, void *Y);

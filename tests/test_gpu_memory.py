@@ -56,3 +56,28 @@ def test_without_memory_for_the_bases(solver):
     assert wt.lib().wt3d_debug_fail_alloc(0) == 0
     Y = s.solve(B, tol=1e-10, maxit=60)
     assert np.linalg.norm(X - Y) <= 1e-4 * np.linalg.norm(X)
+
+
+def test_nothing_runs_after_an_error():
+    """A call that fails has finished with its caller's buffers: here before its first
+    pass, with the columns' conversion queued behind the caller's own work."""
+    import ctypes
+    import torch
+    dims = (24, 22, 20)
+    g = Grid(*dims, 20.0, pmld=5 * 20.0, fst=1)
+    L = wt.lib()
+    with wt.Solver(g) as s:
+        s.set_model(*model.layered_random(*dims, 20.0, seed=1))
+        s.factor(2 * np.pi)
+        F = torch.randn((32, s.n), dtype=torch.complex128, device="cuda")
+        X = torch.zeros_like(F)
+        work = torch.zeros(1 << 27, device="cuda")
+        p = lambda t: ctypes.c_void_p(t.data_ptr())
+        torch.cuda.synchronize()
+        for _ in range(400):      # 1 GB each: 60 ms and more
+            work.mul_(1.0)
+        L.wt3d_debug_fail_alloc(3)     # digits 1, 2; the pass's schedule
+        rc = L.wt3d_solve_device(s._h, 32, p(F), p(X), 1e-10, 10, None, None, 0)
+        idle = L.wt3d_debug_idle(s._h)
+        assert L.wt3d_debug_fail_alloc(0) == 0
+        assert rc == wt.WT3D_ERR_NOMEM and idle == 1

@@ -613,6 +613,7 @@ int solve_dev_cm(wt3d_solver *h, int nrhs, const double2 *d_B, double2 *d_X, dou
                  int *iters, bool adjoint)
 {
     if (!h->have_factor) { set_error("solve before factor"); return WT3D_ERR_STATE; }
+    StreamDone drained{h->sts};
     if (int rc = after_legacy(h, h->sts)) return rc;
     const long long n = h->n;
     int worst_rc = WT3D_OK, maxits = 0;
@@ -1068,6 +1069,7 @@ int wt3d_set_background(wt3d_solver *h, const float *vp, const float *vs, const 
     const long long nn = h->n / 3;
     int rc;
     if (!h->bgro.p && ((rc = h->bgda.alloc(nn)) || (rc = h->bgmu.alloc(nn)) || (rc = h->bgro.alloc(nn)))) return rc;
+    StreamDone drained{h->st};
     StreamBuf<float> dvp, dvs, drho;   // per-call temporaries in stream order (see StreamBuf)
     if ((rc = dvp.alloc(nn, h->st)) || (rc = dvs.alloc(nn, h->st)) || (rc = drho.alloc(nn, h->st))) return rc;
     WT_CUDA(cudaMemcpyAsync(dvp.p, vp, sizeof(float) * nn, cudaMemcpyHostToDevice, h->st));
@@ -1102,6 +1104,7 @@ int wt3d_rhs_planewave(wt3d_solver *h, const wt3d_layered1d *m, int nsrc, const 
                               h->st)))
         return rc;
     const int nl = m->nl;
+    StreamDone drained{h->st};
     if ((rc = product_prepare(h, h->st, nsrc, false, h->abg.p))) return rc;
     ProductDone done{h};
     for (int c0 = 0; c0 < nsrc; c0 += MAXRHS) {
@@ -1151,6 +1154,7 @@ int wt3d_set_values_c64(wt3d_solver *h, const float _Complex *a)
 {
     if (!h || !a) { set_error("null pointer"); return WT3D_ERR_ARG; }
     const long long nin = h->vmap.p ? h->nnz_in : h->nnz;   // caller entries
+    StreamDone drained{h->st};
     StreamBuf<float2> tmp;   // per-call, in stream order (see StreamBuf)
     int rc = tmp.alloc(nin, h->st);
     if (rc) return rc;
@@ -1171,6 +1175,7 @@ int wt3d_set_values_c128(wt3d_solver *h, const double _Complex *a)
 {
     if (!h || !a) { set_error("null pointer"); return WT3D_ERR_ARG; }
     if (h->vmap.p) {
+        StreamDone drained{h->st};
         StreamBuf<double2> tmp;
         int rc = tmp.alloc(h->nnz_in, h->st);
         if (rc) return rc;
@@ -1204,6 +1209,7 @@ static int solve_host(wt3d_solver *h, int nrhs, const double _Complex *B, double
 {
     if (!h || nrhs < 1 || !B || !X) { set_error("wt3d_solve: bad arguments"); return WT3D_ERR_ARG; }
     if (!h->have_factor) { set_error("solve before factor"); return WT3D_ERR_STATE; }
+    StreamDone drained{h->sts};
     StreamBuf<double2> dB, dX;   // per-call, in the solve stream's order (see StreamBuf)
     int rc;
     if ((rc = dB.alloc((size_t)h->n * nrhs, h->sts)) || (rc = dX.alloc((size_t)h->n * nrhs, h->sts))) return rc;
@@ -1232,6 +1238,7 @@ int wt3d_apply(wt3d_solver *h, int nrhs, const double _Complex *X, double _Compl
     if (!h || nrhs < 1 || !X || !Y) { set_error("wt3d_apply: bad arguments"); return WT3D_ERR_ARG; }
     if (!h->have_values) { set_error("no operator"); return WT3D_ERR_STATE; }
     const long long n = h->n;
+    StreamDone drained{h->st};
     StreamBuf<double2> dX;   // per-call, in stream order (see StreamBuf)
     int rc = dX.alloc((size_t)n * nrhs, h->st);
     if (rc || (rc = product_prepare(h, h->st, nrhs, false, nullptr))) return rc;
@@ -1255,6 +1262,7 @@ int wt3d_apply_device(wt3d_solver *h, int nrhs, const void *d_X, void *d_Y)
     if (int rc0 = after_legacy(h, h->st)) return rc0;
     if (!h->have_values) { set_error("no operator"); return WT3D_ERR_STATE; }
     const long long n = h->n;
+    StreamDone drained{h->st};
     if (int rc = product_prepare(h, h->st, nrhs, false, nullptr)) return rc;
     ProductDone done{h};
     for (int c0 = 0; c0 < nrhs; c0 += MAXRHS) {
@@ -1320,6 +1328,7 @@ int wt3d_misfit_gradient(wt3d_solver *h, int nsrc, const void *d_F, const void *
     const long long nd = (long long)nsrc * nrec * 3;
     // taken and released in the order of h->st; the solves on h->sts start after
     // the synchronisation below and are done when they return
+    StreamDone drained{h->st};
     StreamBuf<double2> X, S, Lm, dd, dp, dr;
     StreamBuf<long long> drec;
     StreamBuf<double> dg;
@@ -1400,6 +1409,7 @@ int wt3d_rhs_sources(wt3d_solver *h, int nsrc, const double *xyz, const int *com
         const std::complex<double> v = sterm ? reinterpret_cast<const std::complex<double> *>(sterm)[j] : 1.0;
         st[j] = make_double2(v.real(), v.imag());
     }
+    StreamDone drained{h->st};
     StreamBuf<int> dcol, dcmp;
     StreamBuf<long long> dnd;
     StreamBuf<double> dw;
@@ -1435,6 +1445,7 @@ int wt3d_sample_receivers(wt3d_solver *h, int nrhs, const void *d_U, int nrec, c
         w.insert(w.end(), b.begin(), b.end());
         start.push_back((int)nd.size());
     }
+    StreamDone drained{h->st};
     StreamBuf<int> dstart;
     StreamBuf<long long> dnd;
     StreamBuf<double> dw;
@@ -1755,6 +1766,7 @@ extern "C" int wt3d_profile_solve(wt3d_solver *h, int m, double *out)
         rc = h->e64->profile_schedule(*sc, h->st, out);
     }
     if (rc) return rc;
+    StreamDone drained{h->st};
     ProductDone done{h};
     if ((rc = product_prepare(h, h->st, m, false, nullptr))) return rc;
     cudaEventRecord(h->ev0, h->st);
@@ -1833,6 +1845,12 @@ extern "C" int wt3d_debug_fail_alloc(int nth)
     return left;
 }
 
+// Whether nothing is running or queued on the handle's streams.
+extern "C" int wt3d_debug_idle(wt3d_solver *h)
+{
+    return h && cudaStreamQuery(h->st) == cudaSuccess && cudaStreamQuery(h->sts) == cudaSuccess;
+}
+
 // Y = op(A) X, host complex128 arrays (column-major), as the solves form it.
 extern "C" int wt3d_debug_product(wt3d_solver *h, int adjoint, int nrhs, const void *X, void *Y)
 {
@@ -1842,6 +1860,7 @@ extern "C" int wt3d_debug_product(wt3d_solver *h, int adjoint, int nrhs, const v
     DevVec<double2> d;
     if (int rc = d.alloc((size_t)h->n * nrhs)) return rc;
     WT_CUDA(cudaMemcpy(d.p, X, bytes, cudaMemcpyHostToDevice));
+    StreamDone drained{h->st};
     if (int rc = product_prepare(h, h->st, nrhs, adjoint != 0, nullptr)) return rc;
     ProductDone done{h};
     for (int c0 = 0; c0 < nrhs; c0 += MAXRHS) {

@@ -67,6 +67,16 @@ struct DevVec {
     DevVec &operator=(const DevVec &) = delete;
 };
 
+// Waits for a stream at the end of its scope.  Declared before the buffers of a call,
+// so that on every way out, errors included, nothing of the call is running any more
+// when it returns (its caller may free what it passed in, and buffers released on
+// another stream would be given to others while still in use), and the buffers'
+// release has been seen, without which the pool cannot be trimmed.
+struct StreamDone {
+    cudaStream_t st;
+    ~StreamDone() { cudaStreamSynchronize(st); }
+};
+
 // Stream-ordered device buffer from the scratch pool.  Releasing a cudaMalloc
 // buffer with cudaFree waits for the whole device, so a per-call temporary of one
 // handle would wait for another handle's factorisation; these buffers are
