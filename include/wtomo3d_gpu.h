@@ -318,6 +318,15 @@ int wt3d_memcpy(wt3d_solver *h, void *dst, const void *src, long long bytes);
 /* Free and total device memory of the current device. */
 int wt3d_mem_info(double *free_bytes, double *total_bytes);
 
+/* The pool of the current device that calls take their temporaries from:
+ * bytes that it holds (they are not in wt3d_mem_info's free bytes) and those
+ * in use.  The rest is kept between calls, up to 16 GB while a handle exists;
+ * the library's own allocations take it back when they would fail, other
+ * allocators of the process do not: wt3d_scratch_trim returns it to the
+ * device, for them. */
+int wt3d_scratch_info(double *reserved_bytes, double *used_bytes);
+int wt3d_scratch_trim(void);
+
 /* Device memory of a handle for grid g, before creating it (host analysis
  * only, cached per grid): out[0] = bytes a factored handle holds on its own,
  * out[1] = additional bytes once plane-wave sources are built (background

@@ -81,3 +81,22 @@ def test_nothing_runs_after_an_error():
         idle = L.wt3d_debug_idle(s._h)
         assert L.wt3d_debug_fail_alloc(0) == 0
         assert rc == wt.WT3D_ERR_NOMEM and idle == 1
+
+
+def test_pool_of_temporaries(solver):
+    """What the pool keeps between calls is counted, and returned when asked for."""
+    s = solver
+    s.solve(point_forces(s.grid, 16, 0), tol=1e-10, maxit=60)
+    held, used = wt.scratch_info()
+    assert held > 0 and used == 0
+    free, _ = wt.mem_info()
+    wt.scratch_trim()
+    assert wt.scratch_info() == (0.0, 0.0)
+    assert wt.mem_info()[0] > free
+
+
+def test_no_pool_without_handles():
+    """A call without a handle leaves nothing behind in the pool."""
+    g = Grid(*DIMS, 20.0, pmld=3 * 20.0, fst=1)
+    wt.assemble(g, *model.layered_random(*DIMS, 20.0, seed=1), 2 * np.pi)
+    assert wt.scratch_info() == (0.0, 0.0)

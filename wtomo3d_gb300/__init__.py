@@ -136,6 +136,7 @@ def lib():
         L.wt3d_batch_buffers.argtypes = [vp, ctypes.c_int, ctypes.POINTER(vp), ctypes.POINTER(vp)]
         L.wt3d_memcpy.argtypes = [vp, vp, vp, ctypes.c_longlong]
         L.wt3d_mem_info.argtypes = [ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_double)]
+        L.wt3d_scratch_info.argtypes = L.wt3d_mem_info.argtypes
         L.wt3d_source_weights.argtypes = [ctypes.POINTER(Grid)] + [ctypes.c_double] * 3 + [ctypes.c_int,
                                           ctypes.c_double, ctypes.c_int, vp, vp, ctypes.POINTER(ctypes.c_int)]
         L.wt3d_rhs_sources.argtypes = [vp, ctypes.c_int, vp, vp, vp, ctypes.c_int, ctypes.c_double, vp]
@@ -232,6 +233,19 @@ def mem_info():
     f, t = ctypes.c_double(), ctypes.c_double()
     _check(lib().wt3d_mem_info(ctypes.byref(f), ctypes.byref(t)))
     return f.value, t.value
+
+
+def scratch_info():
+    """(held, used) bytes of the pool that calls take their temporaries from; what
+    is held and not used is free to handles and calls, but not in mem_info()."""
+    r, u = ctypes.c_double(), ctypes.c_double()
+    _check(lib().wt3d_scratch_info(ctypes.byref(r), ctypes.byref(u)))
+    return r.value, u.value
+
+
+def scratch_trim():
+    """Returns the pool's unused bytes to the device, for other allocators."""
+    _check(lib().wt3d_scratch_trim())
 
 
 def solver_bytes(grid, precision=PREC_MIXED):

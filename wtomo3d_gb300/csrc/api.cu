@@ -21,12 +21,20 @@ void set_error(const std::string &msg) { g_err = msg; }
 static thread_local int g_fail_alloc = 0;   // allocations until the one that fails, 0 for none
 bool alloc_is_to_fail() { return g_fail_alloc > 0 && --g_fail_alloc == 0; }
 
-// One pool per device, made at its first use and kept for the process; empty
-// between handles.  A stream takes memory that another has released only where
-// that release has completed: no stream is made to wait for another's work.
+// One pool per device, made at its first use and kept for the process.  It keeps
+// memory between calls while a handle exists; without one, what a call has released
+// goes back to the device at the next synchronisation.  A stream takes memory that
+// another has released only where that release has completed: no stream is made to
+// wait for another's work.
 static std::mutex g_pool_mu;
 static std::map<int, cudaMemPool_t> g_pools;
-static std::atomic<int> g_handles{0};
+static int g_handles = 0;   // under g_pool_mu
+
+static void pool_threshold(cudaMemPool_t pool)
+{
+    unsigned long long keep = g_handles > 0 ? SCRATCH_KEEP : 0;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+}
 
 cudaMemPool_t scratch_pool()
 {
@@ -44,9 +52,8 @@ cudaMemPool_t scratch_pool()
         cudaGetLastError();
         pool = nullptr;
     } else {
-        unsigned long long keep = SCRATCH_KEEP;
         int off = 0;
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        pool_threshold(pool);
         cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &off);
     }
     g_pools[dev] = pool;
@@ -58,6 +65,19 @@ void scratch_trim()
     std::lock_guard<std::mutex> lk(g_pool_mu);
     for (auto &kv : g_pools)
         if (kv.second) cudaMemPoolTrimTo(kv.second, 0);
+}
+
+// A handle comes (change 1) or goes (-1): the last one takes the pools' memory with it.
+static void count_handle(int change)
+{
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    g_handles += change;
+    if (g_handles > 1 || (g_handles == 1 && change < 0)) return;
+    for (auto &kv : g_pools)
+        if (kv.second) {
+            pool_threshold(kv.second);
+            if (g_handles == 0) cudaMemPoolTrimTo(kv.second, 0);
+        }
 }
 
 // Spread sources: F[src_col[e] * n + 3 node[e] + comp[e]] += w[e] * sterm[e]
@@ -185,7 +205,7 @@ struct wt3d_solver {
     bool have_model = false, have_values = false, have_factor = false;
     long long kernels_solve = 0;
     wt3d_stats stats{};
-    wt3d_solver() { g_handles.fetch_add(1); }
+    wt3d_solver() { count_handle(1); }
     ~wt3d_solver()
     {
         if (st) cudaStreamSynchronize(st);
@@ -198,7 +218,7 @@ struct wt3d_solver {
         if (st) cudaStreamDestroy(st);
         if (sts) cudaStreamDestroy(sts);
         if (pin) cudaFreeHost(pin);
-        if (g_handles.fetch_sub(1) == 1) scratch_trim();
+        count_handle(-1);
     }
 };
 
@@ -236,7 +256,7 @@ int have_gpu()
 }
 
 // Digits of op(A) (abg - A with abg != nullptr) for the tensor-core products of a
-// call with up to m columns, until product_done.  Grid operators and 8 or more
+// call with up to m columns, until ProductDone.  Grid operators and blocks of 8 or more
 // columns only: with fewer the FP64 kernel is as fast (0.5 ms for one column of
 // 48^3, 0.9 for four), and without the memory it does the work too.
 struct ProductDone {
@@ -747,18 +767,15 @@ int wt3d_pattern(int nx, int ny, int nz, int base, int *irptr, int *jcptr)
     if (rc) return rc;
     long long nnz = wt3d_pattern_nnz(nx, ny, nz);
     long long n = 3LL * nx * ny * nz;
-    int *di = nullptr, *dj = nullptr;
-    WT_CUDA(cudaMalloc(&di, sizeof(int) * (n + 1)));
-    if (cudaMalloc(&dj, sizeof(int) * nnz) != cudaSuccess) { cudaFree(di); set_error("cudaMalloc"); return WT3D_ERR_NOMEM; }
-    rc = device_pattern(nx, ny, nz, base, di, dj, 0);
-    if (!rc && (cudaMemcpy(irptr, di, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost) != cudaSuccess ||
-                cudaMemcpy(jcptr, dj, sizeof(int) * nnz, cudaMemcpyDeviceToHost) != cudaSuccess)) {
+    DevVec<int> di, dj;
+    if ((rc = di.alloc(n + 1)) || (rc = dj.alloc(nnz))) return rc;
+    if ((rc = device_pattern(nx, ny, nz, base, di.p, dj.p, 0))) return rc;
+    if (cudaMemcpy(irptr, di.p, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost) != cudaSuccess ||
+        cudaMemcpy(jcptr, dj.p, sizeof(int) * nnz, cudaMemcpyDeviceToHost) != cudaSuccess) {
         set_error("wt3d_pattern: copy back failed");
-        rc = WT3D_ERR_CUDA;
+        return WT3D_ERR_CUDA;
     }
-    cudaFree(di);
-    cudaFree(dj);
-    return rc;
+    return WT3D_OK;
 }
 
 int wt3d_assemble_device(const wt3d_grid *g, const float *d_vp, const float *d_vs, const float *d_rho,
@@ -794,6 +811,7 @@ int wt3d_assemble(const wt3d_grid *g, const float *vp, const float *vs, const fl
     WT_CUDA(cudaMemcpy(drho.p, rho, sizeof(float) * nn, cudaMemcpyHostToDevice));
     if ((rc = device_pattern(g->nx, g->ny, g->nz, 0, di.p, dj.p, 0))) return rc;
     if ((rc = wt3d_assemble_device(g, dvp.p, dvs.p, drho.p, omega_re, omega_im, di.p, da.p, nullptr))) return rc;
+    WT_CUDA(cudaStreamSynchronize(nullptr));   // without a handle the pool gives its memory back here
     WT_CUDA(cudaMemcpy(a, da.p, sizeof(double2) * nnz, cudaMemcpyDeviceToHost));
     return WT3D_OK;
 }
@@ -1518,6 +1536,28 @@ int wt3d_mem_info(double *free_bytes, double *total_bytes)
     WT_CUDA(cudaMemGetInfo(&f, &t));
     if (free_bytes) *free_bytes = (double)f;
     if (total_bytes) *total_bytes = (double)t;
+    return WT3D_OK;
+}
+
+int wt3d_scratch_info(double *reserved_bytes, double *used_bytes)
+{
+    unsigned long long r = 0, u = 0;
+    int dev = 0;
+    WT_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    auto it = g_pools.find(dev);
+    if (it != g_pools.end() && it->second) {
+        WT_CUDA(cudaMemPoolGetAttribute(it->second, cudaMemPoolAttrReservedMemCurrent, &r));
+        WT_CUDA(cudaMemPoolGetAttribute(it->second, cudaMemPoolAttrUsedMemCurrent, &u));
+    }
+    if (reserved_bytes) *reserved_bytes = (double)r;
+    if (used_bytes) *used_bytes = (double)u;
+    return WT3D_OK;
+}
+
+int wt3d_scratch_trim(void)
+{
+    scratch_trim();
     return WT3D_OK;
 }
 

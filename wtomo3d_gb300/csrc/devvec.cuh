@@ -7,8 +7,9 @@
 namespace wt3d {
 
 // Memory pool of the current device for per-call temporaries (api.cu): keeps up
-// to SCRATCH_KEEP bytes between calls, and nothing once the last handle is gone
-// or an allocation fails (scratch_trim).  nullptr where pools cannot be made.
+// to SCRATCH_KEEP bytes between calls while a handle exists, and gives back what it
+// does not use when an allocation of the library fails (scratch_trim) or a caller
+// asks (wt3d_scratch_trim).  nullptr where pools cannot be made.
 constexpr unsigned long long SCRATCH_KEEP = 16ull << 30;
 cudaMemPool_t scratch_pool();
 void scratch_trim();

@@ -374,17 +374,21 @@ class GpuBackend:
         return r + extra + 2.0 * g.n * self.max_batch * 16      # + the batch buffers
 
     def can_open(self, key, freeing):
-        """Free device memory (plus what the evictions release) covers the new
-        handle, a factorisation workspace of its grid unless every workspace
-        the grid may have is held already, the Krylov bases of a slow solve and
-        a margin."""
+        """Free device memory (with what the pool of temporaries keeps unused, and
+        what the evictions release) covers the new handle, a factorisation
+        workspace of its grid unless every workspace the grid may have is held
+        already, the Krylov bases and operator digits of a slow solve and a
+        margin."""
         g = self.grid(key[0])
         _, _, ws = self.wt.solver_bytes(g, self.precision)
         with self._lock:
             shared = self._open.get(tuple(key[0]), 0) >= self.workspaces
-        transient = (0.0 if shared else 1.25 * ws) + 17.0 * g.n * 32 * 16 + 4e9
+        # 288 x 32 bytes per unknown for the bases at the most; the digits: 88 x 16,
+        # as many entries of a byte, six integers
+        transient = (0.0 if shared else 1.25 * ws) + (288.0 * 32 + 94 * 16 + 24) * g.n + 4e9
         free, _ = self.wt.mem_info()
-        return free + freeing >= self.bytes_needed(key) + transient
+        held, used = self.wt.scratch_info()
+        return free + held - used + freeing >= self.bytes_needed(key) + transient
 
     def open(self, key):
         dims, seed, freq = key
