@@ -413,6 +413,24 @@ int wt3d_debug_product(wt3d_solver *h, int adjoint, int nrhs, const void *X, voi
 int wt3d_debug_gemm(int path, int M, int N, int K, const void *A, int lda, const void *B, int ldb, void *C,
                     int ldc);
 
+/* One product of the substitution passes on host arrays (complex64, or
+ * complex128 with precision WT3D_PREC_FP64), for checks of its kernels:
+ * out (out_rows x nc) = op(A) in, or with sub out -= op(A) in, op(A) = A
+ * (M x K) or, with herm, A^H (A K x M), rows lda apart; in is in_rows x nc.
+ * tri 1 or 2: the lower (unit diagonal) or upper triangle of A, M = K.  Input
+ * row k is in_map[k], output row i out_map[i] (null: k and i).  K is cut into
+ * units of chunk (a multiple of 32 up to 1024) that add up.  nc is 1, 4, 8, 16
+ * or 32.  kernel 0: multiply-adds through shared memory, 1: one column through
+ * registers (complex128 with herm only), 2: tensor cores (complex64, 8 columns
+ * and more), -1: as a pass with such units chooses. */
+int wt3d_debug_skinny_kernel(int precision, int kernel, int herm, int tri, int sub, int M, int K, int nc, int chunk,
+                             const void *A, int lda, const void *in, const int *in_map, int in_rows, void *out,
+                             const int *out_map, int out_rows);
+
+/* The same in complex64 with kernel -1, without maps, into a cleared out. */
+int wt3d_debug_skinny(int herm, int tri, int M, int K, int nc, int chunk, const void *A, int lda, const void *in,
+                      void *out);
+
 /* Device-resident timing of the GEMM kernels: average ms of `iters`
  * launches of C -= A B (M x K by K x N complex64, device-filled operands);
  * path 1 = tensor-core kernel (operand split excluded), 0 = SIMT kernel,

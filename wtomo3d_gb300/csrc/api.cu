@@ -1915,23 +1915,42 @@ extern "C" int wt3d_debug_product(wt3d_solver *h, int adjoint, int nrhs, const v
     return WT3D_OK;
 }
 
-// One product of the substitution passes on host complex64 arrays, as its kernel
-// computes it: out (M x nc) = op(A) in (K x nc), op(A) = A (M x K) or, with herm,
-// A^H (A K x M), rows lda apart; tri 1 or 2: A is a packed block inverse (M = K) and
-// its lower (unit) or upper triangle is meant.  K is cut into units of chunk rows;
-// one column with units of more than 64 rows goes to the kernel of large grids.
-extern "C" int wt3d_debug_skinny(int herm, int tri, int M, int K, int nc, int chunk, const void *A, int lda,
-                                 const void *in, void *out)
+// One product of the substitution passes on host arrays, in units of chunk rows of K:
+// out (out_rows x nc) = or -= (sub) op(A) in (in_rows x nc), op(A) = A (M x K) or, with
+// herm, A^H (A K x M), rows lda apart; tri 1 or 2: A is a packed block inverse (M = K)
+// and its lower (unit) or upper triangle is meant.  Input row k is in_map[k] and output
+// row i out_map[i], or k and i without maps.  kernel 0: k_skinny, 1: k_gemv (one
+// column; complex128 with herm only), 2: k_skinny_tc (complex64, 8 columns and more),
+// -1: as a pass with such units chooses, one column with more than 64 rows as on large
+// grids.
+template <class T>
+static int debug_skinny(int kernel, int herm, int tri, int sub, int M, int K, int nc, int chunk, const void *A, int lda,
+                        const void *in, const int *in_map, int in_rows, void *out, const int *out_map, int out_rows)
 {
-    if (nc != sk_columns(nc) || chunk < 32 || chunk % 32 || chunk > SK_KMAX || (tri && M != K)) return WT3D_ERR_ARG;
-    const size_t na = (size_t)(herm ? K : M) * lda;
-    DevVec<cx<float>> dA, dB, dC;
+    constexpr bool f32 = std::is_same<T, float>::value;
+    if (M < 1 || K < 1 || nc != sk_columns(nc) || chunk < 32 || chunk % 32 || chunk > SK_KMAX || (tri && M != K) ||
+        lda < (herm ? M : K))
+        return WT3D_ERR_ARG;
+    if (kernel < 0) kernel = f32 && sk_tensor(nc, chunk) ? 2 : nc == 1 && chunk > 64 ? 1 : 0;
+    if (kernel > 2 || (kernel == 1 && (nc != 1 || (!f32 && !herm))) || (kernel == 2 && (!f32 || nc < 8))) return WT3D_ERR_ARG;
+    auto in_range = [](const int *map, int m, int rows) {
+        for (int i = 0; i < m; i++)
+            if ((map ? map[i] : i) < 0 || (map ? map[i] : i) >= rows) return false;
+        return true;
+    };
+    if (!in_range(in_map, K, in_rows) || !in_range(out_map, M, out_rows)) return WT3D_ERR_ARG;
+    const size_t na = (size_t)(herm ? K : M) * lda, nin = (size_t)in_rows * nc, nout = (size_t)out_rows * nc;
+    DevVec<cx<T>> dA, dB, dC;
+    DevVec<int> dbm, dcm;
     DevVec<SkUnit> du;
     int rc;
-    if ((rc = dA.alloc(na)) || (rc = dB.alloc((size_t)K * nc)) || (rc = dC.alloc((size_t)M * nc))) return rc;
-    WT_CUDA(cudaMemcpy(dA.p, A, sizeof(cx<float>) * na, cudaMemcpyHostToDevice));
-    WT_CUDA(cudaMemcpy(dB.p, in, sizeof(cx<float>) * K * nc, cudaMemcpyHostToDevice));
-    WT_CUDA(cudaMemset(dC.p, 0, sizeof(cx<float>) * M * nc));
+    if ((rc = dA.alloc(na)) || (rc = dB.alloc(nin)) || (rc = dC.alloc(nout)) ||
+        (in_map && (rc = dbm.upload(std::vector<int>(in_map, in_map + K)))) ||
+        (out_map && (rc = dcm.upload(std::vector<int>(out_map, out_map + M)))))
+        return rc;
+    WT_CUDA(cudaMemcpy(dA.p, A, sizeof(cx<T>) * na, cudaMemcpyHostToDevice));
+    WT_CUDA(cudaMemcpy(dB.p, in, sizeof(cx<T>) * nin, cudaMemcpyHostToDevice));
+    WT_CUDA(cudaMemcpy(dC.p, out, sizeof(cx<T>) * nout, cudaMemcpyHostToDevice));
     std::vector<SkUnit> hu;
     for (int r0 = 0; r0 < M; r0 += SK_M) {
         int k0 = 0, k1 = K;
@@ -1939,19 +1958,40 @@ extern "C" int wt3d_debug_skinny(int herm, int tri, int M, int K, int nc, int ch
         for (int k = k0; k < k1; k += chunk) {
             SkUnit u{};
             u.A = herm ? dA.p + (size_t)k * lda + r0 : dA.p + (size_t)r0 * lda + k;
+            u.bmap = in_map ? dbm.p + k : nullptr;
+            u.cmap = out_map ? dcm.p + r0 : nullptr;
             u.b0 = k; u.c0 = r0; u.lda = lda; u.M = std::min(SK_M, M - r0); u.K = std::min(chunk, k1 - k);
-            u.flags = (tri == 1 ? SK_LOWER : tri == 2 ? SK_UPPER : 0) | (k1 - k0 > chunk ? SK_ATOM : 0);
+            u.flags = (tri == 1 ? SK_LOWER : tri == 2 ? SK_UPPER : 0) | (sub ? SK_SUB : 0) |
+                      (k1 - k0 > chunk ? SK_ATOM : 0);
             u.d = k - r0;
             hu.push_back(u);
         }
     }
     if ((rc = du.upload(hu))) return rc;
-    Engine<float>::sk_attributes();
-    if (sk_tensor(nc, chunk)) sk_tensor_launch(nc, herm != 0, du.p, (int)hu.size(), dB.p, dC.p, 0);
-    else Engine<float>::sk_launch(nc, nc == 1 && chunk > 64, herm != 0, du.p, (int)hu.size(), dB.p, dC.p, 0);
+    Engine<T>::sk_attributes();
+    if constexpr (f32)
+        if (kernel == 2) sk_tensor_launch(nc, herm != 0, du.p, (int)hu.size(), dB.p, dC.p, 0);
+    if (kernel < 2) Engine<T>::sk_launch(nc, kernel == 1, herm != 0, du.p, (int)hu.size(), dB.p, dC.p, 0);
     WT_CUDA(cudaGetLastError());
-    WT_CUDA(cudaMemcpy(out, dC.p, sizeof(cx<float>) * M * nc, cudaMemcpyDeviceToHost));
+    WT_CUDA(cudaMemcpy(out, dC.p, sizeof(cx<T>) * nout, cudaMemcpyDeviceToHost));
     return WT3D_OK;
+}
+
+extern "C" int wt3d_debug_skinny_kernel(int precision, int kernel, int herm, int tri, int sub, int M, int K, int nc,
+                                        int chunk, const void *A, int lda, const void *in, const int *in_map,
+                                        int in_rows, void *out, const int *out_map, int out_rows)
+{
+    if (precision == WT3D_PREC_MIXED)
+        return debug_skinny<float>(kernel, herm, tri, sub, M, K, nc, chunk, A, lda, in, in_map, in_rows, out, out_map, out_rows);
+    return debug_skinny<double>(kernel, herm, tri, sub, M, K, nc, chunk, A, lda, in, in_map, in_rows, out, out_map, out_rows);
+}
+
+extern "C" int wt3d_debug_skinny(int herm, int tri, int M, int K, int nc, int chunk, const void *A, int lda,
+                                 const void *in, void *out)
+{
+    if (M < 1 || nc < 1) return WT3D_ERR_ARG;
+    memset(out, 0, sizeof(cx<float>) * M * nc);
+    return debug_skinny<float>(-1, herm, tri, 0, M, K, nc, chunk, A, lda, in, nullptr, K, out, nullptr, M);
 }
 
 // Select the CUDA device for the calling thread (multi-GPU replicas: one

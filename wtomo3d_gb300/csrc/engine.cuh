@@ -96,12 +96,14 @@ public:
     static constexpr int SBW = SB<T>;   // columns per diagonal block of the substitutions
     // units a launch of k_skinny is cut into, and the shortest K of a unit
     static constexpr int SK_SLOTS = 152 * 8, SK_KMIN = 64;
-    // factor entries from which the products of a pass over one column are k_gemv's (all of
-    // A^H are).  One kernel for a whole pass: launches of two that need different splits
+    // complex64 factor entries from which the products of a pass over one column are
+    // k_gemv's (all of A^H are).  One kernel for a whole pass: launches of two that need different splits
     // of L1 and shared memory wait for each other's SMs, and choosing by launch lost 10 %.
     // Milliseconds per pass, k_skinny and k_gemv: 14x12x13 0.158 and 0.169, 20^3 0.268 and
     // 0.279, 29x27x25 (1.2e8 entries) 0.50 and 0.47, 40^3 1.54 and 1.29, 64x64x48 5.4 and
     // 4.2; A^H: 14x12x13 0.111 and 0.109, 20^3 0.27 and 0.20, 64x64x48 5.7 and 4.0.
+    // complex128 (calls of one pass): 14x12x13 0.35 and 0.37, 24x22x20 1.31 and 1.43,
+    // 40^3 6.57 and 6.71, so none forward; A^H 0.37 and 0.34, 1.27 and 1.28, 6.42 and 6.10.
     static constexpr double GEMV_MIN_ENTRIES = 8e7;
     // outer block width of the two-level LU (WT3D_WB: a multiple of KB, 512 by default)
     const int WB = [] {
@@ -265,8 +267,9 @@ public:
     static void sk_launch(int nc, bool gemv, bool herm, const SkUnit *u, int n, const cx<T> *in, cx<T> *out,
                           cudaStream_t st)
     {
-        if (gemv) {
-            sk_chain(herm ? k_gemv<T, true> : k_gemv<T, false>, 0, u, n, in, out, st);
+        if (gemv) {   // complex128: A^H only
+            if (herm) sk_chain(k_gemv<T, true>, 0, u, n, in, out, st);
+            else if constexpr (sizeof(T) == 4) sk_chain(k_gemv<T, false>, 0, u, n, in, out, st);
             return;
         }
         if (nc == 1) sk_launch_n<1>(herm, u, n, in, out, st);
@@ -658,7 +661,7 @@ public:
                 }, tri ? LK_SUBSTEP : LK_TCGEMM, fl, by});
                 return;
             }
-        const bool gemv = nc == 1 && (herm || (double)fac.n >= GEMV_MIN_ENTRIES);
+        const bool gemv = nc == 1 && (herm || (sizeof(T) == 4 && (double)fac.n >= GEMV_MIN_ENTRIES));
         sc.launches.push_back({[psc, u0, nu, nc, gemv, herm, in, out](cudaStream_t st) {
             sk_launch(nc, gemv, herm, psc->sk.p + u0, nu, in, out, st);
         }, tri ? LK_SUBSTEP : LK_GEMM, fl, by});

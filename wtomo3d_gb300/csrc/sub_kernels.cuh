@@ -451,7 +451,8 @@ __global__ void __launch_bounds__(SK_TH) k_skinny(const SkUnit *__restrict__ uni
     }
 }
 
-// The products with one column, except forward passes of small grids.  Bound by
+// The products with one column, except forward passes of small grids and of
+// complex128.  Bound by
 // reading A, once, so entries go from memory to registers without a stop in shared
 // memory: as stored, a warp reads eight rows at a time, 32 neighbouring k each; of
 // A^H, a warp reads whole stored rows, a lane per output row.  The loads are a tile
