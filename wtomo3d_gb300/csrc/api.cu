@@ -259,9 +259,14 @@ int have_gpu()
 // call with up to m columns, until ProductDone.  Grid operators and blocks of 8 or more
 // columns only: with fewer the FP64 kernel is as fast (0.5 ms for one column of
 // 48^3, 0.9 for four), and without the memory it does the work too.
+void product_done(wt3d_solver *h)
+{
+    h->epA.release();
+    h->epE.release();
+}
 struct ProductDone {
     wt3d_solver *h;
-    ~ProductDone() { h->epA.release(); h->epE.release(); }
+    ~ProductDone() { product_done(h); }
 };
 unsigned char *digits_below(const wt3d_solver *h)
 {
@@ -654,6 +659,7 @@ int solve_dev_cm(wt3d_solver *h, int nrhs, const double2 *d_B, double2 *d_X, dou
         to_columns(h, h->sts, m, h->Xn.p, d_X + (long long)c0 * n);
     }
     cudaEventRecord(h->ev1, h->sts);
+    product_done(h);   // before the wait, so that no other is needed for it
     WT_CUDA(cudaStreamSynchronize(h->sts));
     if (int rc = h->e32 ? h->e32->check_tc_err() : h->e64->check_tc_err()) return rc;
     h->stats.t_solve_ms = ms_between(h->ev0, h->ev1);
@@ -1235,6 +1241,8 @@ static int solve_host(wt3d_solver *h, int nrhs, const double _Complex *B, double
     rc = solve_dev_cm(h, nrhs, dB.p, dX.p, tol, maxit, relres, iters, adjoint);
     if (rc && rc != WT3D_ERR_NOCONV) return rc;
     WT_CUDA(cudaMemcpyAsync(X, dX.p, sizeof(double2) * h->n * nrhs, cudaMemcpyDeviceToHost, h->sts));
+    dB.release();
+    dX.release();
     WT_CUDA(cudaStreamSynchronize(h->sts));
     return rc;
 }
@@ -1290,6 +1298,7 @@ int wt3d_apply_device(wt3d_solver *h, int nrhs, const void *d_X, void *d_Y)
         to_columns(h, h->st, m, h->Rn.p, (double2 *)d_Y + (long long)c0 * n);
     }
     WT_CUDA(cudaGetLastError());
+    product_done(h);
     WT_CUDA(cudaStreamSynchronize(h->st));
     return WT3D_OK;
 }
