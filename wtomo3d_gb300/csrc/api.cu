@@ -366,8 +366,9 @@ int solve_host_buffer(wt3d_solver *h)
 // the current iterate, h->Rn = B - op(A) Xn and bnorm2/rnorm2 the squared
 // column norms of B and R; on exit Xn is the new iterate.  Classical
 // Gram-Schmidt applied twice; Givens rotations and the small least-squares
-// problems per column on the host.  The restart length is the longest, up to
-// GM_KMAX, whose bases take no more than GM_BYTES per row: 10 for 32 columns of
+// problems per column on the host.  The restart length is the longest from 8 up to
+// GM_KMAX whose bases take no more than GM_BYTES per row (8 take 288 x 32 with 32
+// columns in complex128): 10 for 32 columns of
 // complex64 factors, 16 for up to 16 columns (WT3D_GMRES_RESTART sets another,
 // 1..16).  Every restart forgets what the basis has learnt of the few slow
 // modes: 64^3 at 1 Hz, 4 adjoint columns, took 19 to 27 passes with a restart of

@@ -29,7 +29,7 @@
 //
 // Errors against extended precision, 2-norm over the product, 13x12x11: random
 // fields 4.7e-17 (FP64 kernel 1.6e-16), wave fields 4.3e-17 (1.4e-15).  32 columns
-// of 64x64x48 in 3.1 ms instead of 8.8; the digits of the operator, 0.6 ms, are
+// of 64x64x48 in 3.2 ms instead of 8.8; the digits of the operator, 0.3 ms, are
 // made once per call.
 #pragma once
 #include "refine_kernels.cuh"

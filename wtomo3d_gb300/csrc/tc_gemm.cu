@@ -539,7 +539,7 @@ long long tc_workspace_floats(const GemmTask<float> *g, int n)
 bool tc_eligible(const GemmTask<float> &g)
 {
     // large enough that the tensor-core tile (128 x 128 complex) is not mostly
-    // padding; the narrow right-hand-side blocks of the solves stay on SIMT
+    // padding
     return g.M >= 64 && g.N >= 96 && g.K >= 32;
 }
 
