@@ -7,7 +7,8 @@
 // not the bound.  Every operand is h + m + l of 8 bits each, all 24 bits of FP32 and
 // (BF16 has FP32's exponents) whatever the magnitudes of the entries beside it; an
 // entry of A below 2^-110 is held to 2^-134, and one of X likewise against its column's
-// largest of 16 k, as the columns are scaled by powers of two.  Two halves in FP16
+// largest of 16 k, as the columns are scaled by powers of two; from 3.39e38 on an
+// entry rounds to infinity.  Two halves in FP16
 // with three products take 2/3 to 3/4 of the time of a pass, but hold 22 bits, and
 // fewer of an entry below 2^-16 of the largest of its row or column in 16 k.
 // l h + h l + m m + m h + h m + h h of a k16 step is summed by the tensor cores, whose
