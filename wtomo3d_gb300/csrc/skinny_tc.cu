@@ -3,14 +3,14 @@
 //
 // On the FP32 pipe these products are bound by its 73 TF/s (36 - 39 TF/s
 // reached: at 32 columns a factor entry costs 128 multiply-adds for its 8 bytes).
-// mma.sync in BF16 does 604 TF/s here, so that six products of split operands are
-// not the bound.  Every operand is h + m + l of 8 bits each, all 24 bits of FP32 and
-// (BF16 has FP32's exponents) whatever the magnitudes of the entries beside it; an
-// entry of A below 2^-110 is held to 2^-134, and one of X likewise against its column's
-// largest of 16 k, as the columns are scaled by powers of two; from 3.39e38 on an
-// entry rounds to infinity.  Two halves in FP16
-// with three products take 2/3 to 3/4 of the time of a pass, but hold 22 bits, and
-// fewer of an entry below 2^-16 of the largest of its row or column in 16 k.
+// mma.sync in BF16 does 604 TF/s here, eight times that, for six products of split
+// operands.  Every operand is h + m + l of 8 bits each, all 24 bits of FP32 and (BF16
+// has FP32's exponents) whatever the magnitudes of the entries beside it; an entry of
+// A below 2^-110 is held to 2^-134, and one of X likewise against its column's largest
+// of 16 k, as the columns are scaled by powers of two; from 3.39e38 on an entry rounds
+// to infinity.  Two halves in FP16 with three products take 2/3 to 3/4 of the time of
+// a pass, but hold 22 bits, and fewer of an entry below 2^-16 of the largest of its
+// row or column in 16 k.
 // l h + h l + m m + m h + h m + h h of a k16 step is summed by the tensor cores, whose
 // additions truncate, and only then added to FP32 sums with rounded operations: the
 // error is 1.6e-7 at K = 1024 and 6e-8 at K = 32 (Gaussian entries), with FP32
@@ -19,7 +19,9 @@
 // memory and kept its sums in tensor memory reached 63 TF/s on the largest blocks.
 //
 // A pass of 64x64x48 with 32, 16, 8 columns: 15.4, 10.5, 7.1 ms with FP32 products,
-// 12.4, 8.0, 6.6 ms with these; 48^3 with 32: 8.2 and 6.7 ms.
+// 12.4, 8.0, 6.6 ms with these; 48^3 with 32: 8.2 and 6.7 ms.  Bound by the tensor
+// pipe: half busy on 24576 x 1024 entries and 32 columns, 1.26 waves of CTAs, and the
+// order of the products (one, two or four chains of them at a time) changes nothing.
 #include <cuda_bf16.h>
 #include "sub_kernels.cuh"
 
