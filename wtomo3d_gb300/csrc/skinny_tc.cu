@@ -3,7 +3,7 @@
 //
 // On the FP32 pipe these products are bound by its 73 TF/s (36 - 39 TF/s
 // reached: at 32 columns a factor entry costs 128 multiply-adds for its 8 bytes).
-// mma.sync in BF16 does 604 TF/s here, eight times that, for six products of split
+// 16-bit mma.sync does 604 TF/s here (FP16), eight times that, for six products of split
 // operands.  Every operand is h + m + l of 8 bits each, all 24 bits of FP32 and (BF16
 // has FP32's exponents) whatever the magnitudes of the entries beside it; an entry of
 // A below 2^-110 is held to 2^-134, and one of X likewise against its column's largest
